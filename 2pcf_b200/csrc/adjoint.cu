@@ -126,7 +126,7 @@ __device__ __forceinline__ void adj_pair(float sx, float sy, const float4 l, con
   const float d2 = fmaf(dy, dy, dx2);
   float r;
   if (LOGB) {
-    const float rs = rsqrtf(d2);
+    const float rs = rsqrt_ftz(d2);
     r = rs * rs;
   } else {
     r = __frcp_rn(d2);
@@ -181,7 +181,7 @@ __device__ __forceinline__ void adj_terms2(float2 nsx, float2 nsy, float sz, con
   d2 = fma2(dy, dy, dx2);
   float2 r;
   if (LOGB) {
-    const float2 rs = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+    const float2 rs = make_float2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y));
     r = mul2(rs, rs);
   } else {
     r = make_float2(__frcp_rn(d2.x), __frcp_rn(d2.y));
@@ -872,7 +872,7 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     a.dsum = dsum[t];
     // item cost: the source groups play the lens-group role, the lens grid the source grid
     tdesc[t].lens_cat = si; tdesc[t].src_cat = li; tdesc[t].item_base = 0; tdesc[t].lens_acc_off = -1;
-    tdesc[t].margin = margin;
+    tdesc[t].margin = margin; tdesc[t].split = 1;
     if (hc[li] > 0)
       for (int g = 0; g < ngroups[si]; ++g) items.push_back(make_int2(t, g));
   }

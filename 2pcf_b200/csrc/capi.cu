@@ -183,16 +183,20 @@ struct SrcIn {
   const float *x, *y, *z, *f1, *f2, *w, *m;
 };
 
-struct LensBuilt {
-  int n_valid = 0;
+// Lens groups of one size (the work items of one pair kernel).
+struct LensGroups {
   int n_groups = 0;
-  float4* rec = nullptr;
-  float* zs = nullptr;
-  int* perm = nullptr;
   int* group_start = nullptr;
   float4* group_box = nullptr;
   std::vector<int> patch_groups;  // [n_patch_eff + 1], host
   int* d_patch_groups = nullptr;
+};
+struct LensBuilt {
+  int n_valid = 0;
+  float4* rec = nullptr;
+  float* zs = nullptr;
+  int* perm = nullptr;
+  LensGroups by[2];  // [1]: for k_pairs_series, [0]: for the other pair kernels
 };
 
 struct SrcBuilt {
@@ -214,15 +218,39 @@ struct Batch {
   std::vector<LensBuilt> lb;
   std::vector<TaskDesc> tdesc;
   std::vector<char> want_lens;
+  std::vector<char> kind;       // pair kernel of each task: 1 = k_pairs_series (pairs_series.cu), 0 = the others
   int n_items = 0, grid = 0;
-  PairParams P{};
-  PairLaunch L{};
-  int* head = nullptr;  // [0] queue head, [1] error flags
+  PairParams P[2];              // by kind; P[k].n_items = 0: no launch
+  PairLaunch L[2];
+  int* head = nullptr;  // [0], [2] queue heads, [1] error flags
   double* item_sums = nullptr;
   double* lens_acc = nullptr;
   long long lens_acc_elems = 0;
   std::vector<double*> dpatch;
 };
+
+bool wants_lens(const tpcf_result& o) {
+  return o.xi_E_marks || o.xi_B_marks || o.K_marks || o.w_marks || o.marks_weight || o.lens_sums || o.lens_raw;
+}
+
+// Whether a source catalogue is dense enough for k_pairs_series: the
+// half-diagonal of a 32-source sub-chunk (sources spread evenly over their
+// bounding box) against the width of the last bin.  Log bins (the kernel's
+// milliseconds / k_pairs', 100 k lenses on 600' x 600', theta_max 100'):
+// ratio 0.08: 3.3 / 5.0, 0.12: 2.08 / 2.22, 0.17: 1.60 / 1.38 and 6.7 / 6.0,
+// 0.26: 4.5 / 2.6 -- wider sub-chunks straddle several edges and few
+// combinations are far.  In the other spacings k_pairs searches the bin of
+// every pair: 0.34: 7.3 / 12.9, 0.77: 3.2 / 4.7, 1.1: 3.0 / 3.4, 1.7: 2.9 / 1.6.
+bool series_pays(int n_valid, double ex, double ey, const tpcf_bins* bins, const double* edges) {
+  if (n_valid < kChunk) return false;
+  const double half = std::sqrt(0.5 * kChunk * ex * ey / n_valid);
+  const double width = edges[bins->n_bin] - edges[bins->n_bin - 1];
+  return half <= (bins->spacing == TPCF_LOG ? 0.14 : 1.1) * width;
+}
+
+// A task with fewer lens groups than kSplitItems / 2 is cut into several items
+// per group (at most kMaxSplit).
+constexpr int kSplitItems = 8192, kMaxSplit = 8;
 
 void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<SrcIn> srcs, const std::vector<int>& tl,
                  const std::vector<int>& ts, const tpcf_bins* bins, int n_patch, const tpcf_result* outs, Batch& B) {
@@ -338,13 +366,17 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   int tch = 2;
   if (!sph && c->opts.group_size > 0 && c->opts.group_size <= bt) bt = c->opts.group_size;
   if (!sph && c->opts.tile_chunks == 1) tch = 1;
-  const int lens_group = sph ? bt : 32;
 
   const double Rd = bins->x_max;
   float R = (float)(Rd * (1.0 + 1e-6));
+  const char* var_env = std::getenv("TPCF_PAIR_VARIANT");
+  B.variant = var_env ? std::atoi(var_env) : 0;
+  bool any_lens = false;
+  for (int t = 0; t < nT; ++t) any_lens = any_lens || wants_lens(outs[t]);
 
   // ---- source grids
   std::vector<GridDesc> grids(nS);
+  std::vector<char> src_series(nS, 0);
   for (int i = 0; i < nS; ++i) {
     const SrcIn& s = srcs[i];
     GridDesc& g = grids[i];
@@ -358,6 +390,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     }
     double cell = c->opts.cell_size > 0 ? c->opts.cell_size : Rd / 16.0;
     const double span = std::max((double)ex, (double)ey);
+    const bool series = !sph && !any_lens && B.variant == 0 && series_pays(n_valid, ex, ey, bins, e.data());
+    src_series[i] = series;
     if (!c->opts.use_grid) cell = span * 2.0 + 1.0;
     // keep the grid below 2^24 cells
     while ((span / cell + 2.0) * (span / cell + 2.0) > (double)(1 << 24)) cell *= 1.5;
@@ -369,8 +403,9 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     g.ncx = ncx; g.ncy = ncy; g.n_valid = n_valid;
     int* cs = (int*)ws_alloc(c, sizeof(int) * (ncells + 1));
     const int n_chunks = std::max((n_valid + kChunk - 1) / kChunk, 1);
-    SrcPair* pairs = sph ? nullptr : (SrcPair*)ws_alloc(c, sizeof(SrcPair) * (kChunk / 2) * n_chunks);
-    ChunkMeta* cmeta = sph ? nullptr : (ChunkMeta*)ws_alloc(c, sizeof(ChunkMeta) * n_chunks);
+    SrcPair* pairs = sph || series ? nullptr : (SrcPair*)ws_alloc(c, sizeof(SrcPair) * (kChunk / 2) * n_chunks);
+    ChunkMeta* cmeta = sph || series ? nullptr : (ChunkMeta*)ws_alloc(c, sizeof(ChunkMeta) * n_chunks);
+    float* srec = series ? (float*)ws_alloc(c, series_bytes(n_valid, mode, has_m, has_z)) : nullptr;
     SrcRecS* recs = sph ? (SrcRecS*)ws_alloc(c, sizeof(SrcRecS) * std::max(n_valid, 1)) : nullptr;
     if (s.n > 0) {
       unsigned* k0 = (unsigned*)ws_alloc(c, sizeof(unsigned) * s.n);
@@ -390,6 +425,9 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
       if (sph)
         counted(c, launch_src_gather_sph(i1, n_valid, mode, lamS[i], s.y, s.z, s.f1, s.f2, s.w, s.m, recs, st),
                 "src gather");
+      else if (series)
+        counted(c, launch_src_series(i1, n_valid, mode, has_m, has_z, s.x, s.y, s.z, s.f1, s.f2, s.w, s.m, srec, st),
+                "src gather");
       else
         counted(c, launch_src_pairs(i1, n_valid, mode, s.x, s.y, s.z, s.f1, s.f2, s.w, s.m, pairs, cmeta, st),
                 "src gather");
@@ -401,6 +439,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     g.recs = recs;
     g.pairs = pairs;
     g.meta = cmeta;
+    g.series = srec;
   }
   // FP32 guard on the reach of a task's rows and cells: the rounding scale of
   // the coordinates its two catalogues hold, so that a task's tiles (and its
@@ -416,10 +455,11 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     return (float)(1e-5 * (std::max(extent[li], extent[nL + si]) + Rd) + 1e-4 * grids[si].cell);
   };
 
-  // ---- lens catalogues: sort by (patch, Hilbert index), groups of <= lens_group lenses
+  // ---- lens catalogues: sort by (patch, Hilbert index), groups for each pair kernel that reads them
   std::vector<LensBuilt>& lb = B.lb;
   lb.assign(nL, LensBuilt{});
-  std::vector<LensDesc> ldesc(nL);
+  std::vector<LensDesc> ldesc(2 * nL);  // [kind * nL + catalogue]
+  const int lens_group[2] = {sph ? bt : 32, series_lens_group()};
   for (int i = 0; i < nL; ++i) {
     const LensIn& l = lens[i];
     LensBuilt& LB = lb[i];
@@ -450,63 +490,74 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
         for (int p = 1; p <= n_patch_eff; ++p) off[p] = LB.n_valid;
       }
     }
-    std::vector<int> gstart;
-    LB.patch_groups.assign(n_patch_eff + 1, 0);
-    for (int p = 0; p < n_patch_eff; ++p) {
-      LB.patch_groups[p] = (int)gstart.size();
-      for (int s0 = off[p]; s0 < off[p + 1]; s0 += lens_group) gstart.push_back(s0);
-    }
-    LB.patch_groups[n_patch_eff] = (int)gstart.size();
-    LB.n_groups = (int)gstart.size();
-    gstart.push_back(LB.n_valid);
-    LB.group_start = (int*)ws_alloc(c, sizeof(int) * gstart.size());
-    check(cudaMemcpyAsync(LB.group_start, gstart.data(), sizeof(int) * gstart.size(), cudaMemcpyHostToDevice, st), "H2D groups");
-    LB.d_patch_groups = (int*)ws_alloc(c, sizeof(int) * (n_patch_eff + 1));
-    check(cudaMemcpyAsync(LB.d_patch_groups, LB.patch_groups.data(), sizeof(int) * (n_patch_eff + 1),
-                          cudaMemcpyHostToDevice, st), "H2D patch groups");
     float4* pos = nullptr;
     if (sph) {
       pos = (float4*)ws_alloc(c, sizeof(float4) * 2 * std::max(LB.n_valid, 1));
       if (LB.n_valid > 0) counted(c, launch_lens_pos_sph(LB.perm, LB.n_valid, lamL[i], l.y, pos, st), "lens pos");
     }
-    LB.group_box = (float4*)ws_alloc(c, sizeof(float4) * std::max(LB.n_groups, 1));
-    counted(c, launch_group_box(LB.rec, LB.group_start, LB.n_groups, LB.group_box, st), "group box");
-    check(cudaStreamSynchronize(st), "sync groups");  // host vectors above must outlive the async copies
-    LensDesc& d = ldesc[i];
-    d.rec = LB.rec; d.z = LB.zs; d.group_start = LB.group_start; d.group_box = LB.group_box;
-    d.n_valid = LB.n_valid; d.n_groups = LB.n_groups;
-    d.pos = pos;
+    for (int k = 0; k < 2; ++k) {
+      bool used = false;
+      for (int t = 0; t < nT; ++t) used = used || (tl[t] == i && src_series[ts[t]] == k);
+      LensGroups& LG = LB.by[k];
+      LG.patch_groups.assign(n_patch_eff + 1, 0);
+      if (!used) continue;
+      std::vector<int> gstart;
+      for (int p = 0; p < n_patch_eff; ++p) {
+        LG.patch_groups[p] = (int)gstart.size();
+        for (int s0 = off[p]; s0 < off[p + 1]; s0 += lens_group[k]) gstart.push_back(s0);
+      }
+      LG.patch_groups[n_patch_eff] = (int)gstart.size();
+      LG.n_groups = (int)gstart.size();
+      gstart.push_back(LB.n_valid);
+      LG.group_start = (int*)ws_alloc(c, sizeof(int) * gstart.size());
+      check(cudaMemcpyAsync(LG.group_start, gstart.data(), sizeof(int) * gstart.size(), cudaMemcpyHostToDevice, st), "H2D groups");
+      LG.d_patch_groups = (int*)ws_alloc(c, sizeof(int) * (n_patch_eff + 1));
+      check(cudaMemcpyAsync(LG.d_patch_groups, LG.patch_groups.data(), sizeof(int) * (n_patch_eff + 1),
+                            cudaMemcpyHostToDevice, st), "H2D patch groups");
+      LG.group_box = (float4*)ws_alloc(c, sizeof(float4) * std::max(LG.n_groups, 1));
+      counted(c, launch_group_box(LB.rec, LG.group_start, LG.n_groups, LG.group_box, st), "group box");
+      check(cudaStreamSynchronize(st), "sync groups");  // host vectors above must outlive the async copies
+      LensDesc& d = ldesc[k * nL + i];
+      d.rec = LB.rec; d.z = LB.zs; d.group_start = LG.group_start; d.group_box = LG.group_box;
+      d.n_valid = LB.n_valid; d.n_groups = LG.n_groups;
+      d.pos = pos;
+    }
   }
 
   // ---- tasks and work items
   Phase ph_items("tpcf: work items");
   std::vector<TaskDesc>& tdesc = B.tdesc;
   tdesc.assign(nT, TaskDesc{});
-  std::vector<int2> items;
+  std::vector<int2> items[2];
+  int n_items = 0;
+  B.kind.assign(nT, 0);
   B.want_lens.assign(nT, 0);
   long long lens_acc_elems = 0;
   for (int t = 0; t < nT; ++t) {
     TaskDesc& d = tdesc[t];
-    d.lens_cat = tl[t];
+    const int kind = B.kind[t] = src_series[ts[t]];
+    d.lens_cat = kind * nL + tl[t];
     d.src_cat = ts[t];
     d.margin = task_margin(tl[t], ts[t]);
-    d.item_base = (int)items.size();
-    for (int g = 0; g < lb[tl[t]].n_groups; ++g) items.push_back(make_int2(t, g));
-    const tpcf_result& o = outs[t];
-    B.want_lens[t] =
-        (o.xi_E_marks || o.xi_B_marks || o.K_marks || o.w_marks || o.marks_weight || o.lens_sums || o.lens_raw) ? 1 : 0;
+    d.item_base = n_items;
+    const int ng = lb[tl[t]].by[kind].n_groups;
+    // few lens groups: several items per group keep the SMs' warps busy (a
+    // property of the task alone, so its sums do not depend on the batch)
+    d.split = !sph && !any_lens && ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
+    for (int i = 0; i < ng * d.split; ++i) items[kind].push_back(make_int2(t, i));
+    n_items += ng * d.split;
+    B.want_lens[t] = wants_lens(outs[t]) ? 1 : 0;
     d.lens_acc_off = -1;
     if (B.want_lens[t]) {
       d.lens_acc_off = lens_acc_elems;
       lens_acc_elems += (long long)kQ * nb * std::max(lb[tl[t]].n_valid, 1);
     }
   }
-  const int n_items = (int)items.size();
   TaskDesc* d_tasks = (TaskDesc*)ws_alloc(c, sizeof(TaskDesc) * std::max(nT, 1));
-  LensDesc* d_lens = (LensDesc*)ws_alloc(c, sizeof(LensDesc) * std::max(nL, 1));
+  LensDesc* d_lens = (LensDesc*)ws_alloc(c, sizeof(LensDesc) * 2 * std::max(nL, 1));
   GridDesc* d_grids = (GridDesc*)ws_alloc(c, sizeof(GridDesc) * std::max(nS, 1));
   check(cudaMemcpyAsync(d_tasks, tdesc.data(), sizeof(TaskDesc) * nT, cudaMemcpyHostToDevice, st), "H2D tasks");
-  check(cudaMemcpyAsync(d_lens, ldesc.data(), sizeof(LensDesc) * nL, cudaMemcpyHostToDevice, st), "H2D lens desc");
+  check(cudaMemcpyAsync(d_lens, ldesc.data(), sizeof(LensDesc) * 2 * nL, cudaMemcpyHostToDevice, st), "H2D lens desc");
   check(cudaMemcpyAsync(d_grids, grids.data(), sizeof(GridDesc) * nS, cudaMemcpyHostToDevice, st), "H2D grid desc");
   double* item_sums = (double*)ws_alloc(c, sizeof(double) * kQ * nb * std::max(n_items, 1));
   double* lens_acc = lens_acc_elems ? (double*)ws_alloc(c, sizeof(double) * lens_acc_elems) : nullptr;
@@ -519,33 +570,34 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   check(cudaMemcpyAsync(d_e2, e2.data(), sizeof(double) * (nb + 1), cudaMemcpyHostToDevice, st), "H2D edges");
   check(cudaMemcpyAsync(d_e2f, e2f.data(), sizeof(float) * (nb + 1), cudaMemcpyHostToDevice, st), "H2D edges f");
 
-  int2* d_items = (int2*)ws_alloc(c, sizeof(int2) * std::max(n_items, 1));
-  int n_run = 0;
-  if (n_items > 0) {
-    int2* d_items0 = (int2*)ws_alloc(c, sizeof(int2) * n_items);
-    check(cudaMemcpyAsync(d_items0, items.data(), sizeof(int2) * n_items, cudaMemcpyHostToDevice, st), "H2D items");
-    unsigned long long* ck0 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n_items);
-    unsigned long long* ck1 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n_items);
-    int* o0 = (int*)ws_alloc(c, sizeof(int) * n_items);
-    int* o1 = (int*)ws_alloc(c, sizeof(int) * n_items);
+  int2* d_items[2] = {nullptr, nullptr};
+  int n_run[2] = {0, 0};
+  for (int k = 0; k < 2; ++k) {
+    const int n = (int)items[k].size();
+    if (n == 0) continue;
+    d_items[k] = (int2*)ws_alloc(c, sizeof(int2) * n);
+    int2* d_items0 = (int2*)ws_alloc(c, sizeof(int2) * n);
+    check(cudaMemcpyAsync(d_items0, items[k].data(), sizeof(int2) * n, cudaMemcpyHostToDevice, st), "H2D items");
+    unsigned long long* ck0 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n);
+    unsigned long long* ck1 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n);
+    int* o0 = (int*)ws_alloc(c, sizeof(int) * n);
+    int* o1 = (int*)ws_alloc(c, sizeof(int) * n);
     if (sph)
-      counted(c, launch_item_cost_sph(d_items0, n_items, d_tasks, d_lens, d_grids, R, ck0, o0, st),
-              "item cost");
+      counted(c, launch_item_cost_sph(d_items0, n, d_tasks, d_lens, d_grids, R, ck0, o0, st), "item cost");
     else
-      counted(c, launch_item_cost(d_items0, n_items, d_tasks, d_lens, d_grids, R, ck0, o0, st), "item cost");
+      counted(c, launch_item_cost(d_items0, n, d_tasks, d_lens, d_grids, R, ck0, o0, st), "item cost");
     size_t tb = 0;
-    check(sort_pairs_u64_desc(nullptr, tb, ck0, ck1, o0, o1, n_items, st), "sort size");
+    check(sort_pairs_u64_desc(nullptr, tb, ck0, ck1, o0, o1, n, st), "sort size");
     void* tmp = ws_alloc(c, tb);
-    check(sort_pairs_u64_desc(tmp, tb, ck0, ck1, o0, o1, n_items, st), "sort items");
+    check(sort_pairs_u64_desc(tmp, tb, ck0, ck1, o0, o1, n, st), "sort items");
     const int sc = c->opts.shard_count > 1 ? c->opts.shard_count : 1;
     const int si = sc > 1 ? c->opts.shard_index : 0;
-    counted(c, launch_permute_items(d_items0, o1, n_items, si, sc, d_items, st), "permute items");
-    n_run = sc > 1 ? (n_items - si + sc - 1) / sc : n_items;
+    counted(c, launch_permute_items(d_items0, o1, n, si, sc, d_items[k], st), "permute items");
+    n_run[k] = sc > 1 ? (n - si + sc - 1) / sc : n;
   }
-  PairParams& P = B.P;
-  P = PairParams{};
-  P.tasks = d_tasks; P.lenses = d_lens; P.grids = d_grids; P.items = d_items; P.n_items = n_run;
-  P.nb = nb; P.queue_head = head; P.item_sums = item_sums; P.lens_acc = lens_acc; P.err = err;
+  PairParams P{};
+  P.tasks = d_tasks; P.lenses = d_lens; P.grids = d_grids;
+  P.nb = nb; P.item_sums = item_sums; P.lens_acc = lens_acc; P.err = err;
   P.e2 = d_e2; P.e2f = d_e2f; P.R = R;
   if (logb) {  // t = log2(theta^2) A + B (planar: theta^2 = d2)
     const double l0 = std::log2(e[0] * e[0]), l1 = std::log2(e[nb] * e[nb]);
@@ -564,12 +616,20 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   // sources (at 4096 one lens and bin of the 2 M x 0.5 M clustered
   // workload reached 1.05e-6 of its sum|terms|)
   P.flush_src = lens_acc ? 1024 : 4096;
+  P.far_bin = series_far_bin(e2.data(), nb);
   P.debug_skip_tile = c->skip_tile + 1;
   P.wait_limit = c->wait_limit;
-  const char* var_env = std::getenv("TPCF_PAIR_VARIANT");
-  B.variant = var_env ? std::atoi(var_env) : 0;
-  if (n_items > 0 && !sph)
-    counted(c, prepare_pairs(P, mode, has_m, has_z, logb, bt, tch, B.variant, c->num_sms, &B.L), "pair kernel");
+  for (int k = 0; k < 2; ++k) {
+    B.P[k] = P;
+    B.P[k].items = d_items[k];
+    B.P[k].n_items = n_run[k];
+    B.P[k].queue_head = head + 2 * k;
+    if (n_run[k] == 0 || sph) continue;
+    if (k == 1)
+      counted(c, prepare_pairs_series(B.P[k], mode, has_m, has_z, logb, bt, c->num_sms, &B.L[k]), "pair kernel");
+    else
+      counted(c, prepare_pairs(B.P[k], mode, has_m, has_z, logb, bt, tch, B.variant, c->num_sms, &B.L[k]), "pair kernel");
+  }
 
   B.mode = mode; B.sph = sph; B.sharded = sharded; B.use_patch_any = use_patch_any;
   B.has_m = has_m; B.has_z = has_z; B.logb = logb;
@@ -605,11 +665,14 @@ void batch_launch(tpcf_ctx* c, Batch& B, bool timed) {
       check(cudaEventRecord(ev0, st), "event record");
     }
     if (B.sph) {
-      counted(c, launch_pairs_sph(B.P, B.mode, B.has_m, B.has_z, B.logb, B.bt, c->num_sms, st, &B.grid),
+      counted(c, launch_pairs_sph(B.P[0], B.mode, B.has_m, B.has_z, B.logb, B.bt, c->num_sms, st, &B.grid),
               "pair kernel");
     } else {
-      B.grid = B.L.grid;
-      counted(c, launch_prepared(B.L, B.P, st), "pair kernel");
+      for (int k = 0; k < 2; ++k) {
+        if (B.P[k].n_items == 0) continue;
+        B.grid = B.L[k].grid;
+        counted(c, launch_prepared(B.L[k], B.P[k], st), "pair kernel");
+      }
     }
     if (timed) {
       check(cudaEventRecord(ev1, st), "event record");
@@ -618,9 +681,9 @@ void batch_launch(tpcf_ctx* c, Batch& B, bool timed) {
     }
   }
   for (int t = 0; t < B.nT; ++t) {
-    const LensBuilt& LB = B.lb[B.tl[t]];
-    if (B.n_items > 0 && LB.n_groups > 0)
-      counted(c, launch_patch_reduce(B.item_sums, B.tdesc[t].item_base, LB.d_patch_groups, B.n_patch_eff, nb,
+    const LensGroups& LG = B.lb[B.tl[t]].by[(int)B.kind[t]];
+    if (B.n_items > 0 && LG.n_groups > 0)
+      counted(c, launch_patch_reduce(B.item_sums, B.tdesc[t].item_base, B.tdesc[t].split, LG.d_patch_groups, B.n_patch_eff, nb,
                                      B.dpatch[t], st), "patch reduce");
     else
       check(cudaMemsetAsync(B.dpatch[t], 0, sizeof(double) * kQ * nb * B.n_patch_eff, st), "memset patch");

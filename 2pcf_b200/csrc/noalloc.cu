@@ -240,7 +240,7 @@ tpcf_status run_noalloc(tpcf_ctx* c, const float* xA, const float* yA, const flo
   counted(c, cudaGetLastError(), "groups");
   counted(c, launch_group_box(lrec, gstart, n_groups, gbox, st), "group box");
   TaskDesc td{};
-  td.lens_cat = 0; td.src_cat = 0; td.item_base = 0; td.lens_acc_off = -1; td.margin = margin;
+  td.lens_cat = 0; td.src_cat = 0; td.item_base = 0; td.lens_acc_off = -1; td.margin = margin; td.split = 1;
   LensDesc ld{};
   ld.rec = lrec; ld.z = zs; ld.group_start = gstart; ld.group_box = gbox; ld.n_valid = nl_valid;
   ld.n_groups = n_groups;
@@ -269,7 +269,7 @@ tpcf_status run_noalloc(tpcf_ctx* c, const float* xA, const float* yA, const flo
     }
     int grid = 0;
     counted(c, launch_pairs(P, 0, has_m, has_z, logb, bt, 2, 0, c->num_sms, st, &grid), "pair kernel");
-    counted(c, launch_patch_reduce(item_sums, 0, pgroups, 1, nb, psum, st), "patch reduce");
+    counted(c, launch_patch_reduce(item_sums, 0, 1, pgroups, 1, nb, psum, st), "patch reduce");
   } else {
     check(cudaMemsetAsync(psum, 0, sizeof(double) * kQ * nb, st), "clear sums");
   }

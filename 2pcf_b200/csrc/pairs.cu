@@ -35,6 +35,7 @@
 #include <cstdio>
 
 #include "pair_hist.cuh"
+#include "pair_tiles.cuh"
 #include "tpcf_device.cuh"
 #include "tpcf_internal.cuh"
 #include "tpcf_kernels.h"
@@ -111,7 +112,7 @@ __device__ __forceinline__ void do_pair(float lx, float ly, float lz, const floa
   // d2 = 0 is in range: there d = sqrt(0) = 0 exactly (as in the reference).
   float d, r;
   if (LOGB) {
-    const float rs = rsqrtf(d2);
+    const float rs = rsqrt_ftz(d2);
     d = d2 * rs;
     r = rs * rs;
   } else {
@@ -183,7 +184,7 @@ __device__ __forceinline__ void pair_terms2(const LensP& L, const float4 xy, con
   const float2 dx2 = mul2(dxp, dxp);
   d2 = fma2(dyp, dyp, dx2);
   if (LOGB) {
-    const float2 rs = make_float2(rsqrtf(d2.x), rsqrtf(d2.y));
+    const float2 rs = make_float2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y));
     d = mul2(d2, rs);
     r = mul2(rs, rs);
   } else {
@@ -402,81 +403,6 @@ extern "C" int tpcf_debug_mode_stats(unsigned long long* out) {
 }
 #endif
 
-// ------------------------------------------------------------- tile ring --
-// Each warp walks the cell rows of its work item 32 at a time, lane r holding
-// the source span [s0, s1) of row c0 + r.  A row's span covers the sub-chunks
-// [s0 / 32, ceil(s1 / 32)); its first and last sub-chunks are partial when s0
-// or s1 is not a multiple of 32.  Tile k of the pass is the (k - first)-th
-// group of TCH sub-chunks of the row whose prefix of tile counts contains k.
-struct TileGeom {
-  int c0, n, lo0, hiL;
-};
-template <int TCH>
-__device__ __forceinline__ int tiles_of_span(int s, int e) {
-  if (e <= s) return 0;
-  const int nc = ((e + kChunk - 1) >> 5) - (s >> 5);
-  return (nc + TCH - 1) / TCH;
-}
-// Called by all 32 lanes with the same k (0 <= k < the pass's tile count);
-// incl = this lane's inclusive prefix of tile counts, s0/s1 its row's span.
-template <int TCH>
-__device__ __forceinline__ TileGeom tile_of(int k, int incl, int ntr, int s0, int s1) {
-  const int r = __popc(__ballot_sync(0xffffffffu, incl <= k));  // first row with incl > k
-  const int s = __shfl_sync(0xffffffffu, s0, r);
-  const int e = __shfl_sync(0xffffffffu, s1, r);
-  const int first = __shfl_sync(0xffffffffu, incl - ntr, r);
-  const int kk = k - first;
-  const int cA = s >> 5, cB = (e + kChunk - 1) >> 5;
-  TileGeom t;
-  t.c0 = cA + kk * TCH;
-  t.n = min(TCH, cB - t.c0);
-  t.lo0 = kk == 0 ? (s & (kChunk - 1)) : 0;
-  t.hiL = (t.c0 + t.n == cB && (e & (kChunk - 1))) ? (e & (kChunk - 1)) : kChunk;
-  return t;
-}
-
-// Fold this warp's 32 histogram columns into its FP64 sums (times the lens
-// factors val*w or w) and, when lens_col is set, each lane's per-lens FP64
-// column (zeroed before the launch; a lens's pairs between two folds fall in
-// few bins, so only its non-zero cells are added, as fire-and-forget FP64
-// reductions: each column has one writer, so the adds land in program order
-// and the result is deterministic, and no load latency is waited for); then
-// clear the columns.  Called by all lanes of the warp.
-template <int QA, int BT>
-__device__ __forceinline__ void warp_fold(const float* hist, float* hcol, double* wsum, const double* fvw,
-                                          const double* fw, int nb, double* lens_col, size_t lens_stride, int warp,
-                                          int lane) {
-  __syncwarp();
-  if (lens_col) {
-    for (int q = 0; q < kQ; ++q) {
-      const int qa = (q == QK && QA == 5) ? QW : q;
-      for (int b = 0; b < nb; ++b) {
-        const float v = hcol[(b * QA + qa) * BT];
-        if (v != 0.f) atomicAdd(lens_col + (size_t)(q * nb + b) * lens_stride, (double)v);
-      }
-    }
-  }
-  const int cb = warp * 32;
-  for (int e = lane; e < kQ * nb; e += 32) {
-    const int q = e / nb, b = e - q * nb;
-    if (q == QK && QA == 5) continue;  // K == w: copied from the w row at item end
-    const float* row = hist + (b * QA + q) * BT + cb;
-    double s = 0.0;
-    if (q == QN) {
-      for (int l = 0; l < 32; ++l) s += (double)row[(l + lane) & 31];
-    } else {
-      const double* f = ((q == QGT || q == QGX) ? fvw : fw) + cb;
-      for (int l = 0; l < 32; ++l) {
-        const int c = (l + lane) & 31;
-        s = fma((double)row[c], f[c], s);
-      }
-    }
-    wsum[e] += s;
-  }
-  __syncwarp();
-  for (int e = 0; e < nb * QA; ++e) hcol[e * BT] = 0.f;
-}
-
 // ------------------------------------------------------------ pair kernel --
 // Every warp is independent: it takes its own work items (32 lenses, one per
 // lane, against every source row the group's theta_max neighbourhood touches)
@@ -550,7 +476,7 @@ __global__ void __launch_bounds__(BT, kPairMinBlocks) k_pairs(const PairParams P
     const TaskDesc T = P.tasks[it.x];
     const LensDesc LD = P.lenses[T.lens_cat];
     const GridDesc G = P.grids[T.src_cat];
-    const int g = it.y;
+    const int g = it.y / T.split, part = it.y - g * T.split;
     const int gs = LD.group_start[g];
     const int nl = LD.group_start[g + 1] - gs;
     const bool act = lane < nl;
@@ -577,11 +503,11 @@ __global__ void __launch_bounds__(BT, kPairMinBlocks) k_pairs(const PairParams P
     int cy0, cy1;
     row_range(G, box, P.R, T.margin, cy0, cy1);
 
-    for (int c0 = cy0; c0 <= cy1 && !aborted; c0 += kRowsPerPass) {
-      const int nr = min(kRowsPerPass, cy1 - c0 + 1);
+    for (int c0 = cy0 + part; c0 <= cy1 && !aborted; c0 += kRowsPerPass * T.split) {
       int s0 = 0, s1 = 0;
-      if (lane < nr) {
-        const int2 sp = row_span(G, box, P.R, T.margin, c0 + lane);
+      const int row = c0 + lane * T.split;
+      if (row <= cy1) {
+        const int2 sp = row_span(G, box, P.R, T.margin, row);
         s0 = sp.x;
         s1 = sp.y > sp.x ? sp.y : sp.x;
       }
@@ -687,7 +613,7 @@ __global__ void __launch_bounds__(BT, kPairMinBlocks) k_pairs(const PairParams P
     }
     if (aborted) break;
     warp_fold<QA, BT>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, warp, lane);
-    double* out = P.item_sums + (size_t)(T.item_base + g) * kQ * nb;
+    double* out = P.item_sums + (size_t)(T.item_base + it.y) * kQ * nb;
     for (int e = lane; e < kQ * nb; e += 32) {
       const int src = (e / nb == QK && QA == 5) ? e - (QK - QW) * nb : e;
       out[e] = wsum[src];
@@ -996,15 +922,16 @@ __global__ void k_item_cost(const int2* __restrict__ items, int n_items, const T
   const TaskDesc T = tasks[it.x];
   const LensDesc L = lenses[T.lens_cat];
   const GridDesc G = grids[T.src_cat];
-  const float4 box = L.group_box[it.y];
+  const int g = it.y / T.split, part = it.y - g * T.split;
+  const float4 box = L.group_box[g];
   int cy0, cy1;
   row_range(G, box, R, T.margin, cy0, cy1);
   unsigned long long s = 0;
-  for (int cy = cy0; cy <= cy1; ++cy) {
+  for (int cy = cy0 + part; cy <= cy1; cy += T.split) {
     const int2 sp = row_span(G, box, R, T.margin, cy);
     if (sp.y > sp.x) s += (unsigned long long)(sp.y - sp.x);
   }
-  const unsigned long long nl = (unsigned long long)(L.group_start[it.y + 1] - L.group_start[it.y]);
+  const unsigned long long nl = (unsigned long long)(L.group_start[g + 1] - L.group_start[g]);
   cost[i] = item_key(s * nl + 1, i);
   order[i] = i;
 }
@@ -1049,20 +976,20 @@ __global__ void k_dfma_peak(double* out, int iters, double a, double b) {
 }
 
 // Per-patch FP64 sums from item sums, fixed order (deterministic).
-// patch_groups[p] .. patch_groups[p+1] are the groups of patch p.  Block
+// patch_groups[p] .. patch_groups[p+1] are the groups of patch p, `split` items each.  Block
 // (p, c) covers the 32 sums e = 32 c + lane of patch p: warp w adds the groups
 // g0 + w, g0 + w + 8, ... (lane-contiguous loads), then the 8 warp sums are
 // added in warp order.
 constexpr int kReduceWarps = 8;
 __global__ void __launch_bounds__(32 * kReduceWarps) k_patch_reduce(const double* __restrict__ item_sums, int item_base,
-                                                                   const int* __restrict__ patch_groups, int n_patch,
+                                                                   int split, const int* __restrict__ patch_groups, int n_patch,
                                                                    int nb, double* patch_sums) {
   __shared__ double part[kReduceWarps][32];
   const int p = blockIdx.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int e = blockIdx.y * 32 + lane;
   const int ne = kQ * nb;
-  const int g0 = patch_groups[p], g1 = patch_groups[p + 1];
+  const int g0 = patch_groups[p] * split, g1 = patch_groups[p + 1] * split;
   double s = 0.0;
   if (e < ne) {
 #pragma unroll 4
@@ -1280,10 +1207,10 @@ cudaError_t launch_dfma_peak(double* out, int blocks, int threads, int iters, cu
   k_dfma_peak<<<blocks, threads, 0, st>>>(out, iters, 0.999999999, 1e-13);
   return cudaGetLastError();
 }
-cudaError_t launch_patch_reduce(const double* item_sums, int item_base, const int* patch_groups, int n_patch, int nb,
-                                double* patch_sums, cudaStream_t st) {
+cudaError_t launch_patch_reduce(const double* item_sums, int item_base, int split, const int* patch_groups, int n_patch,
+                                int nb, double* patch_sums, cudaStream_t st) {
   if (n_patch > 0)
-    k_patch_reduce<<<dim3(n_patch, (kQ * nb + 31) / 32), 32 * kReduceWarps, 0, st>>>(item_sums, item_base, patch_groups,
+    k_patch_reduce<<<dim3(n_patch, (kQ * nb + 31) / 32), 32 * kReduceWarps, 0, st>>>(item_sums, item_base, split, patch_groups,
                                                                                     n_patch, nb, patch_sums);
   return cudaGetLastError();
 }

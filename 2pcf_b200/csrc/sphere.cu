@@ -111,7 +111,7 @@ __device__ __forceinline__ void sph_terms(const LensS& L, const float4 a, const 
   const float dz = (a.z - L.h.z) + (b.z - L.l.z);
   d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
   // series path: binned pairs have d2 > 0; otherwise c = 0 exactly at d2 = 0
-  const float c = SMALL ? d2 * rsqrtf(d2) : sqrtf(d2);
+  const float c = SMALL ? d2 * rsqrt_ftz(d2) : sqrtf(d2);
   th = chord_theta<SMALL>(d2, c);
   if (MODE == 0) {
     const float A = fmaf(dy, L.ey, dx * L.ex);
@@ -135,7 +135,7 @@ template <bool LOGB>
 __device__ __forceinline__ int pair_bin_s(float d2, const LensS& L, const float4 a, const float4 b,
                                           const BinCtx& C) {
   if (LOGB) {
-    const float t = fmaf(__log2f(chord_theta2(d2)), C.A, C.B);
+    const float t = fmaf(lg2_ftz(chord_theta2(d2)), C.A, C.B);
     const float tf = floorf(t);
     const float fr = t - tf;
     int bin = __float2int_rz(tf);
@@ -170,8 +170,8 @@ __device__ __forceinline__ int classify_s(const LensS& L, const float4 mn, const
   const float dmax2 = fmaf(dzh, dzh, fmaf(dyh, dyh, dxh * dxh));
   int b0, b1;
   if (LOGB) {
-    b0 = __float2int_rd(fmaf(__log2f(chord_theta2(dmin2)), C.A, C.B) - C.eps);
-    b1 = __float2int_rd(fmaf(__log2f(chord_theta2(dmax2)), C.A, C.B) + C.eps);
+    b0 = __float2int_rd(fmaf(lg2_ftz(chord_theta2(dmin2)), C.A, C.B) - C.eps);
+    b1 = __float2int_rd(fmaf(lg2_ftz(chord_theta2(dmax2)), C.A, C.B) + C.eps);
   } else {
     b0 = edge_index_f32(dmin2 * (1.f - C.eps), C.e2f, C.nb);
     b1 = edge_index_f32(dmax2 * (1.f + C.eps), C.e2f, C.nb);
@@ -266,7 +266,7 @@ __device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, f
   const float2 dz = add2(add2(lo2(s.hzp), L.nhz), add2(lo2(s.lzq), L.nlz));
   d2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
   if (SMALL) {
-    const float2 c = mul2(d2, make_float2(rsqrtf(d2.x), rsqrtf(d2.y)));
+    const float2 c = mul2(d2, make_float2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y)));
     th = mul2(c, fma2(d2, fma2(d2, fma2(d2, dup2(6.9754464e-4f), dup2(4.6875e-3f)), dup2(4.16666679e-2f)),
                       dup2(1.f)));
   } else {

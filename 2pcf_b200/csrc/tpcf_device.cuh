@@ -21,6 +21,20 @@ __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); 
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 __device__ __forceinline__ float sum2(float2 v) { return v.x + v.y; }
 
+// MUFU reciprocal square root and logarithm without the denormal scaling of
+// the default forms (three more instructions each): their arguments are squared
+// distances, 0 or far above 1e-38; lg2 of 0 is -inf, rsqrt of 0 is inf.
+__device__ __forceinline__ float rsqrt_ftz(float v) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float lg2_ftz(float v) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 // ------------------------------------------------------------ PTX helpers --
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -161,7 +175,7 @@ struct BinCtx {
 template <bool LOGB>
 __device__ __forceinline__ int pair_bin(float d2, float lx, float ly, float sx, float sy, const BinCtx& C) {
   if (LOGB) {
-    const float t = fmaf(__log2f(d2), C.A, C.B);
+    const float t = fmaf(lg2_ftz(d2), C.A, C.B);
     const float tf = floorf(t);
     const float fr = t - tf;
     int b = __float2int_rz(tf);
@@ -201,8 +215,8 @@ __device__ __forceinline__ int classify(float lx, float ly, const float4 box, co
   const float dmax2 = fmaf(dyh, dyh, dxh * dxh);
   int b0, b1;
   if (LOGB) {
-    b0 = __float2int_rd(fmaf(__log2f(dmin2), C.A, C.B) - C.eps);
-    b1 = __float2int_rd(fmaf(__log2f(dmax2), C.A, C.B) + C.eps);
+    b0 = __float2int_rd(fmaf(lg2_ftz(dmin2), C.A, C.B) - C.eps);
+    b1 = __float2int_rd(fmaf(lg2_ftz(dmax2), C.A, C.B) + C.eps);
   } else {
     b0 = edge_index_f32(dmin2 * (1.f - C.eps), C.e2f, C.nb);
     b1 = edge_index_f32(dmax2 * (1.f + C.eps), C.e2f, C.nb);
@@ -233,8 +247,8 @@ __device__ __forceinline__ int classify_edges(float lx, float ly, const float4 b
   const float dmax2 = fmaf(dyh, dyh, dxh * dxh);
   int b0, b1;
   if (LOGB) {
-    b0 = __float2int_rd(fmaf(__log2f(dmin2), C.A, C.B) - C.eps);
-    b1 = __float2int_rd(fmaf(__log2f(dmax2), C.A, C.B) + C.eps);
+    b0 = __float2int_rd(fmaf(lg2_ftz(dmin2), C.A, C.B) - C.eps);
+    b1 = __float2int_rd(fmaf(lg2_ftz(dmax2), C.A, C.B) + C.eps);
   } else {
     b0 = edge_index_f32(dmin2 * (1.f - C.eps), C.e2f, C.nb);
     b1 = edge_index_f32(dmax2 * (1.f + C.eps), C.e2f, C.nb);

@@ -88,6 +88,7 @@ struct GridDesc {
   const SrcRecS* recs;    // [n_valid], sorted by cell (sphere), else nullptr
   const SrcPair* pairs;   // planar sources: [ceil(n_valid/32) * 16] in sub-chunk form
   const ChunkMeta* meta;  // [ceil(n_valid/32)]
+  const float* series;    // sub-chunk records with moments (k_pairs_series), else nullptr
 };
 
 struct LensDesc {
@@ -105,6 +106,8 @@ struct TaskDesc {
   int src_cat;
   int item_base;            // row of (task, group 0) in item_sums
   float margin;             // FP32 guard on the reach of this task's rows and cells
+  int split;                // work items per lens group, each with every split-th cell row (1 for most)
+  int pad;
   long long lens_acc_off;   // element offset of this task's per-lens sums, -1 = none
 };
 
@@ -112,7 +115,7 @@ struct PairParams {
   const TaskDesc* tasks;
   const LensDesc* lenses;
   const GridDesc* grids;
-  const int2* items;        // (task, group) in processing order
+  const int2* items;        // (task, group * split + part) in processing order
   int n_items;
   int nb;
   int* queue_head;
@@ -124,6 +127,7 @@ struct PairParams {
   float R;                  // search radius: theta_max with a relative margin
   float binA, binB;         // log spacing: t = lg2(d2)*binA + binB
   float eps;                // guard band half-width in t units (log) or relative (generic)
+  int far_bin;              // k_pairs_series: first bin of the far sums
   int flush_src;            // FP32 histogram -> FP64 after this many sources (0: 4096)
   // Fault injection for tests only (0 in every product call): 1 + the ring
   // index of a source tile whose bulk copy is never issued, so that the waits

@@ -23,6 +23,16 @@ struct PairLaunch {
 };
 cudaError_t prepare_pairs(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int bt, int tch,
                           int variant, int num_sms, PairLaunch* L);
+// The same for the kernel of calls without per-lens outputs (pairs_series.cu),
+// whose sub-chunk records are series_bytes long and made by launch_src_series.
+cudaError_t prepare_pairs_series(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int bt, int num_sms,
+                                 PairLaunch* L);
+int series_lens_group();  // lenses per work item
+int series_far_bin(const double* e2, int nb);
+size_t series_bytes(int n_valid, int mode, bool has_m, bool has_z);
+cudaError_t launch_src_series(const int* idx, int n_valid, int mode, bool has_m, bool has_z, const float* x,
+                              const float* y, const float* z, const float* f1, const float* f2, const float* w,
+                              const float* m, float* rec, cudaStream_t st);
 cudaError_t launch_prepared(const PairLaunch& L, const PairParams& P, cudaStream_t st);
 
 // Spherical pair kernel (sphere.cu); P.grids[*].recs and P.lenses[*].pos set.
@@ -72,8 +82,8 @@ cudaError_t launch_permute_items(const int2* items, const int* order, int n, int
                                  cudaStream_t st);
 cudaError_t launch_ffma_peak(float* out, int blocks, int threads, int iters, cudaStream_t st);
 cudaError_t launch_dfma_peak(double* out, int blocks, int threads, int iters, cudaStream_t st);
-cudaError_t launch_patch_reduce(const double* item_sums, int item_base, const int* patch_groups, int n_patch,
-                                int nb, double* patch_sums, cudaStream_t st);
+cudaError_t launch_patch_reduce(const double* item_sums, int item_base, int split, const int* patch_groups,
+                                int n_patch, int nb, double* patch_sums, cudaStream_t st);
 cudaError_t launch_lens_outputs(const double* acc, const float4* rec, const int* perm, int n_valid, int nb,
                                 float* xi_E, float* xi_B, float* K_m, float* w_m, float* marks_weight,
                                 double* lens_sums, double* lens_raw, cudaStream_t st);

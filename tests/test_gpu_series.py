@@ -1,0 +1,110 @@
+"""The series pair kernel (dense source catalogues without per-lens outputs):
+sub-chunk moments, direct passes at bin edges, ragged groups and sub-chunks,
+against the FP64 oracle.  Bar as in test_gpu_pairs: n_pairs bit-exact, every sum
+within 1e-6 of the oracle's sum of |terms| (FP32 pair terms, FP64 sums; the series
+is truncated below 1e-7 of a sub-chunk's sum of |terms|)."""
+import numpy as np
+import pytest
+
+from parity import check_sums
+
+pytestmark = pytest.mark.gpu
+
+N_SRC, BOX = 60_001, 60.0   # sub-chunks of about 1.4' a side, the last one ragged
+
+
+def f32(a):
+    return np.ascontiguousarray(a, np.float32)
+
+
+def catalogues(seed, n_lens, n_src=N_SRC, z=False):
+    rng = np.random.default_rng(seed)
+    L = dict(x=f32(rng.uniform(0, BOX, n_lens)), y=f32(rng.uniform(0, BOX, n_lens)),
+             z=f32(rng.uniform(0, 0.8, n_lens)) if z else np.zeros(n_lens, np.float32),
+             val=f32(rng.normal(0.01, 0.02, n_lens)), w=f32(rng.uniform(0.5, 1.5, n_lens)))
+    S = dict(x=f32(rng.uniform(0, BOX, n_src)), y=f32(rng.uniform(0, BOX, n_src)),
+             z=f32(rng.uniform(0.1, 1.2, n_src)) if z else np.ones(n_src, np.float32),
+             e1=f32(rng.normal(0, .26, n_src)), e2=f32(rng.normal(0, .26, n_src)),
+             w=f32(rng.uniform(0.5, 1.5, n_src)), m=f32(rng.normal(0, .03, n_src)) if z else np.zeros(n_src, np.float32))
+    return L, S
+
+
+def shear(tpcf, ctx, L, S, bins, **kw):
+    return tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"], S["e1"],
+                                      S["e2"], S["w"], S["m"], bins, calculate_marks=False, ctx=ctx, **kw)
+
+
+@pytest.mark.parametrize("n_lens,z", [(1, False), (63, False), (64, True), (65, False), (200, True)])
+def test_log_bins(tpcf, oracle, ctx, n_lens, z):
+    L, S = catalogues(60 + n_lens, n_lens, z=z)
+    bins = tpcf.create_bins(0.3, 25.0, 8)
+    res = shear(tpcf, ctx, L, S, bins)
+    check_sums(f"series log {n_lens} lenses z={z}", res, oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
+
+
+@pytest.mark.parametrize("spacing,lo", [("lin", 0.0), ("sqrt", 0.5), ("ihs", 0.2)])
+def test_other_spacings(tpcf, oracle, ctx, spacing, lo):
+    L, S = catalogues(71, 70)
+    bins = tpcf.create_bins(lo, 20.0, 12, spacing=spacing, p=0.5)
+    res = shear(tpcf, ctx, L, S, bins)
+    check_sums(f"series {spacing}", res, oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
+
+
+def test_coincident_pair_in_the_first_linear_bin(tpcf, oracle, ctx):
+    """A lens on a source with x_min = 0: the pair counts, its d is 0, its g
+    terms are 0/0 in bin 0 and nowhere else."""
+    L, S = catalogues(72, 66)
+    L["x"][5], L["y"][5] = S["x"][777], S["y"][777]
+    bins = tpcf.create_bins(0.0, 20.0, 10, spacing="lin")
+    res = shear(tpcf, ctx, L, S, bins)
+    can = oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq)
+    np.testing.assert_array_equal(res.n_pairs, can["n_pairs"].astype(np.int64))
+    assert np.isnan(res.sum_gt[0]) and np.all(np.isfinite(res.sum_gt[1:]))
+    assert np.all(np.abs(res.sum_gt[1:] - can["sum_gt"][1:]) <= 1e-6 * can["abs_gt"][1:])
+    np.testing.assert_allclose(res.sum_dw, can["sum_dw"], rtol=1e-6)
+
+
+def test_kappa_auto_correlation(tpcf, oracle, ctx):
+    rng = np.random.default_rng(73)
+    n = 20_011
+    x, y = f32(rng.uniform(0, BOX, n)), f32(rng.uniform(0, BOX, n))
+    k, w = f32(rng.normal(0, .02, n)), f32(rng.uniform(0.5, 1.5, n))
+    kb = f32(rng.normal(0, .01, n))
+    bins = tpcf.create_bins(0.5, 25.0, 5)
+    res = tpcf.scalar_kappa_tpcf(x, y, k, w, x, y, k, kb, w, bins, calculate_marks=False, ctx=ctx)
+    L = dict(x=x, y=y, val=k, w=w)
+    K = dict(x=x, y=y, kappa_E=k, kappa_B=kb, w=w)
+    check_sums("series kappa auto", res, oracle.canon_pairs(oracle.KAPPA, L, K, bins.bin_edges_sq))
+
+
+def test_pairs_on_the_edges(tpcf, oracle, ctx):
+    """Dense rings within a few ulp of every edge: decided in FP64."""
+    bins = tpcf.create_bins(1.0, 25.0, 6)
+    rng = np.random.default_rng(74)
+    n = 60_000
+    d = bins.bin_edges[rng.integers(0, 7, n)] * (1.0 + rng.integers(-40, 41, n) * 1e-8)
+    a = rng.uniform(0, 2 * np.pi, n)
+    _, S = catalogues(74, 1, n_src=n)
+    S["x"], S["y"] = f32(30 + d * np.cos(a)), f32(30 + d * np.sin(a))
+    L = dict(x=np.full(3, 30, np.float32), y=np.full(3, 30, np.float32), z=np.zeros(3, np.float32),
+             val=np.ones(3, np.float32), w=np.ones(3, np.float32))
+    res = shear(tpcf, ctx, L, S, bins)
+    check_sums("series rings", res, oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
+
+
+def test_patches_and_mixed_batch(tpcf, oracle, ctx):
+    """A dense and a sparse source catalogue in one batch (two pair kernels):
+    each task as when launched alone, patch sums adding up to the totals."""
+    rng = np.random.default_rng(75)
+    L, S = catalogues(75, 150)
+    _, S2 = catalogues(76, 1, n_src=500)
+    bins = tpcf.create_bins(0.5, 25.0, 8)
+    lab = rng.integers(0, 5, 150).astype(np.int32)
+    lc = tpcf.LensCatalog(L["x"], L["y"], L["val"], L["w"], L["z"])
+    sc = [tpcf.ShapeCatalog(s["x"], s["y"], s["e1"], s["e2"], s["w"], s["z"], s["m"]) for s in (S, S2)]
+    both = tpcf.batch_shear_2pcf([lc], sc, [(0, 0), (0, 1)], bins, lens_patches=[lab], n_patch=5, ctx=ctx)
+    for i, s in enumerate((S, S2)):
+        check_sums(f"series mixed batch {i}", both[i], oracle.canon_pairs(oracle.SHEAR, L, s, bins.bin_edges_sq))
+        one = tpcf.batch_shear_2pcf([lc], [sc[i]], [(0, 0)], bins, lens_patches=[lab], n_patch=5, ctx=ctx)[0]
+        np.testing.assert_array_equal(one.patch_sums, both[i].patch_sums)
+        np.testing.assert_array_equal(both[i].patch_sums[:, 5].sum(0), both[i].n_pairs)
