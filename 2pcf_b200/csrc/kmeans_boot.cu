@@ -50,76 +50,211 @@ __global__ void k_km_init_labels(int* labels, long long n, int k) {
   }
 }
 
-// Assign each point to its nearest centroid; accumulate fixed-point sums of
-// x*w, y*w and w per cluster and count the reassignments.
-__global__ void k_km_assign(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ w,
-                            long long n, const float2* __restrict__ cen, int k, float min_init, double sp_scale,
-                            double sw_scale, int* labels, unsigned long long* acc, unsigned long long* n_re,
-                            const int* state) {
-  if (state[0]) return;  // converged in an earlier pass of this batch
+// One Lloyd pass: assign each point to its nearest centroid, move the
+// fixed-point sums of x*w, y*w and w by the points that changed cluster (the
+// first pass adds every point), then, in the block that finishes last, set the
+// centroids and evaluate the stopping rule of src/kmeans.f90:118-137: the run
+// stops after a pass with no reassignment, a reassigned fraction below tol,
+// or max_iter + 1 passes.
+//
+// Most points are settled by a bound, not by k distances: far[i] holds a lower
+// bound on the distance from point i to every centroid but its own, plus the
+// total drift D (the sum over the passes of the largest centroid move) at the
+// time it was formed; half[j] is half the distance from centroid j to its
+// nearest neighbour.  If the FP32 distance u to its own centroid stays below
+// far[i] - D or half[own] by a relative 4e-6 -- ten times what FP32 rounding can
+// move either -- its centroid is the strict nearest in FP32 too, and its label
+// stands.  (half settles most points while a few centroids still move far.)
+// The others are listed per tile of the block and search all centroids, eight
+// lanes per point, by the reference's rule: smallest correctly rounded
+// sqrt(dx*dx + dy*dy), the first one on a tie, below min_init.  The labels are
+// those of the plain search in every pass.
+//
+// 1 M points, 100 centroids: 21.5 ms for the call when every pass formed every
+// distance and re-summed every point, 8.6 ms with far alone, 6.6 ms with both and
+// one wave of blocks (32 registers; 222 passes of 10 to 30 us: the latency of
+// the chain label -> centroid -> search -> last block, not its traffic).
+struct KmState {
+  int done, passes;
+  float drift;
+  int pad;
+  unsigned long long arrived;  // blocks done (low half) and points that changed cluster (high half)
+};
+constexpr int kKmThreads = 512, kKmTile = 2048;
+constexpr int kKmHalf = 512;  // half is formed for up to this many centroids (k^2 distances a pass)
+__global__ void __launch_bounds__(kKmThreads, 4) k_km_pass(const float* __restrict__ x, const float* __restrict__ y,
+                                                        const float* __restrict__ w, long long n, float2* cen, int k,
+                                                        float min_init, int sp, int sw, int* labels, float* far,
+                                                        float* half, unsigned long long* acc, float tol, int max_iter,
+                                                        KmState* state) {
+  if (state->done) return;  // converged in an earlier pass of this batch
   extern __shared__ unsigned char sm[];
   float2* c = reinterpret_cast<float2*>(sm);
   unsigned long long* a = reinterpret_cast<unsigned long long*>(c + k);
-  for (int j = threadIdx.x; j < k; j += blockDim.x) c[j] = cen[j];
+  float* h = reinterpret_cast<float*>(a + 3 * k);
+  __shared__ int list[kKmTile];
+  __shared__ int n_list;
+  __shared__ unsigned n_changed;
+  __shared__ unsigned long long before;
+  __shared__ float smove[kKmThreads / 32];
+  const bool first = state->passes == 0;
+  const float D = state->drift;
+  const double sp_scale = ldexp(1.0, sp), sw_scale = ldexp(1.0, sw);
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    c[j] = cen[j];
+    h[j] = half[j];
+  }
   for (int j = threadIdx.x; j < 3 * k; j += blockDim.x) a[j] = 0ull;
-  __syncthreads();
-  unsigned long long re = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float xi = x[i], yi = y[i];
-    float best = min_init;
-    int bi = -1;
-    // the correctly rounded sqrt (as the reference) only where it can win:
-    // q > best^2 (1 + 1e-5) gives sqrt(q) > best whatever the roundings
-    float tsq = __fmul_rn(min_init, min_init) * 1.00001f;
-    for (int j = 0; j < k; ++j) {
-      const float dx = __fsub_rn(xi, c[j].x), dy = __fsub_rn(yi, c[j].y);
-      const float q = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-      if (q > tsq) continue;
-      const float d = __fsqrt_rn(q);
-      if (d < best) {
-        best = d;
-        bi = j;
-        tsq = __fmul_rn(best, best) * 1.00001f;
+  unsigned re = 0;
+  if (threadIdx.x == 0) n_changed = 0;
+  for (long long t0 = (long long)blockIdx.x * kKmTile; t0 < n; t0 += (long long)gridDim.x * kKmTile) {
+    if (threadIdx.x == 0) n_list = 0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kKmTile / kKmThreads; ++u) {
+      const long long i = t0 + u * kKmThreads + threadIdx.x;
+      bool open = i < n;
+      if (open && !first) {
+        const int l = labels[i];
+        if (l >= 0) {
+          const float dx = x[i] - c[l].x, dy = y[i] - c[l].y;
+          const float d = sqrtf(dx * dx + dy * dy) * 1.000004f;
+          open = !((d < h[l] || d < far[i] - D) && d < 0.999f * min_init);
+        }
+      }
+      if (open) list[atomicAdd(&n_list, 1)] = (int)(i - t0);
+    }
+    __syncthreads();
+    const int nl = n_list;
+    // eight lanes per point: lane v takes centroids v, v + 8, ..
+    for (int q0 = threadIdx.x >> 3; q0 < (nl + 3) / 4 * 4; q0 += kKmThreads / 8) {  // whole warps
+      const bool live = q0 < nl;
+      const long long i = t0 + list[live ? q0 : 0];
+      const float xi = x[i], yi = y[i];
+      const int old = labels[i];
+      // the two smallest squared distances and where the smallest is (a NaN
+      // centroid is no candidate)
+      float q1 = INFINITY, q2 = INFINITY;
+      int bi = -1;
+#pragma unroll 4
+      for (int j = threadIdx.x & 7; j < k; j += 8) {
+        const float dx = __fsub_rn(xi, c[j].x), dy = __fsub_rn(yi, c[j].y);
+        const float q = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+        q2 = fminf(q2, fmaxf(q1, q));
+        bi = q < q1 ? j : bi;
+        q1 = fminf(q1, q);
+      }
+#pragma unroll
+      for (int o = 4; o; o >>= 1) {
+        const float p1 = __shfl_xor_sync(0xffffffffu, q1, o), p2 = __shfl_xor_sync(0xffffffffu, q2, o);
+        const int pi = __shfl_xor_sync(0xffffffffu, bi, o);
+        q2 = fminf(fmaxf(q1, p1), fminf(q2, p2));
+        bi = p1 < q1 ? pi : bi;
+        q1 = fminf(q1, p1);
+      }
+      if (!live || (threadIdx.x & 7)) continue;
+      far[i] = (sqrtf(q2) * 0.999998f + D) * 0.9999998f;  // nearest of the others
+      // The reference compares correctly rounded square roots and keeps the first
+      // of equal ones: settled by the squares unless the two smallest nearly agree.
+      if (!(q2 > q1 * 1.000001f)) {
+        float best = min_init;
+        bi = -1;
+        for (int j = 0; j < k; ++j) {
+          const float dx = __fsub_rn(xi, c[j].x), dy = __fsub_rn(yi, c[j].y);
+          const float q = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+          if (!(q <= q1 * 1.000002f)) continue;
+          const float d = __fsqrt_rn(q);
+          if (d < best) {
+            best = d;
+            bi = j;
+          }
+        }
+        far[i] = 0.f;  // no bound
+      } else if (!(__fsqrt_rn(q1) < min_init)) {
+        bi = -1;
+      }
+      if (bi != old) {
+        labels[i] = bi;
+        ++re;
+      }
+      if (first || bi != old) {
+        const double wi = (double)w[i];
+        const long long vx = __double2ll_rn((double)xi * wi * sp_scale), vy = __double2ll_rn((double)yi * wi * sp_scale),
+                        vw = __double2ll_rn(wi * sw_scale);
+        if (bi >= 0) {
+          atomicAdd(&a[3 * bi + 0], (unsigned long long)vx);
+          atomicAdd(&a[3 * bi + 1], (unsigned long long)vy);
+          atomicAdd(&a[3 * bi + 2], (unsigned long long)vw);
+        }
+        if (!first && old >= 0) {
+          atomicAdd(&a[3 * old + 0], (unsigned long long)(-vx));
+          atomicAdd(&a[3 * old + 1], (unsigned long long)(-vy));
+          atomicAdd(&a[3 * old + 2], (unsigned long long)(-vw));
+        }
       }
     }
-    if (bi != labels[i]) {
-      labels[i] = bi;
-      ++re;
-    }
-    if (bi >= 0) {
-      const double wi = (double)w[i];
-      atomicAdd(&a[3 * bi + 0], (unsigned long long)__double2ll_rn((double)xi * wi * sp_scale));
-      atomicAdd(&a[3 * bi + 1], (unsigned long long)__double2ll_rn((double)yi * wi * sp_scale));
-      atomicAdd(&a[3 * bi + 2], (unsigned long long)__double2ll_rn(wi * sw_scale));
-    }
+    __syncthreads();
   }
   __syncthreads();
   for (int j = threadIdx.x; j < 3 * k; j += blockDim.x)
     if (a[j]) atomicAdd(&acc[j], a[j]);
-  for (int o = 16; o; o >>= 1) re += __shfl_xor_sync(0xffffffffu, re, o);
-  if ((threadIdx.x & 31) == 0 && re) atomicAdd(n_re, re);
+  if (re) atomicAdd(&n_changed, re);
+  // the last block to arrive sees every block's sums
+  __threadfence();
+  __syncthreads();
+  const unsigned long long mine = ((unsigned long long)n_changed << 32) + 1ull;
+  if (threadIdx.x == 0) before = atomicAdd(&state->arrived, mine);
+  __syncthreads();
+  if ((unsigned)before != gridDim.x - 1) return;
+  const unsigned r = (unsigned)((before + mine) >> 32);
+  __threadfence();
+  float move = 0.f;
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    const double W = ldexp((double)(long long)__ldcg(&acc[3 * j + 2]), -sw);
+    const double cx = ldexp((double)(long long)__ldcg(&acc[3 * j + 0]), -sp) / W;
+    const double cy = ldexp((double)(long long)__ldcg(&acc[3 * j + 1]), -sp) / W;
+    const float2 nc = make_float2((float)cx, (float)cy);
+    const float dx = nc.x - c[j].x, dy = nc.y - c[j].y;
+    move = fmaxf(move, sqrtf(dx * dx + dy * dy) * 1.000002f);  // (NaN: an empty cluster, no candidate any more)
+    cen[j] = nc;
+    c[j] = nc;
+  }
+  __syncthreads();
+  if (k <= kKmHalf) {  // 8 threads per centroid
+    for (int j0 = 0; j0 < k; j0 += kKmThreads / 8) {
+      const int j = j0 + (threadIdx.x >> 3);
+      float q = INFINITY;
+      if (j < k)
+        for (int i = threadIdx.x & 7; i < k; i += 8) {
+          const float dx = c[i].x - c[j].x, dy = c[i].y - c[j].y;
+          if (i != j) q = fminf(q, dx * dx + dy * dy);
+        }
+      for (int o = 4; o; o >>= 1) q = fminf(q, __shfl_xor_sync(0xffffffffu, q, o));
+      if (j < k && (threadIdx.x & 7) == 0) half[j] = 0.5f * sqrtf(q) * 0.999996f;
+    }
+  }
+  for (int o = 16; o; o >>= 1) move = fmaxf(move, __shfl_xor_sync(0xffffffffu, move, o));
+  if ((threadIdx.x & 31) == 0) smove[threadIdx.x >> 5] = move;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int v = 1; v < kKmThreads / 32; ++v) move = fmaxf(move, smove[v]);
+    state->drift = (D + move) * 1.0000002f;
+    const int it = state->passes + 1;
+    state->passes = it;
+    state->arrived = 0ull;
+    if (r == 0u || (float)r / (float)n < tol || it > max_iter) state->done = 1;
+  }
 }
 
 // Centroids from the fixed-point sums (two's-complement int64), then clear
-// them; then the stopping rule of src/kmeans.f90:118-137 on the device:
-// state = {done, passes}; the run stops after a pass with no reassignment, a
-// reassigned fraction below tol, or max_iter + 1 passes.  Without state only
-// the centroids are updated.
-__global__ void k_km_update(unsigned long long* acc, int k, int sp, int sw, float2* cen, unsigned long long* n_re,
-                            long long n, float tol, int max_iter, int* state) {
-  if (state && state[0]) return;
+// them (equal-weight k-means).
+__global__ void k_km_update(unsigned long long* acc, int k, int sp, int sw, float2* cen) {
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
     const double W = ldexp((double)(long long)acc[3 * j + 2], -sw);
     const double cx = ldexp((double)(long long)acc[3 * j + 0], -sp) / W;
     const double cy = ldexp((double)(long long)acc[3 * j + 1], -sp) / W;
     cen[j] = make_float2((float)cx, (float)cy);
     acc[3 * j + 0] = acc[3 * j + 1] = acc[3 * j + 2] = 0ull;
-  }
-  if (state && threadIdx.x == 0) {
-    const int it = ++state[1];
-    const unsigned long long re = *n_re;
-    *n_re = 0ull;
-    if (re == 0ull || (float)re / (float)n < tol || it > max_iter) state[0] = 1;
   }
 }
 
@@ -482,33 +617,33 @@ tpcf_status tpcf_kmeans(tpcf_ctx* c, const float* x, const float* y, const float
     const int sp = fixed_scale(n, amax * wmax), sw = fixed_scale(n, wmax);
     int* lab = (int*)ws_alloc(c, sizeof(int) * n);
     float2* dcen = (float2*)ws_alloc(c, sizeof(float2) * k);
-    unsigned long long* acc = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * (3 * k + 2));
-    unsigned long long* n_re = acc + 3 * k;
-    int* state = reinterpret_cast<int*>(acc + 3 * k + 1);  // {done, passes}
+    unsigned long long* acc = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * 3 * k);
+    float* far = (float*)ws_alloc(c, sizeof(float) * n);
+    float* half = (float*)ws_alloc(c, sizeof(float) * k);
+    KmState* state = (KmState*)ws_alloc(c, sizeof(KmState));
     check(cudaMemcpyAsync(dcen, cen.data(), sizeof(float2) * k, cudaMemcpyHostToDevice, st), "H2D centroids");
-    check(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * (3 * k + 2), st), "memset acc");
+    check(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * 3 * k, st), "memset acc");
+    check(cudaMemsetAsync(half, 0, sizeof(float) * k, st), "memset half");
+    check(cudaMemsetAsync(state, 0, sizeof(KmState), st), "memset state");
     k_km_init_labels<<<std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(lab, n, k);
     counted(c, cudaGetLastError(), "init labels");
-    const size_t smem = sizeof(float2) * k + sizeof(unsigned long long) * 3 * k;
-    check(cudaFuncSetAttribute(k_km_assign, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
-    const int blocks = std::max(1, std::min<int>((int)((n + 255) / 256), c->num_sms * 4));
-    // Lloyd passes in batches of kPassBatch with the stopping rule evaluated on
-    // the device (k_km_update): one host synchronisation per batch; passes
-    // after convergence return at once.
-    constexpr int kPassBatch = 8;
-    int hstate[2] = {0, 0};
-    for (int done_passes = 0; !hstate[0] && done_passes <= max_iter; done_passes += kPassBatch) {
-      for (int b = 0; b < kPassBatch; ++b) {
-        k_km_assign<<<blocks, 256, smem, st>>>(x, y, w, n, dcen, k, diam * 10.0f, std::ldexp(1.0, sp),
-                                               std::ldexp(1.0, sw), lab, acc, n_re, state);
-        counted(c, cudaGetLastError(), "k-means assign");
-        k_km_update<<<1, 256, 0, st>>>(acc, k, sp, sw, dcen, n_re, n, reassign_tol, max_iter, state);
-        counted(c, cudaGetLastError(), "k-means update");
+    const size_t smem = (sizeof(float2) + sizeof(unsigned long long) * 3 + sizeof(float)) * k;
+    check(cudaFuncSetAttribute(k_km_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+    const int blocks = (int)std::max<long long>(1, std::min<long long>((n + kKmTile - 1) / kKmTile, c->num_sms * 4));
+    // Lloyd passes in batches (8, 16, then 32) with the stopping rule evaluated
+    // on the device: one host synchronisation per batch; passes after
+    // convergence return at once.
+    KmState hstate{};
+    for (int batch = 8; !hstate.done; batch = std::min(32, batch * 2)) {
+      for (int b = 0; b < batch; ++b) {
+        k_km_pass<<<blocks, kKmThreads, smem, st>>>(x, y, w, n, dcen, k, diam * 10.0f, sp, sw, lab, far, half, acc,
+                                                    reassign_tol, max_iter, state);
+        counted(c, cudaGetLastError(), "k-means pass");
       }
-      check(cudaMemcpyAsync(hstate, state, sizeof(hstate), cudaMemcpyDeviceToHost, st), "D2H k-means state");
+      check(cudaMemcpyAsync(&hstate, state, sizeof(hstate), cudaMemcpyDeviceToHost, st), "D2H k-means state");
       check(cudaStreamSynchronize(st), "sync k-means");
     }
-    const int it = hstate[1];
+    const int it = hstate.passes;
     copy_out(c, labels_out, lab, sizeof(int) * n);
     if (centroids_out) copy_out(c, centroids_out, dcen, sizeof(float2) * k);
     check(cudaStreamSynchronize(st), "sync outputs");
@@ -685,7 +820,7 @@ tpcf_status tpcf_kmeans_equal(tpcf_ctx* c, const float* x, const float* y, const
       counted(c, cudaGetLastError(), "k-means sweep");
       k_km_sums<<<sblocks, 256, ssm, st>>>(x, y, w, lab, n, k, std::ldexp(1.0, sp), std::ldexp(1.0, sw), acc);
       counted(c, cudaGetLastError(), "k-means sums");
-      k_km_update<<<1, 256, 0, st>>>(acc, k, sp, sw, dcen, nullptr, n, 0.f, 0, nullptr);
+      k_km_update<<<1, 256, 0, st>>>(acc, k, sp, sw, dcen);
       counted(c, cudaGetLastError(), "k-means update");
       check(cudaMemcpyAsync(&hre, n_re, sizeof(hre), cudaMemcpyDeviceToHost, st), "D2H n_re");
       check(cudaMemcpyAsync(hw.data(), wfix, sizeof(long long) * k, cudaMemcpyDeviceToHost, st), "D2H weights");
