@@ -97,6 +97,11 @@ void begin_call(tpcf_ctx* c) {
   check(cudaSetDevice(c->device), "cudaSetDevice");
 }
 
+cudaStream_t aux_stream(tpcf_ctx* c) {
+  if (!c->aux_stream) check(cudaStreamCreateWithFlags(&c->aux_stream, cudaStreamNonBlocking), "second stream");
+  return c->aux_stream;
+}
+
 void vlog(tpcf_ctx* c, const char* fmt, ...) {
   if (!c->opts.verbose) return;
   va_list ap;
@@ -864,6 +869,7 @@ tpcf_status tpcf_destroy(tpcf_ctx* c) {
   cudaStreamSynchronize(c->stream);
   for (auto& s : c->slots)
     if (s.ptr) cudaFree(s.ptr);
+  if (c->aux_stream) cudaStreamDestroy(c->aux_stream);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
   return TPCF_OK;

@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -628,22 +629,55 @@ __global__ void k_unit_mult(unsigned long long seed, long long n_units, long lon
   }
 }
 
-// Field sums: out[(g * n_field + fi) * R + r] = sum over the field's blocks.
-// One warp per output: lane l adds blocks l, l + 32, ... of the field, then
-// the lanes are combined by a fixed shuffle tree (the same order every run).
-__global__ void k_marks_reduce(const double* __restrict__ partial, const MarksField* __restrict__ fields,
-                               int n_field, int n_blocks, int n_map_g, int R, double* __restrict__ out) {
-  const int t = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (t >= n_map_g * n_field * R) return;  // whole warps
-  const int r = t % R, fi = (t / R) % n_field, g = t / (R * n_field);
+// Field sums of several passes: pass p (of blockIdx.z), map or resample g of the
+// pass: out[((p MG + g) * n_field + fi) * R + r] = sum over the field's blocks.
+// A block covers 32 consecutive outputs of one field: warp v adds blocks v,
+// v + 16, ... (256-byte loads of a block's row), then the warps' sums are added in
+// warp order (the same order every run).  One warp per output, each lane on
+// another block's row, read 32 bytes for every 8 it used: 7.1 us a pass at 435
+// blocks x 976 outputs.
+constexpr int kMarksReduceWarps = 16;
+__global__ void __launch_bounds__(32 * kMarksReduceWarps) k_marks_reduce(const double* __restrict__ partial,
+                                                                        const MarksField* __restrict__ fields,
+                                                                        int n_field, int n_blocks, int n_map_g, int R,
+                                                                        double* __restrict__ out) {
+  __shared__ double part[kMarksReduceWarps][32];
+  const int lane = threadIdx.x & 31, v = threadIdx.x >> 5;
+  // n_map_g: maps of the last pass; the others hold kMapGroup
+  const int p = blockIdx.z, g_p = p + 1 < (int)gridDim.z ? kMapGroup : n_map_g;
+  const int fi = blockIdx.y, e = blockIdx.x * 32 + lane, ne = g_p * R;
+  partial += (size_t)p * n_blocks * kMapGroup * R;
+  out += (size_t)p * kMapGroup * n_field * R;
   const int c0 = fields[fi].chunk0;
   const int c1 = fi + 1 < n_field ? fields[fi + 1].chunk0 : n_blocks;
   double s = 0.0;
-  for (int c = c0 + lane; c < c1; c += 32) s += partial[((size_t)c * n_map_g + g) * R + r];
+  if (e < ne) {
+#pragma unroll 8
+    for (int c = c0 + v; c < c1; c += kMarksReduceWarps) s += partial[(size_t)c * ne + e];
+  }
+  part[v][lane] = s;
+  __syncthreads();
+  if (v == 0 && e < ne) {
+    double t = part[0][lane];
 #pragma unroll
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[t] = s;
+    for (int k = 1; k < kMarksReduceWarps; ++k) t += part[k][lane];
+    out[((size_t)(e / R) * n_field + fi) * R + e % R] = t;
+  }
+}
+// g: maps of the last of the n_pass passes.
+cudaError_t launch_marks_reduce(const double* part, const MarksField* df, int n_field, int nblk, int n_pass, int g,
+                                int R, double* out, cudaStream_t st) {
+  const int e = (n_pass > 1 ? kMapGroup : g) * R;
+  k_marks_reduce<<<dim3((e + 31) / 32, n_field, n_pass), 32 * kMarksReduceWarps, 0, st>>>(part, df, n_field, nblk, g, R,
+                                                                                         out);
+  return cudaGetLastError();
+}
+// Passes whose partial sums are kept (up to 64 MiB) before one reduction of all
+// of them: a reduction of one pass is all latency (6 us).  250 k lenses, 1000
+// resamples: 3.88 ms for the call with one pass kept, 3.26 ms with 18.
+int marks_passes_kept(int nblk, int R, int n_pass) {
+  const size_t one = sizeof(double) * (size_t)std::max(nblk, 1) * kMapGroup * R;
+  return (int)std::max<size_t>(1, std::min<size_t>((size_t)n_pass, ((size_t)64 << 20) / one));
 }
 
 // With timing enabled (tpcf_set_timing), CUDA events on the call's stream
@@ -672,6 +706,44 @@ struct PassTimer {
       ms += t;
     }
     c->last_pair_ms = ms;
+  }
+};
+
+// Order of the draws and the sums of a marks bootstrap.  With overlap the
+// draws run on the context's second stream: a buffer is drawn into once the
+// sums over its last contents are done, and summed once it is drawn.  Without,
+// everything is on the call's stream.  The destructor waits for the second
+// stream, so a call that fails midway leaves nothing running on the workspace.
+struct DrawStream {
+  tpcf_ctx* c;
+  cudaStream_t aux = nullptr;
+  std::unique_ptr<Event> drawn[2], free_[2];
+  bool busy[2] = {false, false};
+  DrawStream(tpcf_ctx* ctx, bool overlap) : c(ctx) {
+    if (!overlap) return;
+    for (int b = 0; b < 2; ++b) drawn[b].reset(new Event), free_[b].reset(new Event);
+    cudaStream_t a = aux_stream(c);
+    check(cudaEventRecord(free_[0]->e, c->stream), "event record");
+    check(cudaStreamWaitEvent(a, free_[0]->e, 0), "stream wait");  // after all earlier work of the call
+    aux = a;
+  }
+  ~DrawStream() {
+    if (aux) cudaStreamSynchronize(aux);
+  }
+  cudaStream_t begin(int b) {
+    if (!aux) return c->stream;
+    if (busy[b]) check(cudaStreamWaitEvent(aux, free_[b]->e, 0), "stream wait");
+    return aux;
+  }
+  void end(int b) {
+    if (!aux) return;
+    check(cudaEventRecord(drawn[b]->e, aux), "event record");
+    check(cudaStreamWaitEvent(c->stream, drawn[b]->e, 0), "stream wait");
+  }
+  void used(int b) {
+    if (!aux) return;
+    check(cudaEventRecord(free_[b]->e, c->stream), "event record");
+    busy[b] = true;
   }
 };
 
@@ -760,7 +832,9 @@ extern "C" tpcf_status tpcf_xi_from_marks(tpcf_ctx* c, int32_t n_field, const tp
     check(cudaMemcpyAsync(df, hf.data(), sizeof(MarksField) * n_field, cudaMemcpyHostToDevice, st), "H2D fields");
     const int R = 3 * nb + 1;
     std::vector<double> sums((size_t)n_map * n_field * R, 0.0);
-    double* part = (double*)ws_alloc(c, sizeof(double) * (size_t)std::max(nblk, 1) * kMapGroup * R);
+    const size_t part_pass = (size_t)std::max(nblk, 1) * kMapGroup * R;
+    const int n_keep = marks_passes_kept(nblk, R, (n_map + kMapGroup - 1) / kMapGroup);
+    double* part = (double*)ws_alloc(c, sizeof(double) * part_pass * n_keep);
     // the sums of every pass stay on the device until one copy after the
     // last pass, so the host queues all passes without waiting on any
     double* dout = (double*)ws_alloc(c, sizeof(double) * sums.size());
@@ -768,22 +842,24 @@ extern "C" tpcf_status tpcf_xi_from_marks(tpcf_ctx* c, int32_t n_field, const tp
     check(cudaMemsetAsync(derr, 0, sizeof(unsigned), st), "memset");
     const int MG = marks_group(nb);
     PassTimer timer(c);
+    int kept = 0;
     for (int m0 = 0; m0 < n_map; m0 += MG) {
       const int g = std::min(MG, n_map - m0);
-      if (nblk > 0) {
-        timer.mark(st);
-        counted(c, launch_marks_partials(df, n_field, nblk, chunk, MapFactors{m0}, g, nb, part, derr, c->skip_tile,
-                                      c->wait_limit, st),
-                "marks partials");
-        timer.mark(st);
-      }
-      const int tot = g * n_field * R;
       double* dpass = dout + (size_t)m0 * n_field * R;
-      if (nblk > 0) {
-        k_marks_reduce<<<(tot + 7) / 8, 256, 0, st>>>(part, df, n_field, nblk, g, R, dpass);
-        counted(c, cudaGetLastError(), "marks reduce");
-      } else {
-        check(cudaMemsetAsync(dpass, 0, sizeof(double) * tot, st), "memset");
+      if (nblk == 0) {
+        check(cudaMemsetAsync(dpass, 0, sizeof(double) * g * n_field * R, st), "memset");
+        continue;
+      }
+      timer.mark(st);
+      counted(c, launch_marks_partials(df, n_field, nblk, chunk, MapFactors{m0}, g, nb, part + part_pass * kept, derr,
+                                       c->skip_tile, c->wait_limit, st),
+              "marks partials");
+      timer.mark(st);
+      if (++kept == n_keep || m0 + g == n_map) {
+        counted(c, launch_marks_reduce(part, df, n_field, nblk, kept, g, R,
+                                       dpass - (size_t)(kept - 1) * MG * n_field * R, st),
+                "marks reduce");
+        kept = 0;
       }
     }
     check(cudaMemcpyAsync(sums.data(), dout, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, st), "D2H sums");
@@ -880,8 +956,21 @@ extern "C" tpcf_status tpcf_marks_bootstrap(tpcf_ctx* c, int32_t n_field, const 
     MarksField* df = (MarksField*)ws_alloc(c, sizeof(MarksField) * n_field);
     check(cudaMemcpyAsync(df, hf.data(), sizeof(MarksField) * n_field, cudaMemcpyHostToDevice, st), "H2D fields");
     const int R = 3 * nb + 1;
-    int* mbuf = multiplicity ? nullptr : (int*)ws_alloc(c, sizeof(int) * (size_t)kMapGroup * n_units);
-    double* part = (double*)ws_alloc(c, sizeof(double) * (size_t)std::max(nblk, 1) * kMapGroup * R);
+    // Multiplicities drawn here (16 M scattered atomic increments per pass of 16
+    // resamples of 1 M lenses, bound by L2 atomics) run on a second stream into
+    // one of two buffers while the other is summed (bound by FP64): 250 k
+    // lenses, 1000 resamples: the call takes 3.26 ms against 4.10 ms in line (fewer
+    // draw blocks, to leave the sums more room, are slower: 444: 3.67 ms).  One
+    // buffer, and no overlap, beyond 1 GiB.
+    const size_t mbytes = sizeof(int) * (size_t)kMapGroup * n_units;
+    const int n_buf = multiplicity ? 0 : mbytes <= ((size_t)1 << 30) ? 2 : 1;
+    int* mbuf[2] = {nullptr, nullptr};
+    for (int b = 0; b < n_buf; ++b) mbuf[b] = (int*)ws_alloc(c, mbytes);
+    DrawStream draws(c, n_buf == 2);
+    const size_t part_pass = (size_t)std::max(nblk, 1) * kMapGroup * R;
+    const int n_keep = marks_passes_kept(nblk, R, (n_boot + kMapGroup - 1) / kMapGroup);
+    int kept = 0;
+    double* part = (double*)ws_alloc(c, sizeof(double) * part_pass * n_keep);
     std::vector<double> sums((size_t)n_boot * n_field * R, 0.0);
     // the sums of every pass stay on the device until one copy after the
     // last pass, so the host queues all passes without waiting on any
@@ -897,24 +986,31 @@ extern "C" tpcf_status tpcf_marks_bootstrap(tpcf_ctx* c, int32_t n_field, const 
       if (multiplicity) {
         mult = dmult_all + (size_t)s0 * n_units;
       } else {
-        check(cudaMemsetAsync(mbuf, 0, sizeof(int) * (size_t)G * n_units, st), "memset mult");
+        const int b = n_buf == 2 ? (s0 / MG) & 1 : 0;
+        cudaStream_t ds = draws.begin(b);
+        check(cudaMemsetAsync(mbuf[b], 0, sizeof(int) * (size_t)G * n_units, ds), "memset mult");
         const long long work = (n_draw + 3) / 4 * G;
-        k_unit_mult<<<(unsigned)std::min<long long>((work + 255) / 256, 148 * 16), 256, 0, st>>>(seed, n_units, n_draw,
-                                                                                                 s0, G, mbuf);
+        k_unit_mult<<<(unsigned)std::min<long long>((work + 255) / 256, 148 * 16), 256, 0, ds>>>(seed, n_units, n_draw,
+                                                                                                 s0, G, mbuf[b]);
         counted(c, cudaGetLastError(), "bootstrap draws");
-        mult = mbuf;
+        draws.end(b);
+        mult = mbuf[b];
       }
       if (nblk > 0) {
         timer.mark(st);
         counted(c,
-                launch_marks_partials(df, n_field, nblk, chunk, MultFactors{mult, dunit, n_units}, G, nb, part, derr,
+                launch_marks_partials(df, n_field, nblk, chunk, MultFactors{mult, dunit, n_units}, G, nb,
+                                      part + part_pass * kept, derr,
                                       c->skip_tile, c->wait_limit, st),
                 "bootstrap partials");
         timer.mark(st);
-        const int tot = G * n_field * R;
-        k_marks_reduce<<<(tot + 7) / 8, 256, 0, st>>>(part, df, n_field, nblk, G, R,
-                                                       dout + (size_t)s0 * n_field * R);
-        counted(c, cudaGetLastError(), "bootstrap reduce");
+        if (!multiplicity) draws.used((n_buf == 2 ? (s0 / MG) & 1 : 0));
+        if (++kept == n_keep || s0 + G == n_boot) {
+          counted(c, launch_marks_reduce(part, df, n_field, nblk, kept, G, R,
+                                         dout + (size_t)(s0 - (kept - 1) * MG) * n_field * R, st),
+                  "bootstrap reduce");
+          kept = 0;
+        }
       }
     }
     check(cudaMemcpyAsync(sums.data(), dout, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, st), "D2H sums");

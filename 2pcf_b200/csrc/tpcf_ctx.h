@@ -43,6 +43,7 @@ struct tpcf_ctx {
   int num_sms = 0;
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
+  cudaStream_t aux_stream = nullptr;  // second stream of a call (aux_stream()), made on first use
   tpcf_opts opts{};
   std::string err;
   std::vector<tpcf::Slot> slots;
@@ -72,5 +73,16 @@ template <class T>
 const T* stage(tpcf_ctx* c, const T* p, int64_t n);
 void copy_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes);
 void begin_call(tpcf_ctx* c);
+cudaStream_t aux_stream(tpcf_ctx* c);
+
+// An event of one call (no timing); destroyed with the object, which CUDA
+// defers until the event has completed.
+struct Event {
+  cudaEvent_t e = nullptr;
+  Event() { check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event"); }
+  ~Event() { cudaEventDestroy(e); }
+  Event(const Event&) = delete;
+  Event& operator=(const Event&) = delete;
+};
 tpcf_status canonical_edges(const tpcf_bins* b, double* e, double* e2);
 }  // namespace tpcf
