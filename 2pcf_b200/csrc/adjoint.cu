@@ -505,24 +505,6 @@ __global__ void k_adj_lens_gather(const int* __restrict__ idx, int n_valid, cons
 }
 
 // Source Hilbert keys over the source box (source validity: finite, z >= 0).
-__global__ void k_adj_src_keys(const float* __restrict__ x, const float* __restrict__ y,
-                               const float* __restrict__ z, long long n, float4 box, unsigned long long* keys,
-                               int* idx) {
-  const float sxs = 65535.f / fmaxf(box.z - box.x, 1e-30f), sys = 65535.f / fmaxf(box.w - box.y, 1e-30f);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float xi = x[i], yi = y[i];
-    const bool v = isfinite(xi) && isfinite(yi) && !(z && z[i] < 0.f);
-    unsigned long long key = ~0ull;
-    if (v) {
-      const unsigned qx = (unsigned)clamp_floor((xi - box.x) * sxs, 0, 65535);
-      const unsigned qy = (unsigned)clamp_floor((yi - box.y) * sys, 0, 65535);
-      key = hilbert_index(qx, qy, 16);
-    }
-    keys[i] = key;
-    idx[i] = (int)i;
-  }
-}
-
 __global__ void k_adj_src_gather(const int* __restrict__ idx, int n_valid, const float* __restrict__ x,
                                  const float* __restrict__ y, const float* __restrict__ z,
                                  const float* __restrict__ e1, const float* __restrict__ e2,
@@ -733,23 +715,17 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
 
   // boxes and counts: lens catalogues (kind 1), then source catalogues (kind 0)
   const int ncat = nL + nS;
-  int* box_ord = (int*)ws_alloc(c, sizeof(int) * 8 * ncat);
-  unsigned long long* cnt = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * ncat);
-  int* pr = (int*)ws_alloc(c, sizeof(int) * 2 * ncat);
-  float* boxf = (float*)ws_alloc(c, sizeof(float) * 8 * ncat);
-  counted(c, launch_bbox_init(box_ord, cnt, pr, ncat, st), "bbox init");
+  Boxes BX;
+  BX.begin(c, ncat);
   for (int i = 0; i < nL; ++i)
     counted(c, launch_bbox(lens[i].x, lens[i].y, lens[i].z, lens[i].w, nullptr, nullptr, lens[i].n, 1,
-                           box_ord + 8 * i, cnt + i, pr + 2 * i, st), "bbox lens");
+                           BX.d_box + 8 * i, BX.d_cnt + i, BX.d_pr + 2 * i, st), "bbox lens");
   for (int i = 0; i < nS; ++i)
     counted(c, launch_bbox(srcs[i].x, srcs[i].y, srcs[i].z, nullptr, nullptr, nullptr, srcs[i].n, 0,
-                           box_ord + 8 * (nL + i), cnt + nL + i, pr + 2 * (nL + i), st), "bbox src");
-  counted(c, launch_bbox_finish(box_ord, boxf, 8 * ncat, st), "bbox finish");
-  std::vector<float> hb(8 * ncat);
-  std::vector<unsigned long long> hc(ncat);
-  check(cudaMemcpyAsync(hb.data(), boxf, sizeof(float) * 8 * ncat, cudaMemcpyDeviceToHost, st), "D2H box");
-  check(cudaMemcpyAsync(hc.data(), cnt, sizeof(unsigned long long) * ncat, cudaMemcpyDeviceToHost, st), "D2H count");
-  check(cudaStreamSynchronize(st), "sync box");
+                           BX.d_box + 8 * (nL + i), BX.d_cnt + nL + i, BX.d_pr + 2 * (nL + i), st), "bbox src");
+  BX.read(c);
+  const std::vector<float>& hb = BX.box;
+  const std::vector<unsigned long long>& hc = BX.cnt;
 
   // outputs, zero for sources with no pair
   std::vector<float*> o_e1(nS), o_e2(nS), o_w(nS), o_m(nS);
@@ -798,7 +774,7 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
       int* i1 = (int*)ws_alloc(c, sizeof(int) * l.n);
       int cell_bits = 1;
       while (cell_bits < 32 && (1ull << cell_bits) <= (unsigned long long)ncells) ++cell_bits;
-      const int mb = std::min(16, (32 - cell_bits) & ~1);
+      const int mb = cell_hilbert_bits(l.n, ncells, cell_bits);
       k_adj_lens_keys<<<(unsigned)std::min<long long>((l.n + 255) / 256, 4096), 256, 0, st>>>(
           l.x, l.y, l.z, l.w, l.n, x0, y0, g.inv_cell, ncx, ncy, mb, k0, i0);
       counted(c, cudaGetLastError(), "lens keys");
@@ -832,17 +808,17 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     gbox[i] = (float4*)ws_alloc(c, sizeof(float4) * std::max(ngroups[i], 1));
     if (ns == 0) continue;
     const float* b = &hb[8 * (nL + i)];
-    unsigned long long* k0 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * s.n);
-    unsigned long long* k1 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * s.n);
+    unsigned* k0 = (unsigned*)ws_alloc(c, sizeof(unsigned) * s.n);
+    unsigned* k1 = (unsigned*)ws_alloc(c, sizeof(unsigned) * s.n);
     int* i0 = (int*)ws_alloc(c, sizeof(int) * s.n);
     int* i1 = (int*)ws_alloc(c, sizeof(int) * s.n);
-    k_adj_src_keys<<<(unsigned)std::min<long long>((s.n + 255) / 256, 4096), 256, 0, st>>>(
-        s.x, s.y, s.z, s.n, make_float4(b[0], b[1], b[2], b[3]), k0, i0);
-    counted(c, cudaGetLastError(), "source keys");
+    const int half = std::min(15, lens_key_bits(s.n, 1).half);  // one patch: 32-bit keys
+    counted(c, launch_lens_keys(s.x, s.y, s.z, nullptr, nullptr, s.n, make_float4(b[0], b[1], b[2], b[3]), half, 1, k0,
+                                i0, st), "source keys");
     size_t tb = 0;
-    check(sort_pairs_u64(nullptr, tb, k0, k1, i0, i1, (int)s.n, st), "sort size");
+    check(sort_pairs_u32(nullptr, tb, k0, k1, i0, i1, (int)s.n, 2 * half + 1, st), "sort size");
     void* tmp = ws_alloc(c, tb);
-    check(sort_pairs_u64(tmp, tb, k0, k1, i0, i1, (int)s.n, st), "sort sources");
+    check(sort_pairs_u32(tmp, tb, k0, k1, i0, i1, (int)s.n, 2 * half + 1, st), "sort sources");
     k_adj_src_gather<<<(ns + 255) / 256, 256, 0, st>>>(i1, ns, s.x, s.y, s.z, s.e1, s.e2, s.w, s.m, s0[i], s1[i],
                                                          perm[i]);
     counted(c, cudaGetLastError(), "source gather");
@@ -860,7 +836,8 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
   // tasks, their D sums and the work items (task, source group)
   std::vector<AdjTask> at(nT);
   std::vector<double*> dsum(nT, nullptr);
-  std::vector<int2> items;
+  std::vector<int2> ranges;  // {task, first item}
+  int n_items = 0;
   std::vector<TaskDesc> tdesc(nT);
   for (int t = 0; t < nT; ++t) {
     const int li = tasks[t].lens, si = tasks[t].src;
@@ -873,10 +850,11 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     // item cost: the source groups play the lens-group role, the lens grid the source grid
     tdesc[t].lens_cat = si; tdesc[t].src_cat = li; tdesc[t].item_base = 0; tdesc[t].lens_acc_off = -1;
     tdesc[t].margin = margin; tdesc[t].split = 1;
-    if (hc[li] > 0)
-      for (int g = 0; g < ngroups[si]; ++g) items.push_back(make_int2(t, g));
+    if (hc[li] > 0 && ngroups[si] > 0) {
+      ranges.push_back(make_int2(t, n_items));
+      n_items += ngroups[si];
+    }
   }
-  const int n_items = (int)items.size();
   if (n_items > 0) {
     std::vector<LensDesc> gdesc(nS);
     for (int i = 0; i < nS; ++i) {
@@ -891,21 +869,10 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     check(cudaMemcpyAsync(d_td, tdesc.data(), sizeof(TaskDesc) * nT, cudaMemcpyHostToDevice, st), "H2D");
     check(cudaMemcpyAsync(d_gd, gdesc.data(), sizeof(LensDesc) * nS, cudaMemcpyHostToDevice, st), "H2D");
     check(cudaMemcpyAsync(d_lg, lgrid.data(), sizeof(GridDesc) * nL, cudaMemcpyHostToDevice, st), "H2D");
-    int2* items0 = (int2*)ws_alloc(c, sizeof(int2) * n_items);
-    int2* d_items = (int2*)ws_alloc(c, sizeof(int2) * n_items);
-    check(cudaMemcpyAsync(items0, items.data(), sizeof(int2) * n_items, cudaMemcpyHostToDevice, st), "H2D items");
-    // costliest items first (in cost bands, space order inside a band): cost =
-    // lenses in the rows of each source group
-    unsigned long long* ck0 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n_items);
-    unsigned long long* ck1 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n_items);
-    int* o0 = (int*)ws_alloc(c, sizeof(int) * n_items);
-    int* o1 = (int*)ws_alloc(c, sizeof(int) * n_items);
-    counted(c, launch_item_cost(items0, n_items, d_td, d_gd, d_lg, R, ck0, o0, st), "item cost");
-    size_t tb = 0;
-    check(sort_pairs_u64_desc(nullptr, tb, ck0, ck1, o0, o1, n_items, st), "sort size");
-    void* tmp = ws_alloc(c, tb);
-    check(sort_pairs_u64_desc(tmp, tb, ck0, ck1, o0, o1, n_items, st), "sort items");
-    counted(c, launch_permute_items(items0, o1, n_items, 0, 1, d_items, st), "permute items");
+    // costliest items first (in cost bands): cost = lenses in the rows of each
+    // source group
+    int n_run = 0;
+    int2* d_items = order_items(c, ranges, n_items, d_td, d_gd, d_lg, R, false, 0, 1, &n_run);
     double* de2 = (double*)ws_alloc(c, sizeof(double) * (nb + 1));
     float* de2f = (float*)ws_alloc(c, sizeof(float) * (nb + 1));
     float4* dcoef = (float4*)ws_alloc(c, sizeof(float4) * coef.size());

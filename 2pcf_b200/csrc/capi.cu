@@ -91,6 +91,86 @@ void copy_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes) {
   check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, c->stream), "output copy");
 }
 
+void put_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes) {
+  if (!dst || bytes == 0) return;
+  if (is_device_ptr(dst))
+    check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream), "output copy");
+  else
+    std::memcpy(dst, src, bytes);
+}
+
+void Boxes::begin(tpcf_ctx* c, int n) {
+  ncat = n;
+  d_cnt = (unsigned long long*)ws_alloc(c, (sizeof(unsigned long long) + 10 * sizeof(int)) * n);
+  d_box = reinterpret_cast<int*>(d_cnt + n);
+  d_pr = d_box + 8 * n;
+  counted(c, launch_bbox_init(d_box, d_cnt, d_pr, n, c->stream), "bbox init");
+}
+void Boxes::read(tpcf_ctx* c) {
+  std::vector<unsigned char> h((sizeof(unsigned long long) + 10 * sizeof(int)) * ncat);
+  check(cudaMemcpyAsync(h.data(), d_cnt, h.size(), cudaMemcpyDeviceToHost, c->stream), "D2H boxes");
+  check(cudaStreamSynchronize(c->stream), "sync boxes");
+  cnt.resize(ncat);
+  std::memcpy(cnt.data(), h.data(), sizeof(unsigned long long) * ncat);
+  const unsigned char* b = h.data() + sizeof(unsigned long long) * ncat;
+  box.resize(8 * ncat);
+  for (int i = 0; i < 8 * ncat; ++i) {  // undo the order-preserving integer form
+    int o;
+    std::memcpy(&o, b + sizeof(int) * i, sizeof(int));
+    o = o >= 0 ? o : o ^ 0x7fffffff;
+    std::memcpy(&box[i], &o, sizeof(int));
+  }
+  pr.resize(2 * ncat);
+  std::memcpy(pr.data(), b + sizeof(int) * 8 * ncat, sizeof(int) * 2 * ncat);
+}
+
+LensKeyBits lens_key_bits(int64_t n, int n_patch) {
+  LensKeyBits k{};
+  int pb = 1;
+  while (((int64_t)n_patch >> pb) > 0) ++pb;
+  k.half = 2;
+  while (k.half < 16 && ((int64_t)1 << (2 * k.half)) < 16 * n) ++k.half;
+  k.wide = 2 * k.half + pb > 32;
+  k.total = 2 * k.half + pb;
+  return k;
+}
+int cell_hilbert_bits(int64_t n, unsigned ncells, int cell_bits) {
+  int half = 1;
+  while (half < 8 && ((int64_t)1 << (2 * half)) * ncells < 16 * n) ++half;
+  return std::min(2 * half, (32 - cell_bits) & ~1);
+}
+
+int2* order_items(tpcf_ctx* c, const std::vector<int2>& ranges, int n, const TaskDesc* tasks, const LensDesc* lenses,
+                  const GridDesc* grids, float R, bool sph, int shard_index, int shard_count, int* n_run) {
+  cudaStream_t st = c->stream;
+  *n_run = shard_count > 1 ? (n - shard_index + shard_count - 1) / shard_count : n;
+  if (n == 0) return nullptr;
+  int2* dr = (int2*)ws_alloc(c, sizeof(int2) * ranges.size());
+  check(cudaMemcpyAsync(dr, ranges.data(), sizeof(int2) * ranges.size(), cudaMemcpyHostToDevice, st), "H2D ranges");
+  int2* items = (int2*)ws_alloc(c, sizeof(int2) * n);
+  int2* out = (int2*)ws_alloc(c, sizeof(int2) * n);
+  unsigned* band = (unsigned*)ws_alloc(c, sizeof(unsigned) * n);
+  if (sph)
+    counted(c, launch_item_cost_sph(dr, (int)ranges.size(), n, tasks, lenses, grids, R, items, band, st), "item cost");
+  else
+    counted(c, launch_item_cost(dr, (int)ranges.size(), n, tasks, lenses, grids, R, items, band, st), "item cost");
+  if (shard_count <= 1 && n <= item_order_max()) {
+    counted(c, launch_item_order(items, band, n, out, st), "item order");
+    return out;
+  }
+  unsigned* band1 = (unsigned*)ws_alloc(c, sizeof(unsigned) * n);
+  int* o0 = (int*)ws_alloc(c, sizeof(int) * n);
+  int* o1 = (int*)ws_alloc(c, sizeof(int) * n);
+  counted(c, launch_iota32(o0, n, st), "item index");
+  size_t tb = 0;
+  check(sort_bands_desc(nullptr, tb, band, band1, o0, o1, n, st), "sort size");
+  void* tmp = ws_alloc(c, tb);
+  check(sort_bands_desc(tmp, tb, band, band1, o0, o1, n, st), "sort items");
+  counted(c, launch_permute_items(items, o1, n, shard_count > 1 ? shard_index : 0, std::max(1, shard_count), out, st),
+          "permute items");
+  return out;
+}
+
 void begin_call(tpcf_ctx* c) {
   c->next_slot = 0;
   c->h2d_bytes = 0;
@@ -193,8 +273,7 @@ struct LensGroups {
   int n_groups = 0;
   int* group_start = nullptr;
   float4* group_box = nullptr;
-  std::vector<int> patch_groups;  // [n_patch_eff + 1], host
-  int* d_patch_groups = nullptr;
+  int* d_patch_groups = nullptr;  // [n_patch_eff + 1]
 };
 struct LensBuilt {
   int n_valid = 0;
@@ -322,25 +401,18 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
 
   // ---- bounding boxes, z ranges, max |m|, counts, patch ranges (one sync)
   const int ncat = nL + nS;
-  int* box_ord = (int*)ws_alloc(c, sizeof(int) * 8 * ncat);
-  unsigned long long* cnt = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * ncat);
-  int* pr = (int*)ws_alloc(c, sizeof(int) * 2 * ncat);
-  float* boxf = (float*)ws_alloc(c, sizeof(float) * 8 * ncat);
-  counted(c, launch_bbox_init(box_ord, cnt, pr, ncat, st), "bbox init");
+  Boxes BX;
+  BX.begin(c, ncat);
   for (int i = 0; i < nL; ++i)
     counted(c, launch_bbox(lens[i].x, lens[i].y, lens[i].z, lens[i].w, lens[i].patch, nullptr, lens[i].n, 1,
-                           box_ord + 8 * i, cnt + i, pr + 2 * i, st), "bbox lens");
+                           BX.d_box + 8 * i, BX.d_cnt + i, BX.d_pr + 2 * i, st), "bbox lens");
   for (int i = 0; i < nS; ++i)
     counted(c, launch_bbox(srcs[i].x, srcs[i].y, srcs[i].z, nullptr, nullptr, srcs[i].m, srcs[i].n, 0,
-                           box_ord + 8 * (nL + i), cnt + nL + i, pr + 2 * (nL + i), st), "bbox src");
-  counted(c, launch_bbox_finish(box_ord, boxf, 8 * ncat, st), "bbox finish");
-  std::vector<float> hbox(8 * ncat);
-  std::vector<unsigned long long> hcnt(ncat);
-  std::vector<int> hpr(2 * ncat);
-  check(cudaMemcpyAsync(hbox.data(), boxf, sizeof(float) * 8 * ncat, cudaMemcpyDeviceToHost, st), "D2H box");
-  check(cudaMemcpyAsync(hcnt.data(), cnt, sizeof(unsigned long long) * ncat, cudaMemcpyDeviceToHost, st), "D2H count");
-  check(cudaMemcpyAsync(hpr.data(), pr, sizeof(int) * 2 * ncat, cudaMemcpyDeviceToHost, st), "D2H prange");
-  check(cudaStreamSynchronize(st), "sync bbox");
+                           BX.d_box + 8 * (nL + i), BX.d_cnt + nL + i, BX.d_pr + 2 * (nL + i), st), "bbox src");
+  BX.read(c);
+  const std::vector<float>& hbox = BX.box;
+  const std::vector<unsigned long long>& hcnt = BX.cnt;
+  const std::vector<int>& hpr = BX.pr;
   for (int i = 0; i < nL; ++i)
     if (lens[i].patch && hcnt[i] > 0 && (hpr[2 * i] < 0 || hpr[2 * i + 1] >= n_patch))
       throw Failure(TPCF_ERR_INVALID_ARG, "patch label outside [0, n_patch)");
@@ -419,7 +491,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
       int* i1 = (int*)ws_alloc(c, sizeof(int) * s.n);
       int cell_bits = 1;
       while (cell_bits < 32 && (1ull << cell_bits) <= (unsigned long long)ncells) ++cell_bits;
-      const int mb = std::min(16, (32 - cell_bits) & ~1);  // within-cell Hilbert bits
+      const int mb = cell_hilbert_bits(s.n, ncells, cell_bits);
       counted(c, launch_src_keys(s.x, s.y, s.z, s.n, x0, y0, g.inv_cell, ncx, ncy, mb, k0, i0, st), "src keys");
       const int end_bit = cell_bits + mb;
       size_t tb = 0;
@@ -475,20 +547,31 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     LB.perm = (int*)ws_alloc(c, sizeof(int) * std::max(LB.n_valid, 1));
     std::vector<int> off(n_patch_eff + 1, 0);
     if (l.n > 0 && LB.n_valid > 0) {
-      unsigned long long* k0 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * l.n);
-      unsigned long long* k1 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * l.n);
       int* i0 = (int*)ws_alloc(c, sizeof(int) * l.n);
       int* i1 = (int*)ws_alloc(c, sizeof(int) * l.n);
-      float4 box = make_float4(b[0], b[1], b[2], b[3]);
-      counted(c, launch_lens_keys(l.x, l.y, l.z, l.w, l.patch, l.n, box, k0, i0, st), "lens keys");
-      size_t tb = 0;
-      check(sort_pairs_u64(nullptr, tb, k0, k1, i0, i1, (int)l.n, st), "sort size");
-      void* tmp = ws_alloc(c, tb);
-      check(sort_pairs_u64(tmp, tb, k0, k1, i0, i1, (int)l.n, st), "sort lenses");
+      const float4 box = make_float4(b[0], b[1], b[2], b[3]);
+      const LensKeyBits kb = lens_key_bits(l.n, n_patch_eff);
+      int* doff = l.patch ? (int*)ws_alloc(c, sizeof(int) * (n_patch_eff + 1)) : nullptr;
+      auto sort = [&](auto* k0, auto* k1, auto sorter) {
+        counted(c, launch_lens_keys(l.x, l.y, l.z, l.w, l.patch, l.n, box, kb.half, n_patch_eff, k0, i0, st),
+                "lens keys");
+        size_t tb = 0;
+        check(sorter(nullptr, tb, k0, k1, i0, i1, (int)l.n, kb.total, st), "sort size");
+        void* tmp = ws_alloc(c, tb);
+        check(sorter(tmp, tb, k0, k1, i0, i1, (int)l.n, kb.total, st), "sort lenses");
+        if (doff) counted(c, launch_patch_offsets(k1, LB.n_valid, n_patch_eff, 2 * kb.half, doff, st), "patch offsets");
+      };
+      if (kb.wide) {
+        auto* k0 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * l.n);
+        auto* k1 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * l.n);
+        sort(k0, k1, sort_pairs_u64);
+      } else {
+        auto* k0 = (unsigned*)ws_alloc(c, sizeof(unsigned) * l.n);
+        auto* k1 = (unsigned*)ws_alloc(c, sizeof(unsigned) * l.n);
+        sort(k0, k1, sort_pairs_u32);
+      }
       counted(c, launch_lens_gather(i1, LB.n_valid, l.x, l.y, l.z, l.val, l.w, LB.rec, LB.zs, LB.perm, st), "lens gather");
       if (l.patch) {
-        int* doff = (int*)ws_alloc(c, sizeof(int) * (n_patch_eff + 1));
-        counted(c, launch_patch_offsets(k1, LB.n_valid, n_patch_eff, doff, st), "patch offsets");
         check(cudaMemcpyAsync(off.data(), doff, sizeof(int) * (n_patch_eff + 1), cudaMemcpyDeviceToHost, st), "D2H off");
         check(cudaStreamSynchronize(st), "sync offsets");
       } else {
@@ -504,24 +587,31 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
       bool used = false;
       for (int t = 0; t < nT; ++t) used = used || (tl[t] == i && src_series[ts[t]] == k);
       LensGroups& LG = LB.by[k];
-      LG.patch_groups.assign(n_patch_eff + 1, 0);
       if (!used) continue;
-      std::vector<int> gstart;
-      for (int p = 0; p < n_patch_eff; ++p) {
-        LG.patch_groups[p] = (int)gstart.size();
-        for (int s0 = off[p]; s0 < off[p + 1]; s0 += lens_group[k]) gstart.push_back(s0);
+      if (n_patch_eff == 1) {
+        LG.n_groups = (LB.n_valid + lens_group[k] - 1) / lens_group[k];
+        LG.group_start = (int*)ws_alloc(c, sizeof(int) * (LG.n_groups + 1));
+        LG.d_patch_groups = (int*)ws_alloc(c, sizeof(int) * 2);
+        counted(c, launch_uniform_groups(LG.n_groups, LB.n_valid, lens_group[k], LG.group_start, LG.d_patch_groups, st),
+                "groups");
+      } else {
+        std::vector<int> gstart, pg(n_patch_eff + 1);
+        for (int p = 0; p < n_patch_eff; ++p) {
+          pg[p] = (int)gstart.size();
+          for (int s0 = off[p]; s0 < off[p + 1]; s0 += lens_group[k]) gstart.push_back(s0);
+        }
+        pg[n_patch_eff] = (int)gstart.size();
+        LG.n_groups = (int)gstart.size();
+        gstart.push_back(LB.n_valid);
+        LG.group_start = (int*)ws_alloc(c, sizeof(int) * gstart.size());
+        check(cudaMemcpyAsync(LG.group_start, gstart.data(), sizeof(int) * gstart.size(), cudaMemcpyHostToDevice, st), "H2D groups");
+        LG.d_patch_groups = (int*)ws_alloc(c, sizeof(int) * (n_patch_eff + 1));
+        check(cudaMemcpyAsync(LG.d_patch_groups, pg.data(), sizeof(int) * (n_patch_eff + 1), cudaMemcpyHostToDevice, st),
+              "H2D patch groups");
+        check(cudaStreamSynchronize(st), "sync groups");  // host vectors above must outlive the async copies
       }
-      LG.patch_groups[n_patch_eff] = (int)gstart.size();
-      LG.n_groups = (int)gstart.size();
-      gstart.push_back(LB.n_valid);
-      LG.group_start = (int*)ws_alloc(c, sizeof(int) * gstart.size());
-      check(cudaMemcpyAsync(LG.group_start, gstart.data(), sizeof(int) * gstart.size(), cudaMemcpyHostToDevice, st), "H2D groups");
-      LG.d_patch_groups = (int*)ws_alloc(c, sizeof(int) * (n_patch_eff + 1));
-      check(cudaMemcpyAsync(LG.d_patch_groups, LG.patch_groups.data(), sizeof(int) * (n_patch_eff + 1),
-                            cudaMemcpyHostToDevice, st), "H2D patch groups");
       LG.group_box = (float4*)ws_alloc(c, sizeof(float4) * std::max(LG.n_groups, 1));
       counted(c, launch_group_box(LB.rec, LG.group_start, LG.n_groups, LG.group_box, st), "group box");
-      check(cudaStreamSynchronize(st), "sync groups");  // host vectors above must outlive the async copies
       LensDesc& d = ldesc[k * nL + i];
       d.rec = LB.rec; d.z = LB.zs; d.group_start = LG.group_start; d.group_box = LG.group_box;
       d.n_valid = LB.n_valid; d.n_groups = LG.n_groups;
@@ -533,8 +623,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   Phase ph_items("tpcf: work items");
   std::vector<TaskDesc>& tdesc = B.tdesc;
   tdesc.assign(nT, TaskDesc{});
-  std::vector<int2> items[2];
-  int n_items = 0;
+  std::vector<int2> ranges[2];  // {task, first item among its kind}
+  int n_kind[2] = {0, 0}, n_items = 0;
   B.kind.assign(nT, 0);
   B.want_lens.assign(nT, 0);
   long long lens_acc_elems = 0;
@@ -549,7 +639,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     // few lens groups: several items per group keep the SMs' warps busy (a
     // property of the task alone, so its sums do not depend on the batch)
     d.split = !sph && !any_lens && ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
-    for (int i = 0; i < ng * d.split; ++i) items[kind].push_back(make_int2(t, i));
+    if (ng > 0) ranges[kind].push_back(make_int2(t, n_kind[kind]));
+    n_kind[kind] += ng * d.split;
     n_items += ng * d.split;
     B.want_lens[t] = wants_lens(outs[t]) ? 1 : 0;
     d.lens_acc_off = -1;
@@ -558,48 +649,35 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
       lens_acc_elems += (long long)kQ * nb * std::max(lb[tl[t]].n_valid, 1);
     }
   }
-  TaskDesc* d_tasks = (TaskDesc*)ws_alloc(c, sizeof(TaskDesc) * std::max(nT, 1));
-  LensDesc* d_lens = (LensDesc*)ws_alloc(c, sizeof(LensDesc) * 2 * std::max(nL, 1));
-  GridDesc* d_grids = (GridDesc*)ws_alloc(c, sizeof(GridDesc) * std::max(nS, 1));
-  check(cudaMemcpyAsync(d_tasks, tdesc.data(), sizeof(TaskDesc) * nT, cudaMemcpyHostToDevice, st), "H2D tasks");
-  check(cudaMemcpyAsync(d_lens, ldesc.data(), sizeof(LensDesc) * 2 * nL, cudaMemcpyHostToDevice, st), "H2D lens desc");
-  check(cudaMemcpyAsync(d_grids, grids.data(), sizeof(GridDesc) * nS, cudaMemcpyHostToDevice, st), "H2D grid desc");
+  // descriptors and edges: one copy
+  std::vector<float> e2f(nb + 1);
+  for (int i = 0; i <= nb; ++i) e2f[i] = (float)e2[i];
+  const size_t o_tasks = 0, o_lens = o_tasks + sizeof(TaskDesc) * nT, o_grid = o_lens + sizeof(LensDesc) * 2 * nL,
+               o_e2 = o_grid + sizeof(GridDesc) * nS, o_e2f = o_e2 + sizeof(double) * (nb + 1),
+               n_blob = o_e2f + sizeof(float) * (nb + 1);
+  static_assert(sizeof(TaskDesc) % 8 == 0 && sizeof(LensDesc) % 8 == 0 && sizeof(GridDesc) % 8 == 0, "aligned parts");
+  std::vector<unsigned char> blob(n_blob);
+  std::memcpy(blob.data() + o_tasks, tdesc.data(), sizeof(TaskDesc) * nT);
+  std::memcpy(blob.data() + o_lens, ldesc.data(), sizeof(LensDesc) * 2 * nL);
+  std::memcpy(blob.data() + o_grid, grids.data(), sizeof(GridDesc) * nS);
+  std::memcpy(blob.data() + o_e2, e2.data(), sizeof(double) * (nb + 1));
+  std::memcpy(blob.data() + o_e2f, e2f.data(), sizeof(float) * (nb + 1));
+  unsigned char* d_blob = (unsigned char*)ws_alloc(c, n_blob);
+  check(cudaMemcpyAsync(d_blob, blob.data(), n_blob, cudaMemcpyHostToDevice, st), "H2D descriptors");
+  TaskDesc* d_tasks = (TaskDesc*)(d_blob + o_tasks);
+  LensDesc* d_lens = (LensDesc*)(d_blob + o_lens);
+  GridDesc* d_grids = (GridDesc*)(d_blob + o_grid);
+  double* d_e2 = (double*)(d_blob + o_e2);
+  float* d_e2f = (float*)(d_blob + o_e2f);
   double* item_sums = (double*)ws_alloc(c, sizeof(double) * kQ * nb * std::max(n_items, 1));
   double* lens_acc = lens_acc_elems ? (double*)ws_alloc(c, sizeof(double) * lens_acc_elems) : nullptr;
   int* head = (int*)ws_alloc(c, sizeof(int) * 4);
   unsigned* err = (unsigned*)(head + 1);
-  double* d_e2 = (double*)ws_alloc(c, sizeof(double) * (nb + 1));
-  float* d_e2f = (float*)ws_alloc(c, sizeof(float) * (nb + 1));
-  std::vector<float> e2f(nb + 1);
-  for (int i = 0; i <= nb; ++i) e2f[i] = (float)e2[i];
-  check(cudaMemcpyAsync(d_e2, e2.data(), sizeof(double) * (nb + 1), cudaMemcpyHostToDevice, st), "H2D edges");
-  check(cudaMemcpyAsync(d_e2f, e2f.data(), sizeof(float) * (nb + 1), cudaMemcpyHostToDevice, st), "H2D edges f");
-
   int2* d_items[2] = {nullptr, nullptr};
   int n_run[2] = {0, 0};
-  for (int k = 0; k < 2; ++k) {
-    const int n = (int)items[k].size();
-    if (n == 0) continue;
-    d_items[k] = (int2*)ws_alloc(c, sizeof(int2) * n);
-    int2* d_items0 = (int2*)ws_alloc(c, sizeof(int2) * n);
-    check(cudaMemcpyAsync(d_items0, items[k].data(), sizeof(int2) * n, cudaMemcpyHostToDevice, st), "H2D items");
-    unsigned long long* ck0 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n);
-    unsigned long long* ck1 = (unsigned long long*)ws_alloc(c, sizeof(unsigned long long) * n);
-    int* o0 = (int*)ws_alloc(c, sizeof(int) * n);
-    int* o1 = (int*)ws_alloc(c, sizeof(int) * n);
-    if (sph)
-      counted(c, launch_item_cost_sph(d_items0, n, d_tasks, d_lens, d_grids, R, ck0, o0, st), "item cost");
-    else
-      counted(c, launch_item_cost(d_items0, n, d_tasks, d_lens, d_grids, R, ck0, o0, st), "item cost");
-    size_t tb = 0;
-    check(sort_pairs_u64_desc(nullptr, tb, ck0, ck1, o0, o1, n, st), "sort size");
-    void* tmp = ws_alloc(c, tb);
-    check(sort_pairs_u64_desc(tmp, tb, ck0, ck1, o0, o1, n, st), "sort items");
-    const int sc = c->opts.shard_count > 1 ? c->opts.shard_count : 1;
-    const int si = sc > 1 ? c->opts.shard_index : 0;
-    counted(c, launch_permute_items(d_items0, o1, n, si, sc, d_items[k], st), "permute items");
-    n_run[k] = sc > 1 ? (n - si + sc - 1) / sc : n;
-  }
+  for (int k = 0; k < 2; ++k)
+    d_items[k] = order_items(c, ranges[k], n_kind[k], d_tasks, d_lens, d_grids, R, sph, c->opts.shard_index,
+                             c->opts.shard_count, &n_run[k]);
   PairParams P{};
   P.tasks = d_tasks; P.lenses = d_lens; P.grids = d_grids;
   P.nb = nb; P.item_sums = item_sums; P.lens_acc = lens_acc; P.err = err;
@@ -648,7 +726,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   B.lens_acc = lens_acc;
   B.lens_acc_elems = lens_acc_elems;
   B.dpatch.assign(nT, nullptr);
-  for (int t = 0; t < nT; ++t) B.dpatch[t] = (double*)ws_alloc(c, sizeof(double) * kQ * nb * n_patch_eff);
+  double* dpatch = (double*)ws_alloc(c, sizeof(double) * kQ * nb * n_patch_eff * nT);
+  for (int t = 0; t < nT; ++t) B.dpatch[t] = dpatch + (size_t)t * kQ * nb * n_patch_eff;
 }
 
 // The pair kernel and the per-patch reductions of a prepared batch: device
@@ -701,12 +780,12 @@ void batch_finish(tpcf_ctx* c, Batch& B, const tpcf_bins* bins, tpcf_result* out
   Phase ph_reduce("tpcf: outputs");
   cudaStream_t st = c->stream;
   const int nb = B.nb, nT = B.nT, n_patch_eff = B.n_patch_eff, n_patch = B.n_patch;
-  std::vector<std::vector<double>> hpatch(nT);
+  const size_t per_task = (size_t)kQ * nb * n_patch_eff;
+  std::vector<double> hpatch(per_task * nT);
+  check(cudaMemcpyAsync(hpatch.data(), B.dpatch[0], sizeof(double) * per_task * nT, cudaMemcpyDeviceToHost, st),
+        "D2H patch");
   for (int t = 0; t < nT; ++t) {
     const LensBuilt& LB = B.lb[B.tl[t]];
-    hpatch[t].resize((size_t)kQ * nb * n_patch_eff);
-    check(cudaMemcpyAsync(hpatch[t].data(), B.dpatch[t], sizeof(double) * kQ * nb * n_patch_eff,
-                          cudaMemcpyDeviceToHost, st), "D2H patch");
     if (B.want_lens[t]) {
       const tpcf_result& o = outs[t];
       const int64_t nA = B.lens_n[B.tl[t]];
@@ -762,7 +841,7 @@ void batch_finish(tpcf_ctx* c, Batch& B, const tpcf_bins* bins, tpcf_result* out
     tpcf_result& o = outs[t];
     std::vector<double> tot((size_t)kQ * nb, 0.0);
     for (int p = 0; p < n_patch_eff; ++p)
-      for (int q = 0; q < kQ * nb; ++q) tot[q] += hpatch[t][(size_t)p * kQ * nb + q];
+      for (int q = 0; q < kQ * nb; ++q) tot[q] += hpatch[per_task * t + (size_t)p * kQ * nb + q];
     std::vector<double> sdw(nb), sgt(nb), sgx(nb), sw(nb), sK(nb);
     std::vector<int64_t> np(nb);
     std::vector<float> mt(nb), gt(nb), gx(nb), ww(nb);
@@ -775,26 +854,26 @@ void batch_finish(tpcf_ctx* c, Batch& B, const tpcf_bins* bins, tpcf_result* out
       gx[b] = sK[b] > 0 ? (float)(sgx[b] / sK[b]) : 0.f;
       ww[b] = (float)sw[b];
     }
-    copy_out(c, o.sum_dw, sdw.data(), sizeof(double) * nb);
-    copy_out(c, o.sum_gt, sgt.data(), sizeof(double) * nb);
-    copy_out(c, o.sum_gx, sgx.data(), sizeof(double) * nb);
-    copy_out(c, o.sum_w, sw.data(), sizeof(double) * nb);
-    copy_out(c, o.sum_K, sK.data(), sizeof(double) * nb);
-    copy_out(c, o.n_pairs, np.data(), sizeof(int64_t) * nb);
-    copy_out(c, o.theta, centers.data(), sizeof(float) * nb);
+    put_out(c, o.sum_dw, sdw.data(), sizeof(double) * nb);
+    put_out(c, o.sum_gt, sgt.data(), sizeof(double) * nb);
+    put_out(c, o.sum_gx, sgx.data(), sizeof(double) * nb);
+    put_out(c, o.sum_w, sw.data(), sizeof(double) * nb);
+    put_out(c, o.sum_K, sK.data(), sizeof(double) * nb);
+    put_out(c, o.n_pairs, np.data(), sizeof(int64_t) * nb);
+    put_out(c, o.theta, centers.data(), sizeof(float) * nb);
     if (!B.sharded) {
-      copy_out(c, o.mean_theta, mt.data(), sizeof(float) * nb);
-      copy_out(c, o.g_t, gt.data(), sizeof(float) * nb);
-      copy_out(c, o.g_x, gx.data(), sizeof(float) * nb);
-      copy_out(c, o.weights, ww.data(), sizeof(float) * nb);
+      put_out(c, o.mean_theta, mt.data(), sizeof(float) * nb);
+      put_out(c, o.g_t, gt.data(), sizeof(float) * nb);
+      put_out(c, o.g_x, gx.data(), sizeof(float) * nb);
+      put_out(c, o.weights, ww.data(), sizeof(float) * nb);
     }
     if (o.patch_sums && B.use_patch_any) {
       std::vector<double> ps((size_t)n_patch * 6 * nb);
       for (int p = 0; p < n_patch; ++p)
         for (int r = 0; r < 6; ++r)
           for (int b = 0; b < nb; ++b)
-            ps[((size_t)p * 6 + r) * nb + b] = hpatch[t][(size_t)p * kQ * nb + pub_row[r] * nb + b];
-      copy_out(c, o.patch_sums, ps.data(), sizeof(double) * ps.size());
+            ps[((size_t)p * 6 + r) * nb + b] = hpatch[per_task * t + (size_t)p * kQ * nb + pub_row[r] * nb + b];
+      put_out(c, o.patch_sums, ps.data(), sizeof(double) * ps.size());
     }
     check(cudaStreamSynchronize(st), "sync outputs");  // host staging vectors are freed at scope exit
   }

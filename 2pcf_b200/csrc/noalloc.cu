@@ -208,16 +208,18 @@ tpcf_status run_noalloc(tpcf_ctx* c, const float* xA, const float* yA, const flo
   float* zs = (float*)cv.take(sizeof(float) * std::max(nl_valid, 1));
   int* perm = (int*)cv.take(sizeof(int) * std::max(nl_valid, 1));
   if (nA > 0 && nl_valid > 0) {
-    unsigned long long* k0 = (unsigned long long*)cv.take(sizeof(unsigned long long) * nA);
-    unsigned long long* k1 = (unsigned long long*)cv.take(sizeof(unsigned long long) * nA);
+    unsigned* k0 = (unsigned*)cv.take(sizeof(unsigned) * nA);
+    unsigned* k1 = (unsigned*)cv.take(sizeof(unsigned) * nA);
+    const int half = std::min(15, lens_key_bits(nA, 1).half);  // one patch: 32-bit keys
+    const int key_bits = 2 * half + 1;
     int* i0 = (int*)cv.take(sizeof(int) * nA);
     int* i1 = (int*)cv.take(sizeof(int) * nA);
     size_t tb = 0;
-    check(sort_pairs_u64(nullptr, tb, k0, k1, i0, i1, (int)nA, st), "sort size");
+    check(sort_pairs_u32(nullptr, tb, k0, k1, i0, i1, (int)nA, key_bits, st), "sort size");
     void* tmp = cv.take(tb);
     const float4 lbox = make_float4(hbox[0], hbox[1], hbox[2], hbox[3]);
-    counted(c, launch_lens_keys(xA, yA, zA, wA, nullptr, nA, lbox, k0, i0, st), "lens keys");
-    check(sort_pairs_u64(tmp, tb, k0, k1, i0, i1, (int)nA, st), "sort lenses");
+    counted(c, launch_lens_keys(xA, yA, zA, wA, nullptr, nA, lbox, half, 1, k0, i0, st), "lens keys");
+    check(sort_pairs_u32(tmp, tb, k0, k1, i0, i1, (int)nA, key_bits, st), "sort lenses");
     counted(c, launch_lens_gather(i1, nl_valid, xA, yA, zA, valA, wA, lrec, zs, perm, st), "lens gather");
   }
   constexpr int kGroup = 32;

@@ -839,26 +839,28 @@ __global__ void k_src_pairs(const int* __restrict__ idx, int n_valid, int n_chun
 }
 
 
-// Lens sort keys: (patch << 32) | Hilbert index of (x, y) on a 2^16 grid over
-// the box (groups of 32 consecutive lenses of one patch: a third less box
-// diagonal than Morton order on the tomography lenses); invalid lenses get ~0
-// and sort last.
+// Lens sort keys: (patch << 2 half) | Hilbert index of (x, y) on a 2^half grid
+// over the box (groups of consecutive lenses of one patch: a third less box
+// diagonal than Morton order on the tomography lenses); invalid lenses get
+// patch n_patch and sort last.
+template <class Key>
 __global__ void k_lens_keys(const float* __restrict__ x, const float* __restrict__ y,
                             const float* __restrict__ z, const float* __restrict__ w,
-                            const int* __restrict__ patch, long long n, float4 box,
-                            unsigned long long* keys, int* idx) {
-  const float sx = 65535.f / fmaxf(box.z - box.x, 1e-30f);
-  const float sy = 65535.f / fmaxf(box.w - box.y, 1e-30f);
+                            const int* __restrict__ patch, long long n, float4 box, int half, int n_patch,
+                            Key* keys, int* idx) {
+  const int top = (1 << half) - 1;
+  const float sx = (float)top / fmaxf(box.z - box.x, 1e-30f);
+  const float sy = (float)top / fmaxf(box.w - box.y, 1e-30f);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const float xi = x[i], yi = y[i];
-    bool v = isfinite(xi) && isfinite(yi) && w[i] != 0.f;
+    bool v = isfinite(xi) && isfinite(yi) && (!w || w[i] != 0.f);
     if (z && z[i] < 0.f) v = false;
-    unsigned long long key = ~0ull;
+    Key key = (Key)n_patch << (2 * half);
     if (v) {
-      const unsigned qx = (unsigned)clamp_floor((xi - box.x) * sx, 0, 65535);
-      const unsigned qy = (unsigned)clamp_floor((yi - box.y) * sy, 0, 65535);
-      const unsigned long long p = patch ? (unsigned long long)(unsigned)patch[i] : 0ull;
-      key = (p << 32) | hilbert_index(qx, qy, 16);
+      const unsigned qx = (unsigned)clamp_floor((xi - box.x) * sx, 0, top);
+      const unsigned qy = (unsigned)clamp_floor((yi - box.y) * sy, 0, top);
+      const Key p = patch ? (Key)(unsigned)patch[i] : (Key)0;
+      key = (p << (2 * half)) | (Key)hilbert_index(qx, qy, half);
     }
     keys[i] = key;
     idx[i] = (int)i;
@@ -878,16 +880,28 @@ __global__ void k_lens_gather(const int* __restrict__ idx, int n_valid, const fl
 }
 
 // off[p] = first sorted lens with patch >= p, for p in [0, n_patch].
-__global__ void k_patch_offsets(const unsigned long long* __restrict__ keys, int n_valid, int n_patch, int* off) {
+template <class Key>
+__global__ void k_patch_offsets(const Key* __restrict__ keys, int n_valid, int n_patch, int shift, int* off) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p > n_patch) return;
-  const unsigned long long t = (unsigned long long)(unsigned)p << 32;
+  const Key t = (Key)(unsigned)p << shift;
   int lo = 0, hi = n_valid;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
     if (keys[mid] < t) lo = mid + 1; else hi = mid;
   }
   off[p] = lo;
+}
+
+// Groups of `size` consecutive lenses of one patch: starts [n_groups + 1] and
+// the patch's group range {0, n_groups}.
+__global__ void k_uniform_groups(int n_groups, int n_valid, int size, int* start, int* patch_groups) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g <= n_groups) start[g] = min(g * size, n_valid);
+  if (g == 0) {
+    patch_groups[0] = 0;
+    patch_groups[1] = n_groups;
+  }
 }
 
 // One warp per group: bounding box of its lenses.
@@ -911,14 +925,15 @@ __global__ void k_group_box(const float4* __restrict__ rec, const int* __restric
   if (lane == 0) box[g] = make_float4(mnx, mny, mxx, mxy);
 }
 
-// Estimated cost of each work item: lenses x sources in its rows.  Key for a
-// descending sort (longest items first).
-__global__ void k_item_cost(const int2* __restrict__ items, int n_items, const TaskDesc* __restrict__ tasks,
-                            const LensDesc* __restrict__ lenses, const GridDesc* __restrict__ grids, float R,
-                            unsigned long long* cost, int* order) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_items) return;
-  const int2 it = items[i];
+// Work items and their cost bands (cost = lenses x sources in the item's
+// rows); 8 threads per item share its rows.
+__global__ void k_item_cost(const int2* __restrict__ ranges, int n_ranges, int n_items,
+                            const TaskDesc* __restrict__ tasks, const LensDesc* __restrict__ lenses,
+                            const GridDesc* __restrict__ grids, float R, int2* __restrict__ items,
+                            unsigned* __restrict__ band) {
+  const int i = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 3), v = threadIdx.x & 7;
+  const bool live = i < n_items;
+  const int2 it = item_at(ranges, n_ranges, live ? i : n_items - 1);
   const TaskDesc T = tasks[it.x];
   const LensDesc L = lenses[T.lens_cat];
   const GridDesc G = grids[T.src_cat];
@@ -927,13 +942,53 @@ __global__ void k_item_cost(const int2* __restrict__ items, int n_items, const T
   int cy0, cy1;
   row_range(G, box, R, T.margin, cy0, cy1);
   unsigned long long s = 0;
-  for (int cy = cy0 + part; cy <= cy1; cy += T.split) {
+  for (int cy = cy0 + part + v * T.split; cy <= cy1; cy += 8 * T.split) {
     const int2 sp = row_span(G, box, R, T.margin, cy);
     if (sp.y > sp.x) s += (unsigned long long)(sp.y - sp.x);
   }
+#pragma unroll
+  for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (!live || v) return;
   const unsigned long long nl = (unsigned long long)(L.group_start[g + 1] - L.group_start[g]);
-  cost[i] = item_key(s * nl + 1, i);
-  order[i] = i;
+  items[i] = it;
+  band[i] = cost_band(s * nl + 1);
+}
+
+// Items by descending cost band in one block (up to kOrderMax items; five
+// launches of a radix sort otherwise, 58 us against 6 us for 5000 items).  The
+// order inside a band is not fixed: every item sums into its own slot, so the
+// order changes no result (shards, which must agree on it, sort instead).
+constexpr int kOrderMax = 16384;
+__global__ void __launch_bounds__(1024) k_item_order(const int2* __restrict__ items, const unsigned* __restrict__ band,
+                                                     int n, int2* __restrict__ out) {
+  __shared__ int count[kCostBands], base[kCostBands];
+  __shared__ int wsum[kCostBands / 32];
+  const int t = threadIdx.x;
+  if (t < kCostBands) count[t] = 0;
+  __syncthreads();
+  for (int i = t; i < n; i += 1024) atomicAdd(&count[kCostBands - 1 - band[i]], 1);
+  __syncthreads();
+  int v = 0, incl = 0;
+  if (t < kCostBands) {  // exclusive scan, highest band first
+    v = incl = count[t];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((t & 31) >= o) incl += u;
+    }
+    if ((t & 31) == 31) wsum[t >> 5] = incl;
+  }
+  __syncthreads();
+  if (t < kCostBands) {
+    int add = 0;
+    for (int k = 0; k < (t >> 5); ++k) add += wsum[k];
+    base[t] = incl - v + add;
+  }
+  __syncthreads();
+  for (int i = t; i < n; i += 1024) out[atomicAdd(&base[kCostBands - 1 - band[i]], 1)] = items[i];
+}
+__global__ void k_iota32(int* v, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) v[i] = i;
 }
 
 // out[j] = items[order[j*count + index]]: shard `index` of `count`, taking every
@@ -977,10 +1032,10 @@ __global__ void k_dfma_peak(double* out, int iters, double a, double b) {
 
 // Per-patch FP64 sums from item sums, fixed order (deterministic).
 // patch_groups[p] .. patch_groups[p+1] are the groups of patch p, `split` items each.  Block
-// (p, c) covers the 32 sums e = 32 c + lane of patch p: warp w adds the groups
-// g0 + w, g0 + w + 8, ... (lane-contiguous loads), then the 8 warp sums are
-// added in warp order.
-constexpr int kReduceWarps = 8;
+// (p, c) covers the 32 sums e = 32 c + lane of patch p: warp w adds the items
+// g0 + w, g0 + w + kReduceWarps, ... (lane-contiguous loads), then the warp sums
+// are added in warp order.
+constexpr int kReduceWarps = 32;  // 5000 items of one patch: 63 us with 8 warps
 __global__ void __launch_bounds__(32 * kReduceWarps) k_patch_reduce(const double* __restrict__ item_sums, int item_base,
                                                                    int split, const int* __restrict__ patch_groups, int n_patch,
                                                                    int nb, double* patch_sums) {
@@ -992,7 +1047,7 @@ __global__ void __launch_bounds__(32 * kReduceWarps) k_patch_reduce(const double
   const int g0 = patch_groups[p] * split, g1 = patch_groups[p + 1] * split;
   double s = 0.0;
   if (e < ne) {
-#pragma unroll 4
+#pragma unroll 8
     for (int g = g0 + w; g < g1; g += kReduceWarps) s += item_sums[(size_t)(item_base + g) * ne + e];
   }
   part[w][lane] = s;
@@ -1169,29 +1224,53 @@ cudaError_t launch_src_pairs(const int* idx, int n_valid, int mode, const float*
                                                      meta);
   return cudaGetLastError();
 }
+template <class Key>
 cudaError_t launch_lens_keys(const float* x, const float* y, const float* z, const float* w, const int* patch,
-                             long long n, float4 box, unsigned long long* keys, int* idx, cudaStream_t st) {
-  if (n > 0) k_lens_keys<<<gdim(n, 256), 256, 0, st>>>(x, y, z, w, patch, n, box, keys, idx);
+                             long long n, float4 box, int half, int n_patch, Key* keys, int* idx, cudaStream_t st) {
+  if (n > 0) k_lens_keys<Key><<<gdim(n, 256), 256, 0, st>>>(x, y, z, w, patch, n, box, half, n_patch, keys, idx);
   return cudaGetLastError();
 }
+template cudaError_t launch_lens_keys<unsigned>(const float*, const float*, const float*, const float*, const int*,
+                                                long long, float4, int, int, unsigned*, int*, cudaStream_t);
+template cudaError_t launch_lens_keys<unsigned long long>(const float*, const float*, const float*, const float*,
+                                                          const int*, long long, float4, int, int,
+                                                          unsigned long long*, int*, cudaStream_t);
 cudaError_t launch_lens_gather(const int* idx, int n_valid, const float* x, const float* y, const float* z,
                                const float* val, const float* w, float4* rec, float* zs, int* perm, cudaStream_t st) {
   if (n_valid > 0) k_lens_gather<<<(n_valid + 255) / 256, 256, 0, st>>>(idx, n_valid, x, y, z, val, w, rec, zs, perm);
   return cudaGetLastError();
 }
-cudaError_t launch_patch_offsets(const unsigned long long* keys, int n_valid, int n_patch, int* off, cudaStream_t st) {
-  k_patch_offsets<<<(n_patch + 1 + 255) / 256, 256, 0, st>>>(keys, n_valid, n_patch, off);
+template <class Key>
+cudaError_t launch_patch_offsets(const Key* keys, int n_valid, int n_patch, int shift, int* off, cudaStream_t st) {
+  k_patch_offsets<Key><<<(n_patch + 1 + 255) / 256, 256, 0, st>>>(keys, n_valid, n_patch, shift, off);
+  return cudaGetLastError();
+}
+template cudaError_t launch_patch_offsets<unsigned>(const unsigned*, int, int, int, int*, cudaStream_t);
+template cudaError_t launch_patch_offsets<unsigned long long>(const unsigned long long*, int, int, int, int*,
+                                                              cudaStream_t);
+cudaError_t launch_uniform_groups(int n_groups, int n_valid, int size, int* start, int* patch_groups,
+                                  cudaStream_t st) {
+  k_uniform_groups<<<(n_groups + 1 + 255) / 256, 256, 0, st>>>(n_groups, n_valid, size, start, patch_groups);
   return cudaGetLastError();
 }
 cudaError_t launch_group_box(const float4* rec, const int* gstart, int n_groups, float4* box, cudaStream_t st) {
   if (n_groups > 0) k_group_box<<<(n_groups + 7) / 8, 256, 0, st>>>(rec, gstart, n_groups, box);
   return cudaGetLastError();
 }
-cudaError_t launch_item_cost(const int2* items, int n_items, const TaskDesc* tasks, const LensDesc* lenses,
-                             const GridDesc* grids, float R, unsigned long long* cost, int* order,
+cudaError_t launch_item_cost(const int2* ranges, int n_ranges, int n_items, const TaskDesc* tasks,
+                             const LensDesc* lenses, const GridDesc* grids, float R, int2* items, unsigned* band,
                              cudaStream_t st) {
   if (n_items > 0)
-    k_item_cost<<<(n_items + 127) / 128, 128, 0, st>>>(items, n_items, tasks, lenses, grids, R, cost, order);
+    k_item_cost<<<(n_items + 31) / 32, 256, 0, st>>>(ranges, n_ranges, n_items, tasks, lenses, grids, R, items, band);
+  return cudaGetLastError();
+}
+int item_order_max() { return kOrderMax; }
+cudaError_t launch_item_order(const int2* items, const unsigned* band, int n, int2* out, cudaStream_t st) {
+  k_item_order<<<1, 1024, 0, st>>>(items, band, n, out);
+  return cudaGetLastError();
+}
+cudaError_t launch_iota32(int* v, int n, cudaStream_t st) {
+  k_iota32<<<(n + 255) / 256, 256, 0, st>>>(v, n);
   return cudaGetLastError();
 }
 cudaError_t launch_permute_items(const int2* items, const int* order, int n, int index, int count, int2* out,
@@ -1229,12 +1308,13 @@ cudaError_t sort_pairs_u32(void* tmp, size_t& tmp_bytes, const unsigned* kin, un
   return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kin, kout, vin, vout, n, 0, end_bit, st);
 }
 cudaError_t sort_pairs_u64(void* tmp, size_t& tmp_bytes, const unsigned long long* kin, unsigned long long* kout,
-                           const int* vin, int* vout, int n, cudaStream_t st) {
-  return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kin, kout, vin, vout, n, 0, 64, st);
+                           const int* vin, int* vout, int n, int end_bit, cudaStream_t st) {
+  return cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kin, kout, vin, vout, n, 0, end_bit, st);
 }
-cudaError_t sort_pairs_u64_desc(void* tmp, size_t& tmp_bytes, const unsigned long long* kin,
-                                unsigned long long* kout, const int* vin, int* vout, int n, cudaStream_t st) {
-  return cub::DeviceRadixSort::SortPairsDescending(tmp, tmp_bytes, kin, kout, vin, vout, n, 0, 64, st);
+cudaError_t sort_bands_desc(void* tmp, size_t& tmp_bytes, const unsigned* kin, unsigned* kout, const int* vin,
+                            int* vout, int n, cudaStream_t st) {
+  static_assert(kCostBands == 512, "nine key bits");
+  return cub::DeviceRadixSort::SortPairsDescending(tmp, tmp_bytes, kin, kout, vin, vout, n, 0, 9, st);
 }
 
 }  // namespace tpcf

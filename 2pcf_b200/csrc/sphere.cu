@@ -819,12 +819,13 @@ __global__ void k_unit_vectors(const float* __restrict__ lam, const float* __res
   }
 }
 
-__global__ void k_item_cost_sph(const int2* __restrict__ items, int n_items, const TaskDesc* __restrict__ tasks,
-                                const LensDesc* __restrict__ lenses, const GridDesc* __restrict__ grids, float R,
-                                unsigned long long* cost, int* order) {
+__global__ void k_item_cost_sph(const int2* __restrict__ ranges, int n_ranges, int n_items,
+                                const TaskDesc* __restrict__ tasks, const LensDesc* __restrict__ lenses,
+                                const GridDesc* __restrict__ grids, float R, int2* __restrict__ items,
+                                unsigned* __restrict__ band) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_items) return;
-  const int2 it = items[i];
+  const int2 it = item_at(ranges, n_ranges, i);
   const TaskDesc T = tasks[it.x];
   const LensDesc L = lenses[T.lens_cat];
   const GridDesc G = grids[T.src_cat];
@@ -842,8 +843,8 @@ __global__ void k_item_cost_sph(const int2* __restrict__ items, int n_items, con
       if (sp[j].y > sp[j].x) s += (unsigned long long)(sp[j].y - sp[j].x);
   }
   const unsigned long long nl = (unsigned long long)(L.group_start[it.y + 1] - L.group_start[it.y]);
-  cost[i] = item_key(s * nl + 1, i);
-  order[i] = i;
+  items[i] = it;
+  band[i] = cost_band(s * nl + 1);
 }
 
 // --------------------------------------------------------- host launchers --
@@ -919,12 +920,12 @@ cudaError_t launch_unit_vectors(const float* lam, const float* phi, long long n,
   if (n > 0) k_unit_vectors<<<gdim_s(n, 256), 256, 0, st>>>(lam, phi, n, hi, lo);
   return cudaGetLastError();
 }
-cudaError_t launch_item_cost_sph(const int2* items, int n_items, const TaskDesc* tasks, const LensDesc* lenses,
-                                 const GridDesc* grids, float R, unsigned long long* cost, int* order,
+cudaError_t launch_item_cost_sph(const int2* ranges, int n_ranges, int n_items, const TaskDesc* tasks,
+                                 const LensDesc* lenses, const GridDesc* grids, float R, int2* items, unsigned* band,
                                  cudaStream_t st) {
   if (n_items > 0)
-    k_item_cost_sph<<<(n_items + 127) / 128, 128, 0, st>>>(items, n_items, tasks, lenses, grids, R, cost,
-                                                            order);
+    k_item_cost_sph<<<(n_items + 127) / 128, 128, 0, st>>>(ranges, n_ranges, n_items, tasks, lenses, grids, R, items,
+                                                            band);
   return cudaGetLastError();
 }
 

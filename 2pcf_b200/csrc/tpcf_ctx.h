@@ -71,9 +71,42 @@ void check(cudaError_t e, const char* what);
 void counted(tpcf_ctx* c, cudaError_t e, const char* what);
 template <class T>
 const T* stage(tpcf_ctx* c, const T* p, int64_t n);
+// Puts `bytes` of host memory at dst (host or device; a device copy is complete
+// for the caller once the stream is).
+void put_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes);
 void copy_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes);
 void begin_call(tpcf_ctx* c);
 cudaStream_t aux_stream(tpcf_ctx* c);
+// The bounding boxes, counts and patch ranges of ncat catalogues on the device
+// (launch_bbox accumulates into them) and their copy on the host.
+struct Boxes {
+  int ncat = 0;
+  unsigned long long* d_cnt = nullptr;  // [ncat], then box_ord [8 ncat], pr [2 ncat]
+  int* d_box = nullptr;
+  int* d_pr = nullptr;
+  std::vector<float> box;               // [8 ncat]: minx miny maxx maxy minz maxz max|m| 0
+  std::vector<unsigned long long> cnt;
+  std::vector<int> pr;
+  void begin(tpcf_ctx* c, int n);       // allocates and clears
+  void read(tpcf_ctx* c);               // one copy, one wait
+};
+// Sort-key bits of n lenses in n_patch patches: 2 half Hilbert bits (cells of
+// less than a sixteenth of an object on average; a radix sort pays per 8 bits)
+// under the patch bits; wide: more than 32 in all (64-bit keys).
+struct LensKeyBits {
+  int half, total;
+  bool wide;
+};
+LensKeyBits lens_key_bits(int64_t n, int n_patch);
+// Hilbert bits within a cell of the source sort key.
+int cell_hilbert_bits(int64_t n, unsigned ncells, int cell_bits);
+struct TaskDesc;
+struct LensDesc;
+struct GridDesc;
+// The work items of the ranges {task, first item} (n in all) on the device,
+// costliest first; with shard_count > 1 every shard_count-th of them.
+int2* order_items(tpcf_ctx* c, const std::vector<int2>& ranges, int n, const TaskDesc* tasks, const LensDesc* lenses,
+                  const GridDesc* grids, float R, bool sph, int shard_index, int shard_count, int* n_run);
 
 // An event of one call (no timing); destroyed with the object, which CUDA
 // defers until the event has completed.

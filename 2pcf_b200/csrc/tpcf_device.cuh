@@ -108,15 +108,22 @@ __device__ __forceinline__ int2 row_span(const GridDesc& G, float4 box, float R,
   return make_int2(G.cell_start[base + cx0], G.cell_start[base + cx1 + 1]);
 }
 
-// Sort key of work item i (items are built in task, then lens-group order,
-// and lens groups follow (patch, Hilbert) order): the item's cost in bands of
-// 2^(1/8) (about 9%) on top, the item index below.  Sorted descending, the
-// costliest items start first (load balance), and inside one band the items
-// run in task and space order, so that the warps resident at one time read
-// the same rows of one source grid and those stay in L2.
-__device__ __forceinline__ unsigned long long item_key(unsigned long long cost, int i) {
-  const unsigned band = (unsigned)(__log2f((float)cost) * 8.f);
-  return ((unsigned long long)band << 32) | (unsigned)i;
+// Cost band of a work item: log2 of its cost in steps of 2^(1/8) (about 9%),
+// below kCostBands.  The costliest bands start first (load balance); inside
+// one band the items run in task and space order, so that the warps resident
+// at one time read the same rows of one source grid and those stay in L2.
+constexpr int kCostBands = 512;
+__device__ __forceinline__ unsigned cost_band(unsigned long long cost) {
+  return min((unsigned)(__log2f((float)cost) * 8.f), (unsigned)kCostBands - 1u);
+}
+// Work item i of the concatenated ranges {task, first item}: (task, item of the task).
+__device__ __forceinline__ int2 item_at(const int2* __restrict__ ranges, int n_ranges, int i) {
+  int lo = 0, hi = n_ranges;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (ranges[mid].y <= i) lo = mid; else hi = mid;
+  }
+  return make_int2(ranges[lo].x, i - ranges[lo].y);
 }
 
 // Position of cell (qx, qy) of a 2^bits x 2^bits grid (bits <= 16) along the

@@ -46,8 +46,8 @@ cudaError_t launch_lens_pos_sph(const int* perm, int n_valid, const float* lam, 
                                 cudaStream_t st);
 cudaError_t launch_unit_vectors(const float* lam, const float* phi, long long n, float* hi, float* lo,
                                 cudaStream_t st);
-cudaError_t launch_item_cost_sph(const int2* items, int n_items, const TaskDesc* tasks, const LensDesc* lenses,
-                                 const GridDesc* grids, float R, unsigned long long* cost, int* order,
+cudaError_t launch_item_cost_sph(const int2* ranges, int n_ranges, int n_items, const TaskDesc* tasks,
+                                 const LensDesc* lenses, const GridDesc* grids, float R, int2* items, unsigned* band,
                                  cudaStream_t st);
 
 cudaError_t launch_bbox_init(int* box_ord, unsigned long long* count, int* prange, int n, cudaStream_t st);
@@ -67,17 +67,25 @@ cudaError_t launch_cell_start(const unsigned* keys, long long n, unsigned ncells
 cudaError_t launch_src_pairs(const int* idx, int n_valid, int mode, const float* x, const float* y,
                              const float* z, const float* f1, const float* f2, const float* w, const float* m,
                              SrcPair* pairs, ChunkMeta* meta, cudaStream_t st);
+// Key: unsigned or unsigned long long, 2 half + bits of n_patch wide.
+template <class Key>
 cudaError_t launch_lens_keys(const float* x, const float* y, const float* z, const float* w, const int* patch,
-                             long long n, float4 box, unsigned long long* keys, int* idx, cudaStream_t st);
+                             long long n, float4 box, int half, int n_patch, Key* keys, int* idx, cudaStream_t st);
 cudaError_t launch_lens_gather(const int* idx, int n_valid, const float* x, const float* y, const float* z,
                                const float* val, const float* w, float4* rec, float* zs, int* perm,
                                cudaStream_t st);
-cudaError_t launch_patch_offsets(const unsigned long long* keys, int n_valid, int n_patch, int* off,
-                                 cudaStream_t st);
+template <class Key>
+cudaError_t launch_patch_offsets(const Key* keys, int n_valid, int n_patch, int shift, int* off, cudaStream_t st);
+cudaError_t launch_uniform_groups(int n_groups, int n_valid, int size, int* start, int* patch_groups,
+                                  cudaStream_t st);
 cudaError_t launch_group_box(const float4* rec, const int* gstart, int n_groups, float4* box, cudaStream_t st);
-cudaError_t launch_item_cost(const int2* items, int n_items, const TaskDesc* tasks, const LensDesc* lenses,
-                             const GridDesc* grids, float R, unsigned long long* cost, int* order,
+// Work items of the concatenated ranges {task, first item} and their cost bands.
+cudaError_t launch_item_cost(const int2* ranges, int n_ranges, int n_items, const TaskDesc* tasks,
+                             const LensDesc* lenses, const GridDesc* grids, float R, int2* items, unsigned* band,
                              cudaStream_t st);
+int item_order_max();
+cudaError_t launch_item_order(const int2* items, const unsigned* band, int n, int2* out, cudaStream_t st);
+cudaError_t launch_iota32(int* v, int n, cudaStream_t st);
 cudaError_t launch_permute_items(const int2* items, const int* order, int n, int index, int count, int2* out,
                                  cudaStream_t st);
 cudaError_t launch_ffma_peak(float* out, int blocks, int threads, int iters, cudaStream_t st);
@@ -93,8 +101,8 @@ cudaError_t launch_cov(const double* x, int n_s, int D, double* cov, cudaStream_
 cudaError_t sort_pairs_u32(void* tmp, size_t& tmp_bytes, const unsigned* kin, unsigned* kout, const int* vin,
                            int* vout, int n, int end_bit, cudaStream_t st);
 cudaError_t sort_pairs_u64(void* tmp, size_t& tmp_bytes, const unsigned long long* kin, unsigned long long* kout,
-                           const int* vin, int* vout, int n, cudaStream_t st);
-cudaError_t sort_pairs_u64_desc(void* tmp, size_t& tmp_bytes, const unsigned long long* kin,
-                                unsigned long long* kout, const int* vin, int* vout, int n, cudaStream_t st);
+                           const int* vin, int* vout, int n, int end_bit, cudaStream_t st);
+cudaError_t sort_bands_desc(void* tmp, size_t& tmp_bytes, const unsigned* kin, unsigned* kout, const int* vin,
+                            int* vout, int n, cudaStream_t st);
 
 }  // namespace tpcf
