@@ -8,13 +8,16 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "sph_canon.cuh"
@@ -97,6 +100,82 @@ void put_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes) {
     check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream), "output copy");
   else
     std::memcpy(dst, src, bytes);
+}
+
+void copy_out_large(tpcf_ctx* c, const std::vector<HostCopy>& v) {
+  struct Piece {
+    char* dst;
+    const char* src;
+    size_t bytes, off;
+  };
+  std::vector<HostCopy> host;
+  size_t total = 0;
+  for (const HostCopy& h : v) {
+    if (!h.dst || !h.bytes) continue;
+    cudaPointerAttributes a{};
+    const bool pageable = cudaPointerGetAttributes(&a, h.dst) == cudaSuccess && a.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    if (pageable && h.bytes >= kPinnedPiece / 2) {
+      host.push_back(h);
+      total += h.bytes;
+    } else {
+      copy_out(c, h.dst, h.src, h.bytes);
+    }
+  }
+  const size_t want = std::min(total, kPinnedMax);
+  if (c->pinned_bytes < want) {
+    if (c->pinned) cudaFreeHost(c->pinned);
+    c->pinned = nullptr;
+    c->pinned_bytes = 0;
+    if (cudaHostAlloc(&c->pinned, want, cudaHostAllocDefault) == cudaSuccess) {
+      c->pinned_bytes = want;
+    } else {  // no pinned memory: plain copies
+      cudaGetLastError();
+      c->pinned = nullptr;
+      for (const HostCopy& h : host) copy_out(c, h.dst, h.src, h.bytes);
+      host.clear();
+    }
+  }
+  size_t h = 0, done = 0;  // the next byte to copy: host[h] + done
+  while (h < host.size()) {
+    std::vector<Piece> pieces;
+    size_t off = 0;
+    while (h < host.size() && off < c->pinned_bytes) {
+      const size_t n = std::min({kPinnedPiece, host[h].bytes - done, c->pinned_bytes - off});
+      pieces.push_back({(char*)host[h].dst + done, (const char*)host[h].src + done, n, off});
+      off += n;
+      done += n;
+      if (done == host[h].bytes) {
+        ++h;
+        done = 0;
+      }
+    }
+    std::vector<std::unique_ptr<Event>> ev;
+    for (const Piece& p : pieces) {
+      check(cudaMemcpyAsync((char*)c->pinned + p.off, p.src, p.bytes, cudaMemcpyDeviceToHost, c->stream), "D2H piece");
+      ev.emplace_back(new Event);
+      check(cudaEventRecord(ev.back()->e, c->stream), "event record");
+    }
+    std::atomic<size_t> next{0};
+    std::atomic<int> bad{cudaSuccess};
+    auto work = [&]() {
+      cudaSetDevice(c->device);
+      for (size_t i; (i = next.fetch_add(1)) < pieces.size();) {
+        const cudaError_t e = cudaEventSynchronize(ev[i]->e);
+        if (e != cudaSuccess) bad = e;
+        else std::memcpy(pieces[i].dst, (char*)c->pinned + pieces[i].off, pieces[i].bytes);
+      }
+    };
+    const size_t nt = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), pieces.size()});
+    std::vector<std::thread> pool;
+    try {
+      for (size_t t = 1; t < nt; ++t) pool.emplace_back(work);
+    } catch (...) {  // fewer threads than asked for: the others do the work
+    }
+    work();
+    for (std::thread& t : pool) t.join();
+    check((cudaError_t)bad.load(), "output copy");
+  }
 }
 
 void Boxes::begin(tpcf_ctx* c, int n) {
@@ -335,6 +414,7 @@ bool series_pays(int n_valid, double ex, double ey, const tpcf_bins* bins, const
 // A task with fewer lens groups than kSplitItems / 2 is cut into several items
 // per group (at most kMaxSplit).
 constexpr int kSplitItems = 8192, kMaxSplit = 8;
+constexpr size_t kSplitLensBytes = (size_t)256 << 20;  // per-lens sums of a split task at most
 
 void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<SrcIn> srcs, const std::vector<int>& tl,
                  const std::vector<int>& ts, const tpcf_bins* bins, int n_patch, const tpcf_result* outs, Batch& B) {
@@ -638,7 +718,11 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     const int ng = lb[tl[t]].by[kind].n_groups;
     // few lens groups: several items per group keep the SMs' warps busy (a
     // property of the task alone, so its sums do not depend on the batch)
-    d.split = !sph && !any_lens && ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
+    d.split = !sph && ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
+    // the parts of a group add into per-lens columns of their own (k_lens_outputs sums them)
+    const size_t lens_bytes = sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1);
+    if (wants_lens(outs[t]))
+      while (d.split > 1 && lens_bytes * d.split > kSplitLensBytes) --d.split;
     if (ng > 0) ranges[kind].push_back(make_int2(t, n_kind[kind]));
     n_kind[kind] += ng * d.split;
     n_items += ng * d.split;
@@ -646,7 +730,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     d.lens_acc_off = -1;
     if (B.want_lens[t]) {
       d.lens_acc_off = lens_acc_elems;
-      lens_acc_elems += (long long)kQ * nb * std::max(lb[tl[t]].n_valid, 1);
+      lens_acc_elems += (long long)kQ * nb * std::max(lb[tl[t]].n_valid, 1) * d.split;
     }
   }
   // descriptors and edges: one copy
@@ -782,6 +866,7 @@ void batch_finish(tpcf_ctx* c, Batch& B, const tpcf_bins* bins, tpcf_result* out
   const int nb = B.nb, nT = B.nT, n_patch_eff = B.n_patch_eff, n_patch = B.n_patch;
   const size_t per_task = (size_t)kQ * nb * n_patch_eff;
   std::vector<double> hpatch(per_task * nT);
+  std::vector<HostCopy> large;
   check(cudaMemcpyAsync(hpatch.data(), B.dpatch[0], sizeof(double) * per_task * nT, cudaMemcpyDeviceToHost, st),
         "D2H patch");
   for (int t = 0; t < nT; ++t) {
@@ -807,17 +892,21 @@ void batch_finish(tpcf_ctx* c, Batch& B, const tpcf_bins* bins, tpcf_result* out
       if (!marks_all && (xE || xB || Km || wm))
         throw Failure(TPCF_ERR_INVALID_ARG, "xi_E_marks, xi_B_marks, K_marks and w_marks go together");
       if (LB.n_valid > 0 && B.n_items > 0 && B.lens_acc)
-        counted(c, launch_lens_outputs(B.lens_acc + B.tdesc[t].lens_acc_off, LB.rec, LB.perm, LB.n_valid, nb, xE,
+        counted(c, launch_lens_outputs(B.lens_acc + B.tdesc[t].lens_acc_off, B.tdesc[t].split, LB.rec, LB.perm, LB.n_valid, nb, xE,
                                        xB, Km, wm, mw, ls, lr, st), "lens outputs");
-      if (xE && xE != (void*)o.xi_E_marks) copy_out(c, o.xi_E_marks, xE, mb);
-      if (xB && xB != (void*)o.xi_B_marks) copy_out(c, o.xi_B_marks, xB, mb);
-      if (Km && Km != (void*)o.K_marks) copy_out(c, o.K_marks, Km, mb);
-      if (wm && wm != (void*)o.w_marks) copy_out(c, o.w_marks, wm, mb);
-      if (mw && mw != (void*)o.marks_weight) copy_out(c, o.marks_weight, mw, sizeof(float) * nA);
-      if (ls && ls != (void*)o.lens_sums) copy_out(c, o.lens_sums, ls, sizeof(double) * 6 * nb * nA);
-      if (lr && lr != (void*)o.lens_raw) copy_out(c, o.lens_raw, lr, sizeof(double) * 6 * nb * nA);
+      auto out = [&](void* user, const void* dev, size_t bytes) {
+        if (dev && dev != user) large.push_back({user, dev, bytes});
+      };
+      out(o.xi_E_marks, xE, mb);
+      out(o.xi_B_marks, xB, mb);
+      out(o.K_marks, Km, mb);
+      out(o.w_marks, wm, mb);
+      out(o.marks_weight, mw, sizeof(float) * nA);
+      out(o.lens_sums, ls, sizeof(double) * 6 * nb * nA);
+      out(o.lens_raw, lr, sizeof(double) * 6 * nb * nA);
     }
   }
+  copy_out_large(c, large);
   unsigned herr = 0;
   check(cudaMemcpyAsync(&herr, B.head + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st), "D2H err");
   check(cudaStreamSynchronize(st), "sync results");
@@ -948,6 +1037,7 @@ tpcf_status tpcf_destroy(tpcf_ctx* c) {
   cudaStreamSynchronize(c->stream);
   for (auto& s : c->slots)
     if (s.ptr) cudaFree(s.ptr);
+  if (c->pinned) cudaFreeHost(c->pinned);
   if (c->aux_stream) cudaStreamDestroy(c->aux_stream);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;

@@ -666,7 +666,7 @@ tpcf_status tpcf_kmeans(tpcf_ctx* c, const float* x, const float* y, const float
       check(cudaStreamSynchronize(st), "sync k-means");
     }
     const int it = hstate.passes;
-    copy_out(c, labels_out, lab, sizeof(int) * n);
+    copy_out_large(c, {{labels_out, lab, sizeof(int) * (size_t)n}});
     if (centroids_out) copy_out(c, centroids_out, dcen, sizeof(float2) * k);
     check(cudaStreamSynchronize(st), "sync outputs");
     if (n_iter_out) *n_iter_out = it;

@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(BT, kPairMinBlocks) k_pairs(const PairParams P
       vw = (double)r.z * (double)r.w;
       w = (double)r.w;
       if (HAS_Z) lz = LD.z[gs + lane];
-      if (P.lens_acc && T.lens_acc_off >= 0) lens_col = P.lens_acc + T.lens_acc_off + gs + lane;
+      if (P.lens_acc && T.lens_acc_off >= 0) lens_col = P.lens_acc + T.lens_acc_off + (size_t)part * kQ * nb * LD.n_valid + gs + lane;
     }
     LensP LP;
     LP.nlx = dup2(-lx);
@@ -1060,9 +1060,10 @@ __global__ void __launch_bounds__(32 * kReduceWarps) k_patch_reduce(const double
 }
 
 // Per-lens outputs in input order from per-lens FP64 sums [kQ][nb][n_valid]
-// (sorted order, no lens factors).  Outputs must be zeroed beforehand (masked
+// (sorted order, no lens factors), the `split` parts of the
+// task added in order.  Outputs must be zeroed beforehand (masked
 // lenses keep 0, as in the reference).
-__global__ void k_lens_outputs(const double* __restrict__ acc, const float4* __restrict__ rec,
+__global__ void k_lens_outputs(const double* __restrict__ acc, int split, const float4* __restrict__ rec,
                                const int* __restrict__ perm, int n_valid, int nb, float* xi_E, float* xi_B,
                                float* K_m, float* w_m, float* marks_weight, double* lens_sums, double* lens_raw) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1071,13 +1072,20 @@ __global__ void k_lens_outputs(const double* __restrict__ acc, const float4* __r
   const double vw = (double)r.z * (double)r.w, w = (double)r.w;
   const size_t i = (size_t)perm[s];
   double mw = 0.0;
+  const size_t part = (size_t)kQ * nb * n_valid;
+  auto sum = [&](int q, int b) {
+    const double* a = acc + (size_t)(q * nb + b) * n_valid + s;
+    double v = a[0];
+    for (int p = 1; p < split; ++p) v += a[p * part];
+    return v;
+  };
   for (int b = 0; b < nb; ++b) {
-    const double gt = acc[(size_t)(QGT * nb + b) * n_valid + s] * vw;
-    const double gx = acc[(size_t)(QGX * nb + b) * n_valid + s] * vw;
-    const double ww = acc[(size_t)(QW * nb + b) * n_valid + s] * w;
-    const double dw = acc[(size_t)(QDW * nb + b) * n_valid + s] * w;
-    const double nn = acc[(size_t)(QN * nb + b) * n_valid + s];
-    const double kk = acc[(size_t)(QK * nb + b) * n_valid + s] * w;
+    const double gt = sum(QGT, b) * vw;
+    const double gx = sum(QGX, b) * vw;
+    const double ww = sum(QW, b) * w;
+    const double dw = sum(QDW, b) * w;
+    const double nn = sum(QN, b);
+    const double kk = sum(QK, b) * w;
     if (xi_E) {
       xi_E[i * nb + b] = (float)gt;
       xi_B[i * nb + b] = (float)gx;
@@ -1095,11 +1103,11 @@ __global__ void k_lens_outputs(const double* __restrict__ acc, const float4* __r
     }
     if (lens_raw) {
       double* o = lens_raw + i * 6 * nb;
-      o[0 * nb + b] = acc[(size_t)(QDW * nb + b) * n_valid + s];
-      o[1 * nb + b] = acc[(size_t)(QGT * nb + b) * n_valid + s];
-      o[2 * nb + b] = acc[(size_t)(QGX * nb + b) * n_valid + s];
-      o[3 * nb + b] = acc[(size_t)(QW * nb + b) * n_valid + s];
-      o[4 * nb + b] = acc[(size_t)(QK * nb + b) * n_valid + s];
+      o[0 * nb + b] = sum(QDW, b);
+      o[1 * nb + b] = sum(QGT, b);
+      o[2 * nb + b] = sum(QGX, b);
+      o[3 * nb + b] = sum(QW, b);
+      o[4 * nb + b] = sum(QK, b);
       o[5 * nb + b] = nn;
     }
     mw += ww;
@@ -1293,11 +1301,11 @@ cudaError_t launch_patch_reduce(const double* item_sums, int item_base, int spli
                                                                                     n_patch, nb, patch_sums);
   return cudaGetLastError();
 }
-cudaError_t launch_lens_outputs(const double* acc, const float4* rec, const int* perm, int n_valid, int nb,
+cudaError_t launch_lens_outputs(const double* acc, int split, const float4* rec, const int* perm, int n_valid, int nb,
                                 float* xi_E, float* xi_B, float* K_m, float* w_m, float* marks_weight,
                                 double* lens_sums, double* lens_raw, cudaStream_t st) {
   if (n_valid > 0)
-    k_lens_outputs<<<(n_valid + 127) / 128, 128, 0, st>>>(acc, rec, perm, n_valid, nb, xi_E, xi_B, K_m, w_m,
+    k_lens_outputs<<<(n_valid + 127) / 128, 128, 0, st>>>(acc, split, rec, perm, n_valid, nb, xi_E, xi_B, K_m, w_m,
                                                           marks_weight, lens_sums, lens_raw);
   return cudaGetLastError();
 }

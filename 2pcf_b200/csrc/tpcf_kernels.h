@@ -92,7 +92,7 @@ cudaError_t launch_ffma_peak(float* out, int blocks, int threads, int iters, cud
 cudaError_t launch_dfma_peak(double* out, int blocks, int threads, int iters, cudaStream_t st);
 cudaError_t launch_patch_reduce(const double* item_sums, int item_base, int split, const int* patch_groups,
                                 int n_patch, int nb, double* patch_sums, cudaStream_t st);
-cudaError_t launch_lens_outputs(const double* acc, const float4* rec, const int* perm, int n_valid, int nb,
+cudaError_t launch_lens_outputs(const double* acc, int split, const float4* rec, const int* perm, int n_valid, int nb,
                                 float* xi_E, float* xi_B, float* K_m, float* w_m, float* marks_weight,
                                 double* lens_sums, double* lens_raw, cudaStream_t st);
 
