@@ -718,7 +718,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     const int ng = lb[tl[t]].by[kind].n_groups;
     // few lens groups: several items per group keep the SMs' warps busy (a
     // property of the task alone, so its sums do not depend on the batch)
-    d.split = !sph && ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
+    // (the sphere's items are blocks of up to 128 lenses)
+    d.split = ng > 0 ? std::max(1, std::min(kMaxSplit, (sph ? kSplitItems / 2 : kSplitItems) / ng)) : 1;
     // the parts of a group add into per-lens columns of their own (k_lens_outputs sums them)
     const size_t lens_bytes = sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1);
     if (wants_lens(outs[t]))

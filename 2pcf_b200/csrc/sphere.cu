@@ -180,9 +180,8 @@ __device__ __forceinline__ int classify_s(const LensS& L, const float4 mn, const
   b0 = max(b0, -1);  // every bin below 0 or from nb up is dropped alike
   b1 = min(b1, C.nb);
   blo = b0;
-  if (b0 == b1) return 1;  // a z cut is applied inside the register paths
-  if (b1 == b0 + 1) return 2;
-  return 3;
+  const int e = b1 - b0;  // bin edges in range; a z cut is applied inside the register paths
+  return e <= 2 ? 1 + e : 4;
 }
 
 template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB, bool SMALL, int NC, int QA>
@@ -291,27 +290,31 @@ __device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, f
   }
 }
 
-// Register sums of one lens over a sub-chunk: all pairs (s*) and, in the
-// one-edge path, the upper side (h*).
+// Register sums of one lens over a sub-chunk: all pairs (s*) and, per edge,
+// the upper side (h*).
+template <int NE>
 struct SphAcc {
-  float2 sgt, sgx, sw, sdw, sk, sn, hgt, hgx, hw, hdw, hk, hn, nc;
+  float2 sgt, sgx, sw, sdw, sk, sn, nc;
+  float2 hgt[NE ? NE : 1], hgx[NE ? NE : 1], hw[NE ? NE : 1], hdw[NE ? NE : 1], hk[NE ? NE : 1], hn[NE ? NE : 1];
 };
-__device__ __forceinline__ void sph_acc_zero(SphAcc& A) {
-  A.sgt = A.sgx = A.sw = A.sdw = A.sk = A.sn = dup2(0.f);
-  A.hgt = A.hgx = A.hw = A.hdw = A.hk = A.hn = A.nc = dup2(0.f);
+template <int NE>
+__device__ __forceinline__ void sph_acc_zero(SphAcc<NE>& A) {
+  A.sgt = A.sgx = A.sw = A.sdw = A.sk = A.sn = A.nc = dup2(0.f);
+#pragma unroll
+  for (int e = 0; e < NE; ++e) A.hgt[e] = A.hgx[e] = A.hw[e] = A.hdw[e] = A.hk[e] = A.hn[e] = dup2(0.f);
 }
 
 // The two pairs of one SrcPairS against a lens (TAIL: only the first; the
 // second half is a copy, masked out).  With a z cut a pair with z_A > z_B
-// (src/tpcf.f90:322) adds nothing.  DUAL also forms the upper-side sums
-// (pairs with d2 >= E, the side a 1.0/0.0 mask from one FP32 compare at
-// Ehi = E (1 + eps), applied by multiplication) and counts the pairs between
-// Elo = E (1 - eps) and Ehi, inside the guard band (A.nc).  Without a z cut
-// the w and K sums of all pairs (and, scalar-scalar, the g sums) are the
-// sub-chunk's totals, so they are not accumulated here.
-template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool DUAL, bool TAIL>
-__device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPairS& s, float Elo, float Ehi,
-                                         SphAcc& A) {
+// (src/tpcf.f90:322) adds nothing.  For each of the NE edges the upper-side
+// sums are formed too (pairs with d2 >= E, the side a 1.0/0.0 mask from one FP32
+// compare at Ehi = E (1 + eps), applied by multiplication), and the pairs
+// between Elo = E (1 - eps) and Ehi, inside the guard band, are counted (A.nc).
+// Without a z cut the w and K sums of all pairs (and, scalar-scalar, the g sums)
+// are the sub-chunk's totals, so they are not accumulated here.
+template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NE, bool TAIL>
+__device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPairS& s, const float* Elo,
+                                         const float* Ehi, SphAcc<NE>& A) {
   constexpr bool LI = !HAS_Z;
   float2 d2, th, r, X, Y;
   sph_terms2<MODE, SMALL>(L, s, d2, th, r, X, Y);
@@ -335,9 +338,10 @@ __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPai
   if (!LI) A.sw = add2(A.sw, w);
   A.sdw = fma2(th, w, A.sdw);
   if (MODE == 0 && HAS_M && !LI) A.sk = add2(A.sk, K);
-  if (DUAL) {
-    float2 mh = make_float2(d2.x >= Ehi ? 1.f : 0.f, d2.y >= Ehi ? 1.f : 0.f);
-    const float2 ml = make_float2(d2.x >= Elo ? 1.f : 0.f, d2.y >= Elo ? 1.f : 0.f);
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    float2 mh = make_float2(d2.x >= Ehi[e] ? 1.f : 0.f, d2.y >= Ehi[e] ? 1.f : 0.f);
+    const float2 ml = make_float2(d2.x >= Elo[e] ? 1.f : 0.f, d2.y >= Elo[e] ? 1.f : 0.f);
     if (HAS_Z || TAIL) {
       A.nc = fma2(add2(ml, make_float2(-mh.x, -mh.y)), vm, A.nc);
       mh = mul2(mh, vm);
@@ -346,18 +350,18 @@ __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPai
     }
     const float2 rm = mul2(r, mh);  // r, w, K carry the validity mask already
     const float2 wm = mul2(w, mh);
-    A.hgt = fma2(rm, X, A.hgt);
-    A.hgx = fma2(rm, Y, A.hgx);
-    A.hw = add2(A.hw, wm);
-    A.hdw = fma2(th, wm, A.hdw);
-    A.hn = add2(A.hn, mh);
-    if (MODE == 0 && HAS_M) A.hk = fma2(K, mh, A.hk);
+    A.hgt[e] = fma2(rm, X, A.hgt[e]);
+    A.hgx[e] = fma2(rm, Y, A.hgx[e]);
+    A.hw[e] = add2(A.hw[e], wm);
+    A.hdw[e] = fma2(th, wm, A.hdw[e]);
+    A.hn[e] = add2(A.hn[e], mh);
+    if (MODE == 0 && HAS_M) A.hk[e] = fma2(K, mh, A.hk[e]);
   }
 }
 
 // Sums over all pairs of a sub-chunk; ss = {sum p, sum q, sum w, sum K}.
-template <int MODE, bool HAS_M, bool HAS_Z, int QA>
-__device__ __forceinline__ void sph_totals(const SphAcc& A, int cnt, const float4 ss, float* tot) {
+template <int MODE, bool HAS_M, bool HAS_Z, int QA, int NE>
+__device__ __forceinline__ void sph_totals(const SphAcc<NE>& A, int cnt, const float4 ss, float* tot) {
   constexpr bool LI = !HAS_Z;
   tot[QGT] = (LI && MODE == 1) ? ss.x : sum2(A.sgt);
   tot[QGX] = (LI && MODE == 1) ? ss.y : sum2(A.sgx);
@@ -371,58 +375,71 @@ __device__ __forceinline__ void sph_totals(const SphAcc& A, int cnt, const float
 template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NC, int QA>
 __device__ __forceinline__ void chunk_single_s(const SrcPairS* __restrict__ S, int cnt, const LensS2& L, float lz,
                                                int cls, int blo, float* __restrict__ hcol, const float4 ss) {
-  SphAcc A;
+  SphAcc<0> A;
   sph_acc_zero(A);
   const int np = cnt >> 1;
 #pragma unroll 2
-  for (int k = 0; k < np; ++k) sph_step<MODE, HAS_M, HAS_Z, SMALL, false, false>(L, lz, S[k], 0.f, 0.f, A);
+  for (int k = 0; k < np; ++k) sph_step<MODE, HAS_M, HAS_Z, SMALL, 0, false>(L, lz, S[k], nullptr, nullptr, A);
   if (cnt & 1)
-    sph_step<MODE, HAS_M, HAS_Z, SMALL, false, true>(L, lz, dup_pair_s(src_of_s(S, cnt - 1)), 0.f, 0.f, A);
+    sph_step<MODE, HAS_M, HAS_Z, SMALL, 0, true>(L, lz, dup_pair_s(src_of_s(S, cnt - 1)), nullptr, nullptr, A);
   if (cls != 1) return;
   float acc[QA];
   sph_totals<MODE, HAS_M, HAS_Z, QA>(A, cnt, ss, acc);
   hist_add<QA, NC>(hcol, blo, acc);
 }
 
-// Class 2: pairs in bins blo and blo+1 (either may be out of range, then it is
-// dropped); the edge between them is e2f[blo+1].
-template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NC, int QA>
-__device__ __forceinline__ void chunk_dual_s(const SrcPairS* __restrict__ S, int cnt, const LensS& Lf,
-                                             const LensS2& L, float lz, int cls, int blo, float* __restrict__ hcol,
-                                             const BinCtx& C, const float4 ss) {
-  // lanes of class 1 (or 0) keep an edge no pair reaches
-  const float E = C.e2f[min(max(blo + 1, 0), C.nb)];
-  const float Elo = (cls == 2) ? E * (1.f - C.eps_rel) : 3.0e38f;
-  const float Ehi = (cls == 2) ? E * (1.f + C.eps_rel) : 3.0e38f;
-  SphAcc A;
+// Classes 2 and 3: pairs in bins blo .. blo + NE across NE = 1 or 2 edges (a bin
+// outside [0, nb) is dropped); edge e is e2f[blo + 1 + e].  Bin blo + j receives
+// h[j-1] - h[j] with h[-1] = all and h[NE] = 0, as in the planar kernel.
+template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NC, int QA, int NE>
+__device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, int cnt, const LensS& Lf,
+                                              const LensS2& L, float lz, int cls, int blo, float* __restrict__ hcol,
+                                              const BinCtx& C, const float4 ss) {
+  float Elo[NE], Ehi[NE];
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {  // lanes with fewer edges keep one no pair reaches
+    const bool on = e < cls - 1;
+    const float E = C.e2f[min(max(blo + 1 + e, 0), C.nb)];
+    Elo[e] = on ? E * (1.f - C.eps_rel) : 3.0e38f;
+    Ehi[e] = on ? E * (1.f + C.eps_rel) : 3.0e38f;
+  }
+  SphAcc<NE> A;
   sph_acc_zero(A);
   const int np = cnt >> 1;
 #pragma unroll 2
-  for (int k = 0; k < np; ++k) sph_step<MODE, HAS_M, HAS_Z, SMALL, true, false>(L, lz, S[k], Elo, Ehi, A);
+  for (int k = 0; k < np; ++k) sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, false>(L, lz, S[k], Elo, Ehi, A);
   if (cnt & 1)
-    sph_step<MODE, HAS_M, HAS_Z, SMALL, true, true>(L, lz, dup_pair_s(src_of_s(S, cnt - 1)), Elo, Ehi, A);
+    sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, true>(L, lz, dup_pair_s(src_of_s(S, cnt - 1)), Elo, Ehi, A);
   if (cls == 0) return;
   if (sum2(A.nc) != 0.f) {  // rare: a pair inside the guard band; the sub-chunk is binned pair by pair
     for (int j = 0; j < cnt; ++j) do_pair_s<MODE, HAS_M, HAS_Z, SMALL, SMALL, NC, QA>(Lf, lz, src_of_s(S, j), hcol, C);
     return;
   }
-  float tot[QA], hi[QA];
-  sph_totals<MODE, HAS_M, HAS_Z, QA>(A, cnt, ss, tot);
-  hi[QGT] = sum2(A.hgt);
-  hi[QGX] = sum2(A.hgx);
-  hi[QW] = sum2(A.hw);
-  hi[QDW] = sum2(A.hdw);
-  hi[QN] = sum2(A.hn);
-  if (MODE == 0 && HAS_M) hi[QK] = sum2(A.hk);
-  if (cls == 1) {
-    hist_add<QA, NC>(hcol, blo, tot);
-    return;
-  }
-  float lo[QA];
+  float prev[QA];
+  sph_totals<MODE, HAS_M, HAS_Z, QA>(A, cnt, ss, prev);
 #pragma unroll
-  for (int q = 0; q < QA; ++q) lo[q] = tot[q] - hi[q];
-  if (blo >= 0) hist_add<QA, NC>(hcol, blo, lo);
-  if (blo + 1 < C.nb) hist_add<QA, NC>(hcol, blo + 1, hi);
+  for (int j = 0; j <= NE; ++j) {
+    float up[QA];
+#pragma unroll
+    for (int q = 0; q < QA; ++q) up[q] = 0.f;
+    if (j < NE) {
+      up[QGT] = sum2(A.hgt[j < NE ? j : 0]);
+      up[QGX] = sum2(A.hgx[j < NE ? j : 0]);
+      up[QW] = sum2(A.hw[j < NE ? j : 0]);
+      up[QDW] = sum2(A.hdw[j < NE ? j : 0]);
+      up[QN] = sum2(A.hn[j < NE ? j : 0]);
+      if (MODE == 0 && HAS_M) up[QK] = sum2(A.hk[j < NE ? j : 0]);
+    }
+    const int bin = blo + j;
+    if (j <= cls - 1 && bin >= 0 && bin < C.nb) {
+      float v[QA];
+#pragma unroll
+      for (int q = 0; q < QA; ++q) v[q] = prev[q] - up[q];
+      hist_add<QA, NC>(hcol, bin, v);
+    }
+#pragma unroll
+    for (int q = 0; q < QA; ++q) prev[q] = up[q];
+  }
 }
 
 // ------------------------------------------------------------ cell runs -----
@@ -569,7 +586,7 @@ __global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
     const TaskDesc T = P.tasks[it.x];
     const LensDesc LD = P.lenses[T.lens_cat];
     const GridDesc G = P.grids[T.src_cat];
-    const int g = it.y;
+    const int g = it.y / T.split, part = it.y - g * T.split;  // this item's rows: every T.split-th
     const int gs = LD.group_start[g];
     const int nl = LD.group_start[g + 1] - gs;
     const bool act = tid < nl;
@@ -583,7 +600,7 @@ __global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
       vw = (double)r.z * (double)r.w;
       w = (double)r.w;
       if (HAS_Z) lz = LD.z[gs + tid];
-      if (P.lens_acc && T.lens_acc_off >= 0) lens_col = P.lens_acc + T.lens_acc_off + gs + tid;
+      if (P.lens_acc && T.lens_acc_off >= 0) lens_col = P.lens_acc + T.lens_acc_off + (size_t)part * kQ * nb * LD.n_valid + gs + tid;
     } else {
       Lf = lens_frame(make_float4(1.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f));
     }
@@ -600,13 +617,13 @@ __global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
     bool full;
     sph_reach(G, box, P.R, T.margin, dl, full);
 
-    for (int c0 = cy0; c0 <= cy1; c0 += kRowsS) {
-      const int nr = min(kRowsS, cy1 - c0 + 1);
+    for (int c0 = cy0 + part; c0 <= cy1; c0 += kRowsS * T.split) {
+      const int nr = min(kRowsS, (cy1 - c0) / T.split + 1);
       const int ns = 3 * nr;
       __syncthreads();
       for (int r = tid; r < nr; r += BT) {
         int2 sp[3];
-        const int k = sph_row_spans(G, box, P.R, T.margin, c0 + r, dl, full, sp);
+        const int k = sph_row_spans(G, box, P.R, T.margin, c0 + r * T.split, dl, full, sp);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           const int2 v = j < k ? sp[j] : make_int2(0, 0);
@@ -729,7 +746,9 @@ __global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
             if (m == 1) {
               chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, BT, QA>(Sc, cnt, LP, lz, cls, blo, hcol, subsum[sc]);
             } else if (m == 2) {
-              chunk_dual_s<MODE, HAS_M, HAS_Z, SMALL, BT, QA>(Sc, cnt, Lf, LP, lz, cls, blo, hcol, C, subsum[sc]);
+              chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, BT, QA, 1>(Sc, cnt, Lf, LP, lz, cls, blo, hcol, C, subsum[sc]);
+            } else if (m == 3) {
+              chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, BT, QA, 2>(Sc, cnt, Lf, LP, lz, cls, blo, hcol, C, subsum[sc]);
             } else if (act) {
               for (int j = 0; j < cnt; ++j)
                 do_pair_s<MODE, HAS_M, HAS_Z, LOGB, SMALL, BT, QA>(Lf, lz, src_of_s(Sc, j), hcol, C);
@@ -747,7 +766,7 @@ __global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
     }
     flush_hist<QA, BT>(hist, bsum, fvw, fw, nb, lens_col, lens_stride);
     __syncthreads();
-    double* out = P.item_sums + (size_t)(T.item_base + g) * kQ * nb;
+    double* out = P.item_sums + (size_t)(T.item_base + it.y) * kQ * nb;
     for (int e = tid; e < kQ * nb; e += BT) {
       const int q = e / nb;
       out[e] = (q == QK && QA == 5) ? bsum[e - (QK - QW) * nb] : bsum[e];
@@ -829,20 +848,21 @@ __global__ void k_item_cost_sph(const int2* __restrict__ ranges, int n_ranges, i
   const TaskDesc T = tasks[it.x];
   const LensDesc L = lenses[T.lens_cat];
   const GridDesc G = grids[T.src_cat];
-  const float4 box = L.group_box[it.y];
+  const int g = it.y / T.split, part = it.y - g * T.split;
+  const float4 box = L.group_box[g];
   int cy0, cy1;
   row_range(G, box, R, T.margin, cy0, cy1);
   float dl;
   bool full;
   sph_reach(G, box, R, T.margin, dl, full);
   unsigned long long s = 0;
-  for (int cy = cy0; cy <= cy1; ++cy) {
+  for (int cy = cy0 + part; cy <= cy1; cy += T.split) {
     int2 sp[3];
     const int k = sph_row_spans(G, box, R, T.margin, cy, dl, full, sp);
     for (int j = 0; j < k; ++j)
       if (sp[j].y > sp[j].x) s += (unsigned long long)(sp[j].y - sp[j].x);
   }
-  const unsigned long long nl = (unsigned long long)(L.group_start[it.y + 1] - L.group_start[it.y]);
+  const unsigned long long nl = (unsigned long long)(L.group_start[g + 1] - L.group_start[g]);
   items[i] = it;
   band[i] = cost_band(s * nl + 1);
 }
