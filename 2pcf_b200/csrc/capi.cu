@@ -519,7 +519,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   int bt = 128;
   while (bt > 32 && (size_t)nb * qa * bt * 4 > 100 * 1024) bt /= 2;
   // planar: bt threads per block, each warp one 32-lens group at a time, tiles
-  // of tch sub-chunks; sphere: one bt-lens group per block
+  // of tch sub-chunks
   int tch = 2;
   if (!sph && c->opts.group_size > 0 && c->opts.group_size <= bt) bt = c->opts.group_size;
   if (!sph && c->opts.tile_chunks == 1) tch = 1;
@@ -563,7 +563,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     SrcPair* pairs = sph || series ? nullptr : (SrcPair*)ws_alloc(c, sizeof(SrcPair) * (kChunk / 2) * n_chunks);
     ChunkMeta* cmeta = sph || series ? nullptr : (ChunkMeta*)ws_alloc(c, sizeof(ChunkMeta) * n_chunks);
     float* srec = series ? (float*)ws_alloc(c, series_bytes(n_valid, mode, has_m, has_z)) : nullptr;
-    SrcRecS* recs = sph ? (SrcRecS*)ws_alloc(c, sizeof(SrcRecS) * std::max(n_valid, 1)) : nullptr;
+    void* sphc = sph ? ws_alloc(c, sph_src_bytes(n_valid)) : nullptr;
     if (s.n > 0) {
       unsigned* k0 = (unsigned*)ws_alloc(c, sizeof(unsigned) * s.n);
       unsigned* k1 = (unsigned*)ws_alloc(c, sizeof(unsigned) * s.n);
@@ -580,7 +580,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
       check(sort_pairs_u32(tmp, tb, k0, k1, i0, i1, (int)s.n, end_bit, st), "sort sources");
       counted(c, launch_cell_start(k1, s.n, ncells, mb, cs, st), "cell start");
       if (sph)
-        counted(c, launch_src_gather_sph(i1, n_valid, mode, lamS[i], s.y, s.z, s.f1, s.f2, s.w, s.m, recs, st),
+        counted(c, launch_src_gather_sph(i1, n_valid, mode, lamS[i], s.y, s.z, s.f1, s.f2, s.w, s.m, sphc, st),
                 "src gather");
       else if (series)
         counted(c, launch_src_series(i1, n_valid, mode, has_m, has_z, s.x, s.y, s.z, s.f1, s.f2, s.w, s.m, srec, st),
@@ -593,7 +593,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     }
     g.cell_start = cs;
     g.rec = nullptr;
-    g.recs = recs;
+    g.sph = sphc;
     g.pairs = pairs;
     g.meta = cmeta;
     g.series = srec;
@@ -616,7 +616,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   std::vector<LensBuilt>& lb = B.lb;
   lb.assign(nL, LensBuilt{});
   std::vector<LensDesc> ldesc(2 * nL);  // [kind * nL + catalogue]
-  const int lens_group[2] = {sph ? bt : 32, series_lens_group()};
+  const int lens_group[2] = {32, series_lens_group()};
   for (int i = 0; i < nL; ++i) {
     const LensIn& l = lens[i];
     LensBuilt& LB = lb[i];
@@ -718,8 +718,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     const int ng = lb[tl[t]].by[kind].n_groups;
     // few lens groups: several items per group keep the SMs' warps busy (a
     // property of the task alone, so its sums do not depend on the batch)
-    // (the sphere's items are blocks of up to 128 lenses)
-    d.split = ng > 0 ? std::max(1, std::min(kMaxSplit, (sph ? kSplitItems / 2 : kSplitItems) / ng)) : 1;
+    d.split = ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
     // the parts of a group add into per-lens columns of their own (k_lens_outputs sums them)
     const size_t lens_bytes = sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1);
     if (wants_lens(outs[t]))
@@ -834,7 +833,7 @@ void batch_launch(tpcf_ctx* c, Batch& B, bool timed) {
       check(cudaEventRecord(ev0, st), "event record");
     }
     if (B.sph) {
-      counted(c, launch_pairs_sph(B.P[0], B.mode, B.has_m, B.has_z, B.logb, B.bt, c->num_sms, st, &B.grid),
+      counted(c, launch_pairs_sph(B.P[0], B.mode, B.has_m, B.has_z, B.logb, c->num_sms, st, &B.grid),
               "pair kernel");
     } else {
       for (int k = 0; k < 2; ++k) {

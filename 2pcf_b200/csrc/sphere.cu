@@ -29,6 +29,7 @@
 #include <cstdio>
 
 #include "pair_hist.cuh"
+#include "pair_tiles.cuh"
 #include "sph_canon.cuh"
 #include "tpcf_device.cuh"
 #include "tpcf_internal.cuh"
@@ -67,6 +68,11 @@ __device__ __forceinline__ int slow_bin_s(float4 ha, float4 la, float4 hb, float
 }
 
 // ------------------------------------------------------------ pair terms ----
+// One source in scalar form: a = {hi, p}, b = {lo, q}, c = {w, K, z, 0}.
+struct __align__(16) SrcRecS {
+  float4 a, b, c;
+};
+
 // One lens: unit vector hi/lo and its local east/north basis.
 struct LensS {
   float4 h, l;
@@ -203,12 +209,11 @@ __device__ __forceinline__ void do_pair_s(const LensS& L, float lz, const SrcRec
   if (MODE == 0 && HAS_M) h[QK * NC] += s.c.y;
 }
 
-// Two consecutive sources (2k, 2k+1) of a 32-source sub-chunk in shared
-// memory with their fields interleaved, so that a 64-bit register pair holds
-// one field of both (the operand form of the sm_100 packed FP32
-// instructions).  The kernel rewrites each tile in place into this form (the
-// same 96 bytes as the two SrcRecS).  p, q = a.w, b.w of SrcRecS; w, K, z =
-// c.x, c.y, c.z.
+// Two consecutive sources (2k, 2k+1) of a 32-source sub-chunk with their fields
+// interleaved, so that a 64-bit register pair holds one field of both (the
+// operand form of the sm_100 packed FP32 instructions).  The source grid is
+// stored in this form.  hi, lo: parts of the unit vector; p = -e1 w, q = -e2 w
+// (scalar-scalar kE w, kB w), K = (1 + m) w.
 struct __align__(16) SrcPairS {
   float4 hxy;  // hi.x0 hi.x1 hi.y0 hi.y1
   float4 hzp;  // hi.z0 hi.z1 p0 p1
@@ -217,8 +222,14 @@ struct __align__(16) SrcPairS {
   float4 wk;   // w0 w1 K0 K1
   float4 zz;   // z0 z1 0 0
 };
-static_assert(sizeof(SrcPairS) == 2 * sizeof(SrcRecS), "a SrcPairS rewrites two SrcRecS in place");
-
+// A sub-chunk as it lies in HBM and is copied into shared memory: the 3-D box
+// of its hi parts widened by 2^-23 per side (the hi/lo split of both ends moves
+// u_B - u_A by at most 2^-24), its {p, q, w, K} sums, its sources.
+struct __align__(16) ChunkS {
+  float4 mn, mx, sum;
+  SrcPairS src[kChunk / 2];
+};
+static_assert(sizeof(ChunkS) % 16 == 0, "copied in 16-byte units");
 // Source j of a sub-chunk in SrcPairS form, as a SrcRecS.
 __device__ __forceinline__ SrcRecS src_of_s(const SrcPairS* __restrict__ S, int j) {
   const float* f = reinterpret_cast<const float*>(S + (j >> 1)) + (j & 1);
@@ -227,19 +238,6 @@ __device__ __forceinline__ SrcRecS src_of_s(const SrcPairS* __restrict__ S, int 
   r.b = make_float4(f[8], f[10], f[12], f[14]);
   r.c = make_float4(f[16], f[18], f[20], 0.f);
   return r;
-}
-
-// One source in both halves of a SrcPairS (the odd last source of a sub-chunk;
-// the second half is masked out by the step that takes it).
-__device__ __forceinline__ SrcPairS dup_pair_s(const SrcRecS& r) {
-  SrcPairS p;
-  p.hxy = make_float4(r.a.x, r.a.x, r.a.y, r.a.y);
-  p.hzp = make_float4(r.a.z, r.a.z, r.a.w, r.a.w);
-  p.lxy = make_float4(r.b.x, r.b.x, r.b.y, r.b.y);
-  p.lzq = make_float4(r.b.z, r.b.z, r.b.w, r.b.w);
-  p.wk = make_float4(r.c.x, r.c.x, r.c.y, r.c.y);
-  p.zz = make_float4(r.c.z, r.c.z, 0.f, 0.f);
-  return p;
 }
 
 // A lens's constants in packed form: -hi, -lo and the east/north basis.
@@ -263,7 +261,9 @@ __device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, f
   const float2 dx = add2(add2(lo2(s.hxy), L.nhx), add2(lo2(s.lxy), L.nlx));
   const float2 dy = add2(add2(hi2(s.hxy), L.nhy), add2(hi2(s.lxy), L.nly));
   const float2 dz = add2(add2(lo2(s.hzp), L.nhz), add2(lo2(s.lzq), L.nlz));
-  d2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+  // series path (log bins): d2 = 0 is below the first edge; the offsets only keep
+  // its masked terms finite
+  d2 = fma2(dz, dz, fma2(dy, dy, SMALL ? fma2(dx, dx, dup2(1e-30f)) : mul2(dx, dx)));
   if (SMALL) {
     const float2 c = mul2(d2, make_float2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y)));
     th = mul2(c, fma2(d2, fma2(d2, fma2(d2, dup2(6.9754464e-4f), dup2(4.6875e-3f)), dup2(4.16666679e-2f)),
@@ -274,7 +274,7 @@ __device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, f
   if (MODE == 0) {
     const float2 A = fma2(dy, L.ey, mul2(dx, L.ex));
     const float2 B = fma2(dz, L.nz, fma2(dy, L.ny, mul2(dx, L.nx)));
-    const float2 A2 = mul2(A, A);
+    const float2 A2 = SMALL ? fma2(A, A, dup2(1e-30f)) : mul2(A, A);
     const float2 P = fma2(make_float2(-B.x, -B.y), B, A2);
     const float2 sq = fma2(B, B, A2);
     const float2 ab = mul2(A, B);
@@ -304,32 +304,36 @@ __device__ __forceinline__ void sph_acc_zero(SphAcc<NE>& A) {
   for (int e = 0; e < NE; ++e) A.hgt[e] = A.hgx[e] = A.hw[e] = A.hdw[e] = A.hk[e] = A.hn[e] = dup2(0.f);
 }
 
-// The two pairs of one SrcPairS against a lens (TAIL: only the first; the
-// second half is a copy, masked out).  With a z cut a pair with z_A > z_B
+// The two pairs of one SrcPairS against a lens; in a partial sub-chunk (PART)
+// a0, a1 tell which of the two belong to the row span.  With a z cut a pair with z_A > z_B
 // (src/tpcf.f90:322) adds nothing.  For each of the NE edges the upper-side
 // sums are formed too (pairs with d2 >= E, the side a 1.0/0.0 mask from one FP32
 // compare at Ehi = E (1 + eps), applied by multiplication), and the pairs
 // between Elo = E (1 - eps) and Ehi, inside the guard band, are counted (A.nc).
 // Without a z cut the w and K sums of all pairs (and, scalar-scalar, the g sums)
 // are the sub-chunk's totals, so they are not accumulated here.
-template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NE, bool TAIL>
-__device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPairS& s, const float* Elo,
-                                         const float* Ehi, SphAcc<NE>& A) {
-  constexpr bool LI = !HAS_Z;
+template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NE, bool PART>
+__device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPairS& s, bool a0, bool a1,
+                                         const float* Elo, const float* Ehi, SphAcc<NE>& A) {
+  constexpr bool LI = !(HAS_Z || PART);
   float2 d2, th, r, X, Y;
   sph_terms2<MODE, SMALL>(L, s, d2, th, r, X, Y);
   float2 w = lo2(s.wk), K = hi2(s.wk);
-  bool v0 = true, v1 = !TAIL;
+  bool v0 = true, v1 = true;
   if (HAS_Z) {
     v0 = lz <= s.zz.x;
-    v1 = v1 && lz <= s.zz.y;
+    v1 = lz <= s.zz.y;
+  }
+  if (PART) {
+    v0 = v0 && a0;
+    v1 = v1 && a1;
   }
   const float2 vm = make_float2(v0 ? 1.f : 0.f, v1 ? 1.f : 0.f);
-  if (HAS_Z || TAIL) {
+  if (!LI) {
     r = mul2(r, vm);
     w = mul2(w, vm);
     if (MODE == 0 && HAS_M) K = mul2(K, vm);
-    if (HAS_Z) A.sn = add2(A.sn, vm);
+    A.sn = add2(A.sn, vm);
   }
   if (!(LI && MODE == 1)) {
     A.sgt = fma2(r, X, A.sgt);
@@ -342,7 +346,7 @@ __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPai
   for (int e = 0; e < NE; ++e) {
     float2 mh = make_float2(d2.x >= Ehi[e] ? 1.f : 0.f, d2.y >= Ehi[e] ? 1.f : 0.f);
     const float2 ml = make_float2(d2.x >= Elo[e] ? 1.f : 0.f, d2.y >= Elo[e] ? 1.f : 0.f);
-    if (HAS_Z || TAIL) {
+    if (!LI) {
       A.nc = fma2(add2(ml, make_float2(-mh.x, -mh.y)), vm, A.nc);
       mh = mul2(mh, vm);
     } else {
@@ -360,39 +364,45 @@ __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPai
 }
 
 // Sums over all pairs of a sub-chunk; ss = {sum p, sum q, sum w, sum K}.
-template <int MODE, bool HAS_M, bool HAS_Z, int QA, int NE>
-__device__ __forceinline__ void sph_totals(const SphAcc<NE>& A, int cnt, const float4 ss, float* tot) {
-  constexpr bool LI = !HAS_Z;
+template <int MODE, bool HAS_M, bool LI, int QA, int NE>
+__device__ __forceinline__ void sph_totals(const SphAcc<NE>& A, const float4 ss, float* tot) {
   tot[QGT] = (LI && MODE == 1) ? ss.x : sum2(A.sgt);
   tot[QGX] = (LI && MODE == 1) ? ss.y : sum2(A.sgx);
   tot[QW] = LI ? ss.z : sum2(A.sw);
   tot[QDW] = sum2(A.sdw);
-  tot[QN] = HAS_Z ? sum2(A.sn) : (float)cnt;
+  tot[QN] = LI ? (float)kChunk : sum2(A.sn);
   if (MODE == 0 && HAS_M) tot[QK] = LI ? ss.w : sum2(A.sk);
 }
 
+// The sources [lo, hi) of a sub-chunk (all 32 unless PART) against a lens.
+template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NE>
+__device__ __forceinline__ void sph_loop(const SrcPairS* __restrict__ S, int lo, int hi, const LensS2& L, float lz,
+                                         const float* Elo, const float* Ehi, SphAcc<NE>& A) {
+  const int k0 = PART ? lo >> 1 : 0, k1 = PART ? (hi + 1) >> 1 : kChunk / 2;
+#pragma unroll 2
+  for (int k = k0; k < k1; ++k)
+    sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, PART>(L, lz, S[k], !PART || 2 * k >= lo, !PART || 2 * k + 1 < hi, Elo, Ehi,
+                                                  A);
+}
+
 // Class 1: every pair of the chunk is in bin `blo`.
-template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NC, int QA>
-__device__ __forceinline__ void chunk_single_s(const SrcPairS* __restrict__ S, int cnt, const LensS2& L, float lz,
-                                               int cls, int blo, float* __restrict__ hcol, const float4 ss) {
+template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NC, int QA>
+__device__ __forceinline__ void chunk_single_s(const SrcPairS* __restrict__ S, int lo, int hi, const LensS2& L,
+                                               float lz, int cls, int blo, float* __restrict__ hcol, const float4 ss) {
   SphAcc<0> A;
   sph_acc_zero(A);
-  const int np = cnt >> 1;
-#pragma unroll 2
-  for (int k = 0; k < np; ++k) sph_step<MODE, HAS_M, HAS_Z, SMALL, 0, false>(L, lz, S[k], nullptr, nullptr, A);
-  if (cnt & 1)
-    sph_step<MODE, HAS_M, HAS_Z, SMALL, 0, true>(L, lz, dup_pair_s(src_of_s(S, cnt - 1)), nullptr, nullptr, A);
+  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, 0>(S, lo, hi, L, lz, nullptr, nullptr, A);
   if (cls != 1) return;
   float acc[QA];
-  sph_totals<MODE, HAS_M, HAS_Z, QA>(A, cnt, ss, acc);
+  sph_totals<MODE, HAS_M, !(HAS_Z || PART), QA>(A, ss, acc);
   hist_add<QA, NC>(hcol, blo, acc);
 }
 
 // Classes 2 and 3: pairs in bins blo .. blo + NE across NE = 1 or 2 edges (a bin
 // outside [0, nb) is dropped); edge e is e2f[blo + 1 + e].  Bin blo + j receives
 // h[j-1] - h[j] with h[-1] = all and h[NE] = 0, as in the planar kernel.
-template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NC, int QA, int NE>
-__device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, int cnt, const LensS& Lf,
+template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NC, int QA, int NE>
+__device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, int lo, int hi, const LensS& Lf,
                                               const LensS2& L, float lz, int cls, int blo, float* __restrict__ hcol,
                                               const BinCtx& C, const float4 ss) {
   float Elo[NE], Ehi[NE];
@@ -405,18 +415,14 @@ __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, in
   }
   SphAcc<NE> A;
   sph_acc_zero(A);
-  const int np = cnt >> 1;
-#pragma unroll 2
-  for (int k = 0; k < np; ++k) sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, false>(L, lz, S[k], Elo, Ehi, A);
-  if (cnt & 1)
-    sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, true>(L, lz, dup_pair_s(src_of_s(S, cnt - 1)), Elo, Ehi, A);
+  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, NE>(S, lo, hi, L, lz, Elo, Ehi, A);
   if (cls == 0) return;
   if (sum2(A.nc) != 0.f) {  // rare: a pair inside the guard band; the sub-chunk is binned pair by pair
-    for (int j = 0; j < cnt; ++j) do_pair_s<MODE, HAS_M, HAS_Z, SMALL, SMALL, NC, QA>(Lf, lz, src_of_s(S, j), hcol, C);
+    for (int j = lo; j < hi; ++j) do_pair_s<MODE, HAS_M, HAS_Z, SMALL, SMALL, NC, QA>(Lf, lz, src_of_s(S, j), hcol, C);
     return;
   }
   float prev[QA];
-  sph_totals<MODE, HAS_M, HAS_Z, QA>(A, cnt, ss, prev);
+  sph_totals<MODE, HAS_M, !(HAS_Z || PART), QA>(A, ss, prev);
 #pragma unroll
   for (int j = 0; j <= NE; ++j) {
     float up[QA];
@@ -444,15 +450,8 @@ __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, in
 
 // ------------------------------------------------------------ cell runs -----
 constexpr float kTwoPiF = 6.28318548f;      // 2 pi rounded up to FP32
-constexpr int kRowsS = kMaxRows / 4;        // rows per chunk: 3 runs each fit kMaxRows
-#ifndef TPCF_SPH_TILE
-#define TPCF_SPH_TILE 160
-#endif
-// Sources per shared-memory tile (48-byte records): the tile size sets how
-// many blocks share an SM next to the FP32 histogram.
-constexpr int kTileS = TPCF_SPH_TILE;
-static_assert(kTileS % 32 == 0, "tiles hold whole 32-source sub-chunks");
-constexpr int kFlushSrcS = 4096;  // FP32 histogram -> FP64 after about this many sources
+constexpr int kRowsS = 10;  // rows whose (up to three) runs a warp holds at once: lane 3 r + j
+constexpr int kNbufS = 3;   // sub-chunks in flight per warp
 
 // Lambda reach of a work item: full = every cell of a row, else the interval
 // [box.x - dl, box.z + dl] modulo 2 pi.
@@ -496,73 +495,60 @@ __device__ __forceinline__ int sph_row_spans(const GridDesc& G, float4 box, floa
 }
 
 // ------------------------------------------------------------ the kernel ----
-struct SphSmem {
-  size_t tiles, hist, bsum, e2s, fvw, fw, e2f, span0, span1, tpref, subbox, subsum, mbar, misc, total;
+// Shared memory of one warp.
+struct SphWarpSmem {
+  size_t ring, hist, wsum, fvw, fw, mbar, total;
 };
-__host__ __device__ inline size_t align_up_s(size_t v, size_t a) { return (v + a - 1) / a * a; }
-__host__ __device__ inline SphSmem sph_smem_layout(int nb, int qa, int bt) {
-  SphSmem s;
+__host__ __device__ inline SphWarpSmem sph_warp_smem(int nb, int qa) {
+  SphWarpSmem s{};
   size_t o = 0;
-  s.tiles = o; o += 2 * kTileS * sizeof(SrcRecS);
-  s.hist = o;  o += (size_t)nb * qa * bt * sizeof(float);
-  o = align_up_s(o, 16);
-  s.bsum = o;  o += (size_t)kQ * nb * sizeof(double);
-  s.e2s = o;   o += (size_t)(nb + 1) * sizeof(double);
-  s.fvw = o;   o += (size_t)bt * sizeof(double);
-  s.fw = o;    o += (size_t)bt * sizeof(double);
-  s.e2f = o;   o += (size_t)(nb + 1) * sizeof(float);
-  o = align_up_s(o, 16);
-  s.span0 = o; o += kMaxRows * sizeof(int);
-  s.span1 = o; o += kMaxRows * sizeof(int);
-  s.tpref = o; o += (kMaxRows + 1) * sizeof(int);
-  o = align_up_s(o, 16);
-  s.subbox = o; o += 2 * (kTileS / 32) * sizeof(float4);
-  s.subsum = o; o += (kTileS / 32) * sizeof(float4);
-  s.mbar = o;  o += 2 * sizeof(uint64_t);
-  s.misc = o;  o += 16;
-  s.total = align_up_s(o, 128);
+  s.ring = o; o += kNbufS * sizeof(ChunkS);
+  s.hist = o; o += (size_t)nb * qa * 32 * sizeof(float);
+  s.wsum = o; o += (size_t)kQ * nb * sizeof(double);
+  s.fvw = o;  o += 32 * sizeof(double);
+  s.fw = o;   o += 32 * sizeof(double);
+  s.mbar = o; o += kNbufS * sizeof(uint64_t);
+  s.total = (o + 15) / 16 * 16;
   return s;
 }
+__host__ __device__ inline size_t sph_edge_smem(int nb) { return ((size_t)(nb + 1) * 12 + 15) / 16 * 16; }
 
-// Persistent: each block takes (task, lens group) items from the queue and
-// streams the item's source runs through shared memory (bulk copies,
-// double-buffered, bounded waits), as the planar kernel does.
-template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB, int BT>
-// Compiled for 3 blocks per SM (the shared-memory occupancy at 20 bins),
-// which gives the compiler a register budget of up to 170 per thread.
-__global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
+// Persistent, every warp on its own as in the planar kernel: it takes items of
+// 32 lenses from the queue and streams the sub-chunks of the item's source runs
+// through its own ring of buffers (bulk copies, bounded waits).  The tiles were
+// copied for a block of 128 lenses and rewritten into pair form there, between
+// two barriers (barrier stall 1.1 per issued instruction).  Twelve warps per SM
+// (the shared-memory occupancy at 20 bins), up to 168 registers.
+// 100 k x 500 k on the sky, theta_max 200': SKYNOW.
+template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB>
+__global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
   constexpr int QA = (MODE == 0 && HAS_M) ? 6 : 5;
-  constexpr int NW = BT / 32;
   constexpr bool SMALL = LOGB;  // log spacing on the sphere is only chosen with chord(x_max) <= 0.25
   const int nb = P.nb;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   extern __shared__ __align__(128) unsigned char smem[];
-  const SphSmem Ls = sph_smem_layout(nb, QA, BT);
-  SrcRecS* tiles = reinterpret_cast<SrcRecS*>(smem + Ls.tiles);
-  float* hist = reinterpret_cast<float*>(smem + Ls.hist);
-  double* bsum = reinterpret_cast<double*>(smem + Ls.bsum);
-  double* e2s = reinterpret_cast<double*>(smem + Ls.e2s);
-  double* fvw = reinterpret_cast<double*>(smem + Ls.fvw);
-  double* fw = reinterpret_cast<double*>(smem + Ls.fw);
-  float* e2f = reinterpret_cast<float*>(smem + Ls.e2f);
-  int* span0 = reinterpret_cast<int*>(smem + Ls.span0);
-  int* span1 = reinterpret_cast<int*>(smem + Ls.span1);
-  int* tpref = reinterpret_cast<int*>(smem + Ls.tpref);
-  float4* subbox = reinterpret_cast<float4*>(smem + Ls.subbox);
-  float4* subsum = reinterpret_cast<float4*>(smem + Ls.subsum);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + Ls.mbar);
-  int* sh_item = reinterpret_cast<int*>(smem + Ls.misc);
+  double* e2s = reinterpret_cast<double*>(smem);
+  float* e2f = reinterpret_cast<float*>(e2s + nb + 1);
+  const SphWarpSmem W = sph_warp_smem(nb, QA);
+  unsigned char* wb = smem + sph_edge_smem(nb) + (size_t)warp * W.total;
+  ChunkS* ring = reinterpret_cast<ChunkS*>(wb + W.ring);
+  float* hist = reinterpret_cast<float*>(wb + W.hist);
+  double* wsum = reinterpret_cast<double*>(wb + W.wsum);
+  double* fvw = reinterpret_cast<double*>(wb + W.fvw);
+  double* fw = reinterpret_cast<double*>(wb + W.fw);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(wb + W.mbar);
 
-  if (tid == 0) {
-    mbar_init(&mbar[0], 1);
-    mbar_init(&mbar[1], 1);
+  if (lane == 0) {
+    for (int b = 0; b < kNbufS; ++b) mbar_init(&full_bar[b], 1);
     mbar_fence_init();
   }
-  for (int i = tid; i <= nb; i += BT) {
+  for (int i = tid; i <= nb; i += blockDim.x) {
     e2s[i] = P.e2[i];
     e2f[i] = P.e2f[i];
   }
+  float* __restrict__ hcol = hist + lane;
+  for (int e = 0; e < nb * QA; ++e) hcol[e * 32] = 0.f;
   __syncthreads();
   BinCtx C;
   C.A = P.binA; C.B = P.binB; C.eps = P.eps; C.one_m_eps = 1.f - P.eps;
@@ -571,44 +557,45 @@ __global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
   C.lo_g = e2f[0] * (1.f - P.eps);
   C.hi_g = e2f[nb] * (1.f + P.eps);
 
-  uint32_t phase = 0u;
-  uint32_t tcount = 0u;
-  bool timed_out = false;
-  float* __restrict__ hcol = hist + tid;
-  for (int e = 0; e < nb * QA; ++e) hcol[e * BT] = 0.f;
+  const uint32_t wait_limit = P.wait_limit ? P.wait_limit : kWaitPolls;
+  int ring_t = 0;        // ring index of the next sub-chunk this warp consumes
+  int issued_end = 0;    // ring index one past the last sub-chunk this warp issued
+  bool aborted = false;  // a bounded wait ran out: consume and issue nothing more
+  const int flush_src = P.flush_src > 0 ? P.flush_src : 4096;
 
-  for (;;) {
-    if (tid == 0) *sh_item = atomicAdd(P.queue_head, 1);
-    __syncthreads();
-    const int item = *sh_item;
+  while (!aborted) {
+    int item = 0;
+    if (lane == 0) item = atomicAdd(P.queue_head, 1);
+    item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= P.n_items) break;
     const int2 it = P.items[item];
     const TaskDesc T = P.tasks[it.x];
     const LensDesc LD = P.lenses[T.lens_cat];
     const GridDesc G = P.grids[T.src_cat];
+    const ChunkS* __restrict__ src = reinterpret_cast<const ChunkS*>(G.sph);
     const int g = it.y / T.split, part = it.y - g * T.split;  // this item's rows: every T.split-th
     const int gs = LD.group_start[g];
-    const int nl = LD.group_start[g + 1] - gs;
-    const bool act = tid < nl;
+    const bool act = lane < LD.group_start[g + 1] - gs;
     LensS Lf;
     float lz = 0.f;
     double vw = 0.0, w = 0.0;
     double* lens_col = nullptr;
     if (act) {
-      const float4 r = LD.rec[gs + tid];
-      Lf = lens_frame(LD.pos[2 * (gs + tid)], LD.pos[2 * (gs + tid) + 1]);
+      const float4 r = LD.rec[gs + lane];
+      Lf = lens_frame(LD.pos[2 * (gs + lane)], LD.pos[2 * (gs + lane) + 1]);
       vw = (double)r.z * (double)r.w;
       w = (double)r.w;
-      if (HAS_Z) lz = LD.z[gs + tid];
-      if (P.lens_acc && T.lens_acc_off >= 0) lens_col = P.lens_acc + T.lens_acc_off + (size_t)part * kQ * nb * LD.n_valid + gs + tid;
+      if (HAS_Z) lz = LD.z[gs + lane];
+      if (P.lens_acc && T.lens_acc_off >= 0)
+        lens_col = P.lens_acc + T.lens_acc_off + (size_t)part * kQ * nb * LD.n_valid + gs + lane;
     } else {
       Lf = lens_frame(make_float4(1.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f));
     }
     const LensS2 LP = lens_pack(Lf);
-    fvw[tid] = vw;
-    fw[tid] = w;
+    fvw[lane] = vw;
+    fw[lane] = w;
     const size_t lens_stride = (size_t)LD.n_valid;
-    for (int e = tid; e < kQ * nb; e += BT) bsum[e] = 0.0;
+    for (int e = lane; e < kQ * nb; e += 32) wsum[e] = 0.0;
     int since_flush = 0;
     const float4 box = LD.group_box[g];
     int cy0, cy1;
@@ -617,163 +604,105 @@ __global__ void __launch_bounds__(BT, 3) k_pairs_sph(const PairParams P) {
     bool full;
     sph_reach(G, box, P.R, T.margin, dl, full);
 
-    for (int c0 = cy0 + part; c0 <= cy1; c0 += kRowsS * T.split) {
-      const int nr = min(kRowsS, (cy1 - c0) / T.split + 1);
-      const int ns = 3 * nr;
-      __syncthreads();
-      for (int r = tid; r < nr; r += BT) {
+    for (int c0 = cy0 + part; c0 <= cy1 && !aborted; c0 += kRowsS * T.split) {
+      int s0 = 0, s1 = 0;
+      const int r = lane / 3, row = c0 + r * T.split;
+      if (r < kRowsS && row <= cy1) {
         int2 sp[3];
-        const int k = sph_row_spans(G, box, P.R, T.margin, c0 + r * T.split, dl, full, sp);
+        const int k = sph_row_spans(G, box, P.R, T.margin, row, dl, full, sp);
+        const int j = lane - 3 * r;
+        if (j < k) {
+          const int2 v = j == 0 ? sp[0] : j == 1 ? sp[1] : sp[2];
+          s0 = v.x;
+          s1 = v.y > v.x ? v.y : v.x;
+        }
+      }
+      const int ntr = tiles_of_span<1>(s0, s1);
+      int incl = ntr;  // inclusive prefix of the sub-chunk counts over the lanes (runs)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const int2 v = j < k ? sp[j] : make_int2(0, 0);
-          span0[3 * r + j] = v.x;
-          span1[3 * r + j] = v.y > v.x ? v.y : v.x;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int ntiles = __shfl_sync(0xffffffffu, incl, 31);
+      auto issue = [&](int k) {
+        const TileGeom tg = tile_of<1>(k, incl, ntr, s0, s1);
+        const int t = ring_t + k;
+        issued_end = t + 1;
+        if (t + 1 == P.debug_skip_tile) return;  // fault injection (tests): this copy never lands
+        if (lane == 0) {
+          const int b = t % kNbufS;
+          mbar_arrive_tx(&full_bar[b], (uint32_t)sizeof(ChunkS));
+          bulk_g2s(ring + b, src + tg.c0, (uint32_t)sizeof(ChunkS), &full_bar[b]);
         }
-      }
-      __syncthreads();
-      if (tid == 0) {
-        int acc = 0;
-        for (int r = 0; r < ns; ++r) {
-          tpref[r] = acc;
-          acc += (span1[r] - span0[r] + kTileS - 1) / kTileS;
-        }
-        tpref[ns] = acc;
-      }
-      __syncthreads();
-      const int ntiles = tpref[ns];
-      int rc = 0, ri = 0;
-      if (tid == 0 && ntiles > 0) {
-        while (tpref[ri + 1] <= 0) ++ri;
-        const int s0 = span0[ri];
-        const int n0 = min(kTileS, span1[ri] - s0);
-        const int bb = tcount & 1u;
-        mbar_arrive_tx(&mbar[bb], (uint32_t)(n0 * sizeof(SrcRecS)));
-        bulk_g2s(tiles + bb * kTileS, G.recs + s0, (uint32_t)(n0 * sizeof(SrcRecS)), &mbar[bb]);
-      }
+      };
+      for (int k = 0; k < kNbufS && k < ntiles; ++k) issue(k);
       for (int k = 0; k < ntiles; ++k) {
-        if (tid == 0 && k + 1 < ntiles) {
-          while (tpref[ri + 1] <= k + 1) ++ri;
-          const int s1 = span0[ri] + (k + 1 - tpref[ri]) * kTileS;
-          const int n1 = min(kTileS, span1[ri] - s1);
-          const int bb = (tcount + k + 1) & 1u;
-          mbar_arrive_tx(&mbar[bb], (uint32_t)(n1 * sizeof(SrcRecS)));
-          bulk_g2s(tiles + bb * kTileS, G.recs + s1, (uint32_t)(n1 * sizeof(SrcRecS)), &mbar[bb]);
+        const int t = ring_t + k;
+        const int b = t % kNbufS;
+        const TileGeom tg = tile_of<1>(k, incl, ntr, s0, s1);
+        const bool ok = __all_sync(0xffffffffu,
+                                   mbar_wait_bounded(&full_bar[b], (uint32_t)(t / kNbufS) & 1u, wait_limit));
+        if (!ok) {  // stop: drain this warp's copies in flight below, report the timeout
+          aborted = true;
+          ring_t = t;
+          break;
         }
-        while (tpref[rc + 1] <= k) ++rc;
-        const int s = span0[rc] + (k - tpref[rc]) * kTileS;
-        const int n = min(kTileS, span1[rc] - s);
-        const int bb = (tcount + k) & 1u;
-        const bool ok = mbar_wait_bounded(&mbar[bb], (phase >> bb) & 1u);
-        phase ^= (1u << bb);
-        // not __restrict__: the sub-chunk pass rewrites these bytes in place
-        const SrcRecS* S = tiles + bb * kTileS;
-        const int nsub = (n + 31) >> 5;
-        if (ok) {
-          // One warp per 32-source sub-chunk: its 3-D box, widened by 2^-23
-          // per side (the hi/lo split of both ends moves u_B - u_A by at most
-          // 2^-24), its sums of p, q, w, K, and the rewrite of its records
-          // into SrcPairS form (lanes 2k, 2k+1 trade halves with one shuffle
-          // round; each lane stores only the 48 bytes of its own record).
-          for (int sc = warp; sc < nsub; sc += NW) {
-            const int j = sc * 32 + lane;
-            float mnx = INFINITY, mny = INFINITY, mnz = INFINITY, mxx = -INFINITY, mxy = -INFINITY,
-                  mxz = -INFINITY;
-            const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            float4 a = z4, b = z4, c = z4;
-            if (j < n) {
-              a = S[j].a;
-              b = S[j].b;
-              c = S[j].c;
-              mnx = mxx = a.x;
-              mny = mxy = a.y;
-              mnz = mxz = a.z;
-            }
-            const bool odd = lane & 1;
-            // even lane keeps {hi.x, hi.y, hi.z, p, lo.x, lo.y} of both, odd lane {lo.z, q, w, K, z}
-            const float r0 = __shfl_xor_sync(0xffffffffu, odd ? a.x : b.z, 1);
-            const float r1 = __shfl_xor_sync(0xffffffffu, odd ? a.y : b.w, 1);
-            const float r2 = __shfl_xor_sync(0xffffffffu, odd ? a.z : c.x, 1);
-            const float r3 = __shfl_xor_sync(0xffffffffu, odd ? a.w : c.y, 1);
-            const float r4 = __shfl_xor_sync(0xffffffffu, odd ? b.x : c.z, 1);
-            const float r5 = __shfl_xor_sync(0xffffffffu, b.y, 1);
-            float4* dst = reinterpret_cast<float4*>(tiles + bb * kTileS + j);
-            if (!odd) {
-              dst[0] = make_float4(a.x, r0, a.y, r1);
-              dst[1] = make_float4(a.z, r2, a.w, r3);
-              dst[2] = make_float4(b.x, r4, b.y, r5);
-            } else {
-              dst[0] = make_float4(r0, b.z, r1, b.w);
-              dst[1] = make_float4(r2, c.x, r3, c.y);
-              dst[2] = make_float4(r4, c.z, 0.f, 0.f);
-            }
-            fence_proxy_async_smem();  // before the bulk copy that later refills this buffer
-            float s0 = a.w, s1 = b.w, s2 = c.x, s3 = c.y;
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-              s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-              s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-              s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-              s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-            }
-            if (lane == 0) subsum[sc] = make_float4(s0, s1, s2, s3);
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-              mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-              mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-              mnz = fminf(mnz, __shfl_xor_sync(0xffffffffu, mnz, o));
-              mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-              mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-              mxz = fmaxf(mxz, __shfl_xor_sync(0xffffffffu, mxz, o));
-            }
-            if (lane == 0) {
-              const float d = 1.1920929e-7f;
-              subbox[2 * sc] = make_float4(mnx - d, mny - d, mnz - d, 0.f);
-              subbox[2 * sc + 1] = make_float4(mxx + d, mxy + d, mxz + d, 0.f);
-            }
-          }
+        const ChunkS* ch = ring + b;
+        const SrcPairS* __restrict__ Sc = ch->src;
+        const int lo = tg.lo0, hi = tg.hiL;
+        const bool partial = lo > 0 || hi < kChunk;
+        int blo = 0;
+        const int cls = act ? classify_s<LOGB, HAS_Z>(Lf, ch->mn, ch->mx, C, blo) : 0;
+        const int m = (int)__reduce_max_sync(0xffffffffu, (unsigned)cls);
+        const float4 ss = ch->sum;
+        if (m == 1) {
+          if (partial)
+            chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, true, 32, QA>(Sc, lo, hi, LP, lz, cls, blo, hcol, ss);
+          else
+            chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, false, 32, QA>(Sc, 0, kChunk, LP, lz, cls, blo, hcol, ss);
+        } else if (m == 2) {
+          if (partial)
+            chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, true, 32, QA, 1>(Sc, lo, hi, Lf, LP, lz, cls, blo, hcol, C, ss);
+          else
+            chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, false, 32, QA, 1>(Sc, 0, kChunk, Lf, LP, lz, cls, blo, hcol, C,
+                                                                       ss);
+        } else if (m == 3) {
+          if (partial)
+            chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, true, 32, QA, 2>(Sc, lo, hi, Lf, LP, lz, cls, blo, hcol, C, ss);
+          else
+            chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, false, 32, QA, 2>(Sc, 0, kChunk, Lf, LP, lz, cls, blo, hcol, C,
+                                                                       ss);
+        } else if (m == 4 && act) {
+          for (int j = lo; j < hi; ++j)
+            do_pair_s<MODE, HAS_M, HAS_Z, LOGB, SMALL, 32, QA>(Lf, lz, src_of_s(Sc, j), hcol, C);
         }
-        if (__syncthreads_or(!ok)) timed_out = true;
-        if (!timed_out) {
-          for (int sc = 0; sc < nsub; ++sc) {
-            const int base = sc * 32;
-            const int cnt = min(32, n - base);
-            int blo = 0;
-            const int cls = act ? classify_s<LOGB, HAS_Z>(Lf, subbox[2 * sc], subbox[2 * sc + 1], C, blo) : 0;
-            const int m = (int)__reduce_max_sync(0xffffffffu, (unsigned)cls);
-            if (m == 0) continue;
-            const SrcPairS* __restrict__ Sc = reinterpret_cast<const SrcPairS*>(S + base);
-            if (m == 1) {
-              chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, BT, QA>(Sc, cnt, LP, lz, cls, blo, hcol, subsum[sc]);
-            } else if (m == 2) {
-              chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, BT, QA, 1>(Sc, cnt, Lf, LP, lz, cls, blo, hcol, C, subsum[sc]);
-            } else if (m == 3) {
-              chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, BT, QA, 2>(Sc, cnt, Lf, LP, lz, cls, blo, hcol, C, subsum[sc]);
-            } else if (act) {
-              for (int j = 0; j < cnt; ++j)
-                do_pair_s<MODE, HAS_M, HAS_Z, LOGB, SMALL, BT, QA>(Lf, lz, src_of_s(Sc, j), hcol, C);
-            }
-          }
-        }
-        since_flush += n;
-        if (since_flush >= (P.flush_src > 0 ? P.flush_src : kFlushSrcS)) {
-          flush_hist<QA, BT>(hist, bsum, fvw, fw, nb, lens_col, lens_stride);
+        since_flush += hi - lo;
+        __syncwarp();  // every lane is done reading buffer b
+        if (k + kNbufS < ntiles) issue(k + kNbufS);
+        if (since_flush >= flush_src) {
+          warp_fold<QA, 32>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, 0, lane);
           since_flush = 0;
         }
-        __syncthreads();
       }
-      tcount += (uint32_t)ntiles;
+      if (!aborted) ring_t += ntiles;
     }
-    flush_hist<QA, BT>(hist, bsum, fvw, fw, nb, lens_col, lens_stride);
-    __syncthreads();
+    if (aborted) break;
+    warp_fold<QA, 32>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, 0, lane);
     double* out = P.item_sums + (size_t)(T.item_base + it.y) * kQ * nb;
-    for (int e = tid; e < kQ * nb; e += BT) {
-      const int q = e / nb;
-      out[e] = (q == QK && QA == 5) ? bsum[e - (QK - QW) * nb] : bsum[e];
+    for (int e = lane; e < kQ * nb; e += 32) {
+      const int from = (e / nb == QK && QA == 5) ? e - (QK - QW) * nb : e;
+      out[e] = wsum[from];
     }
-    __syncthreads();
+    __syncwarp();
   }
-  if (timed_out && tid == 0) atomicOr(P.err, kErrTimeout);
+  if (aborted) {
+    // wait (bounded) for the copies this warp issued and did not consume, so that
+    // none is in flight when the block's shared memory is released
+    for (int t = ring_t; t < issued_end; ++t)
+      if (t + 1 != P.debug_skip_tile) mbar_wait_bounded(&full_bar[t % kNbufS], (uint32_t)(t / kNbufS) & 1u, wait_limit);
+    if (lane == 0) atomicOr(P.err, kErrTimeout);
+  }
 }
 
 // ------------------------------------------------------------ prep kernels --
@@ -789,30 +718,72 @@ __global__ void k_wrap_lambda(const float* __restrict__ x, long long n, float* o
   }
 }
 
-__global__ void k_src_gather_sph(const int* __restrict__ idx, int n_valid, int mode, const float* __restrict__ lam,
-                                 const float* __restrict__ phi, const float* __restrict__ z,
-                                 const float* __restrict__ f1, const float* __restrict__ f2,
-                                 const float* __restrict__ w, const float* __restrict__ m, SrcRecS* rec) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n_valid) return;
-  const int i = idx[s];
+// Cell-sorted sub-chunks: one warp per 32 sources (lanes 2k, 2k+1 trade halves
+// with one shuffle round).  Past the last source the last one is repeated; such
+// copies are outside every row span.
+__global__ void k_src_gather_sph(const int* __restrict__ idx, int n_valid, int n_chunks, int mode,
+                                 const float* __restrict__ lam, const float* __restrict__ phi,
+                                 const float* __restrict__ z, const float* __restrict__ f1,
+                                 const float* __restrict__ f2, const float* __restrict__ w,
+                                 const float* __restrict__ m, ChunkS* __restrict__ out) {
+  const int ch = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (ch >= n_chunks) return;  // whole warps
+  const int s = ch * kChunk + lane;
+  const bool real = s < n_valid;
+  const int i = idx[real ? s : n_valid - 1];
   const float wi = w[i];
-  float4 hi, lo;
-  canon_unit(lam[i], phi[i], hi, lo);
-  SrcRecS r;
+  float4 a, b;
+  canon_unit(lam[i], phi[i], a, b);
+  float K = wi, zi = 0.f;
   if (mode == 0) {
-    hi.w = -(f1[i] * wi);
-    lo.w = -(f2[i] * wi);
-    const float mi = m ? m[i] : 0.f;
-    r.c = make_float4(wi, wi * (1.0f + mi), z ? z[i] : 0.f, 0.f);
+    a.w = -(f1[i] * wi);
+    b.w = -(f2[i] * wi);
+    K = wi * (1.0f + (m ? m[i] : 0.f));
+    zi = z ? z[i] : 0.f;
   } else {
-    hi.w = f1[i] * wi;
-    lo.w = f2[i] * wi;
-    r.c = make_float4(wi, wi, 0.f, 0.f);
+    a.w = f1[i] * wi;
+    b.w = f2[i] * wi;
   }
-  r.a = hi;
-  r.b = lo;
-  rec[s] = r;
+  const bool odd = lane & 1;
+  // even lane keeps {hi.x, hi.y, hi.z, p, lo.x, lo.y} of both, odd lane {lo.z, q, w, K, z}
+  const float r0 = __shfl_xor_sync(0xffffffffu, odd ? a.x : b.z, 1);
+  const float r1 = __shfl_xor_sync(0xffffffffu, odd ? a.y : b.w, 1);
+  const float r2 = __shfl_xor_sync(0xffffffffu, odd ? a.z : wi, 1);
+  const float r3 = __shfl_xor_sync(0xffffffffu, odd ? a.w : K, 1);
+  const float r4 = __shfl_xor_sync(0xffffffffu, odd ? b.x : zi, 1);
+  const float r5 = __shfl_xor_sync(0xffffffffu, b.y, 1);
+  SrcPairS* dst = out[ch].src + (lane >> 1);
+  if (!odd) {
+    dst->hxy = make_float4(a.x, r0, a.y, r1);
+    dst->hzp = make_float4(a.z, r2, a.w, r3);
+    dst->lxy = make_float4(b.x, r4, b.y, r5);
+  } else {
+    dst->lzq = make_float4(r0, b.z, r1, b.w);
+    dst->wk = make_float4(r2, wi, r3, K);
+    dst->zz = make_float4(r4, zi, 0.f, 0.f);
+  }
+  float s0 = real ? a.w : 0.f, s1 = real ? b.w : 0.f, s2 = real ? wi : 0.f, s3 = real ? K : 0.f;
+  float mnx = a.x, mny = a.y, mnz = a.z, mxx = a.x, mxy = a.y, mxz = a.z;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+    mnx = fminf(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
+    mny = fminf(mny, __shfl_xor_sync(0xffffffffu, mny, o));
+    mnz = fminf(mnz, __shfl_xor_sync(0xffffffffu, mnz, o));
+    mxx = fmaxf(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
+    mxy = fmaxf(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
+    mxz = fmaxf(mxz, __shfl_xor_sync(0xffffffffu, mxz, o));
+  }
+  if (lane == 0) {
+    const float d = 1.1920929e-7f;
+    out[ch].mn = make_float4(mnx - d, mny - d, mnz - d, 0.f);
+    out[ch].mx = make_float4(mxx + d, mxy + d, mxz + d, 0.f);
+    out[ch].sum = make_float4(s0, s1, s2, s3);
+  }
 }
 
 // Unit vectors (hi, lo) of the sorted lenses; perm[s] = input index.
@@ -868,49 +839,44 @@ __global__ void k_item_cost_sph(const int2* __restrict__ ranges, int n_ranges, i
 }
 
 // --------------------------------------------------------- host launchers --
-template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB, int BT>
+template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB>
 static cudaError_t launch_sph_t(const PairParams& P, int num_sms, cudaStream_t st, int* grid_out) {
   constexpr int QA = (MODE == 0 && HAS_M) ? 6 : 5;
-  const size_t smem = sph_smem_layout(P.nb, QA, BT).total;
-  auto kern = k_pairs_sph<MODE, HAS_M, HAS_Z, LOGB, BT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t per = sph_warp_smem(P.nb, QA).total;
+  const int bt = sph_edge_smem(P.nb) + 2 * per <= 113 * 1024 ? 64 : 32;  // two blocks per SM at least
+  const size_t smem = sph_edge_smem(P.nb) + per * (bt / 32);
+  auto kern = k_pairs_sph<MODE, HAS_M, HAS_Z, LOGB>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BT, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  int grid = per_sm * num_sms;
-  if (grid > P.n_items) grid = P.n_items;
-  if (grid < 1) grid = 1;
+  const int need = (P.n_items + bt / 32 - 1) / (bt / 32);  // each warp takes items of its own
+  const int grid = max(1, min(per_sm * num_sms, need));
   *grid_out = grid;
-  kern<<<grid, BT, smem, st>>>(P);
+  kern<<<grid, bt, smem, st>>>(P);
   return cudaGetLastError();
 }
 
-template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB>
-static cudaError_t launch_sph_bt(const PairParams& P, int bt, int num_sms, cudaStream_t st, int* grid) {
-  if (bt == 128) return launch_sph_t<MODE, HAS_M, HAS_Z, LOGB, 128>(P, num_sms, st, grid);
-  if (bt == 64) return launch_sph_t<MODE, HAS_M, HAS_Z, LOGB, 64>(P, num_sms, st, grid);
-  return launch_sph_t<MODE, HAS_M, HAS_Z, LOGB, 32>(P, num_sms, st, grid);
+cudaError_t launch_pairs_sph(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int num_sms,
+                             cudaStream_t st, int* grid) {
+  if (mode == 1)
+    return logb ? launch_sph_t<1, false, false, true>(P, num_sms, st, grid)
+                : launch_sph_t<1, false, false, false>(P, num_sms, st, grid);
+  if (has_m) {
+    if (has_z) return logb ? launch_sph_t<0, true, true, true>(P, num_sms, st, grid)
+                           : launch_sph_t<0, true, true, false>(P, num_sms, st, grid);
+    return logb ? launch_sph_t<0, true, false, true>(P, num_sms, st, grid)
+                : launch_sph_t<0, true, false, false>(P, num_sms, st, grid);
+  }
+  if (has_z) return logb ? launch_sph_t<0, false, true, true>(P, num_sms, st, grid)
+                         : launch_sph_t<0, false, true, false>(P, num_sms, st, grid);
+  return logb ? launch_sph_t<0, false, false, true>(P, num_sms, st, grid)
+              : launch_sph_t<0, false, false, false>(P, num_sms, st, grid);
 }
 
-cudaError_t launch_pairs_sph(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int bt, int num_sms,
-                             cudaStream_t st, int* grid) {
-  if (mode == 1) {
-    return logb ? launch_sph_bt<1, false, false, true>(P, bt, num_sms, st, grid)
-                : launch_sph_bt<1, false, false, false>(P, bt, num_sms, st, grid);
-  }
-  if (has_m) {
-    if (has_z) return logb ? launch_sph_bt<0, true, true, true>(P, bt, num_sms, st, grid)
-                           : launch_sph_bt<0, true, true, false>(P, bt, num_sms, st, grid);
-    return logb ? launch_sph_bt<0, true, false, true>(P, bt, num_sms, st, grid)
-                : launch_sph_bt<0, true, false, false>(P, bt, num_sms, st, grid);
-  }
-  if (has_z) return logb ? launch_sph_bt<0, false, true, true>(P, bt, num_sms, st, grid)
-                         : launch_sph_bt<0, false, true, false>(P, bt, num_sms, st, grid);
-  return logb ? launch_sph_bt<0, false, false, true>(P, bt, num_sms, st, grid)
-              : launch_sph_bt<0, false, false, false>(P, bt, num_sms, st, grid);
-}
+size_t sph_src_bytes(int n_valid) { return sizeof(ChunkS) * (size_t)max((n_valid + kChunk - 1) / kChunk, 1); }
 
 static inline unsigned gdim_s(long long n, int b) {
   long long g = (n + b - 1) / b;
@@ -925,9 +891,11 @@ cudaError_t launch_wrap_lambda(const float* x, long long n, float* out, cudaStre
 }
 cudaError_t launch_src_gather_sph(const int* idx, int n_valid, int mode, const float* lam, const float* phi,
                                   const float* z, const float* f1, const float* f2, const float* w, const float* m,
-                                  SrcRecS* rec, cudaStream_t st) {
-  if (n_valid > 0)
-    k_src_gather_sph<<<(n_valid + 255) / 256, 256, 0, st>>>(idx, n_valid, mode, lam, phi, z, f1, f2, w, m, rec);
+                                  void* out, cudaStream_t st) {
+  const int n_chunks = (n_valid + kChunk - 1) / kChunk;
+  if (n_chunks > 0)
+    k_src_gather_sph<<<(n_chunks + 7) / 8, 256, 0, st>>>(idx, n_valid, n_chunks, mode, lam, phi, z, f1, f2, w, m,
+                                                          static_cast<ChunkS*>(out));
   return cudaGetLastError();
 }
 cudaError_t launch_lens_pos_sph(const int* perm, int n_valid, const float* lam, const float* phi, float4* pos,

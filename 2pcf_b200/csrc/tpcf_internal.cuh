@@ -65,19 +65,8 @@ struct __align__(16) ChunkMeta {
   float4 sum;  // {sum p, sum q, sum w, sum K} over its real sources
 };
 
-// A source on the sphere: the unit vector u of (lambda, phi) split into FP32
-// hi + lo parts (u = hi + lo to ~2^-48), so that u_B - u_A keeps full FP32
-// relative precision at small separations.  Shear: a = {hi, -e1*w},
-// b = {lo, -e2*w}, c = {w, (1+m)*w, z, 0}; scalar-scalar: a = {hi, kE*w},
-// b = {lo, kB*w}, c = {w, w, 0, 0}.
-struct __align__(16) SrcRecS {
-  float4 a;
-  float4 b;
-  float4 c;
-};
-
 // Cell grid of one source catalogue.  Planar: cells over (x, y).  Sphere:
-// cells over (lambda reduced to [0, 2 pi), phi), records in `recs`.
+// cells over (lambda reduced to [0, 2 pi), phi), sub-chunks in `sph`.
 struct GridDesc {
   float x0, y0, cell, inv_cell;
   int ncx, ncy;
@@ -85,7 +74,7 @@ struct GridDesc {
   int pad;
   const int* cell_start;  // [ncx*ncy + 1]
   const SrcRec* rec;      // [n_valid], sorted by cell (lens grid of the adjoint)
-  const SrcRecS* recs;    // [n_valid], sorted by cell (sphere), else nullptr
+  const void* sph;        // sphere: ChunkS [ceil(n_valid/32)] (sphere.cu), sorted by cell, else nullptr
   const SrcPair* pairs;   // planar sources: [ceil(n_valid/32) * 16] in sub-chunk form
   const ChunkMeta* meta;  // [ceil(n_valid/32)]
   const float* series;    // sub-chunk records with moments (k_pairs_series), else nullptr

@@ -35,13 +35,14 @@ cudaError_t launch_src_series(const int* idx, int n_valid, int mode, bool has_m,
                               const float* m, float* rec, cudaStream_t st);
 cudaError_t launch_prepared(const PairLaunch& L, const PairParams& P, cudaStream_t st);
 
-// Spherical pair kernel (sphere.cu); P.grids[*].recs and P.lenses[*].pos set.
-cudaError_t launch_pairs_sph(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int bt, int num_sms,
+// Spherical pair kernel (sphere.cu); P.grids[*].sph and P.lenses[*].pos set.
+cudaError_t launch_pairs_sph(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int num_sms,
                              cudaStream_t st, int* grid);
+size_t sph_src_bytes(int n_valid);
 cudaError_t launch_wrap_lambda(const float* x, long long n, float* out, cudaStream_t st);
 cudaError_t launch_src_gather_sph(const int* idx, int n_valid, int mode, const float* lam, const float* phi,
                                   const float* z, const float* f1, const float* f2, const float* w, const float* m,
-                                  SrcRecS* rec, cudaStream_t st);
+                                  void* out, cudaStream_t st);
 cudaError_t launch_lens_pos_sph(const int* perm, int n_valid, const float* lam, const float* phi, float4* pos,
                                 cudaStream_t st);
 cudaError_t launch_unit_vectors(const float* lam, const float* phi, long long n, float* hi, float* lo,
