@@ -283,12 +283,12 @@ __device__ __forceinline__ void chunk_single(const SrcPair* __restrict__ S, int 
 // NE = 1 or 2 edges (a bin outside [0, nb) is dropped); edge e is
 // e2f[blo + 1 + e].  Sums over all pairs (s*) and, per edge, over the pairs on
 // its far side (h*[e]: d2 >= E_e); bin blo + j receives h[j-1] - h[j] with
-// h[-1] = all and h[NE] = 0.  The side of a pair is a 1.0/0.0 mask from one
-// FP32 compare, applied by multiplication.  Each edge is tested at
-// E (1 - eps) and E (1 + eps): a pair between the two lies within the guard
-// band, and then this lane drops its register sums and bins the sub-chunk
-// pair by pair by the canonical rule (rare).  A lane with fewer edges than NE
-// (class 1, or class 2 in a class-3 warp) keeps 3e38 on its unused edges.
+// h[-1] = all and h[NE] = 0.  The side of a pair is a 1.0/0.0 mask from the sign
+// of d2 - E, applied by multiplication.  The smallest |d2 - E| is kept per
+// edge: when it lies within the guard band, this lane drops its register sums
+// and bins the sub-chunk pair by pair by the canonical rule (rare).  A lane with fewer edges than NE
+// (class 1, or class 2 in a class-3 warp) keeps 3e38 on its unused edges (its
+// |d2 - E| is then 3e38 too: out of the band).
 template <int MODE, bool HAS_M, bool HAS_Z, bool PART, bool LOGB, int NC, int QA, int NE>
 __device__ __forceinline__ void chunk_edges(const SrcPair* __restrict__ S, int lo, int hi, const LensP& L, float lx,
                                             float ly, float lz, int cls, int blo, float* __restrict__ hcol,
@@ -297,15 +297,12 @@ __device__ __forceinline__ void chunk_edges(const SrcPair* __restrict__ S, int l
   constexpr bool LI = !MK;
   float2 sgt = dup2(0.f), sgx = dup2(0.f), sw = dup2(0.f), sdw = dup2(0.f), sk = dup2(0.f), sn = dup2(0.f);
   float2 hgt[NE], hgx[NE], hw[NE], hdw[NE], hk[NE], hn[NE];
-  float Elo[NE], Ehi[NE];
-  float2 nc = dup2(0.f);  // pairs inside a guard band (counted, masked)
+  float E[NE], close[NE];  // edges and the smallest |d2 - E|
 #pragma unroll
   for (int e = 0; e < NE; ++e) {
     hgt[e] = hgx[e] = hw[e] = hdw[e] = hk[e] = hn[e] = dup2(0.f);
-    const bool on = e < cls - 1;
-    const float E = C.e2f[min(max(blo + 1 + e, 0), C.nb)];
-    Elo[e] = on ? E * (1.f - C.eps_rel) : 3.0e38f;
-    Ehi[e] = on ? E * (1.f + C.eps_rel) : 3.0e38f;
+    E[e] = e < cls - 1 ? C.e2f[min(max(blo + 1 + e, 0), C.nb)] : 3.0e38f;
+    close[e] = 3.0e38f;
   }
   const int k0 = PART ? (lo >> 1) : 0;
   const int k1 = PART ? ((hi + 1) >> 1) : kChunk / 2;
@@ -334,14 +331,10 @@ __device__ __forceinline__ void chunk_edges(const SrcPair* __restrict__ S, int l
     if (MODE == 0 && HAS_M && !LI) sk = add2(sk, K);
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
-      float2 mh = make_float2(d2.x >= Ehi[e] ? 1.f : 0.f, d2.y >= Ehi[e] ? 1.f : 0.f);
-      const float2 ml = make_float2(d2.x >= Elo[e] ? 1.f : 0.f, d2.y >= Elo[e] ? 1.f : 0.f);
-      if (MK) {
-        nc = fma2(add2(ml, make_float2(-mh.x, -mh.y)), zm, nc);
-        mh = mul2(mh, zm);
-      } else {
-        nc = add2(nc, add2(ml, make_float2(-mh.x, -mh.y)));
-      }
+      const float2 t = add2(d2, dup2(-E[e]));
+      close[e] = fminf(close[e], fminf(fabsf(t.x), fabsf(t.y)));
+      float2 mh = make_float2(t.x >= 0.f ? 1.f : 0.f, t.y >= 0.f ? 1.f : 0.f);
+      if (MK) mh = mul2(mh, zm);
       const float2 rm = mul2(r, mh);
       const float2 wm = mul2(w, mh);
       hgt[e] = fma2(rm, X, hgt[e]);
@@ -353,7 +346,10 @@ __device__ __forceinline__ void chunk_edges(const SrcPair* __restrict__ S, int l
     }
   }
   if (cls == 0) return;
-  if (sum2(nc) != 0.f) {
+  bool band = false;
+#pragma unroll
+  for (int e = 0; e < NE; ++e) band = band || close[e] <= E[e] * C.eps_rel;
+  if (band) {
     for (int j = lo; j < hi; ++j) {
       float4 a, b;
       src_of(S, j, a, b);

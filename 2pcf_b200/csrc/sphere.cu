@@ -294,27 +294,27 @@ __device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, f
 // the upper side (h*).
 template <int NE>
 struct SphAcc {
-  float2 sgt, sgx, sw, sdw, sk, sn, nc;
+  float2 sgt, sgx, sw, sdw, sk, sn;
+  float close[NE ? NE : 1];  // smallest |d2 - E|
   float2 hgt[NE ? NE : 1], hgx[NE ? NE : 1], hw[NE ? NE : 1], hdw[NE ? NE : 1], hk[NE ? NE : 1], hn[NE ? NE : 1];
 };
 template <int NE>
 __device__ __forceinline__ void sph_acc_zero(SphAcc<NE>& A) {
-  A.sgt = A.sgx = A.sw = A.sdw = A.sk = A.sn = A.nc = dup2(0.f);
+  A.sgt = A.sgx = A.sw = A.sdw = A.sk = A.sn = dup2(0.f);
 #pragma unroll
-  for (int e = 0; e < NE; ++e) A.hgt[e] = A.hgx[e] = A.hw[e] = A.hdw[e] = A.hk[e] = A.hn[e] = dup2(0.f);
+  for (int e = 0; e < NE; ++e) A.close[e] = 3.0e38f, A.hgt[e] = A.hgx[e] = A.hw[e] = A.hdw[e] = A.hk[e] = A.hn[e] = dup2(0.f);
 }
 
 // The two pairs of one SrcPairS against a lens; in a partial sub-chunk (PART)
 // a0, a1 tell which of the two belong to the row span.  With a z cut a pair with z_A > z_B
 // (src/tpcf.f90:322) adds nothing.  For each of the NE edges the upper-side
-// sums are formed too (pairs with d2 >= E, the side a 1.0/0.0 mask from one FP32
-// compare at Ehi = E (1 + eps), applied by multiplication), and the pairs
-// between Elo = E (1 - eps) and Ehi, inside the guard band, are counted (A.nc).
+// sums are formed too (pairs with d2 >= E, the side a 1.0/0.0 mask from the sign
+// of d2 - E, applied by multiplication) and the smallest |d2 - E| is kept.
 // Without a z cut the w and K sums of all pairs (and, scalar-scalar, the g sums)
 // are the sub-chunk's totals, so they are not accumulated here.
 template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NE, bool PART>
 __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPairS& s, bool a0, bool a1,
-                                         const float* Elo, const float* Ehi, SphAcc<NE>& A) {
+                                         const float* E, SphAcc<NE>& A) {
   constexpr bool LI = !(HAS_Z || PART);
   float2 d2, th, r, X, Y;
   sph_terms2<MODE, SMALL>(L, s, d2, th, r, X, Y);
@@ -344,14 +344,10 @@ __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPai
   if (MODE == 0 && HAS_M && !LI) A.sk = add2(A.sk, K);
 #pragma unroll
   for (int e = 0; e < NE; ++e) {
-    float2 mh = make_float2(d2.x >= Ehi[e] ? 1.f : 0.f, d2.y >= Ehi[e] ? 1.f : 0.f);
-    const float2 ml = make_float2(d2.x >= Elo[e] ? 1.f : 0.f, d2.y >= Elo[e] ? 1.f : 0.f);
-    if (!LI) {
-      A.nc = fma2(add2(ml, make_float2(-mh.x, -mh.y)), vm, A.nc);
-      mh = mul2(mh, vm);
-    } else {
-      A.nc = add2(A.nc, add2(ml, make_float2(-mh.x, -mh.y)));
-    }
+    const float2 t = add2(d2, dup2(-E[e]));
+    A.close[e] = fminf(A.close[e], fminf(fabsf(t.x), fabsf(t.y)));
+    float2 mh = make_float2(t.x >= 0.f ? 1.f : 0.f, t.y >= 0.f ? 1.f : 0.f);
+    if (!LI) mh = mul2(mh, vm);
     const float2 rm = mul2(r, mh);  // r, w, K carry the validity mask already
     const float2 wm = mul2(w, mh);
     A.hgt[e] = fma2(rm, X, A.hgt[e]);
@@ -377,12 +373,11 @@ __device__ __forceinline__ void sph_totals(const SphAcc<NE>& A, const float4 ss,
 // The sources [lo, hi) of a sub-chunk (all 32 unless PART) against a lens.
 template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NE>
 __device__ __forceinline__ void sph_loop(const SrcPairS* __restrict__ S, int lo, int hi, const LensS2& L, float lz,
-                                         const float* Elo, const float* Ehi, SphAcc<NE>& A) {
+                                         const float* E, SphAcc<NE>& A) {
   const int k0 = PART ? lo >> 1 : 0, k1 = PART ? (hi + 1) >> 1 : kChunk / 2;
 #pragma unroll 2
   for (int k = k0; k < k1; ++k)
-    sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, PART>(L, lz, S[k], !PART || 2 * k >= lo, !PART || 2 * k + 1 < hi, Elo, Ehi,
-                                                  A);
+    sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, PART>(L, lz, S[k], !PART || 2 * k >= lo, !PART || 2 * k + 1 < hi, E, A);
 }
 
 // Class 1: every pair of the chunk is in bin `blo`.
@@ -391,7 +386,7 @@ __device__ __forceinline__ void chunk_single_s(const SrcPairS* __restrict__ S, i
                                                float lz, int cls, int blo, float* __restrict__ hcol, const float4 ss) {
   SphAcc<0> A;
   sph_acc_zero(A);
-  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, 0>(S, lo, hi, L, lz, nullptr, nullptr, A);
+  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, 0>(S, lo, hi, L, lz, nullptr, A);
   if (cls != 1) return;
   float acc[QA];
   sph_totals<MODE, HAS_M, !(HAS_Z || PART), QA>(A, ss, acc);
@@ -405,19 +400,18 @@ template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NC, int Q
 __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, int lo, int hi, const LensS& Lf,
                                               const LensS2& L, float lz, int cls, int blo, float* __restrict__ hcol,
                                               const BinCtx& C, const float4 ss) {
-  float Elo[NE], Ehi[NE];
+  float E[NE];
 #pragma unroll
-  for (int e = 0; e < NE; ++e) {  // lanes with fewer edges keep one no pair reaches
-    const bool on = e < cls - 1;
-    const float E = C.e2f[min(max(blo + 1 + e, 0), C.nb)];
-    Elo[e] = on ? E * (1.f - C.eps_rel) : 3.0e38f;
-    Ehi[e] = on ? E * (1.f + C.eps_rel) : 3.0e38f;
-  }
+  for (int e = 0; e < NE; ++e)  // lanes with fewer edges keep one no pair reaches
+    E[e] = e < cls - 1 ? C.e2f[min(max(blo + 1 + e, 0), C.nb)] : 3.0e38f;
   SphAcc<NE> A;
   sph_acc_zero(A);
-  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, NE>(S, lo, hi, L, lz, Elo, Ehi, A);
+  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, NE>(S, lo, hi, L, lz, E, A);
   if (cls == 0) return;
-  if (sum2(A.nc) != 0.f) {  // rare: a pair inside the guard band; the sub-chunk is binned pair by pair
+  bool band = false;
+#pragma unroll
+  for (int e = 0; e < NE; ++e) band = band || A.close[e] <= E[e] * C.eps_rel;
+  if (band) {  // rare: a pair inside the guard band; the sub-chunk is binned pair by pair
     for (int j = lo; j < hi; ++j) do_pair_s<MODE, HAS_M, HAS_Z, SMALL, SMALL, NC, QA>(Lf, lz, src_of_s(S, j), hcol, C);
     return;
   }
