@@ -200,6 +200,58 @@ __device__ __forceinline__ void adj_terms2(float2 nsx, float2 nsy, float sz, con
   Q = mul2(dx, dy);
 }
 
+// Sub-chunk sums of a source whose pairs cross up to NE bin edges (class cls = 1 +
+// its edges, lowest bin blo; a side outside [0, nb) contributes nothing): per edge
+// the sums over the pairs at or above it, by selects on the sign of d2 - E.  False
+// when a pair lies within the guard band of an edge (A is then not complete).
+template <bool HAS_Z, bool LOGB, bool WX, int NE>
+__device__ __forceinline__ bool adj_edges(const LensPair* __restrict__ Sc, int np, float2 nsx, float2 nsy, float sz,
+                                          int cls, int blo, const float4* coef, const BinCtx& C, float sum_w,
+                                          Acc& A) {
+  constexpr bool LI = !HAS_Z;
+  float E[NE], close[NE];
+  float2 T1 = dup2(0.f), T2 = dup2(0.f), TN = dup2(0.f), H1[NE], H2[NE], HN[NE];
+#pragma unroll
+  for (int e = 0; e < NE; ++e) {
+    E[e] = e < cls - 1 ? C.e2f[min(max(blo + 1 + e, 0), C.nb)] : 3.0e38f;
+    close[e] = 3.0e38f;
+    H1[e] = H2[e] = HN[e] = dup2(0.f);
+  }
+#pragma unroll 2
+  for (int q = 0; q < np; ++q) {
+    float2 d2, F, Pq, Q, w;
+    bool z0, z1;
+    adj_terms2<HAS_Z, LOGB>(nsx, nsy, sz, Sc[q], d2, F, Pq, Q, w, z0, z1);
+    T1 = fma2(F, Pq, T1);
+    T2 = fma2(F, Q, T2);
+    if (!LI) TN = add2(TN, w);
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const float2 dE = add2(d2, dup2(-E[e]));
+      close[e] = fminf(close[e], fminf(fabsf(dE.x), fabsf(dE.y)));
+      const bool u0 = dE.x >= 0.f, u1 = dE.y >= 0.f;
+      const float2 Fm = make_float2(u0 ? F.x : 0.f, u1 ? F.y : 0.f);  // F, w carry the z mask
+      H1[e] = fma2(Fm, Pq, H1[e]);
+      H2[e] = fma2(Fm, Q, H2[e]);
+      HN[e] = add2(HN[e], make_float2(u0 ? w.x : 0.f, u1 ? w.y : 0.f));
+    }
+  }
+  float p1 = sum2(T1), p2 = sum2(T2), pn = LI ? sum_w : sum2(TN);
+  bool band = false;
+#pragma unroll
+  for (int j = 0; j <= NE; ++j) {
+    const float h1 = j < NE ? sum2(H1[j < NE ? j : 0]) : 0.f, h2 = j < NE ? sum2(H2[j < NE ? j : 0]) : 0.f,
+                hn = j < NE ? sum2(HN[j < NE ? j : 0]) : 0.f;
+    const int bin = blo + j;
+    if (j <= cls - 1 && bin >= 0 && bin < C.nb) adj_apply<WX>(coef[bin], p1 - h1, p2 - h2, pn - hn, A);
+    p1 = h1;
+    p2 = h2;
+    pn = hn;
+    if (j < NE) band = band || close[j < NE ? j : 0] <= E[j < NE ? j : 0] * C.eps_rel;
+  }
+  return !band;
+}
+
 template <bool HAS_Z, bool LOGB, bool WX>
 __global__ void __launch_bounds__(BT, kAdjMinBlocks) k_adj(const AdjParams P) {
   constexpr int NW = BT / 32;
@@ -362,7 +414,7 @@ __global__ void __launch_bounds__(BT, kAdjMinBlocks) k_adj(const AdjParams P) {
             const int base = sc * 32;
             const int cnt = min(32, n - base);
             int blo = 0;
-            const int cls = act ? classify<LOGB, HAS_Z, true>(sx, sy, subbox[sc], C, blo) : 0;
+            const int cls = act ? classify_edges<LOGB>(sx, sy, subbox[sc], C, blo) : 0;
             const int m = (int)__reduce_max_sync(0xffffffffu, (unsigned)cls);
             if (m == 0) continue;
             const LensPair* __restrict__ Sc = reinterpret_cast<const LensPair*>(S + base);
@@ -385,60 +437,24 @@ __global__ void __launch_bounds__(BT, kAdjMinBlocks) k_adj(const AdjParams P) {
                 if (!LI) SN = add2(SN, w);
               }
               adj_apply<WX>(kc, sum2(S1), sum2(S2), LI ? subw[sc] : sum2(SN), Ac);
-            } else if (m == 2) {
-              const float4 kl = (cls >= 1 && blo >= 0) ? coef[blo] : make_float4(0.f, 0.f, 0.f, 0.f);
-              // a side outside [x_min, x_max] contributes nothing
-              const float4 kz = make_float4(0.f, 0.f, 0.f, 0.f);
-              const float4 kh = cls == 2 ? (blo + 1 < nb ? coef[blo + 1] : kz) : kl;
-              const float E = cls == 2 ? e2f[blo + 1] : 3.0e38f;
-              const float gE = cls == 2 ? E * C.eps_rel : 0.f;
-              const float2 nE = dup2(-E);
-              bool near = false;  // some pair lies within the guard band of E
-              float2 T1 = dup2(0.f), T2 = dup2(0.f), TN = dup2(0.f), H1 = dup2(0.f), H2 = dup2(0.f), HN = dup2(0.f);
-#pragma unroll 2
-              for (int q = 0; q < np; ++q) {
-                float2 d2, F, Pq, Q, w;
-                bool z0, z1;
-                adj_terms2<HAS_Z, LOGB>(nsx, nsy, sz, Sc[q], d2, F, Pq, Q, w, z0, z1);
-                const float2 dE = add2(d2, nE);
-                near |= fabsf(dE.x) <= gE;
-                near |= fabsf(dE.y) <= gE;
-                const bool u0 = z0 && d2.x >= E, u1 = z1 && d2.y >= E;
-                T1 = fma2(F, Pq, T1);
-                T2 = fma2(F, Q, T2);
-                if (!LI) TN = add2(TN, w);
-                const float2 Fm = make_float2(u0 ? F.x : 0.f, u1 ? F.y : 0.f);
-                H1 = fma2(Fm, Pq, H1);
-                H2 = fma2(Fm, Q, H2);
-                HN = add2(HN, make_float2(u0 ? w.x : 0.f, u1 ? w.y : 0.f));
-              }
-              const float h1 = sum2(H1), h2 = sum2(H2), hn = sum2(HN);
-              const float tn = LI ? subw[sc] : sum2(TN);
-              adj_apply<WX>(kl, sum2(T1) - h1, sum2(T2) - h2, tn - hn, Ac);
-              adj_apply<WX>(kh, h1, h2, hn, Ac);
-              if (near) {  // rare: this lane's sub-chunk again, pair by pair, by the canonical rule
+            } else {
+              bool ok = false;
+              if (m == 2)
+                ok = adj_edges<HAS_Z, LOGB, WX, 1>(Sc, np, nsx, nsy, sz, cls, blo, coef, C, subw[sc], Ac);
+              else if (m == 3)
+                ok = adj_edges<HAS_Z, LOGB, WX, 2>(Sc, np, nsx, nsy, sz, cls, blo, coef, C, subw[sc], Ac);
+              if (!ok && act) {  // more edges, or (rare) a pair in a guard band: pair by pair, by the canonical rule
                 Ac = Acc{0.f, 0.f, 0.f, 0.f, 0.f};
                 for (int j = 0; j < cnt; ++j) {
                   float lz;
                   const float4 l = lens_of(Sc, j, lz);
-                  if (HAS_Z && lz > sz) continue;
+                  if (HAS_Z && lz > sz) continue;  // lens behind source (src/tpcf.f90:322)
                   const float dx = l.x - sx, dy = l.y - sy;
                   const float d2 = fmaf(dy, dy, dx * dx);
                   const int b = pair_bin<LOGB>(d2, l.x, l.y, sx, sy, C);
                   if ((unsigned)b >= (unsigned)nb) continue;
                   adj_pair<LOGB, WX>(sx, sy, l, coef[b], Ac);
                 }
-              }
-            } else if (act) {
-              for (int j = 0; j < cnt; ++j) {
-                float lz;
-                const float4 l = lens_of(Sc, j, lz);
-                if (HAS_Z && lz > sz) continue;  // lens behind source (src/tpcf.f90:322)
-                const float dx = l.x - sx, dy = l.y - sy;
-                const float d2 = fmaf(dy, dy, dx * dx);
-                const int b = pair_bin<LOGB>(d2, l.x, l.y, sx, sy, C);
-                if ((unsigned)b >= (unsigned)nb) continue;
-                adj_pair<LOGB, WX>(sx, sy, l, coef[b], Ac);
               }
             }
             if (cls != 0) {

@@ -212,33 +212,7 @@ __device__ __forceinline__ int edge_index_f32(float v, const float* e2f, int nb)
   return lo;
 }
 
-template <bool LOGB, bool HAS_Z, bool ZREG = false>
-__device__ __forceinline__ int classify(float lx, float ly, const float4 box, const BinCtx& C, int& blo) {
-  const float dxl = fmaxf(fmaxf(box.x - lx, lx - box.z), 0.f);
-  const float dyl = fmaxf(fmaxf(box.y - ly, ly - box.w), 0.f);
-  const float dxh = fmaxf(lx - box.x, box.z - lx);
-  const float dyh = fmaxf(ly - box.y, box.w - ly);
-  const float dmin2 = fmaf(dyl, dyl, dxl * dxl);
-  const float dmax2 = fmaf(dyh, dyh, dxh * dxh);
-  int b0, b1;
-  if (LOGB) {
-    b0 = __float2int_rd(fmaf(lg2_ftz(dmin2), C.A, C.B) - C.eps);
-    b1 = __float2int_rd(fmaf(lg2_ftz(dmax2), C.A, C.B) + C.eps);
-  } else {
-    b0 = edge_index_f32(dmin2 * (1.f - C.eps), C.e2f, C.nb);
-    b1 = edge_index_f32(dmax2 * (1.f + C.eps), C.e2f, C.nb);
-  }
-  if (b1 < 0 || b0 >= C.nb) return 0;
-  b0 = max(b0, -1);  // every bin below 0 or from nb up is dropped alike
-  b1 = min(b1, C.nb);
-  blo = b0;
-  if (HAS_Z && !ZREG) return 3;  // z cut: per-pair path unless the register paths apply it
-  if (b0 == b1) return 1;
-  if (b1 == b0 + 1) return 2;
-  return 3;
-}
-
-// Class of a box for the planar pair kernel: 0 when no pair can be in range,
+// Class of a box for the planar pair and adjoint kernels: 0 when no pair can be in range,
 // else 1 + the number of bin edges its distance range [dmin, dmax] may cross
 // (guard band eps on both ends) for up to two edges, 4 beyond (per-pair
 // binning).  blo = the lowest bin, -1 when the range starts below the first
