@@ -97,17 +97,43 @@ __device__ __forceinline__ void stage_runs(void* dst, int rows, int live_rows, i
   }
 }
 
-// Lens factors of resample/map g for lens jj of a tile.  stage() starts the
-// copies of the raw inputs of one tile into shared memory (all threads);
-// stage_bulk() does the same for a whole, aligned tile (bulk_ok) by
-// bulk_bytes() of one-thread bulk copies signalled on an mbarrier (rows past
-// n_g are not copied); factors() turns the landed raw values into the
-// numerator factor vw and the K factor wm (both 0 for a lens that takes no
-// part).
+// Four values p[0 .. 3] of which the first n exist (the others read as 0);
+// vec: all four exist and p is 16-byte aligned.
+template <class V4, class T>
+__device__ __forceinline__ V4 load4(const T* p, int n, bool vec) {
+  if (vec) return __ldg(reinterpret_cast<const V4*>(p));
+  V4 v = {0, 0, 0, 0};
+  if (n > 0) v.x = __ldg(p);
+  if (n > 1) v.y = __ldg(p + 1);
+  if (n > 2) v.z = __ldg(p + 2);
+  if (n > 3) v.w = __ldg(p + 3);
+  return v;
+}
+template <class V4>
+__device__ __forceinline__ auto comp4(const V4& v, int s) {
+  return s == 0 ? v.x : s == 1 ? v.y : s == 2 ? v.z : v.w;
+}
+
+// Lens factors: the numerator factor vw and the K factor wm of one lens and
+// map or resample, both 0 for a lens that takes no part.  stage() starts the
+// copies of a tile's raw inputs into shared memory (all threads) and factors()
+// reads a landed value; load() reads four lenses' raw inputs of two maps (g,
+// g + 8) into registers and factor() turns one of them into its factors.
 struct MapFactors {  // foreground maps: vw = val w, wm = w
   static constexpr bool kSame = false;  // vw and wm differ: two factor arrays
   int map0;
   static constexpr size_t kRawBytes = sizeof(float) * (2 * kMapGroup + 1) * kRawStride;
+  // moves to the p-th 16 of n maps: how many they are
+  __device__ __forceinline__ int pass(int p, int n) {
+    map0 += p * kMapGroup;
+    return min(kMapGroup, n - p * kMapGroup);
+  }
+  static __device__ __forceinline__ void of(float v, float w, float mw, double& vw, double& wm) {
+    wm = (double)w;
+    vw = (double)v * wm;
+    // calculate_tpcf_from_marks drops lenses with marks weight x weight <= 0
+    if (!((double)mw * wm > 0.0)) vw = wm = 0.0;
+  }
   // raw rows: val of the kMapGroup maps, w of the kMapGroup maps, marks weight
   __device__ __forceinline__ void stage(const MarksField& F, long long t0, int nt, int n_g, unsigned char* raw,
                                         int tid, int nthr) const {
@@ -123,26 +149,30 @@ struct MapFactors {  // foreground maps: vw = val w, wm = w
     const float* mw = F.mw + t0;
     stage_runs(rv + 2 * kMapGroup * kRawStride, 1, 1, nt, vec, [&](int) { return mw; }, tid, nthr);
   }
-  __device__ __forceinline__ bool bulk_ok(const MarksField& F, long long t0, int nt) const {
-    return nt == 64 && al16(F.val) && al16(F.w) && al16(F.mw) && (F.n & 3) == 0 && (t0 & 3) == 0;
-  }
-  __device__ __forceinline__ uint32_t bulk_bytes(int n_g) const { return 256u * (2 * n_g + 1); }
-  __device__ __forceinline__ void stage_bulk(const MarksField& F, long long t0, int n_g, unsigned char* raw,
-                                             uint64_t* bar) const {
-    float* rv = reinterpret_cast<float*>(raw);
-    const size_t o = (size_t)map0 * (size_t)F.n + (size_t)t0;
-    for (int k = 0; k < n_g; ++k) {
-      bulk_g2s(rv + k * kRawStride, F.val + o + (size_t)k * F.n, 256, bar);
-      bulk_g2s(rv + (kMapGroup + k) * kRawStride, F.w + o + (size_t)k * F.n, 256, bar);
-    }
-    bulk_g2s(rv + 2 * kMapGroup * kRawStride, F.mw + t0, 256, bar);
-  }
   __device__ __forceinline__ void factors(const unsigned char* raw, int g, int jj, double& vw, double& wm) const {
     const float* rv = reinterpret_cast<const float*>(raw);
-    wm = (double)rv[(kMapGroup + g) * kRawStride + jj];
-    vw = (double)rv[g * kRawStride + jj] * wm;
-    // calculate_tpcf_from_marks drops lenses with marks weight x weight <= 0
-    if (!((double)rv[2 * kMapGroup * kRawStride + jj] * wm > 0.0)) vw = wm = 0.0;
+    of(rv[g * kRawStride + jj], rv[(kMapGroup + g) * kRawStride + jj], rv[2 * kMapGroup * kRawStride + jj], vw, wm);
+  }
+  struct Raw {
+    float4 v[2], w[2];
+  };
+  __device__ __forceinline__ bool vec_ok(const MarksField& F) const {
+    return al16(F.val) && al16(F.w) && (F.n & 3) == 0;
+  }
+  // Lenses l0 .. l0 + n - 1, n <= 4; vec (the same for the whole warp): n = 4
+  // and l0 a multiple of 4.  Maps past n_g read the last one: their sums are
+  // dropped.
+  __device__ __forceinline__ void load(const MarksField& F, long long l0, int n, bool vec, int n_g, int g,
+                                       Raw& r) const {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const size_t o = (size_t)(map0 + min(g + 8 * k, n_g - 1)) * (size_t)F.n + (size_t)l0;
+      r.v[k] = load4<float4>(F.val + o, n, vec);
+      r.w[k] = load4<float4>(F.w + o, n, vec);
+    }
+  }
+  __device__ __forceinline__ void factor(const Raw& r, int k, int s, float mw, double& vw, double& wm) const {
+    of(comp4(r.v[k], s), comp4(r.w[k], s), mw, vw, wm);
   }
 };
 struct MultFactors {  // resamples: vw = wm = multiplicity of the lens's unit
@@ -151,6 +181,12 @@ struct MultFactors {  // resamples: vw = wm = multiplicity of the lens's unit
   const int* unit;    // unit of each lens (all fields concatenated), or nullptr: the lens itself
   long long n_units;
   static constexpr size_t kRawBytes = sizeof(int) * kMapGroup * kRawStride;
+  __device__ __forceinline__ int pass(int p, int n) {
+    mult += (size_t)p * kMapGroup * (size_t)n_units;
+    return min(kMapGroup, n - p * kMapGroup);
+  }
+  // the bootstraps take every drawn lens (src/tpcf.f90:601, :917, :1248)
+  static __device__ __forceinline__ double of(int m) { return m > 0 ? (double)m : 0.0; }
   __device__ __forceinline__ void stage(const MarksField& F, long long t0, int nt, int n_g, unsigned char* raw,
                                         int tid, int nthr) const {
     int* rm = reinterpret_cast<int*>(raw);
@@ -169,21 +205,31 @@ struct MultFactors {  // resamples: vw = wm = multiplicity of the lens's unit
       cp_async4(rm + g * kRawStride + jj, mult + o, v);
     }
   }
-  __device__ __forceinline__ bool bulk_ok(const MarksField& F, long long t0, int nt) const {
-    return !unit && nt == 64 && al16(mult) && (n_units & 3) == 0 && ((F.lens0 + t0) & 3) == 0;
-  }
-  __device__ __forceinline__ uint32_t bulk_bytes(int n_g) const { return 256u * n_g; }
-  __device__ __forceinline__ void stage_bulk(const MarksField& F, long long t0, int n_g, unsigned char* raw,
-                                             uint64_t* bar) const {
-    int* rm = reinterpret_cast<int*>(raw);
-    const int* m = mult + F.lens0 + t0;
-    for (int k = 0; k < n_g; ++k) bulk_g2s(rm + k * kRawStride, m + (size_t)k * n_units, 256, bar);
-  }
-  // the bootstraps take every drawn lens (src/tpcf.f90:601, :917, :1248)
   __device__ __forceinline__ void factors(const unsigned char* raw, int g, int jj, double& vw, double& wm) const {
-    const int m = reinterpret_cast<const int*>(raw)[g * kRawStride + jj];
-    wm = m > 0 ? (double)m : 0.0;
-    vw = wm;
+    vw = wm = of(reinterpret_cast<const int*>(raw)[g * kRawStride + jj]);
+  }
+  struct Raw {
+    int4 m[2];
+  };
+  __device__ __forceinline__ bool vec_ok(const MarksField& F) const {
+    return !unit && al16(mult) && (n_units & 3) == 0 && (F.lens0 & 3) == 0;
+  }
+  __device__ __forceinline__ void load(const MarksField& F, long long l0, int n, bool vec, int n_g, int g,
+                                       Raw& r) const {
+    const long long gl = F.lens0 + l0;
+    const int4 u = unit ? load4<int4>(unit + gl, n, false) : make_int4(0, 0, 0, 0);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int* m = mult + (size_t)min(g + 8 * k, n_g - 1) * (size_t)n_units;
+      if (unit)
+        r.m[k] = make_int4(n > 0 ? __ldg(m + u.x) : 0, n > 1 ? __ldg(m + u.y) : 0, n > 2 ? __ldg(m + u.z) : 0,
+                           n > 3 ? __ldg(m + u.w) : 0);
+      else
+        r.m[k] = load4<int4>(m + gl, n, vec);
+    }
+  }
+  __device__ __forceinline__ void factor(const Raw& r, int k, int s, float, double& vw, double& wm) const {
+    vw = wm = of(comp4(r.m[k], s));
   }
 };
 
@@ -210,9 +256,7 @@ struct MultFactors {  // resamples: vw = wm = multiplicity of the lens's unit
 // The factors of one lens are stored as [vw of the 16 maps | 2 pad | wm of
 // the 16 maps | 2 pad] (kLensStride doubles): the four 16-byte loads of a
 // warp touch at most four distinct chunks (vw or wm, half 0 or 1), on
-// disjoint banks; in the tensor-core form a B fragment (4 lenses x 8 maps)
-// starts its lens rows 72 words = 8 banks apart, so each half-warp's 16
-// values fall on 32 distinct banks.
+// disjoint banks.
 constexpr int kTileL = 64;
 constexpr int kLensStride = 2 * (kMapGroup + 2);
 constexpr int kWmOffset = kMapGroup + 2;
@@ -243,11 +287,13 @@ __device__ __forceinline__ void convert_factors(const Fac& fac, const unsigned c
 
 template <class Fac>
 __global__ void __launch_bounds__(kMarksThreads, 2) k_marks_partials(const MarksField* __restrict__ fields, int n_field,
-                                                            const Fac fac, int n_g, int n_bin, int tg,
+                                                            Fac fac, int n_maps, int n_bin, int tg,
                                                             long long chunk, double* __restrict__ partial) {
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int TF = kTileL * kLensStride;
   const int R = 3 * n_bin + 1;
+  const int n_g = fac.pass(blockIdx.y, n_maps);
+  partial += (size_t)blockIdx.y * gridDim.x * kMapGroup * R;
   const int nbp = marks_quad_bins(n_bin), nbq = nbp / 4;
   const int ng = blockDim.x / tg;
   double* fac_s = reinterpret_cast<double*>(sm);  // [kTileL][kLensStride] factors of every row
@@ -348,210 +394,230 @@ __global__ void __launch_bounds__(kMarksThreads, 2) k_marks_partials(const Marks
 }
 
 // FP64 tensor-core form for n_bin <= 32 (tcgen05 has no FP64 kind; the FP64
-// tensor instruction of sm_100 is mma.sync m8n8k4 .f64: D[8][8] += A[8][4]
-// B[4][8], 256 FMA per warp instruction against 32 for a warp FFMA64).
+// tensor instruction of sm_100 is mma.sync .f64, here m16n8k16: D[16][8] +=
+// A[16][16] B[16][8], maps by rows by lenses, 2048 FMA per warp instruction
+// against 32 for a warp FFMA64).
 //
-// Rows (A's M dimension) are grouped so that no 8-row m-tile mixes the two
-// factor kinds: the xi_E, xi_B rows (vw factors) fill the first
-// MV = ceil(2 n_bin / 8) m-tiles, the K rows and the marks weight row (wm
-// factors) the next ceil((n_bin + 1) / 8); padding rows read a zeroed area.
-// Lenses are K (four per step), maps N (two n-tiles of 8).  Warp w owns
-// m-tile w for both n-tiles and every lens of the block, so its sums are
-// final for the block: no reduction between warps.  Two accumulator sets
-// (even and odd lens steps) halve the dependent chain of the tensor
-// instructions.
+// The rows of the marks (B's N dimension) are grouped so that no tile of 8 mixes
+// the two factor kinds: the xi_E, xi_B rows (vw factors) fill the first
+// MV = ceil(2 n_bin / 8) tiles, the K rows and the marks weight row (wm
+// factors) the next MK = ceil((n_bin + 1) / 8); padding rows are zeros.  The 16
+// maps are A's rows, so a tile needs one kind of factors.
 //
-// Staging: thread 0 issues bulk copies of a whole tile (the three marks
-// blocks [64][n_bin] as laid out in HBM, the marks weights, the factors' raw
-// rows) signalled on the buffer's mbarrier; partial or unaligned tiles go by
-// per-thread cp.async with zero fill.  Every wait is bounded: a copy that
-// does not land sets kErrTimeout in *err and the block stops.
+// Bound by the FP64 tensor pipe (57 us for 10^6 lenses, 61 rows and 16 maps,
+// as long as the 370 MB of marks and maps take from HBM), so everything else
+// has to stay below it.  Each warp therefore takes lenses of its own (16 at a
+// time, k, k + kDmmaWarps, ... of the block's) and all row tiles of them: a
+// factor is needed by one lane only, which loads its inputs from HBM into
+// registers one group ahead and converts them there; the marks come by bulk
+// copies into the warp's own ring of buffers; no barrier until the end, where
+// the block's warps are summed in order.  With one row tile per warp instead,
+// every warp read all factors from shared memory, written there in a pass
+// between block barriers: 6 wavefronts of shared memory for 2 tensor
+// instructions, where this form has 1.4, and the m8n8k4 form of the instruction
+// instead of m16n8k16: 130 us for that case against 91 now (pipe 67 % busy; 16
+// warps a SM instead of 12 need spills: 114 us; a third buffer: 93).
+//
+// Within a group of 16 the K index 4 s + tq (tq: the lane's index in the
+// fragment) is lens 4 tq + s: any bijection serves, and with this one a lane's
+// four lenses are consecutive, so its inputs are one 16-byte load a map.
 //
 // Staged marks: quantity q of lens jj, bin b at q QS + jj n_bin + b
-// (QS = 64 n_bin rounded up to 4 floats), the marks weights at 3 QS + jj, and
-// 64 zeros at 3 QS + 64 for the padding rows.
-__host__ __device__ inline int marks_dense_slot(int n_bin) { return (kTileL * n_bin + 3) / 4 * 4; }
-__host__ __device__ inline int marks_dmma_buffer(int n_bin) { return 3 * marks_dense_slot(n_bin) + 2 * kTileL; }
+// (QS = 16 n_bin).  Groups that are short or not 16-byte aligned in HBM are
+// copied value by value (cp.async, zeros past the end).  Every wait is
+// bounded: a copy that does not land sets kErrTimeout in *err and the warp
+// stops.
+constexpr int kDmmaLens = 16;   // lenses per group of a warp
+constexpr int kDmmaWarps = 4;
+constexpr int kDmmaRing = 2;    // buffers per warp
+static_assert(kTileL % kDmmaLens == 0, "chunks hold whole groups");
+__host__ __device__ inline int marks_dmma_buffer(int n_bin) { return 3 * kDmmaLens * n_bin; }
 __host__ __device__ inline int marks_vw_tiles(int n_bin) { return (2 * n_bin + 7) / 8; }
 __host__ __device__ inline int marks_m_tiles(int n_bin) { return marks_vw_tiles(n_bin) + (n_bin + 1 + 7) / 8; }
 constexpr int kDmmaMaxBins = 32;
-constexpr int kDmmaMaxThreads = 32 * ((2 * kDmmaMaxBins + 7) / 8 + (kDmmaMaxBins + 1 + 7) / 8);
-// Registers per thread at most: two blocks of kDmmaMaxThreads per SM.
-constexpr int kDmmaRegs = 65536 / (2 * kDmmaMaxThreads) / 8 * 8;
-constexpr size_t kDmmaRawBytes = std::max(MapFactors::kRawBytes, MultFactors::kRawBytes);
-
-__device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-      : "+d"(d0), "+d"(d1)
-      : "d"(a), "d"(b));
+// Blocks a SM: 3 up to 8 row tiles (168 registers, 64 of them sums), 2 beyond.
+__host__ __device__ constexpr int marks_dmma_per_sm(int tiles) { return tiles <= 8 ? 3 : 2; }
+// Output row of row i of the tiles: 0 .. R - 1, or -1 (padding).
+__device__ __forceinline__ int marks_row(int i, int n_bin) {
+  const int v = 8 * marks_vw_tiles(n_bin);
+  if (i < v) return i < 2 * n_bin ? i : -1;
+  return i - v <= n_bin ? 2 * n_bin + i - v : -1;
 }
 
-template <class Fac>
-__global__ void __launch_bounds__(kDmmaMaxThreads, 2) k_marks_dmma(const MarksField* __restrict__ fields, int n_field,
-                                                              const Fac fac, int n_g, int n_bin, long long chunk,
-                                                              double* __restrict__ partial, unsigned* __restrict__ err,
-                                                              int skip_tile, unsigned wait_limit) {
+// d[16][8] += A[16][16] B[16][8]; a[2 s + h]: row gq + 8 h, K 4 s + tq; b[s]: K
+// 4 s + tq, column gq; d[2 h + c]: row gq + 8 h, column 2 tq + c.
+__device__ __forceinline__ void dmma_16816(double (&d)[4], const double (&a)[8], const double (&b)[4]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7, %8, %9, %10, %11}, "
+      "{%12, %13, %14, %15}, {%0, %1, %2, %3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]),
+        "d"(b[2]), "d"(b[3]));
+}
+
+template <class Fac, int MV, int MK>
+__global__ void __launch_bounds__(32 * kDmmaWarps, marks_dmma_per_sm(MV + MK))
+k_marks_dmma(const MarksField* __restrict__ fields, int n_field, Fac fac, int n_maps, int n_bin, long long chunk,
+             double* __restrict__ partial, unsigned* __restrict__ err, int skip_tile, unsigned wait_limit) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ __align__(8) uint64_t full[2];
-  constexpr int TF = kTileL * kLensStride;
+  __shared__ __align__(8) uint64_t full_s[kDmmaWarps][kDmmaRing];
   const int nb = n_bin, R = 3 * nb + 1;
-  const int QS = marks_dense_slot(nb), MS = marks_dmma_buffer(nb);
-  const int MV = marks_vw_tiles(nb);
-  double* fac_s = reinterpret_cast<double*>(sm);  // [kTileL][kLensStride] factors
-  unsigned char* raw = sm + TF * sizeof(double);
-  float* mk = reinterpret_cast<float*>(raw + kDmmaRawBytes);
+  const int n_g = fac.pass(blockIdx.y, n_maps);
+  partial += (size_t)blockIdx.y * gridDim.x * kMapGroup * R;
+  const int QS = kDmmaLens * nb, BS = marks_dmma_buffer(nb);
+  constexpr int NM = MV + MK;  // tiles of the vw and of the wm rows
   const int blk = blockIdx.x;
   int fi = 0;
   while (fi + 1 < n_field && fields[fi + 1].chunk0 <= blk) ++fi;
-  const MarksField& F = fields[fi];
+  const MarksField F = fields[fi];
   const long long j0 = (long long)(blk - F.chunk0) * chunk;
-  const long long j1 = min(F.n, j0 + chunk);
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int mt = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
-  // this lane's A row (row gq of m-tile mt): output row r (-1: padding), the
-  // staged offset of its value for lens 0 and its lens stride
-  int r = -1, aoff = 3 * QS + kTileL, astr = 1;
-  if (mt < MV) {
-    const int rho = mt * 8 + gq;
-    if (rho < 2 * nb) {
-      const int q = rho / nb, b = rho - q * nb;
-      r = rho, aoff = q * QS + b, astr = nb;
-    }
-  } else {
-    const int rho = (mt - MV) * 8 + gq;
-    if (rho < nb) {
-      r = 2 * nb + rho, aoff = 2 * QS + rho, astr = nb;
-    } else if (rho == nb) {
-      r = 3 * nb, aoff = 3 * QS, astr = 1;
-    }
+  const int n_len = (int)min(F.n - j0, chunk);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
+  float* mk = reinterpret_cast<float*>(sm) + warp * kDmmaRing * BS;
+  uint64_t* full = full_s[warp];
+  // this lane's row of the marks (row gq of each tile): staged offset of its
+  // value for lens 4 tq.  Padding is in the last vw tile, the marks weight row
+  // and padding in the last wm tile.
+  int off[NM];
+#pragma unroll
+  for (int i = 0; i < NM; ++i) {
+    const int r = marks_row(8 * i + gq, nb), q = r < 0 ? 0 : r / nb;
+    off[i] = 4 * tq * nb + (r < 0 || q > 2 ? 0 : q * QS + (r - q * nb));
   }
-  // B: lens tq of the step, map gq of the n-tile
-  const double* bsel = ((mt < MV || Fac::kSame) ? fac_s : fac_s + kWmOffset) + gq;
-  const bool two = n_g > 8;  // the second n-tile holds maps
-
-  // raw rows past n_g, lenses past a partial tile and the zero area are never
-  // copied: start from zeros (ordered before the bulk copies by the fence)
-  for (int e = tid; e < (int)(kDmmaRawBytes / 4); e += nthr) reinterpret_cast<float*>(raw)[e] = 0.f;
-  for (int e = tid; e < 2 * MS; e += nthr) mk[e] = 0.f;
-  if (tid == 0) {
-    mbar_init(&full[0], 1);
-    mbar_init(&full[1], 1);
+  const bool vpad = marks_row(8 * (MV - 1) + gq, nb) < 0, wpad = marks_row(8 * (NM - 1) + gq, nb) < 0;
+  const bool wrow = marks_row(8 * (NM - 1) + gq, nb) == 3 * nb;
+  if (lane == 0) {
+#pragma unroll
+    for (int b = 0; b < kDmmaRing; ++b) mbar_init(&full[b], 1);
     mbar_fence_init();
   }
-  fence_proxy_async_smem();
-  __syncthreads();
-  const bool mbulk = (nb & 3) == 0 && al16(F.xiE) && al16(F.xiB) && al16(F.K) && al16(F.mw);
-  uint32_t par = 0;  // bit b: parity of buffer b's next mbarrier phase
+  __syncwarp();
+  const bool mbulk = al16(F.xiE) && al16(F.xiB) && al16(F.K);
+  const bool lvec = al16(F.mw) && fac.vec_ok(F);
   // fault injection for tests (tpcf_debug_inject): the bulk copies of each
-  // block's tile skip_tile are never issued, so the wait on them runs out
-  // after wait_limit polls (both off in every product call)
+  // block's lenses 64 skip_tile .. + 63 are never issued, so the wait on them
+  // runs out after wait_limit polls (both off in every product call)
   const uint32_t polls = wait_limit ? wait_limit : kWaitPolls;
-
-  // starts the copies of tile t0 into buffer b; true when they complete on full[b]
-  auto stage_tile = [&](long long t0, int b) -> bool {
-    const int nt = (int)min((long long)kTileL, j1 - t0);
-    const bool bm = mbulk && nt == kTileL;
-    const bool br = fac.bulk_ok(F, t0, nt);
-    float* mb = mk + b * MS;
-    if ((bm || br) && tid == 0 && (t0 - j0) / kTileL != skip_tile) {
-      mbar_arrive_tx(&full[b], (bm ? 4u * (3 * nb + 1) * kTileL : 0u) + (br ? fac.bulk_bytes(n_g) : 0u));
-      if (bm) {
-        const size_t o = (size_t)t0 * nb;
-        bulk_g2s(mb, F.xiE + o, 4u * kTileL * nb, &full[b]);
-        bulk_g2s(mb + QS, F.xiB + o, 4u * kTileL * nb, &full[b]);
-        bulk_g2s(mb + 2 * QS, F.K + o, 4u * kTileL * nb, &full[b]);
-        bulk_g2s(mb + 3 * QS, F.mw + t0, 4u * kTileL, &full[b]);
+  // groups of this warp: group k starts at lens j0 + first(k)
+  const int n_group = (n_len + kDmmaLens - 1) / kDmmaLens;
+  const int mine = n_group > warp ? (n_group - warp + kDmmaWarps - 1) / kDmmaWarps : 0;
+  auto first = [&](int k) { return (warp + k * kDmmaWarps) * kDmmaLens; };
+  auto bulk = [&](int k) { return mbulk && first(k) + kDmmaLens <= n_len; };
+  // starts the copies of group k into its buffer (bulk copies complete on
+  // full[buffer], others in the warp's k-th cp.async group)
+  auto stage = [&](int k) {
+    const int f = first(k), b = k % kDmmaRing;
+    float* dst = mk + b * BS;
+    const size_t o = (size_t)(j0 + f) * nb;
+    if (bulk(k)) {
+      if (lane == 0 && f / kTileL != skip_tile) {
+        mbar_arrive_tx(&full[b], 4u * BS);
+        bulk_g2s(dst, F.xiE + o, 4u * QS, &full[b]);
+        bulk_g2s(dst + QS, F.xiB + o, 4u * QS, &full[b]);
+        bulk_g2s(dst + 2 * QS, F.K + o, 4u * QS, &full[b]);
       }
-      if (br) fac.stage_bulk(F, t0, n_g, raw, &full[b]);
-    }
-    if (!bm) {  // the marks as laid out in HBM, zero past the tile's end
-      const size_t o = (size_t)t0 * nb;
-      const int nq = nt * nb;
-      const bool vec = (nb & 3) == 0 && al16(F.xiE) && al16(F.xiB) && al16(F.K);
+    } else {
+      const int nq = min(kDmmaLens, n_len - f) * nb;
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const float* src = (q == 0 ? F.xiE : q == 1 ? F.xiB : F.K) + o;
-        float* dst = mb + q * QS;
-        if (vec) {
-          for (int e = tid; e < kTileL * nb / 4; e += nthr)
-            cp_async16(dst + 4 * e, 4 * e < nq ? src + 4 * e : src, 4 * e < nq);
-        } else {
-          for (int e = tid; e < kTileL * nb; e += nthr) cp_async4(dst + e, e < nq ? src + e : src, e < nq);
-        }
+        for (int e = lane; e < QS; e += 32) cp_async4(dst + q * QS + e, e < nq ? src + e : src, e < nq);
       }
-      const float* mw = F.mw + t0;
-      for (int e = tid; e < kTileL; e += nthr) cp_async4(mb + 3 * QS + e, e < nt ? mw + e : mw, e < nt);
     }
-    if (!br) fac.stage(F, t0, nt, n_g, raw, tid, nthr);
-    return bm || br;
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // waits for buffer b's copies; false when a bulk copy did not land in time
-  int wb = 0;
-  uint32_t wpar = 0;
-  auto land = [&](int b, bool bulk) -> bool {
-    cp_async_wait_all();
-    if (!bulk) return true;
-    wb = b, wpar = (par >> b) & 1u;
-    par ^= 1u << b;
-    return mbar_wait_bounded(&full[b], wpar, polls);
+  // waits for group k, with at most kDmmaRing - 1 later groups begun
+  auto land = [&](int k) -> bool {
+    if (bulk(k)) {
+      const bool ok = mbar_wait_bounded(&full[k % kDmmaRing], (uint32_t)(k / kDmmaRing) & 1u, polls);
+      return __all_sync(0xffffffffu, ok);
+    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(kDmmaRing - 1) : "memory");
+    __syncwarp();
+    return true;
+  };
+  // the lane's raw factor inputs and marks weights of group k
+  auto inputs = [&](int k, typename Fac::Raw& r, float4& mw) {
+    const int f = first(k) + 4 * tq, n = min(4, max(0, n_len - f));
+    const bool vec = lvec && first(k) + kDmmaLens <= n_len;
+    fac.load(F, j0 + f, n, vec, n_g, gq, r);
+    mw = load4<float4>(F.mw + j0 + f, n, vec);
   };
 
-  double acc[2][2][2];
+  double acc[NM][4];
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
+  for (int i = 0; i < NM; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0;
 #pragma unroll
-    for (int n = 0; n < 2; ++n) acc[p][n][0] = acc[p][n][1] = 0.0;
-  bool abort = false;
-  if (j0 < j1) abort = __syncthreads_or(!land(0, stage_tile(j0, 0)));
-  if (!abort) {
-    if (j0 < j1) convert_factors(fac, raw, fac_s, tid, nthr);
-    __syncthreads();
+  for (int k = 0; k < kDmmaRing; ++k) {
+    if (k < mine) stage(k);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  int buf = 0;
-  for (long long t0 = j0; t0 < j1 && !abort; t0 += kTileL) {
-    const bool more = t0 + kTileL < j1;
-    // the raw area was read before the last barrier, the other marks buffer
-    // before the one ahead of it
-    const bool nbulk = more && stage_tile(t0 + kTileL, buf ^ 1);
-    const float* ma = mk + buf * MS + aoff + tq * astr;
-    const double* bp = bsel + tq * kLensStride;
-#pragma unroll 8
-    for (int ks = 0; ks < kTileL / 4; ++ks) {
-      const double a = (double)ma[4 * ks * astr];
-      const double* b = bp + 4 * ks * kLensStride;
-      dmma_884(acc[ks & 1][0][0], acc[ks & 1][0][1], a, b[0]);
-      if (two) dmma_884(acc[ks & 1][1][0], acc[ks & 1][1][1], a, b[8]);
-    }
-    // the next tile's copies landed; this tile's factors and marks are no longer read
-    if (__syncthreads_or(more && !land(buf ^ 1, nbulk))) {
-      abort = true;
+  typename Fac::Raw raw, raw_n;
+  float4 mw, mw_n;
+  if (mine > 0) inputs(0, raw, mw);
+  for (int k = 0; k < mine; ++k) {
+    if (k + 1 < mine) inputs(k + 1, raw_n, mw_n);
+    if (!land(k)) {  // flag it, give the warp's copies one more bounded wait, leave
+      if (lane == 0) atomicOr(err, kErrTimeout);
+      for (int q = k; q < min(mine, k + kDmmaRing); ++q) land(q);
       break;
     }
-    if (more) {
-      convert_factors(fac, raw, fac_s, tid, nthr);
-      __syncthreads();
-    }
-    buf ^= 1;
-  }
-  if (abort) {  // a copy did not land: flag it, give it one more bounded wait, leave
-    if (tid == 0) {
-      atomicOr(err, kErrTimeout);
-      mbar_wait_bounded(&full[wb], wpar, polls);
-    }
-    return;
-  }
-  if (r >= 0) {
+    const float* ma = mk + (k % kDmmaRing) * BS;
+    double vw[8], wm[8];
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
+    for (int s = 0; s < 4; ++s)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int map = 8 * n + 2 * tq + i;
-        if (map < n_g) partial[((size_t)blk * n_g + map) * R + r] = acc[0][n][i] + acc[1][n][i];
+      for (int h = 0; h < 2; ++h) fac.factor(raw, h, s, comp4(mw, s), vw[2 * s + h], wm[2 * s + h]);
+#pragma unroll
+    for (int i = 0; i < NM; ++i) {
+      double m[4];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        float v = ma[off[i] + s * nb];
+        if (i == NM - 1 && wrow) v = comp4(mw, s);
+        if ((i == NM - 1 && wpad) || (i == MV - 1 && vpad)) v = 0.f;
+        m[s] = (double)v;
       }
+      dmma_16816(acc[i], Fac::kSame || i < MV ? vw : wm, m);
+    }
+    __syncwarp();  // all lanes have read the buffer
+    if (k + kDmmaRing < mine) stage(k + kDmmaRing);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    raw = raw_n;
+    mw = mw_n;
+  }
+  // the warps' sums, added in warp order
+  __syncthreads();
+  double* red = reinterpret_cast<double*>(sm);  // [warp][NM * 4][32]
+#pragma unroll
+  for (int i = 0; i < NM; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) red[((warp * NM + i) * 4 + c) * 32 + lane] = acc[i][c];
+  __syncthreads();
+  for (int e = tid; e < NM * 128; e += 32 * kDmmaWarps) {
+    const int l = e & 31, c = (e >> 5) & 3;
+    const int r = marks_row(8 * (e >> 7) + 2 * (l & 3) + (c & 1), nb), map = (l >> 2) + 8 * (c >> 1);
+    if (r < 0 || map >= n_g) continue;
+    double t = red[e];
+#pragma unroll
+    for (int v = 1; v < kDmmaWarps; ++v) t += red[v * NM * 128 + e];
+    partial[((size_t)blk * n_g + map) * R + r] = t;
   }
 }
 size_t marks_dmma_smem(int n_bin) {
-  return sizeof(double) * kTileL * kLensStride + kDmmaRawBytes + 2 * sizeof(float) * (size_t)marks_dmma_buffer(n_bin);
+  const size_t ring = sizeof(float) * kDmmaWarps * kDmmaRing * (size_t)marks_dmma_buffer(n_bin);
+  return std::max(ring, sizeof(double) * 128 * kDmmaWarps * marks_m_tiles(n_bin));
+}
+// The kernel compiled for n_bin's numbers of row tiles (they are compile-time so
+// that the loads, conversions and products of all tiles interleave).
+template <class Fac>
+using MarksDmma = void (*)(const MarksField*, int, Fac, int, int, long long, double*, unsigned*, int, unsigned);
+template <class Fac, int NB = 1>
+MarksDmma<Fac> marks_dmma_kernel(int n_bin) {
+  if constexpr (NB > kDmmaMaxBins) {
+    return nullptr;
+  } else {
+    return n_bin == NB ? k_marks_dmma<Fac, (2 * NB + 7) / 8, (NB + 1 + 7) / 8> : marks_dmma_kernel<Fac, NB + 1>(n_bin);
+  }
 }
 
 // Threads per lens group (two per row quad, whole warps) and per block: as
@@ -572,9 +638,7 @@ size_t marks_smem(int n_bin) {
 // only on the input.
 int marks_blocks(int n_bin) {
   if (n_bin > kDmmaMaxBins) return kMarksBlocks;
-  const int bt = 32 * marks_m_tiles(n_bin);
-  const int per_sm = std::min({2048 / bt, 65536 / (bt * kDmmaRegs), 233472 / ((int)marks_dmma_smem(n_bin) + 1024)});
-  return 148 * std::max(1, per_sm);
+  return 148 * marks_dmma_per_sm(marks_m_tiles(n_bin));
 }
 // Lenses per block for n_lens lenses in all: marks_blocks blocks, whole tiles.
 long long marks_chunk(long long n_lens, int n_bin) {
@@ -582,30 +646,29 @@ long long marks_chunk(long long n_lens, int n_bin) {
   const long long per = (n_lens + nbk - 1) / nbk;
   return std::max<long long>(kTileL, (per + kTileL - 1) / kTileL * kTileL);
 }
-// One pass of the partial sums over all fields: the FP64 tensor-core form for
+// The partial sums of n_maps maps or resamples over all fields, 16 to a pass
+// (blockIdx.y; partial sums of a pass follow those of the one before): the FP64 tensor-core form for
 // n_bin <= 32, the FP64 FMA form for wider binnings.
 template <class Fac>
 cudaError_t launch_marks_partials(const MarksField* fields, int n_field, int nblk, long long chunk, const Fac& fac,
-                                  int n_g, int nb, double* part, unsigned* err, int skip_tile, unsigned wait_limit,
+                                  int n_maps, int nb, double* part, unsigned* err, int skip_tile, unsigned wait_limit,
                                   cudaStream_t st) {
+  const dim3 grid(nblk, (n_maps + kMapGroup - 1) / kMapGroup);
   if (nb <= kDmmaMaxBins) {
+    const MarksDmma<Fac> k = marks_dmma_kernel<Fac>(nb);
     const size_t msm = marks_dmma_smem(nb);
-    cudaError_t e = cudaFuncSetAttribute(k_marks_dmma<Fac>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
     if (e != cudaSuccess) return e;
-    k_marks_dmma<Fac><<<nblk, 32 * marks_m_tiles(nb), msm, st>>>(fields, n_field, fac, n_g, nb, chunk, part, err,
-                                                                 skip_tile, wait_limit);
+    k<<<grid, 32 * kDmmaWarps, msm, st>>>(fields, n_field, fac, n_maps, nb, chunk, part, err, skip_tile, wait_limit);
     return cudaGetLastError();
   }
   const size_t msm = marks_smem(nb);
   const int bt = marks_block_threads(nb), tg = marks_group_threads(nb);
   cudaError_t e = cudaFuncSetAttribute(k_marks_partials<Fac>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
   if (e != cudaSuccess) return e;
-  k_marks_partials<Fac><<<nblk, bt, msm, st>>>(fields, n_field, fac, n_g, nb, tg, chunk, part);
+  k_marks_partials<Fac><<<grid, bt, msm, st>>>(fields, n_field, fac, n_maps, nb, tg, chunk, part);
   return cudaGetLastError();
 }
-
-// maps or resamples per pass over the marks
-int marks_group(int) { return kMapGroup; }
 
 // Multiplicities of G resamples s0.. over n_units units: n_draw draws each,
 // counter (d/4, s, 0x2BCF, 0), word d%4, index by multiply-shift (the stream
@@ -673,12 +736,16 @@ cudaError_t launch_marks_reduce(const double* part, const MarksField* df, int n_
   return cudaGetLastError();
 }
 // Passes whose partial sums are kept (up to 64 MiB) before one reduction of all
-// of them: a reduction of one pass is all latency (6 us).  250 k lenses, 1000
-// resamples: 3.88 ms for the call with one pass kept, 3.26 ms with 18.
+// of them: a reduction of one pass is all latency (6 us).
 int marks_passes_kept(int nblk, int R, int n_pass) {
   const size_t one = sizeof(double) * (size_t)std::max(nblk, 1) * kMapGroup * R;
-  return (int)std::max<size_t>(1, std::min<size_t>((size_t)n_pass, ((size_t)64 << 20) / one));
+  // at most 32768: a grid dimension holds 65535
+  return (int)std::max<size_t>(1, std::min<size_t>(std::min<size_t>((size_t)n_pass, 32768), ((size_t)64 << 20) / one));
 }
+
+// Multiplicities of the passes of one launch: what stays in L2 between the
+// draws and the sums.
+constexpr size_t kDrawBytes = (size_t)64 << 20;
 
 // With timing enabled (tpcf_set_timing), CUDA events on the call's stream
 // around every partial-sum launch; total() after the stream has synchronised
@@ -840,27 +907,20 @@ extern "C" tpcf_status tpcf_xi_from_marks(tpcf_ctx* c, int32_t n_field, const tp
     double* dout = (double*)ws_alloc(c, sizeof(double) * sums.size());
     unsigned* derr = (unsigned*)ws_alloc(c, sizeof(unsigned));
     check(cudaMemsetAsync(derr, 0, sizeof(unsigned), st), "memset");
-    const int MG = marks_group(nb);
     PassTimer timer(c);
-    int kept = 0;
-    for (int m0 = 0; m0 < n_map; m0 += MG) {
-      const int g = std::min(MG, n_map - m0);
-      double* dpass = dout + (size_t)m0 * n_field * R;
-      if (nblk == 0) {
-        check(cudaMemsetAsync(dpass, 0, sizeof(double) * g * n_field * R, st), "memset");
-        continue;
-      }
+    if (nblk == 0) check(cudaMemsetAsync(dout, 0, sizeof(double) * sums.size(), st), "memset");
+    // all passes whose partial sums are kept in one launch: their first and last
+    // blocks overlap
+    for (int m0 = 0; m0 < n_map && nblk > 0; m0 += n_keep * kMapGroup) {
+      const int g = std::min(n_keep * kMapGroup, n_map - m0), n_pass = (g + kMapGroup - 1) / kMapGroup;
       timer.mark(st);
-      counted(c, launch_marks_partials(df, n_field, nblk, chunk, MapFactors{m0}, g, nb, part + part_pass * kept, derr,
-                                       c->skip_tile, c->wait_limit, st),
+      counted(c, launch_marks_partials(df, n_field, nblk, chunk, MapFactors{m0}, g, nb, part, derr, c->skip_tile,
+                                       c->wait_limit, st),
               "marks partials");
       timer.mark(st);
-      if (++kept == n_keep || m0 + g == n_map) {
-        counted(c, launch_marks_reduce(part, df, n_field, nblk, kept, g, R,
-                                       dpass - (size_t)(kept - 1) * MG * n_field * R, st),
-                "marks reduce");
-        kept = 0;
-      }
+      counted(c, launch_marks_reduce(part, df, n_field, nblk, n_pass, g - (n_pass - 1) * kMapGroup, R,
+                                     dout + (size_t)m0 * n_field * R, st),
+              "marks reduce");
     }
     check(cudaMemcpyAsync(sums.data(), dout, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, st), "D2H sums");
     unsigned herr = 0;
@@ -958,17 +1018,24 @@ extern "C" tpcf_status tpcf_marks_bootstrap(tpcf_ctx* c, int32_t n_field, const 
     const int R = 3 * nb + 1;
     // Multiplicities drawn here (16 M scattered atomic increments per pass of 16
     // resamples of 1 M lenses, bound by L2 atomics) run on a second stream into
-    // one of two buffers while the other is summed (bound by FP64): 250 k
-    // lenses, 1000 resamples: the call takes 3.26 ms against 4.10 ms in line (fewer
-    // draw blocks, to leave the sums more room, are slower: 444: 3.67 ms).  One
-    // buffer, and no overlap, beyond 1 GiB.
-    const size_t mbytes = sizeof(int) * (size_t)kMapGroup * n_units;
+    // one of two buffers while the other is summed (bound by FP64).  The draws and
+    // sums of as many passes as kDrawBytes holds go in one launch each, so that
+    // the passes' first and last blocks overlap.  250 k lenses, 1000 resamples:
+    // 3.33 ms for the call; one pass a launch 3.49, two 3.40, eight 3.61; in line
+    // 3.45 (the two kernels share the SMs' registers and mostly take turns; fewer
+    // draw blocks, to leave the sums room, are slower: 592: 3.74, and drawing
+    // inside the sum kernel: 4.9).  One buffer, and no overlap, beyond 1 GiB.
+    const size_t part_pass = (size_t)std::max(nblk, 1) * kMapGroup * R;
+    const int n_pass_all = (n_boot + kMapGroup - 1) / kMapGroup;
+    const size_t mpass = sizeof(int) * (size_t)kMapGroup * n_units;
+    int n_keep = marks_passes_kept(nblk, R, n_pass_all);
+    const int n_launch = (int)std::max<size_t>(1, std::min<size_t>(n_keep, kDrawBytes / mpass));
+    n_keep = n_keep / n_launch * n_launch;
+    const size_t mbytes = mpass * n_launch;
     const int n_buf = multiplicity ? 0 : mbytes <= ((size_t)1 << 30) ? 2 : 1;
     int* mbuf[2] = {nullptr, nullptr};
     for (int b = 0; b < n_buf; ++b) mbuf[b] = (int*)ws_alloc(c, mbytes);
     DrawStream draws(c, n_buf == 2);
-    const size_t part_pass = (size_t)std::max(nblk, 1) * kMapGroup * R;
-    const int n_keep = marks_passes_kept(nblk, R, (n_boot + kMapGroup - 1) / kMapGroup);
     int kept = 0;
     double* part = (double*)ws_alloc(c, sizeof(double) * part_pass * n_keep);
     std::vector<double> sums((size_t)n_boot * n_field * R, 0.0);
@@ -978,10 +1045,10 @@ extern "C" tpcf_status tpcf_marks_bootstrap(tpcf_ctx* c, int32_t n_field, const 
     if (nblk == 0) check(cudaMemsetAsync(dout, 0, sizeof(double) * sums.size(), st), "memset");
     unsigned* derr = (unsigned*)ws_alloc(c, sizeof(unsigned));
     check(cudaMemsetAsync(derr, 0, sizeof(unsigned), st), "memset");
-    const int MG = marks_group(nb);
     PassTimer timer(c);
+    const int MG = n_launch * kMapGroup;
     for (int s0 = 0; s0 < n_boot; s0 += MG) {
-      const int G = std::min(MG, n_boot - s0);
+      const int G = std::min(MG, n_boot - s0), n_pass = (G + kMapGroup - 1) / kMapGroup;
       const int* mult;
       if (multiplicity) {
         mult = dmult_all + (size_t)s0 * n_units;
@@ -1005,9 +1072,10 @@ extern "C" tpcf_status tpcf_marks_bootstrap(tpcf_ctx* c, int32_t n_field, const 
                 "bootstrap partials");
         timer.mark(st);
         if (!multiplicity) draws.used((n_buf == 2 ? (s0 / MG) & 1 : 0));
-        if (++kept == n_keep || s0 + G == n_boot) {
-          counted(c, launch_marks_reduce(part, df, n_field, nblk, kept, G, R,
-                                         dout + (size_t)(s0 - (kept - 1) * MG) * n_field * R, st),
+        kept += n_pass;
+        if (kept == n_keep || s0 + G == n_boot) {
+          counted(c, launch_marks_reduce(part, df, n_field, nblk, kept, G - (n_pass - 1) * kMapGroup, R,
+                                         dout + (size_t)(s0 / kMapGroup + n_pass - kept) * kMapGroup * n_field * R, st),
                   "bootstrap reduce");
           kept = 0;
         }
