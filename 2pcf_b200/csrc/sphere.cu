@@ -16,7 +16,7 @@
 // at any separation).  The FP64 guard band re-bins a pair by the canonical
 // rule: u = hi + lo in FP64, c^2 = (dx^2 + dy^2) + dz^2 rounded as written.
 // The one-bin and one-edge sub-chunk paths run on packed FP32 instructions
-// (two pairs per instruction) over tiles rewritten in place into SrcPairS.
+// (two pairs per instruction) over sub-chunks laid out in pair form in HBM (ChunkS).
 //
 // Pruning: a cell grid over (lambda reduced to [0, 2 pi), phi).  The rows of a
 // work item are the phi rows within R of the lens box (angular distance
@@ -513,7 +513,9 @@ __host__ __device__ inline size_t sph_edge_smem(int nb) { return ((size_t)(nb + 
 // copied for a block of 128 lenses and rewritten into pair form there, between
 // two barriers (barrier stall 1.1 per issued instruction).  Twelve warps per SM
 // (the shared-memory occupancy at 20 bins), up to 168 registers.
-// 100 k x 500 k on the sky, theta_max 200': SKYNOW.
+// 100 k x 500 k on the sky, theta_max 200': 13.7 ms for the call with the block-wide form, 10.34 now
+// (two-edge path and items split by cell rows 10.8, warps on their own 10.67, the
+// d2 - E form of the edge paths 10.34).
 template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB>
 __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
   constexpr int QA = (MODE == 0 && HAS_M) ? 6 : 5;
