@@ -784,6 +784,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   // workload reached 1.05e-6 of its sum|terms|)
   P.flush_src = lens_acc ? 1024 : 4096;
   P.far_bin = series_far_bin(e2.data(), nb);
+  int bt_pairs = bt;  // of k_pairs
+  if (!sph && B.variant == 0 && c->opts.group_size == 0 && c->opts.tile_chunks == 0) pair_tile_shape(nb, qa, &bt_pairs, &tch);
   P.debug_skip_tile = c->skip_tile + 1;
   P.wait_limit = c->wait_limit;
   for (int k = 0; k < 2; ++k) {
@@ -795,7 +797,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     if (k == 1)
       counted(c, prepare_pairs_series(B.P[k], mode, has_m, has_z, logb, bt, c->num_sms, &B.L[k]), "pair kernel");
     else
-      counted(c, prepare_pairs(B.P[k], mode, has_m, has_z, logb, bt, tch, B.variant, c->num_sms, &B.L[k]), "pair kernel");
+      counted(c, prepare_pairs(B.P[k], mode, has_m, has_z, logb, bt_pairs, tch, B.variant, c->num_sms, &B.L[k]), "pair kernel");
   }
 
   B.mode = mode; B.sph = sph; B.sharded = sharded; B.use_patch_any = use_patch_any;

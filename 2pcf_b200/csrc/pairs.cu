@@ -31,6 +31,7 @@
 // n_pairs is identical to the FP64 rule of tpcf_canonical_edges.  Other
 // spacings binary-search the FP32 squared edges with a relative guard band.
 
+#include <algorithm>
 #include <cub/cub.cuh>
 #include <cstdio>
 
@@ -51,17 +52,16 @@ namespace tpcf {
 
 constexpr int kDualUnroll = TPCF_DUAL_UNROLL;      // source-loop unrolling of the edge paths
 constexpr int kSingleUnroll = TPCF_SINGLE_UNROLL;  // and of the single-bin path
-// Blocks per SM that the pair kernel is compiled for: the shared-memory
+// Warps per SM that the pair kernel is compiled for: the shared-memory
 // occupancy of 128 threads at 20 bins (51 KB histogram + tiles).  Declaring it
-// gives the compiler a register budget (up to 170 per thread) that it spends
+// gives the compiler a register budget (up to 168 per thread) that it spends
 // on overlapping the packed FP32 chains of the register paths.
-constexpr int kPairMinBlocks = 3;
+constexpr int kPairWarps = 12;
 // Coordinate of the null source that pads the last sub-chunk of a grid: its
 // d2 (~2e36) stays finite in FP32 and its weight and values are zero.
 constexpr float kNullPos = 1.0e18f;
-// Source bytes in flight per warp: NBUF = kWarpRing / (TCH KB) tile buffers
-// of TCH sub-chunks (1 KB each) plus their ChunkMeta.
-constexpr int kWarpRing = 4096;
+// Tile buffers per warp: TCH sub-chunks (1 KB each) plus their ChunkMeta each.
+constexpr int kPairBuf = 2;
 constexpr int kRowsPerPass = 32;  // cell rows whose spans a warp holds at once (one per lane)
 
 // ------------------------------------------------------- shared-memory map --
@@ -76,7 +76,7 @@ __host__ __device__ inline size_t ring_buffer_bytes(int tch) {
 // bt is the number of threads (histogram columns), tch the sub-chunks per tile.
 __host__ __device__ inline PairSmem pair_smem_layout(int nb, int qa, int bt, int tch) {
   const int nw = bt / 32;
-  const int nbuf = kWarpRing / (tch * kChunk * (int)sizeof(SrcRec));
+  const int nbuf = kPairBuf;
   PairSmem s;
   size_t o = 0;
   s.ring = o;  o += (size_t)nw * nbuf * ring_buffer_bytes(tch);
@@ -410,10 +410,9 @@ extern "C" int tpcf_debug_mode_stats(unsigned long long* out) {
 // PATH 0: sub-chunk classification with the register paths (default);
 // PATH 1: per-pair binning for every pair in reach (for A/B measurement).
 template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB, int BT, int TCH, int PATH>
-__global__ void __launch_bounds__(BT, kPairMinBlocks) k_pairs(const PairParams P) {
+__global__ void __launch_bounds__(BT, kPairWarps * 32 / BT) k_pairs(const PairParams P) {
   constexpr int QA = (MODE == 0 && HAS_M) ? 6 : 5;
-  constexpr int NBUF = kWarpRing / (TCH * kChunk * (int)sizeof(SrcRec));
-  static_assert(NBUF >= 2, "at least two tile buffers per warp");
+  constexpr int NBUF = kPairBuf;
   constexpr size_t BUFB = (size_t)TCH * (kChunk * sizeof(SrcRec) + sizeof(ChunkMeta));
   const int nb = P.nb;
   const int tid = threadIdx.x;
@@ -1139,8 +1138,8 @@ static cudaError_t prepare_pairs_t(const PairParams& P, int num_sms, PairLaunch*
 }
 
 // Tile shapes: bt threads per block (128, 64 or 32; each warp takes 32-lens
-// work items of its own) and tch sub-chunks per source tile (2: two 2.1 KB
-// buffers per warp; 1: four 1.1 KB buffers).  variant 1 forces per-pair binning
+// work items of its own) and tch sub-chunks per source tile (two
+// buffers of tch x 1.1 KB per warp).  variant 1 forces per-pair binning
 // (A/B measurement).
 template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB>
 static cudaError_t prepare_pairs_bt(const PairParams& P, int bt, int tch, int variant, int num_sms, PairLaunch* L) {
@@ -1155,6 +1154,26 @@ static cudaError_t prepare_pairs_bt(const PairParams& P, int bt, int tch, int va
 }
 
 size_t pair_smem_bytes(int nb, int qa, int bt, int tch) { return pair_smem_layout(nb, qa, bt, tch).total; }
+
+// Tile shape of a call that sets none, at most *bt threads: the one that keeps
+// the most warps on an SM (228 KB of shared memory, 1 KB of it per block; 12 warps
+// by registers); among equals the one with the longest tiles and largest blocks,
+// whose per-tile work is least.  128 threads x 2 sub-chunks keep 12 warps up to 20
+// bins and 8 beyond or, with shear calibration (a sixth sum per bin), from 18 bins
+// on; there 128 x 1 or 64 x 2 keep 10 or 12: 100 k lenses x 500 k sources, 20
+// bins, shear calibration: kernel 7.91 -> 7.17 ms with 128 x 1; 60 k x
+// 300 k, 35 bins: 4.6 -> 3.34 ms.
+void pair_tile_shape(int nb, int qa, int* bt, int* tch) {
+  const int shapes[4][2] = {{128, 2}, {128, 1}, {64, 2}, {32, 2}};
+  const int bt_max = *bt;
+  int best = 0;
+  for (const auto& s : shapes) {
+    if (s[0] > bt_max) continue;
+    const int blocks = (int)((size_t)(228 * 1024) / (pair_smem_bytes(nb, qa, s[0], s[1]) + 1024));
+    const int warps = std::min(blocks * s[0] / 32, kPairWarps);
+    if (warps > best) best = warps, *bt = s[0], *tch = s[1];
+  }
+}
 
 cudaError_t prepare_pairs(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int bt, int tch,
                           int variant, int num_sms, PairLaunch* L) {

@@ -9,6 +9,7 @@
 namespace tpcf {
 
 size_t pair_smem_bytes(int nb, int qa, int bt, int tch);
+void pair_tile_shape(int nb, int qa, int* bt, int* tch);
 // bt = lenses per group (threads per block), tch = 32-source sub-chunks per
 // source tile; variant 1 bins every pair one by one (A/B measurement).
 cudaError_t launch_pairs(const PairParams& P, int mode, bool has_m, bool has_z, bool logb, int bt, int tch,
