@@ -413,7 +413,7 @@ bool series_pays(int n_valid, double ex, double ey, const tpcf_bins* bins, const
 
 // A task with fewer lens groups than kSplitItems / 2 is cut into several items
 // per group (at most kMaxSplit).
-constexpr int kSplitItems = 8192, kMaxSplit = 8;
+constexpr int kSplitItems = 8192;
 constexpr size_t kSplitLensBytes = (size_t)256 << 20;  // per-lens sums of a split task at most
 
 void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<SrcIn> srcs, const std::vector<int>& tl,

@@ -90,6 +90,9 @@ struct LensDesc {
   const float4* pos;        // sphere: {hi.xyz, 0}, {lo.xyz, 0} per sorted lens, else nullptr
 };
 
+// Items that a lens group of a task is cut into at most.
+constexpr int kMaxSplit = 8;
+
 struct TaskDesc {
   int lens_cat;
   int src_cat;

@@ -1,0 +1,47 @@
+"""Per-lens outputs, transposed bin chunk by bin chunk on the way out: bin counts
+around the chunk (20 bins), lens counts around a block's 32, outputs on the host
+and on the device, one patch and several.  The per-lens bars are those of
+test_gpu_pairs; counts are exact."""
+import numpy as np
+import pytest
+
+from conftest import uniform_shear
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nb", [1, 19, 20, 21, 45])
+@pytest.mark.parametrize("n", [1, 31, 33, 1000])
+def test_against_brute_force(tpcf, oracle, ctx, nb, n):
+    L, S = uniform_shear(n, 700, 100.0, 300 + nb + n, w="uniform")
+    if n > 1:
+        L["w"][::9] = 0.0
+    bins = tpcf.create_bins(1.0, 60.0, nb)
+    res = tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"], S["e1"],
+                                     S["e2"], S["w"], S["m"], bins, calculate_marks=True, lens_sums=True, ctx=ctx)
+    lens = oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq, lens_idx=np.arange(n))["lens"]
+    got = res.lens_sums
+    np.testing.assert_array_equal(got[:, 5], lens[:, 5])
+    # 1e-6 of the lens's sums of term bounds: the terms themselves for the positive
+    # quantities, |val| |e| w for the rotated ones
+    bound = np.abs(lens)
+    bound[:, 1] = bound[:, 2] = np.abs(L["val"])[:, None] * np.hypot(S["e1"], S["e2"]).max() * lens[:, 3]
+    assert np.all(np.abs(got[:, :5] - lens[:, :5]) <= 1e-6 * bound[:, :5])
+    # the FP32 marks are the FP64 sums rounded once
+    for marks, q in ((res.xi_E_marks, 1), (res.xi_B_marks, 2), (res.w_marks, 3), (res.K_marks, 4)):
+        np.testing.assert_array_equal(marks, got[:, q].astype(np.float32))
+    np.testing.assert_allclose(res.marks_weight, got[:, 3].sum(1), rtol=1.2e-7)
+
+
+def test_large_host_outputs(tpcf, ctx):
+    """More per-lens output than the staging pieces hold at once (64 MiB)."""
+    n, nb = 90_000, 20
+    L, S = uniform_shear(n, 400, 300.0, 77)
+    bins = tpcf.create_bins(1.0, 60.0, nb)
+    res = tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"], S["e1"],
+                                     S["e2"], S["w"], S["m"], bins, calculate_marks=False, lens_sums=True, ctx=ctx)
+    assert res.lens_sums.nbytes > 64 << 20
+    np.testing.assert_array_equal(res.lens_sums[:, 5].sum(0), res.n_pairs)
+    for i in range(0, n, 9973):
+        d2 = (np.float64(L["x"][i]) - S["x"]) ** 2 + (np.float64(L["y"][i]) - S["y"]) ** 2
+        np.testing.assert_array_equal(res.lens_sums[i, 5], np.histogram(d2, bins.bin_edges_sq)[0])
