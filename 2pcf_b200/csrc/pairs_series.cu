@@ -45,9 +45,10 @@ namespace tpcf {
 
 namespace {
 
-// 14 warps per SM at 144 registers: the tomography call (25 tasks, 1.24e12
-// pairs) takes 869 ms against 952 ms with 12 warps at 168 registers and 16 warps
-// at 128 registers gain nothing more.
+// At least 14 warps per SM, at most 144 registers: the tomography call (25 tasks,
+// 1.24e12 pairs) takes 869 ms against 952 ms with 12 warps at 168 registers; where
+// the compiler needs 128 or less, as without z cut and calibration, 16 warps fit
+// and gain nothing more.
 constexpr int kSeriesThreads = 64, kSeriesBlocks = 7;
 constexpr float kFarRatio = 0.08f;
 constexpr float kNullPos = 1.0e18f;  // coordinate of a source that takes no part: every term stays finite

@@ -41,7 +41,7 @@ FLOP_PER_PAIR = 26  # shear-scalar, FMA = 2, MUFU = 1 (per binned pair)
 # DRAM bytes read + written by one pair-kernel launch of the default workload,
 # per grid cell side theta_max/D (one-pass ncu captures of
 # dram__bytes_read.sum + dram__bytes_write.sum)
-K_PAIRS_DRAM_BYTES = {16: 69.567e9 + 0.403e9, 24: 68.311e9 + 0.409e9, 32: 65.525e9 + 0.403e9}
+K_PAIRS_DRAM_BYTES = {16: 54.885e9 + 0.163e9}
 SPH_FLOP_PER_PAIR = 52  # spherical shear-scalar: hi/lo unit-vector differences, east/north projection, angle series
 WORKLOAD_DESC = ("tomography: 5 shear bins (0.2,0.5,1.0,1.9,4.0 M) x 5 scalar bins "
                  "(0.1,0.2,0.4,0.7,1.0 M) = 10.0 M objects, 25 cross-pairs in one launch, "
@@ -267,7 +267,7 @@ def marks_timing(tpcf, stream, nb):
         "fallback 6650 GB/s (MEASURED_PEAKS.json absent)"
     p64 = mctx.measure_fp64_peak()
     out["marks_reweight"] = {"maps": n_map, "lenses": n, "n_bin": nbm, "call_ms": ms, "kernel_ms": kms,
-                             "kernel": "k_marks_dmma (FP64 mma.sync m8n8k4)",
+                             "kernel": "k_marks_dmma (FP64 mma.sync m16n8k16)",
                              "call_hbm_frac": byt / (ms * 1e-3) / 1e9 / hbm,
                              "fp64_frac": n * (3 * nbm + 1) * n_map * 2 / (kms * 1e-3) / 1e12 / p64,
                              "roofline": {"bound": "hbm", "achieved": byt / (kms * 1e-3) / 1e9, "peak": hbm,
@@ -573,7 +573,7 @@ def config_timing(k, tpcf, stream, peak, steps=3, warmup=2, with_cpu=True, cpu_s
            "e2e": {"value": pairs_e2e / (ms_e2e * 1e-3) / 1e9, "unit": UNIT, "ms_per_step": ms_e2e,
                    "h2d_bytes_per_step": int(h2d)},
            "roofline": {"bound": "fp32", "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
-                        "kernel": "k_pairs", "kernel_ms": kms,
+                        "kernel": "k_pairs_series" if k in (2, 3) else "k_pairs", "kernel_ms": kms,
                         "flop_per_pair": KAPPA_FLOP_PER_PAIR if k == 2 else
                         ("26 shear, 14 scalar" if k == 1 else FLOP_PER_PAIR)},
            "autotune_ms_per_gpair": {"cell": {f"theta_max/{d}": round(v, 3) for d, v in tune["cell"].items()},
@@ -899,7 +899,7 @@ def main():
         "e2e": {"value": pairs_e2e / (ms_e2e * 1e-3) / 1e9, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h)},
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                     "frac": achieved / peak, "traffic": traffic, "kernel": "k_pairs_sph" if sphere else "k_pairs",
+                     "frac": achieved / peak, "traffic": traffic, "kernel": "k_pairs_sph" if sphere else "k_pairs_series",
                      "flop_per_pair": fpp, "kernel_ms": pair_ms,
                      "peak_source": "measured in this run: FFMA loop (tpcf_measure_fp32_peak); "
                                     "MEASURED_PEAKS.json has no FP32 figure"},
