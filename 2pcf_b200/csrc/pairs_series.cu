@@ -765,7 +765,9 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
   if (lane == 0) {
     float4* o4 = reinterpret_cast<float4*>(out);
     o4[0] = make_float4(mnx, mny, mxx, mxy);
-    o4[1] = make_float4(cx, cy, rad, (float)((double)rad * rad / ((double)kFarRatio * kFarRatio)));
+    // never 0: a lens on the centre of a sub-chunk without extent has no series
+    const float far2 = (float)((double)rad * rad / ((double)kFarRatio * kFarRatio));
+    o4[1] = make_float4(cx, cy, rad, fmaxf(far2, 1.17549435e-38f));
     o4[2] = make_float4((float)sp, (float)sq, (float)sw, (float)sk);
     o4[3] = make_float4(mnz, mxz, 0.f, 0.f);
   }

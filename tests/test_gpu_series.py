@@ -108,3 +108,23 @@ def test_patches_and_mixed_batch(tpcf, oracle, ctx):
         one = tpcf.batch_shear_2pcf([lc], [sc[i]], [(0, 0)], bins, lens_patches=[lab], n_patch=5, ctx=ctx)[0]
         np.testing.assert_array_equal(one.patch_sums, both[i].patch_sums)
         np.testing.assert_array_equal(both[i].patch_sums[:, 5].sum(0), both[i].n_pairs)
+
+
+@pytest.mark.parametrize("n_same", [31, 32, 64])
+def test_coincident_sources_fill_a_sub_chunk(tpcf, oracle, ctx, n_same):
+    """Sources on one point, the first of the sorted catalogue (its lowest corner), and
+    a lens on the same point: with bins from 0 those pairs count, their d is 0 and their
+    g terms are 0/0 in bin 0 and nowhere else, also where they fill whole sub-chunks."""
+    L, S = catalogues(77, 66)
+    S["x"], S["y"] = f32(np.maximum(S["x"], 0.25)), f32(np.maximum(S["y"], 0.25))
+    S["x"][:n_same], S["y"][:n_same] = 0.0, 0.0
+    L["x"][5], L["y"][5] = 0.0, 0.0
+    bins = tpcf.create_bins(0.0, 20.0, 5, spacing="lin")
+    res = shear(tpcf, ctx, L, S, bins)
+    can = oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq)
+    np.testing.assert_array_equal(res.n_pairs, can["n_pairs"].astype(np.int64))
+    assert np.isnan(res.sum_gt[0]) and np.isnan(res.sum_gx[0])
+    assert np.all(np.abs(res.sum_gt[1:] - can["sum_gt"][1:]) <= 1e-6 * can["abs_gt"][1:])
+    assert np.all(np.abs(res.sum_gx[1:] - can["sum_gx"][1:]) <= 1e-6 * can["abs_gx"][1:])
+    np.testing.assert_allclose(res.sum_dw, can["sum_dw"], rtol=1e-6)
+    np.testing.assert_allclose(res.sum_w, can["sum_w"], rtol=1e-6)
