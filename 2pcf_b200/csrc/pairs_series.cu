@@ -94,7 +94,7 @@ __host__ __device__ inline WarpSmem warp_smem(int nb, int nt, int qa, int rec_fl
   size_t o = 0;
   s.ring = o; o += (size_t)kNbuf * kTch * rec_floats * sizeof(float);
   s.hist = o; o += (size_t)nt * qa * 32 * sizeof(float);
-  s.wsum = o; o += (size_t)kQ * nb * sizeof(double);
+  s.wsum = o; o += ((size_t)kQ * nb + 2) * sizeof(double);  // then the scales of the lens factors
   o = (o + 15) / 16 * 16;
   s.lxy = o;  o += 16 * kLpl * sizeof(float4);
   s.lf = o;   o += 16 * kLpl * sizeof(float4);
@@ -133,6 +133,14 @@ __device__ __noinline__ bool above_edge(float lx, float ly, float sx, float sy, 
   const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
   return e == nb ? d2 > e2[e] : d2 >= e2[e];
 }
+
+// Biased exponent of v, 0 for an infinity or NaN.
+__device__ __forceinline__ unsigned exponent_of(double v) {
+  const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+  return e == 0x7ffu ? 0u : e;
+}
+// The power of two with biased exponent e (1 .. 2046).
+__device__ __forceinline__ double pow2_biased(unsigned e) { return __hiloint2double((int)(e << 20), 0); }
 
 struct LaneSrc {
   float x, y, p, q, w, K, z;
@@ -387,22 +395,43 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
     const GridDesc G = P.grids[T.src_cat];
     const int g = it.y / T.split, part_i = it.y - g * T.split;
     const int gs = LD.group_start[g], nl = LD.group_start[g + 1] - gs;
-    // lenses lane and lane + 32 of the group
+    // lenses lane and lane + 32 of the group.  Their factors val w (formed in FP64)
+    // and w enter the FP32 terms, so the group's are scaled by a power of two to at
+    // most 2 and the item's FP64 sums scaled back: products of very small or very
+    // large lens and source weights stay in range.
     float lx[kLpl], ly[kLpl], lz[kLpl], vw[kLpl], w[kLpl];
+    double fv[kLpl], fw[kLpl];
+    unsigned xv = 0, xw = 0;
     bool act[kLpl];
 #pragma unroll
     for (int l = 0; l < kLpl; ++l) {
       const int i = lane + 32 * l;
       act[l] = i < nl;
-      lx[l] = ly[l] = lz[l] = vw[l] = w[l] = 0.f;
+      lx[l] = ly[l] = lz[l] = 0.f;
+      fv[l] = fw[l] = 0.0;
       if (act[l]) {
         const float4 r = LD.rec[gs + i];
         lx[l] = r.x;
         ly[l] = r.y;
-        vw[l] = r.z * r.w;
-        w[l] = r.w;
+        fv[l] = (double)r.z * (double)r.w;
+        fw[l] = (double)r.w;
         if (HAS_Z) lz[l] = LD.z[gs + i];
       }
+      xv = max(xv, exponent_of(fv[l]));
+      xw = max(xw, exponent_of(fw[l]));
+    }
+    xv = __reduce_max_sync(0xffffffffu, xv);
+    xw = __reduce_max_sync(0xffffffffu, xw);
+    xv = xv ? xv : 1023u;
+    xw = xw ? xw : 1023u;
+#pragma unroll
+    for (int l = 0; l < kLpl; ++l) {
+      vw[l] = (float)(fv[l] * pow2_biased(2046u - xv));
+      w[l] = (float)(fw[l] * pow2_biased(2046u - xw));
+    }
+    if (lane == 0) {
+      wsum[kQ * nb] = pow2_biased(xv);
+      wsum[kQ * nb + 1] = pow2_biased(xw);
     }
     for (int e = lane; e < kQ * nb; e += 32) wsum[e] = 0.0;
     __syncwarp();
@@ -681,8 +710,9 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
     fold_far<QA>(hist, wsum, nb, tb, lane);
     double* out = P.item_sums + (size_t)(T.item_base + it.y) * kQ * nb;
     for (int e = lane; e < kQ * nb; e += 32) {
-      const int src = (e / nb == QK && QA == 5) ? e - (QK - QW) * nb : e;
-      out[e] = wsum[src];
+      const int q = e / nb;
+      const int src = (q == QK && QA == 5) ? e - (QK - QW) * nb : e;
+      out[e] = wsum[src] * (q == QN ? 1.0 : wsum[kQ * nb + (q == QGT || q == QGX ? 0 : 1)]);
     }
     __syncwarp();
   }

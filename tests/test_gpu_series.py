@@ -128,3 +128,16 @@ def test_coincident_sources_fill_a_sub_chunk(tpcf, oracle, ctx, n_same):
     assert np.all(np.abs(res.sum_gx[1:] - can["sum_gx"][1:]) <= 1e-6 * can["abs_gx"][1:])
     np.testing.assert_allclose(res.sum_dw, can["sum_dw"], rtol=1e-6)
     np.testing.assert_allclose(res.sum_w, can["sum_w"], rtol=1e-6)
+
+
+@pytest.mark.parametrize("lens_w,src_w,val", [(1e-25, 1e-25, 1.0), (1e-20, 1e-15, 1e-25), (1e22, 1e25, 1.0),
+                                              (1e30, 1e-30, 1e30)])
+def test_very_small_and_large_weights(tpcf, oracle, ctx, lens_w, src_w, val):
+    """Weights in physical units: lens and source factors that each fit FP32 while
+    their product does not."""
+    L, S = catalogues(78, 130)
+    L["w"], L["val"], S["w"] = f32(L["w"] * lens_w), f32(L["val"] * val), f32(S["w"] * src_w)
+    bins = tpcf.create_bins(0.3, 25.0, 8)
+    res = shear(tpcf, ctx, L, S, bins)
+    check_sums(f"series weights {lens_w} {src_w} {val}", res,
+               oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
