@@ -757,7 +757,7 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     const int li = t.lens, si = nL + t.src;
     if (hc[li] > 0 && hc[si] > 0 && hb[8 * li + 5] > hb[8 * si + 4]) has_z = true;
   }
-  const bool logb = bins->spacing == TPCF_LOG;
+  const bool logb = bins->spacing == TPCF_LOG && e2[0] >= kMinLogD2;
   const double Rd = bins->x_max;
   const float R = (float)(Rd * (1.0 + 1e-6));
 

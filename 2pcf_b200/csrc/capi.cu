@@ -514,7 +514,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     }
   }
   // On the sphere log binning maps theta^2 by a series valid for chords <= 0.25.
-  const bool logb = bins->spacing == TPCF_LOG && (!sph || e2[nb] <= 0.0625);
+  const bool logb = bins->spacing == TPCF_LOG && e2[0] >= kMinLogD2 && (!sph || e2[nb] <= 0.0625);
   const int qa = has_m ? 6 : 5;
   int bt = 128;
   while (bt > 32 && (size_t)nb * qa * bt * 4 > 100 * 1024) bt /= 2;

@@ -143,7 +143,7 @@ tpcf_status run_noalloc(tpcf_ctx* c, const float* xA, const float* yA, const flo
 
   const bool has_m = mB != nullptr && hcnt[1] > 0 && hbox[8 + 6] != 0.f;
   const bool has_z = hcnt[0] > 0 && hcnt[1] > 0 && hbox[5] > hbox[8 + 4];
-  const bool logb = bins->spacing == TPCF_LOG;
+  const bool logb = bins->spacing == TPCF_LOG && e2[0] >= kMinLogD2;
   const int qa = has_m ? 6 : 5;
   int bt = 128;
   while (bt > 32 && (size_t)nb * qa * bt * 4 > 100 * 1024) bt /= 2;

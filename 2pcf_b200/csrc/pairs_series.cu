@@ -52,6 +52,7 @@ namespace {
 constexpr int kSeriesThreads = 64, kSeriesBlocks = 7;
 constexpr float kFarRatio = 0.08f;
 constexpr float kNullPos = 1.0e18f;  // coordinate of a source that takes no part: every term stays finite
+constexpr float kMinNormal = 1.17549435e-38f;
 constexpr int kRows = 32;            // cell rows whose spans a warp holds at once (one per lane)
 constexpr int kTch = 3;              // sub-chunks per tile
 // Lenses per lane (a work item holds 64 lenses): the per-sub-chunk work and the
@@ -154,7 +155,8 @@ struct Terms {
   float2 d2, d, Pn, qq, rv, wv, one;
 };
 template <int MODE, bool HAS_Z, bool LOGB>
-__device__ __forceinline__ Terms pair_terms(const float4 a, const float4 f, const float2 lz, const LaneSrc& S) {
+__device__ __forceinline__ Terms pair_terms(const float4 a, const float4 f, const float2 lz, const LaneSrc& S,
+                                            float tiny) {
   Terms T;
   const float2 dx = add2(dup2(S.x), lo2(a));
   const float2 dy = add2(dup2(S.y), hi2(a));
@@ -162,15 +164,17 @@ __device__ __forceinline__ Terms pair_terms(const float4 a, const float4 f, cons
   T.d2 = fma2(dy, dy, dx2);
   float2 r;
   if (LOGB) {
-    // d2 = 0 is below the first edge; the offset only keeps its terms finite
-    const float2 e2 = add2(T.d2, dup2(1e-30f));
+    // d2 = 0 is below the first edge; the offset (1e-9 of that edge) only keeps its
+    // terms finite
+    const float2 e2 = add2(T.d2, dup2(tiny));
     const float2 rs = make_float2(rsqrt_ftz(e2.x), rsqrt_ftz(e2.y));
     T.d = mul2(T.d2, rs);
     r = mul2(rs, rs);
   } else {
     // one Newton step each on sqrt and 1/d^2 (within 1 ulp); d2 = 0 gives
     // d = 0 and r = 0 (the caller sees to its 0/0)
-    const float2 rs = make_float2(T.d2.x > 0.f ? rsqrt_ftz(T.d2.x) : 0.f, T.d2.y > 0.f ? rsqrt_ftz(T.d2.y) : 0.f);
+    const float2 rs = make_float2(T.d2.x >= kMinNormal ? rsqrt_ftz(T.d2.x) : 0.f,
+                                  T.d2.y >= kMinNormal ? rsqrt_ftz(T.d2.y) : 0.f);
     const float2 dd = mul2(T.d2, rs);
     T.d = fma2(fma2(make_float2(-dd.x, -dd.y), dd, T.d2), mul2(rs, dup2(0.5f)), dd);
     const float2 r0 = mul2(rs, rs);
@@ -227,7 +231,7 @@ __device__ __forceinline__ void direct_sums(const float4* lxy, const float4* lf,
   const int np = (cnt + 1) >> 1;
 #pragma unroll(NE < 2 ? 4 : 1)
   for (int i = 0; i < np; ++i) {
-    const Terms T = pair_terms<MODE, HAS_Z, LOGB>(lxy[i], lf[i], HAS_Z ? lz[i] : make_float2(0.f, 0.f), S);
+    const Terms T = pair_terms<MODE, HAS_Z, LOGB>(lxy[i], lf[i], HAS_Z ? lz[i] : make_float2(0.f, 0.f), S, C.tiny);
     if (HAS_Z) A[0].n = add2(A[0].n, T.one), last_one = T.one.x;
     if (!LOGB) dmin = fminf(dmin, fminf(T.one.x > 0.f ? T.d2.x : 1.f, T.one.y > 0.f ? T.d2.y : 1.f));
     float2 ra = T.rv, wa = T.wv;  // at or above the edge below side k
@@ -255,7 +259,7 @@ __device__ __forceinline__ void direct_sums(const float4* lxy, const float4* lf,
 #pragma unroll 1
     for (int i = 0; i < np; ++i) {
       const float4 a = lxy[i];
-      const Terms T = pair_terms<MODE, HAS_Z, LOGB>(a, lf[i], HAS_Z ? lz[i] : make_float2(0.f, 0.f), S);
+      const Terms T = pair_terms<MODE, HAS_Z, LOGB>(a, lf[i], HAS_Z ? lz[i] : make_float2(0.f, 0.f), S, C.tiny);
 #pragma unroll
       for (int k = 0; k < NE; ++k) {
         const float2 t = add2(T.d2, dup2(-E[k]));
@@ -377,6 +381,7 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
   C.eps_rel = kEdgeBand;
   C.lo_g = e2f[0] * (1.f - P.eps);
   C.hi_g = e2f[nb] * (1.f + P.eps);
+  C.tiny = e2f[0] * 1e-9f;
 
   const uint32_t wait_limit = P.wait_limit ? P.wait_limit : kWaitPolls;
   int ring_t = 0;        // ring index of the next tile this warp consumes
@@ -512,7 +517,7 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
             Zx[l] = cen.x - lx[l];
             Zy[l] = cen.y - ly[l];
             Z2[l] = fmaf(Zy[l], Zy[l], Zx[l] * Zx[l]);
-            rs[l] = rsqrt_ftz(fmaxf(Z2[l], 1e-30f));
+            rs[l] = rsqrt_ftz(fmaxf(Z2[l], kMinNormal));
             dc[l] = Z2[l] * rs[l];
             in[l] = bin_range<LOGB>(dc[l], cen.z, C, b0[l], b1[l]) && act[l];
             bool zall = true;
@@ -797,7 +802,7 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
     o4[0] = make_float4(mnx, mny, mxx, mxy);
     // never 0: a lens on the centre of a sub-chunk without extent has no series
     const float far2 = (float)((double)rad * rad / ((double)kFarRatio * kFarRatio));
-    o4[1] = make_float4(cx, cy, rad, fmaxf(far2, 1.17549435e-38f));
+    o4[1] = make_float4(cx, cy, rad, fmaxf(far2, kMinNormal));
     o4[2] = make_float4((float)sp, (float)sq, (float)sw, (float)sk);
     o4[3] = make_float4(mnz, mxz, 0.f, 0.f);
   }

@@ -256,14 +256,14 @@ __device__ __forceinline__ LensS2 lens_pack(const LensS& L) {
 // sph_terms for the two sources of one SrcPairS (packed FP32; each half
 // equals the scalar computation: a.x - h.x = a.x + (-h.x)).
 template <int MODE, bool SMALL>
-__device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, float2& d2, float2& th, float2& r,
-                                           float2& X, float2& Y) {
+__device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, float tiny, float2& d2, float2& th,
+                                           float2& r, float2& X, float2& Y) {
   const float2 dx = add2(add2(lo2(s.hxy), L.nhx), add2(lo2(s.lxy), L.nlx));
   const float2 dy = add2(add2(hi2(s.hxy), L.nhy), add2(hi2(s.lxy), L.nly));
   const float2 dz = add2(add2(lo2(s.hzp), L.nhz), add2(lo2(s.lzq), L.nlz));
-  // series path (log bins): d2 = 0 is below the first edge; the offsets only keep
-  // its masked terms finite
-  d2 = fma2(dz, dz, fma2(dy, dy, SMALL ? fma2(dx, dx, dup2(1e-30f)) : mul2(dx, dx)));
+  // series path (log bins): d2 = 0 is below the first edge; the offsets (1e-9 of
+  // that edge) only keep its masked terms finite
+  d2 = fma2(dz, dz, fma2(dy, dy, SMALL ? fma2(dx, dx, dup2(tiny)) : mul2(dx, dx)));
   if (SMALL) {
     const float2 c = mul2(d2, make_float2(rsqrt_ftz(d2.x), rsqrt_ftz(d2.y)));
     th = mul2(c, fma2(d2, fma2(d2, fma2(d2, dup2(6.9754464e-4f), dup2(4.6875e-3f)), dup2(4.16666679e-2f)),
@@ -274,7 +274,7 @@ __device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, f
   if (MODE == 0) {
     const float2 A = fma2(dy, L.ey, mul2(dx, L.ex));
     const float2 B = fma2(dz, L.nz, fma2(dy, L.ny, mul2(dx, L.nx)));
-    const float2 A2 = SMALL ? fma2(A, A, dup2(1e-30f)) : mul2(A, A);
+    const float2 A2 = SMALL ? fma2(A, A, dup2(tiny)) : mul2(A, A);
     const float2 P = fma2(make_float2(-B.x, -B.y), B, A2);
     const float2 sq = fma2(B, B, A2);
     const float2 ab = mul2(A, B);
@@ -314,10 +314,10 @@ __device__ __forceinline__ void sph_acc_zero(SphAcc<NE>& A) {
 // are the sub-chunk's totals, so they are not accumulated here.
 template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, int NE, bool PART>
 __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPairS& s, bool a0, bool a1,
-                                         const float* E, SphAcc<NE>& A) {
+                                         float tiny, const float* E, SphAcc<NE>& A) {
   constexpr bool LI = !(HAS_Z || PART);
   float2 d2, th, r, X, Y;
-  sph_terms2<MODE, SMALL>(L, s, d2, th, r, X, Y);
+  sph_terms2<MODE, SMALL>(L, s, tiny, d2, th, r, X, Y);
   float2 w = lo2(s.wk), K = hi2(s.wk);
   bool v0 = true, v1 = true;
   if (HAS_Z) {
@@ -373,20 +373,21 @@ __device__ __forceinline__ void sph_totals(const SphAcc<NE>& A, const float4 ss,
 // The sources [lo, hi) of a sub-chunk (all 32 unless PART) against a lens.
 template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NE>
 __device__ __forceinline__ void sph_loop(const SrcPairS* __restrict__ S, int lo, int hi, const LensS2& L, float lz,
-                                         const float* E, SphAcc<NE>& A) {
+                                         float tiny, const float* E, SphAcc<NE>& A) {
   const int k0 = PART ? lo >> 1 : 0, k1 = PART ? (hi + 1) >> 1 : kChunk / 2;
 #pragma unroll 2
   for (int k = k0; k < k1; ++k)
-    sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, PART>(L, lz, S[k], !PART || 2 * k >= lo, !PART || 2 * k + 1 < hi, E, A);
+    sph_step<MODE, HAS_M, HAS_Z, SMALL, NE, PART>(L, lz, S[k], !PART || 2 * k >= lo, !PART || 2 * k + 1 < hi, tiny, E, A);
 }
 
 // Class 1: every pair of the chunk is in bin `blo`.
 template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NC, int QA>
 __device__ __forceinline__ void chunk_single_s(const SrcPairS* __restrict__ S, int lo, int hi, const LensS2& L,
-                                               float lz, int cls, int blo, float* __restrict__ hcol, const float4 ss) {
+                                               float lz, float tiny, int cls, int blo, float* __restrict__ hcol,
+                                               const float4 ss) {
   SphAcc<0> A;
   sph_acc_zero(A);
-  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, 0>(S, lo, hi, L, lz, nullptr, A);
+  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, 0>(S, lo, hi, L, lz, tiny, nullptr, A);
   if (cls != 1) return;
   float acc[QA];
   sph_totals<MODE, HAS_M, !(HAS_Z || PART), QA>(A, ss, acc);
@@ -406,7 +407,7 @@ __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, in
     E[e] = e < cls - 1 ? C.e2f[min(max(blo + 1 + e, 0), C.nb)] : 3.0e38f;
   SphAcc<NE> A;
   sph_acc_zero(A);
-  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, NE>(S, lo, hi, L, lz, E, A);
+  sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, NE>(S, lo, hi, L, lz, C.tiny, E, A);
   if (cls == 0) return;
   bool band = false;
 #pragma unroll
@@ -552,6 +553,7 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
   C.eps_rel = 4e-6f;
   C.lo_g = e2f[0] * (1.f - P.eps);
   C.hi_g = e2f[nb] * (1.f + P.eps);
+  C.tiny = e2f[0] * 1e-9f;
 
   const uint32_t wait_limit = P.wait_limit ? P.wait_limit : kWaitPolls;
   int ring_t = 0;        // ring index of the next sub-chunk this warp consumes
@@ -654,9 +656,9 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
         const float4 ss = ch->sum;
         if (m == 1) {
           if (partial)
-            chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, true, 32, QA>(Sc, lo, hi, LP, lz, cls, blo, hcol, ss);
+            chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, true, 32, QA>(Sc, lo, hi, LP, lz, C.tiny, cls, blo, hcol, ss);
           else
-            chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, false, 32, QA>(Sc, 0, kChunk, LP, lz, cls, blo, hcol, ss);
+            chunk_single_s<MODE, HAS_M, HAS_Z, SMALL, false, 32, QA>(Sc, 0, kChunk, LP, lz, C.tiny, cls, blo, hcol, ss);
         } else if (m == 2) {
           if (partial)
             chunk_edges_s<MODE, HAS_M, HAS_Z, SMALL, true, 32, QA, 1>(Sc, lo, hi, Lf, LP, lz, cls, blo, hcol, C, ss);

@@ -23,7 +23,8 @@ __device__ __forceinline__ float sum2(float2 v) { return v.x + v.y; }
 
 // MUFU reciprocal square root and logarithm without the denormal scaling of
 // the default forms (three more instructions each): their arguments are squared
-// distances, 0 or far above 1e-38; lg2 of 0 is -inf, rsqrt of 0 is inf.
+// distances, 0 or normal (log-spaced binning asks for kMinLogD2); lg2 of 0 is -inf,
+// rsqrt of 0 is inf.
 __device__ __forceinline__ float rsqrt_ftz(float v) {
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
@@ -174,6 +175,7 @@ struct BinCtx {
   float A, B, eps, one_m_eps;
   float eps_rel;     // relative guard on d2 around one FP32 edge (register paths)
   float lo_g, hi_g;  // generic: fast reject bounds e2f[0]*(1-eps), e2f[nb]*(1+eps)
+  float tiny;        // log spacing: 1e-9 of the lowest squared edge (k_pairs_series, k_pairs_sph)
   int nb;
   const double* e2s;
   const float* e2f;

@@ -19,6 +19,10 @@
 namespace tpcf {
 
 constexpr int kMaxBins = 128;
+// Log-spaced binning by lg2(d^2) takes squared distances from here on, where 1e-9
+// of them is still a normal FP32 number (separations above 3.4e-15); below, log
+// bins are searched like the other spacings.
+constexpr double kMinLogD2 = 1.2e-29;
 constexpr int kMaxRows = 256;   // cell rows scanned per chunk of one work item
 constexpr int kTile = 256;      // sources per shared-memory tile
 constexpr int kQ = 6;           // quantities per bin in item/patch/lens sums

@@ -141,3 +141,16 @@ def test_very_small_and_large_weights(tpcf, oracle, ctx, lens_w, src_w, val):
     res = shear(tpcf, ctx, L, S, bins)
     check_sums(f"series weights {lens_w} {src_w} {val}", res,
                oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
+
+
+@pytest.mark.parametrize("unit", [1e-13, 1e-16])
+@pytest.mark.parametrize("spacing,lo", [("log", 0.3), ("lin", 0.0)])
+def test_very_small_coordinates(tpcf, oracle, ctx, spacing, lo, unit):
+    """Positions and bins in a unit that makes squared separations tiny (still normal
+    FP32 numbers): relative accuracy as at any other scale."""
+    L, S = catalogues(79, 130)
+    for c in (L, S):
+        c["x"], c["y"] = f32(c["x"] * unit), f32(c["y"] * unit)
+    bins = tpcf.create_bins(lo * unit, 25.0 * unit, 8, spacing=spacing)
+    res = shear(tpcf, ctx, L, S, bins)
+    check_sums(f"series unit {unit} {spacing}", res, oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))

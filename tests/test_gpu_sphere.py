@@ -169,3 +169,15 @@ def test_latitude_out_of_range_is_rejected(tpcf, sctx):
     bins = tpcf.create_bins(1 * ARCMIN, 60 * ARCMIN, 4)
     with pytest.raises(tpcf.TPCFError):
         run_shear(tpcf, sctx, L, S, bins)
+
+
+def test_very_small_separations(tpcf, oracle, sctx):
+    """One log bin around 1e-13 rad at the origin, where FP32 positions are that fine:
+    the sub-chunks cross its two edges."""
+    rng = np.random.default_rng(21)
+    L, S = shear_cats(rng, 300, 2000, (0, 1, 0, 1), w="uniform")
+    for c in (L, S):
+        c["x"], c["y"] = f32(c["x"] * (1e-12 / D2R)), f32(c["y"] * (1e-12 / D2R))
+    bins = tpcf.create_bins(1e-14, 4e-13, 1)
+    res = run_shear(tpcf, sctx, L, S, bins, calculate_marks=False)
+    assert_parity(res, oracle.canon_sphere(oracle.SHEAR, L, S, bins.chord_edges_sq))
