@@ -285,8 +285,9 @@ __device__ __forceinline__ void chunk_single(const SrcPair* __restrict__ S, int 
 // its far side (h*[e]: d2 >= E_e); bin blo + j receives h[j-1] - h[j] with
 // h[-1] = all and h[NE] = 0.  The side of a pair is a 1.0/0.0 mask from the sign
 // of d2 - E, applied by multiplication.  The smallest |d2 - E| is kept per
-// edge: when it lies within the guard band, this lane drops its register sums
-// and bins the sub-chunk pair by pair by the canonical rule (rare).  A lane with fewer edges than NE
+// edge: when it lies within the guard band, or a sum is not finite (a pair with
+// d = 0), this lane drops its register sums and bins the sub-chunk pair by pair by
+// the canonical rule (rare).  A lane with fewer edges than NE
 // (class 1, or class 2 in a class-3 warp) keeps 3e38 on its unused edges (its
 // |d2 - E| is then 3e38 too: out of the band).
 template <int MODE, bool HAS_M, bool HAS_Z, bool PART, bool LOGB, int NC, int QA, int NE>
@@ -346,7 +347,9 @@ __device__ __forceinline__ void chunk_edges(const SrcPair* __restrict__ S, int l
     }
   }
   if (cls == 0) return;
-  bool band = false;
+  // a pair with d = 0 (1/d^2 infinite, d NaN for log bins) is on a side of its own:
+  // its 0/1 mask does not keep it out of the other sums
+  bool band = !(fabsf(sum2(sdw)) <= kMaxFinite) || (MODE == 0 && !(fabsf(sum2(sgt)) <= kMaxFinite));
 #pragma unroll
   for (int e = 0; e < NE; ++e) band = band || close[e] <= E[e] * C.eps_rel;
   if (band) {

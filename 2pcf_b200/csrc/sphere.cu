@@ -409,10 +409,12 @@ __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, in
   sph_acc_zero(A);
   sph_loop<MODE, HAS_M, HAS_Z, SMALL, PART, NE>(S, lo, hi, L, lz, C.tiny, E, A);
   if (cls == 0) return;
-  bool band = false;
+  // without the offsets of the series path a pair with d = 0 makes the sums infinite
+  // or NaN whatever its mask
+  bool band = MODE == 0 && !SMALL && !(fabsf(sum2(A.sgt)) <= kMaxFinite);
 #pragma unroll
   for (int e = 0; e < NE; ++e) band = band || A.close[e] <= E[e] * C.eps_rel;
-  if (band) {  // rare: a pair inside the guard band; the sub-chunk is binned pair by pair
+  if (band) {  // rare: a pair inside the guard band or at d = 0; the sub-chunk is binned pair by pair
     for (int j = lo; j < hi; ++j) do_pair_s<MODE, HAS_M, HAS_Z, SMALL, SMALL, NC, QA>(Lf, lz, src_of_s(S, j), hcol, C);
     return;
   }

@@ -20,6 +20,7 @@ __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 __device__ __forceinline__ float sum2(float2 v) { return v.x + v.y; }
+constexpr float kMaxFinite = 3.402823466e+38f;
 
 // MUFU reciprocal square root and logarithm without the denormal scaling of
 // the default forms (three more instructions each): their arguments are squared

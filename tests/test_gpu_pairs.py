@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from conftest import uniform_shear
-from parity import check_sums
+from parity import check_lens_sums, check_sums
 
 pytestmark = pytest.mark.gpu
 
@@ -248,3 +248,46 @@ def test_batched_scalar_scalar_equals_single_calls(tpcf, oracle, ctx):
                                      K["w"], bins, calculate_marks=False, ctx=ctx)
         np.testing.assert_array_equal(one.n_pairs, r.n_pairs)
         np.testing.assert_allclose(one.sum_gt, r.sum_gt, rtol=1e-13, atol=1e-13 * np.abs(one.sum_gt).max())
+
+
+@pytest.mark.parametrize("spacing,lo", [("log", 0.7), ("lin", 0.7), ("lin", 0.0)])
+@pytest.mark.parametrize("z", [False, True])
+def test_lenses_on_sources(tpcf, oracle, ctx, spacing, lo, z):
+    """Lenses drawn from the sources, per-lens sums: the pair of each with itself has
+    d = 0.  Below x_min it counts nowhere, though its sub-chunk crosses the first
+    edges; with bins from 0 it is in bin 0 of its lens, where its g terms are 0/0."""
+    L, S = uniform_shear(300, 40_000, 60.0, 31, w="uniform")
+    if z:
+        rng = np.random.default_rng(32)
+        L["z"], S["z"] = rng.uniform(0, 0.5, 300).astype(np.float32), rng.uniform(0.2, 1, 40_000).astype(np.float32)
+    pick = np.arange(0, 40_000, 150)[:266]
+    L["x"][:266], L["y"][:266] = S["x"][pick], S["y"][pick]
+    S["z"][pick[::2]] = 2.0
+    bins = tpcf.create_bins(lo, 20.0, 5, spacing=spacing)
+    res = tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"], S["e1"],
+                                     S["e2"], S["w"], S["m"], bins, calculate_marks=False, lens_sums=True, ctx=ctx)
+    can = canon(oracle, oracle.SHEAR, L, S, bins, lens_idx=np.arange(300))
+    if lo > 0:
+        check_sums(f"lenses on sources {spacing} z={z}", res, can)
+        check_lens_sums(f"lenses on sources {spacing} z={z}, per lens", res.lens_sums, can)
+        return
+    np.testing.assert_array_equal(res.n_pairs, can["n_pairs"].astype(np.int64))
+    same = np.zeros(300, bool)
+    same[:266] = L["z"][:266] <= S["z"][pick]
+    g = res.lens_sums[:, 1:3]
+    assert np.all(np.isnan(g[same][:, :, 0])) and np.all(np.isfinite(g[~same])) and np.all(np.isfinite(g[:, :, 1:]))
+    np.testing.assert_allclose(res.sum_dw, can["sum_dw"], rtol=1e-6)
+
+
+def test_scalar_auto_correlation_per_lens(tpcf, oracle, ctx):
+    """An auto-correlation with marks, its first bin above the spacing of the objects."""
+    rng = np.random.default_rng(33)
+    f = lambda a: np.ascontiguousarray(a, np.float32)
+    n = 20_011
+    x, y, k, w = (f(rng.uniform(0, 60, n)), f(rng.uniform(0, 60, n)), f(rng.normal(0, .02, n)),
+                  f(rng.uniform(.5, 1.5, n)))
+    bins = tpcf.create_bins(0.7, 20.0, 5)
+    res = tpcf.scalar_kappa_tpcf(x, y, k, w, x, y, k, k, w, bins, ctx=ctx)
+    can = canon(oracle, oracle.KAPPA, dict(x=x, y=y, val=k, w=w), dict(x=x, y=y, kappa_E=k, kappa_B=k, w=w), bins)
+    check_sums("auto-correlation with marks", res, can)
+    assert all(np.isfinite(getattr(res, q)).all() for q in ("xi_E_marks", "xi_B_marks", "K_marks", "w_marks"))

@@ -181,3 +181,15 @@ def test_very_small_separations(tpcf, oracle, sctx):
     bins = tpcf.create_bins(1e-14, 4e-13, 1)
     res = run_shear(tpcf, sctx, L, S, bins, calculate_marks=False)
     assert_parity(res, oracle.canon_sphere(oracle.SHEAR, L, S, bins.chord_edges_sq))
+
+
+@pytest.mark.parametrize("spacing", ["log", "lin"])
+def test_lenses_on_sources(tpcf, oracle, sctx, spacing):
+    """Lenses drawn from the sources, x_min above the spacing of the sources: the pair of
+    a lens with itself counts nowhere."""
+    rng = np.random.default_rng(22)
+    L, S = shear_cats(rng, 200, 30_000, (40, 41, -30, -29), w="uniform")
+    L["x"][:150], L["y"][:150] = S["x"][::200][:150], S["y"][::200][:150]
+    bins = tpcf.create_bins(0.7 * ARCMIN, 20 * ARCMIN, 5, spacing=spacing)
+    res = run_shear(tpcf, sctx, L, S, bins, calculate_marks=False)
+    assert_parity(res, oracle.canon_sphere(oracle.SHEAR, L, S, bins.chord_edges_sq))
