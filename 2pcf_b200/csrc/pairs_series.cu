@@ -15,11 +15,11 @@
 //             sum A conj(z)/z  = conj(Z)/Z sum_k M_k (-t)^k + t sum_k N_k (-t)^k,
 //             M_k = sum A (delta/s)^k,  N_k = sum A conj(delta/s) (delta/s)^k
 //           (conj(z)/z = exp(-2 i phi), so the real and imaginary parts are the
-//           g_t and g_x terms of src/tpcf.f90:343-344), to order 5; and with
+//           g_t and g_x terms of src/tpcf.f90:343-344), to order 6; and with
 //           |1 + tau| = sum_ab c_a c_b tau^a conj(tau)^b, c = binomial(1/2, .),
 //             sum w |z| = |Z| sum_ab c_a c_b W_ab t^a conj(t)^b,
 //             W_ab = sum w (delta/s)^a conj(delta/s)^b,
-//           to order 4.  The moments are formed once per catalogue in FP64
+//           to order 5.  The moments are formed once per catalogue in FP64
 //           (k_src_series) and held in FP32.
 //   direct  everything else: the lenses of the group that need it are listed,
 //           lane = source, two lenses per iteration of packed FP32 arithmetic.
@@ -29,9 +29,11 @@
 //           n_pairs is that rule's.  Since a lane keeps its source, p, q, w and
 //           K multiply once per list and not once per pair.
 //
-// Truncation at |t| = kFarRatio = 0.08: rms 2e-8, at most 9e-8 of sum |A|
-// (random 32-source sub-chunks in FP64); it falls as |t|^6, so it lies below the
-// FP32 rounding of a directly formed term (6e-8) nearly everywhere.
+// Truncation at |t| = kFarRatio = 0.08, the worst of any 32 sources: 2 |t|^7 / (1 - |t|)
+// = 4.6e-8 of sum |A| and 2e-8 of sum w |z| (formulas evaluated in FP64: two knots at
+// opposite ends of the sub-chunk reach 4.2e-8 and 1.6e-8, random sub-chunks 9e-9 and
+// 2.5e-9), below the FP32 rounding of a directly formed term (6e-8).  One order less
+// each leaves 5.2e-7 and 2.8e-7 for the two knots.
 
 #include <cstdio>
 
@@ -61,7 +63,7 @@ constexpr int kTch = 3;              // sub-chunks per tile
 // sparse lenses).
 constexpr int kLpl = 2;
 constexpr int kNbuf = 2;             // tiles in flight per warp
-constexpr int kOrder = 5;            // M_0 .. M_5, N_0 .. N_4
+constexpr int kOrder = 6;            // M_0 .. M_6, N_0 .. N_5
 // Guard band around a squared edge, relative: FP32 d2 is within 3e-7 of its
 // exact value and the FP32 edge within 6e-8.
 constexpr float kEdgeBand = 1.0e-6f;
@@ -71,8 +73,9 @@ constexpr int kKeep = 8;
 
 // One sub-chunk record: {box}{cx cy s (s / kFarRatio)^2}{P Q W K sums}{zmin zmax 0 0},
 // shear: kOrder + 1 times {M_re N_re M_im N_im}, then the distance series
-// {W00 W11/4 W22/64 0}{W10, -W21/8}{-W20/4, W31/16}{W30/8, -5/64 W40}, then the
-// fields of the 32 sources, each [32]: x y p q w (K) (z).
+// {W00 W11/4 W22/64 0}{W10, -W21/8}{-W20/4, W31/16}{W30/8, -5/128 W41}
+// {-5/64 W40, 7/128 W50}{-W32/64, 0}, then the fields of the 32 sources, each [32]:
+// x y p q w (K) (z).
 struct RecShape {
   int g, d, src, fields, floats;
 };
@@ -80,7 +83,7 @@ __host__ __device__ constexpr RecShape rec_shape(int mode, bool has_m, bool has_
   RecShape r{};
   r.g = 16;
   r.d = r.g + (mode == 0 ? 4 * (kOrder + 1) : 0);
-  r.src = r.d + 16;
+  r.src = r.d + 24;
   r.fields = 5 + (has_m ? 1 : 0) + (has_z ? 1 : 0);
   r.floats = r.src + kChunk * r.fields;
   return r;
@@ -569,7 +572,9 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
 #pragma unroll
               for (int l = 0; l < kLpl; ++l) gt[l] = sums.x, gx[l] = sums.y;
             }
-            const float4 q0 = ld4(rec + R.d), q1 = ld4(rec + R.d + 4), q2 = ld4(rec + R.d + 8), q3 = ld4(rec + R.d + 12);
+            const float4 q0 = ld4(rec + R.d), q1 = ld4(rec + R.d + 4), q2 = ld4(rec + R.d + 8), q3 = ld4(rec + R.d + 12),
+                         q4 = ld4(rec + R.d + 16);
+            const float2 q5 = *reinterpret_cast<const float2*>(rec + R.d + 20);
 #pragma unroll
             for (int l = 0; l < kLpl; ++l) {
               const float tt = fmaf(tx[l], tx[l], ty[l] * ty[l]);
@@ -578,9 +583,10 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
               auto step = [&](float2 a, float2 c) {
                 return fma2(dup2(tx[l]), a, fma2(make_float2(-ty[l], ty[l]), make_float2(a.y, a.x), c));
               };
-              float2 a = step(hi2(q3), lo2(q3));
+              float2 a = step(hi2(q4), lo2(q4));
+              a = step(a, fma2(tt2, hi2(q3), lo2(q3)));
               a = step(a, fma2(tt2, hi2(q2), lo2(q2)));
-              a = step(a, fma2(tt2, hi2(q1), lo2(q1)));
+              a = step(a, fma2(tt2, fma2(tt2, q5, hi2(q1)), lo2(q1)));
               const float p0 = fmaf(tt, fmaf(tt, q0.z, q0.y), q0.x);
               dw[l] = dc[l] * (p0 + fmaf(tx[l], a.x, -(ty[l] * a.y)));
             }
@@ -808,7 +814,7 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
   }
   const double uu = ux * ux + uy * uy;
   double re = 1.0, im = 0.0;  // (delta / s)^k
-  double W[5][2];             // sum w (delta/s)^k
+  double W[6][2];             // w (delta/s)^k
   for (int k = 0; k <= kOrder; ++k) {
     const double Mr = dp * re - dq * im, Mi = dp * im + dq * re;
     if (mode == 0) {
@@ -818,7 +824,7 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
       if (lane == 0)
         *reinterpret_cast<float4*>(out + R.g + 4 * k) = make_float4((float)a, (float)b, (float)e, (float)g);
     }
-    if (k < 5) {
+    if (k < 6) {
       W[k][0] = dw * re;
       W[k][1] = dw * im;
     }
@@ -827,19 +833,25 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
     re = nr;
   }
   const double w11 = red(dw * uu), w22 = red(dw * uu * uu);
-  double v[12];
+  double v[18];
   v[0] = red(W[1][0]), v[1] = red(W[1][1]);
   v[2] = red(W[1][0] * uu), v[3] = red(W[1][1] * uu);
   v[4] = red(W[2][0]), v[5] = red(W[2][1]);
   v[6] = red(W[2][0] * uu), v[7] = red(W[2][1] * uu);
   v[8] = red(W[3][0]), v[9] = red(W[3][1]);
   v[10] = red(W[4][0]), v[11] = red(W[4][1]);
+  v[12] = red(W[3][0] * uu), v[13] = red(W[3][1] * uu);
+  v[14] = red(W[5][0]), v[15] = red(W[5][1]);
+  v[16] = red(W[1][0] * uu * uu), v[17] = red(W[1][1] * uu * uu);
   if (lane == 0) {
     float4* o4 = reinterpret_cast<float4*>(out + R.d);
     o4[0] = make_float4((float)sw, (float)(w11 / 4), (float)(w22 / 64), 0.f);
     o4[1] = make_float4((float)v[0], (float)v[1], (float)(-v[2] / 8), (float)(-v[3] / 8));
     o4[2] = make_float4((float)(-v[4] / 4), (float)(-v[5] / 4), (float)(v[6] / 16), (float)(v[7] / 16));
-    o4[3] = make_float4((float)(v[8] / 8), (float)(v[9] / 8), (float)(-5 * v[10] / 64), (float)(-5 * v[11] / 64));
+    o4[3] = make_float4((float)(v[8] / 8), (float)(v[9] / 8), (float)(-5 * v[12] / 128), (float)(-5 * v[13] / 128));
+    o4[4] = make_float4((float)(-5 * v[10] / 64), (float)(-5 * v[11] / 64), (float)(7 * v[14] / 128),
+                        (float)(7 * v[15] / 128));
+    o4[5] = make_float4((float)(-v[16] / 64), (float)(-v[17] / 64), 0.f, 0.f);
   }
 }
 

@@ -154,3 +154,34 @@ def test_very_small_coordinates(tpcf, oracle, ctx, spacing, lo, unit):
     bins = tpcf.create_bins(lo * unit, 25.0 * unit, 8, spacing=spacing)
     res = shear(tpcf, ctx, L, S, bins)
     check_sums(f"series unit {unit} {spacing}", res, oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
+
+
+def test_sub_chunks_of_two_knots(tpcf, oracle, ctx):
+    """Every sub-chunk two knots of sources with equal values, 31 and 1 of them at its
+    two ends, just far enough for the series: all their truncation errors add up.
+    Truncation is at most 4.6e-8 (g) and 2e-8 (d) of the terms; FP32 gives 1/d^2 and d
+    errors of up to 2.6e-7 and 1.3e-7 (twice and once the 2^-22.9 of a reciprocal
+    square root) of either sign at 225 different distances, so their mean stays well
+    below half of that: bars of 2.5e-7 of the sum of |e| w and 1.5e-7 of the sum of d w."""
+    rng = np.random.default_rng(80)
+    gy, gx = np.meshgrid(30.0 + 60.0 * np.arange(15), 30.0 + 60.0 * np.arange(15), indexing="ij")
+    gx, gy = gx.ravel(), gy.ravel()
+    end = np.where(np.arange(32) < 31, 1.0, -1.0)
+    n_fill = 100_000   # away from every lens: the catalogue is dense on average
+    x = np.concatenate([(gx[:, None] + end).ravel(), rng.uniform(840, 900, n_fill)])
+    y = np.concatenate([np.repeat(gy, 32), rng.uniform(960, 1000, n_fill)])
+    n = x.size
+    S = dict(x=f32(x), y=f32(y), z=np.ones(n, np.float32), e1=np.full(n, .3, np.float32),
+             e2=np.full(n, .1, np.float32), w=np.ones(n, np.float32), m=np.zeros(n, np.float32))
+    r, a = rng.uniform(12.55, 12.75, gx.size), np.radians(70.0)
+    L = dict(x=f32(gx - r * np.cos(a)), y=f32(gy - r * np.sin(a)), z=np.zeros(gx.size, np.float32),
+             val=np.ones(gx.size, np.float32), w=np.ones(gx.size, np.float32))
+    bins = tpcf.create_bins(8.0, 20.0, 1, spacing="lin")
+    res = shear(tpcf, ctx, L, S, bins)
+    can = oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq)
+    assert can["n_pairs"][0] == 32 * 225
+    check_sums("series knots", res, can)
+    d_g = np.hypot(res.sum_gt[0] - can["sum_gt"][0], res.sum_gx[0] - can["sum_gx"][0]) / (32 * 225 * np.hypot(.3, .1))
+    d_d = abs(res.sum_dw[0] - can["sum_dw"][0]) / can["sum_dw"][0]
+    print("knots:", d_g, d_d)
+    assert d_g <= 2.5e-7 and d_d <= 1.5e-7
