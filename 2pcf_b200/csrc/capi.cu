@@ -528,12 +528,10 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   float R = (float)(Rd * (1.0 + 1e-6));
   const char* var_env = std::getenv("TPCF_PAIR_VARIANT");
   B.variant = var_env ? std::atoi(var_env) : 0;
-  bool any_lens = false;
-  for (int t = 0; t < nT; ++t) any_lens = any_lens || wants_lens(outs[t]);
 
   // ---- source grids
   std::vector<GridDesc> grids(nS);
-  std::vector<char> src_series(nS, 0);
+  B.kind.assign(nT, 0);
   for (int i = 0; i < nS; ++i) {
     const SrcIn& s = srcs[i];
     GridDesc& g = grids[i];
@@ -547,8 +545,15 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     }
     double cell = c->opts.cell_size > 0 ? c->opts.cell_size : Rd / 16.0;
     const double span = std::max((double)ex, (double)ey);
-    const bool series = !sph && !any_lens && B.variant == 0 && series_pays(n_valid, ex, ey, bins, e.data());
-    src_series[i] = series;
+    // the pair kernel of each of its tasks, by the task and this catalogue alone;
+    // records for each kernel that reads it
+    const bool dense = !sph && B.variant == 0 && series_pays(n_valid, ex, ey, bins, e.data());
+    bool series = false, other = false;
+    for (int t = 0; t < nT; ++t)
+      if (ts[t] == i) {
+        B.kind[t] = dense && !wants_lens(outs[t]);
+        (B.kind[t] ? series : other) = true;
+      }
     if (!c->opts.use_grid) cell = span * 2.0 + 1.0;
     // keep the grid below 2^24 cells
     while ((span / cell + 2.0) * (span / cell + 2.0) > (double)(1 << 24)) cell *= 1.5;
@@ -560,8 +565,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     g.ncx = ncx; g.ncy = ncy; g.n_valid = n_valid;
     int* cs = (int*)ws_alloc(c, sizeof(int) * (ncells + 1));
     const int n_chunks = std::max((n_valid + kChunk - 1) / kChunk, 1);
-    SrcPair* pairs = sph || series ? nullptr : (SrcPair*)ws_alloc(c, sizeof(SrcPair) * (kChunk / 2) * n_chunks);
-    ChunkMeta* cmeta = sph || series ? nullptr : (ChunkMeta*)ws_alloc(c, sizeof(ChunkMeta) * n_chunks);
+    SrcPair* pairs = sph || !other ? nullptr : (SrcPair*)ws_alloc(c, sizeof(SrcPair) * (kChunk / 2) * n_chunks);
+    ChunkMeta* cmeta = sph || !other ? nullptr : (ChunkMeta*)ws_alloc(c, sizeof(ChunkMeta) * n_chunks);
     float* srec = series ? (float*)ws_alloc(c, series_bytes(n_valid, mode, has_m, has_z)) : nullptr;
     void* sphc = sph ? ws_alloc(c, sph_src_bytes(n_valid)) : nullptr;
     if (s.n > 0) {
@@ -582,10 +587,10 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
       if (sph)
         counted(c, launch_src_gather_sph(i1, n_valid, mode, lamS[i], s.y, s.z, s.f1, s.f2, s.w, s.m, sphc, st),
                 "src gather");
-      else if (series)
+      if (series)
         counted(c, launch_src_series(i1, n_valid, mode, has_m, has_z, s.x, s.y, s.z, s.f1, s.f2, s.w, s.m, srec, st),
                 "src gather");
-      else
+      if (pairs)
         counted(c, launch_src_pairs(i1, n_valid, mode, s.x, s.y, s.z, s.f1, s.f2, s.w, s.m, pairs, cmeta, st),
                 "src gather");
     } else {
@@ -600,7 +605,9 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   }
   // FP32 guard on the reach of a task's rows and cells: the rounding scale of
   // the coordinates its two catalogues hold, so that a task's tiles (and its
-  // sums, bit for bit) do not depend on the other tasks of a batch
+  // sums, bit for bit) do not depend on the other tasks of a batch (but for a z
+  // cut, whose masks all tasks of a call take when one needs them, and the last
+  // FP64 places of sum_K beside a calibrated catalogue)
   std::vector<double> extent(ncat, 0.0);
   for (int i = 0; i < ncat; ++i) {
     const float* b = &hbox[8 * i];
@@ -665,7 +672,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     }
     for (int k = 0; k < 2; ++k) {
       bool used = false;
-      for (int t = 0; t < nT; ++t) used = used || (tl[t] == i && src_series[ts[t]] == k);
+      for (int t = 0; t < nT; ++t) used = used || (tl[t] == i && B.kind[t] == k);
       LensGroups& LG = LB.by[k];
       if (!used) continue;
       if (n_patch_eff == 1) {
@@ -705,15 +712,15 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   tdesc.assign(nT, TaskDesc{});
   std::vector<int2> ranges[2];  // {task, first item among its kind}
   int n_kind[2] = {0, 0}, n_items = 0;
-  B.kind.assign(nT, 0);
   B.want_lens.assign(nT, 0);
   long long lens_acc_elems = 0;
   for (int t = 0; t < nT; ++t) {
     TaskDesc& d = tdesc[t];
-    const int kind = B.kind[t] = src_series[ts[t]];
+    const int kind = B.kind[t];
     d.lens_cat = kind * nL + tl[t];
     d.src_cat = ts[t];
     d.margin = task_margin(tl[t], ts[t]);
+    d.flush_src = wants_lens(outs[t]) ? kFlushSrcLens : kFlushSrc;
     d.item_base = n_items;
     const int ng = lb[tl[t]].by[kind].n_groups;
     // few lens groups: several items per group keep the SMs' warps busy (a
@@ -776,13 +783,6 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     P.binA = P.binB = 0.f;
     P.eps = 4e-6f;
   }
-  // FP32 histogram folded into FP64 every 4096 sources (each histogram cell
-  // then holds at most 128 register sums of 32 pairs): the per-bin sums of
-  // the call stay within 1e-6 of sum|terms|.  Per-lens outputs are sums of
-  // far fewer terms per cell, so their FP32 partials are folded every 1024
-  // sources (at 4096 one lens and bin of the 2 M x 0.5 M clustered
-  // workload reached 1.05e-6 of its sum|terms|)
-  P.flush_src = lens_acc ? 1024 : 4096;
   P.far_bin = series_far_bin(e2.data(), nb);
   int bt_pairs = bt;  // of k_pairs
   if (!sph && B.variant == 0 && c->opts.group_size == 0 && c->opts.tile_chunks == 0) pair_tile_shape(nb, qa, &bt_pairs, &tch);

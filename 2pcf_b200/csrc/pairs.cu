@@ -457,7 +457,6 @@ __global__ void __launch_bounds__(BT, kPairWarps * 32 / BT) k_pairs(const PairPa
   bool aborted = false;   // a bounded wait ran out: consume and issue nothing more
   float* __restrict__ hcol = hist + tid;
   double* wsum = bsum + (size_t)warp * kQ * nb;
-  const int flush_src = P.flush_src > 0 ? P.flush_src : 4096;
 #ifdef TPCF_MODE_STATS
   __shared__ unsigned long long sh_stats[15];
   if (tid < 15) sh_stats[tid] = 0ull;
@@ -550,6 +549,11 @@ __global__ void __launch_bounds__(BT, kPairWarps * 32 / BT) k_pairs(const PairPa
         for (int j = 0; j < tg.n; ++j) {
           const int lo = j == 0 ? tg.lo0 : 0;
           const int hi = j == tg.n - 1 ? tg.hiL : kChunk;
+          if (since_flush >= T.flush_src) {
+            warp_fold<QA, BT>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, warp, lane);
+            since_flush = 0;
+          }
+          since_flush += hi - lo;
           const bool part = lo > 0 || hi < kChunk;
           const SrcPair* __restrict__ Sc = Tb + j * (kChunk / 2);
           const float4 cbox = Mb[j].box;
@@ -599,13 +603,8 @@ __global__ void __launch_bounds__(BT, kPairWarps * 32 / BT) k_pairs(const PairPa
             }
           }
         }
-        since_flush += tg.n * kChunk - tg.lo0 - (kChunk - tg.hiL);
         __syncwarp();  // every lane is done reading buffer b
         if (k + NBUF < ntiles) issue(k + NBUF);
-        if (since_flush >= flush_src) {
-          warp_fold<QA, BT>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, warp, lane);
-          since_flush = 0;
-        }
       }
       if (!aborted) ring_t += ntiles;
     }

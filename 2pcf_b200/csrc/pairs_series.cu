@@ -282,6 +282,8 @@ __device__ __forceinline__ void direct_sums(const float4* lxy, const float4* lf,
     }
   }
   zero = !LOGB && dmin == 0.f;
+  // (__fmul_rn: products that the callers' additions must not fuse with, so that every
+  // variant of the kernel rounds alike)
   // A[k].n counts the pairs at or above edge k - 1 (k = 0: all)
   float n[NE + 2];
 #pragma unroll
@@ -299,13 +301,13 @@ __device__ __forceinline__ void direct_sums(const float4* lxy, const float4* lf,
       v[k][QGT] = -fmaf(S.p, c, S.q * sn);
       v[k][QGX] = -fmaf(S.q, c, -(S.p * sn));
     } else {
-      v[k][QGT] = S.p * c;
-      v[k][QGX] = S.q * c;
+      v[k][QGT] = __fmul_rn(S.p, c);
+      v[k][QGX] = __fmul_rn(S.q, c);
     }
-    v[k][QW] = S.w * w;
-    v[k][QDW] = S.w * sum2(A[k].d);
+    v[k][QW] = __fmul_rn(S.w, w);
+    v[k][QDW] = __fmul_rn(S.w, sum2(A[k].d));
     v[k][QN] = S.ok ? n[k] - n[k + 1] : 0.f;
-    v[k][QK] = (MODE == 0 && HAS_M) ? S.K * w : 0.f;
+    v[k][QK] = (MODE == 0 && HAS_M) ? __fmul_rn(S.K, w) : 0.f;
   }
 }
 
@@ -390,7 +392,6 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
   int ring_t = 0;        // ring index of the next tile this warp consumes
   int issued_end = 0;    // ring index one past the last tile this warp issued
   bool aborted = false;  // a bounded wait ran out: consume and issue nothing more
-  const int flush_src = P.flush_src > 0 ? P.flush_src : 4096;
 
   while (!aborted) {
     int item = 0;
@@ -521,7 +522,7 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
             Zy[l] = cen.y - ly[l];
             Z2[l] = fmaf(Zy[l], Zy[l], Zx[l] * Zx[l]);
             rs[l] = rsqrt_ftz(fmaxf(Z2[l], kMinNormal));
-            dc[l] = Z2[l] * rs[l];
+            dc[l] = __fmul_rn(Z2[l], rs[l]);
             in[l] = bin_range<LOGB>(dc[l], cen.z, C, b0[l], b1[l]) && act[l];
             bool zall = true;
             if (HAS_Z) {
@@ -563,7 +564,7 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
 #pragma unroll
               for (int l = 0; l < kLpl; ++l) {
                 const float c2 = fmaf(-Zy[l], Zy[l], Zx[l] * Zx[l]) * r[l];
-                const float zz = Zx[l] * Zy[l];
+                const float zz = __fmul_rn(Zx[l], Zy[l]);
                 const float s2 = (zz + zz) * r[l];
                 gt[l] = fmaf(c2, re[l].x, fmaf(s2, im[l].x, fmaf(tx[l], re[l].y, -(ty[l] * im[l].y))));
                 gx[l] = fmaf(c2, im[l].x, fmaf(-s2, re[l].x, fmaf(tx[l], im[l].y, ty[l] * re[l].y)));
@@ -709,7 +710,7 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
         since_flush += tg.n * kChunk - tg.lo0 - (kChunk - tg.hiL);
         __syncwarp();  // every lane is done reading buffer b
         if (k + kNbuf < ntiles) issue(k + kNbuf);
-        if (since_flush >= flush_src) {
+        if (since_flush >= kFlushSrc) {
           fold_far<QA>(hist, wsum, nb, tb, lane);
           since_flush = 0;
         }

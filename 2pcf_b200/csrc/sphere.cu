@@ -561,7 +561,6 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
   int ring_t = 0;        // ring index of the next sub-chunk this warp consumes
   int issued_end = 0;    // ring index one past the last sub-chunk this warp issued
   bool aborted = false;  // a bounded wait ran out: consume and issue nothing more
-  const int flush_src = P.flush_src > 0 ? P.flush_src : 4096;
 
   while (!aborted) {
     int item = 0;
@@ -680,7 +679,7 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
         since_flush += hi - lo;
         __syncwarp();  // every lane is done reading buffer b
         if (k + kNbufS < ntiles) issue(k + kNbufS);
-        if (since_flush >= flush_src) {
+        if (since_flush >= T.flush_src) {
           warp_fold<QA, 32>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, 0, lane);
           since_flush = 0;
         }

@@ -97,13 +97,22 @@ struct LensDesc {
 // Items that a lens group of a task is cut into at most.
 constexpr int kMaxSplit = 8;
 
+// FP32 histogram folded into FP64 every 4096 sources (each histogram cell then
+// holds at most 128 register sums of 32 pairs): the per-bin sums of a call stay
+// within 1e-6 of sum|terms|.  Per-lens outputs are sums of far fewer terms per
+// cell, so their FP32 partials are folded every 1024 sources (at 4096 one lens and
+// bin of the 2 M x 0.5 M clustered workload reached 1.05e-6 of its sum|terms|).
+// k_pairs counts per sub-chunk, so that its folds do not depend on the tile length
+// (k_pairs_series, k_pairs_sph: one tile length).
+constexpr int kFlushSrc = 4096, kFlushSrcLens = 1024;
+
 struct TaskDesc {
   int lens_cat;
   int src_cat;
   int item_base;            // row of (task, group 0) in item_sums
   float margin;             // FP32 guard on the reach of this task's rows and cells
   int split;                // work items per lens group, each with every split-th cell row (1 for most)
-  int pad;
+  int flush_src;            // FP32 sums -> FP64 after this many sources (k_pairs, k_pairs_sph)
   long long lens_acc_off;   // element offset of this task's per-lens sums, -1 = none
 };
 
@@ -124,7 +133,6 @@ struct PairParams {
   float binA, binB;         // log spacing: t = lg2(d2)*binA + binB
   float eps;                // guard band half-width in t units (log) or relative (generic)
   int far_bin;              // k_pairs_series: first bin of the far sums
-  int flush_src;            // FP32 histogram -> FP64 after this many sources (0: 4096)
   // Fault injection for tests only (0 in every product call): 1 + the ring
   // index of a source tile whose bulk copy is never issued, so that the waits
   // on it run out (0: none), and the poll limit of the waits (0: kWaitPolls).

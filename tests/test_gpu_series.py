@@ -185,3 +185,34 @@ def test_sub_chunks_of_two_knots(tpcf, oracle, ctx):
     d_d = abs(res.sum_dw[0] - can["sum_dw"][0]) / can["sum_dw"][0]
     print("knots:", d_g, d_d)
     assert d_g <= 2.5e-7 and d_d <= 1.5e-7
+
+
+def test_tasks_of_a_mixed_batch(tpcf, ctx, monkeypatch):
+    """Tasks with and without marks, calibration in one source catalogue only, dense and
+    sparse sources: each task's sums are those of the task alone, bit for bit (sum_K,
+    which a call without calibration copies from sum_w, to the last places of FP64)."""
+    rng = np.random.default_rng(81)
+    def source(n, m):
+        return tpcf.ShapeCatalog(f32(rng.uniform(0, 300, n)), f32(rng.uniform(0, 300, n)), f32(rng.normal(0, .26, n)),
+                                 f32(rng.normal(0, .26, n)), f32(rng.uniform(.5, 1.5, n)), np.ones(n, np.float32),
+                                 f32(rng.normal(0, .03, n)) if m else np.zeros(n, np.float32))
+    n = 300
+    lens = tpcf.LensCatalog(f32(rng.uniform(0, 300, n)), f32(rng.uniform(0, 300, n)), f32(rng.normal(0, .02, n)),
+                            f32(rng.uniform(.5, 1.5, n)), np.zeros(n, np.float32))
+    src = [source(300_000, False), source(30_000, False), source(40_000, True)]
+    bins = tpcf.create_bins(1.0, 100.0, 20)
+    tasks = [(0, 0, False), (0, 0, True), (0, 1, False), (0, 1, True), (0, 2, False)]
+    alloc = tpcf._alloc_result
+
+    def run(sources, what):
+        marks = iter([t[2] for t in what])
+        monkeypatch.setattr(tpcf, "_alloc_result", lambda nb, nA, _, *a: alloc(nb, nA, next(marks), *a))
+        return tpcf.batch_shear_2pcf([lens], sources, [t[:2] for t in what], bins, ctx=ctx)
+    together = run(src, tasks)
+    for t in range(len(tasks)):
+        alone = run([src[tasks[t][1]]], [(0, 0, tasks[t][2])])[0]
+        for k in ("n_pairs", "sum_gt", "sum_gx", "sum_w", "sum_dw"):
+            np.testing.assert_array_equal(getattr(together[t], k), getattr(alone, k), err_msg=f"task {t} {k}")
+        np.testing.assert_allclose(together[t].sum_K, alone.sum_K, rtol=1e-14)
+        if tasks[t][2]:
+            np.testing.assert_array_equal(together[t].xi_E_marks, alone.xi_E_marks)
