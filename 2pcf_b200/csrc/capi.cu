@@ -414,7 +414,11 @@ bool series_pays(int n_valid, double ex, double ey, const tpcf_bins* bins, const
 // A task with fewer lens groups than kSplitItems / 2 is cut into several items
 // per group (at most kMaxSplit).
 constexpr int kSplitItems = 8192;
-constexpr size_t kSplitLensBytes = (size_t)256 << 20;  // per-lens sums of a split task at most
+// The parts of a group have per-lens sums of their own: at most this much of them for
+// a split task, and for all tasks of a call with split ones.  (Beyond the second limit,
+// with dozens of tasks, the parts of a task do depend on the others: its sums then
+// agree with those of the task alone to FP64 rounding.)
+constexpr size_t kSplitLensBytes = (size_t)256 << 20, kSplitCallBytes = (size_t)1 << 30;
 
 void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<SrcIn> srcs, const std::vector<int>& tl,
                  const std::vector<int>& ts, const tpcf_bins* bins, int n_patch, const tpcf_result* outs, Batch& B) {
@@ -714,6 +718,9 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   int n_kind[2] = {0, 0}, n_items = 0;
   B.want_lens.assign(nT, 0);
   long long lens_acc_elems = 0;
+  auto lens_bytes_of = [&](int t) { return sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1); };
+  size_t call_lens_bytes = 0;
+  for (int t = 0; t < nT; ++t) call_lens_bytes += wants_lens(outs[t]) ? lens_bytes_of(t) : 0;
   for (int t = 0; t < nT; ++t) {
     TaskDesc& d = tdesc[t];
     const int kind = B.kind[t];
@@ -727,9 +734,9 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     // property of the task alone, so its sums do not depend on the batch)
     d.split = ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
     // the parts of a group add into per-lens columns of their own (k_lens_outputs sums them)
-    const size_t lens_bytes = sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1);
     if (wants_lens(outs[t]))
-      while (d.split > 1 && lens_bytes * d.split > kSplitLensBytes) --d.split;
+      while (d.split > 1 && (lens_bytes_of(t) * d.split > kSplitLensBytes || call_lens_bytes * d.split > kSplitCallBytes))
+        --d.split;
     if (ng > 0) ranges[kind].push_back(make_int2(t, n_kind[kind]));
     n_kind[kind] += ng * d.split;
     n_items += ng * d.split;

@@ -45,3 +45,25 @@ def test_large_host_outputs(tpcf, ctx):
     for i in range(0, n, 9973):
         d2 = (np.float64(L["x"][i]) - S["x"]) ** 2 + (np.float64(L["y"][i]) - S["y"]) ** 2
         np.testing.assert_array_equal(res.lens_sums[i, 5], np.histogram(d2, bins.bin_edges_sq)[0])
+
+
+def test_workspace_of_a_batch_of_many_tasks(tpcf):
+    """60 tasks with per-lens sums: the split groups' extra columns are bounded for the
+    call, not only per task (1.7 GB of sums in all, 8 times that with 8 parts each);
+    counts as when launched alone, sums to the FP32 partials' order."""
+    ctx = tpcf.Context(0)
+    L, S = uniform_shear(30_000, 2000, 400.0, 350, w="uniform")
+    lens = tpcf.LensCatalog(L["x"], L["y"], L["val"], L["w"], L["z"])
+    src = tpcf.ShapeCatalog(*(S[k] for k in ("x", "y", "e1", "e2", "w", "z", "m")))
+    bins = tpcf.create_bins(1.0, 20.0, 20)
+    unsplit = 8 * 6 * 20 * 30_000
+    res = tpcf.batch_shear_2pcf([lens], [src], [(0, 0)] * 60, bins, lens_sums="device", ctx=ctx)
+    held = ctx.stats()["workspace_bytes"]
+    alone = tpcf.batch_shear_2pcf([lens], [src], [(0, 0)], bins, lens_sums="device", ctx=ctx)[0]
+    ctx.close()
+    assert held <= 1.25 * (60 * unsplit + (1 << 30))   # a slot is a quarter larger than asked for
+    for r in res:
+        np.testing.assert_array_equal(r.n_pairs, alone.n_pairs)
+        np.testing.assert_allclose(r.sum_w, alone.sum_w, rtol=1e-6)
+        np.testing.assert_array_equal(r.lens_sums[:, 5].cpu().numpy(), alone.lens_sums[:, 5].cpu().numpy())
+    assert abs(alone.lens_sums[:, 3].sum().item() - alone.sum_w.sum()) <= 1e-9 * alone.sum_w.sum()
