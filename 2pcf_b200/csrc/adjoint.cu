@@ -865,7 +865,7 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     a.dsum = dsum[t];
     // item cost: the source groups play the lens-group role, the lens grid the source grid
     tdesc[t].lens_cat = si; tdesc[t].src_cat = li; tdesc[t].item_base = 0; tdesc[t].lens_acc_off = -1;
-    tdesc[t].margin = margin; tdesc[t].split = 1;
+    tdesc[t].margin = margin; tdesc[t].split = tdesc[t].run = 1;
     if (hc[li] > 0 && ngroups[si] > 0) {
       ranges.push_back(make_int2(t, n_items));
       n_items += ngroups[si];

@@ -415,9 +415,9 @@ bool series_pays(int n_valid, double ex, double ey, const tpcf_bins* bins, const
 // per group (at most kMaxSplit).
 constexpr int kSplitItems = 8192;
 // The parts of a group have per-lens sums of their own: at most this much of them for
-// a split task, and for all tasks of a call with split ones.  (Beyond the second limit,
-// with dozens of tasks, the parts of a task do depend on the others: its sums then
-// agree with those of the task alone to FP64 rounding.)
+// a task, and as much more than one part would need for a call.  Beyond the second
+// limit a group's parts are one work item, added one after the other into one set of
+// per-lens sums: the sums per bin and patch are the same bit for bit.
 constexpr size_t kSplitLensBytes = (size_t)256 << 20, kSplitCallBytes = (size_t)1 << 30;
 
 void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<SrcIn> srcs, const std::vector<int>& tl,
@@ -718,9 +718,18 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   int n_kind[2] = {0, 0}, n_items = 0;
   B.want_lens.assign(nT, 0);
   long long lens_acc_elems = 0;
-  auto lens_bytes_of = [&](int t) { return sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1); };
-  size_t call_lens_bytes = 0;
-  for (int t = 0; t < nT; ++t) call_lens_bytes += wants_lens(outs[t]) ? lens_bytes_of(t) : 0;
+  // few lens groups: several parts per group keep the SMs' warps busy (a property
+  // of the task alone, so its sums do not depend on the batch)
+  size_t extra_lens = 0;
+  for (int t = 0; t < nT; ++t) {
+    TaskDesc& d = tdesc[t];
+    const int ng = lb[tl[t]].by[(int)B.kind[t]].n_groups;
+    d.split = ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
+    const size_t lens_bytes = sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1);
+    if (!wants_lens(outs[t])) continue;
+    while (d.split > 1 && lens_bytes * d.split > kSplitLensBytes) --d.split;
+    extra_lens += lens_bytes * (d.split - 1);
+  }
   for (int t = 0; t < nT; ++t) {
     TaskDesc& d = tdesc[t];
     const int kind = B.kind[t];
@@ -730,21 +739,15 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     d.flush_src = wants_lens(outs[t]) ? kFlushSrcLens : kFlushSrc;
     d.item_base = n_items;
     const int ng = lb[tl[t]].by[kind].n_groups;
-    // few lens groups: several items per group keep the SMs' warps busy (a
-    // property of the task alone, so its sums do not depend on the batch)
-    d.split = ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
-    // the parts of a group add into per-lens columns of their own (k_lens_outputs sums them)
-    if (wants_lens(outs[t]))
-      while (d.split > 1 && (lens_bytes_of(t) * d.split > kSplitLensBytes || call_lens_bytes * d.split > kSplitCallBytes))
-        --d.split;
+    d.run = wants_lens(outs[t]) && extra_lens > kSplitCallBytes ? d.split : 1;
     if (ng > 0) ranges[kind].push_back(make_int2(t, n_kind[kind]));
-    n_kind[kind] += ng * d.split;
+    n_kind[kind] += ng * (d.split / d.run);
     n_items += ng * d.split;
     B.want_lens[t] = wants_lens(outs[t]) ? 1 : 0;
     d.lens_acc_off = -1;
     if (B.want_lens[t]) {
       d.lens_acc_off = lens_acc_elems;
-      lens_acc_elems += (long long)kQ * nb * std::max(lb[tl[t]].n_valid, 1) * d.split;
+      lens_acc_elems += (long long)kQ * nb * std::max(lb[tl[t]].n_valid, 1) * (d.split / d.run);
     }
   }
   // descriptors and edges: one copy
@@ -901,7 +904,7 @@ void batch_finish(tpcf_ctx* c, Batch& B, const tpcf_bins* bins, tpcf_result* out
       if (!marks_all && (xE || xB || Km || wm))
         throw Failure(TPCF_ERR_INVALID_ARG, "xi_E_marks, xi_B_marks, K_marks and w_marks go together");
       if (LB.n_valid > 0 && B.n_items > 0 && B.lens_acc)
-        counted(c, launch_lens_outputs(B.lens_acc + B.tdesc[t].lens_acc_off, B.tdesc[t].split, LB.rec, LB.perm, LB.n_valid, nb, xE,
+        counted(c, launch_lens_outputs(B.lens_acc + B.tdesc[t].lens_acc_off, B.tdesc[t].split / B.tdesc[t].run, LB.rec, LB.perm, LB.n_valid, nb, xE,
                                        xB, Km, wm, mw, ls, lr, st), "lens outputs");
       auto out = [&](void* user, const void* dev, size_t bytes) {
         if (dev && dev != user) large.push_back({user, dev, bytes});

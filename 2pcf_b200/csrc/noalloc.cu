@@ -242,7 +242,7 @@ tpcf_status run_noalloc(tpcf_ctx* c, const float* xA, const float* yA, const flo
   counted(c, cudaGetLastError(), "groups");
   counted(c, launch_group_box(lrec, gstart, n_groups, gbox, st), "group box");
   TaskDesc td{};
-  td.lens_cat = 0; td.src_cat = 0; td.item_base = 0; td.lens_acc_off = -1; td.margin = margin; td.split = 1;
+  td.lens_cat = 0; td.src_cat = 0; td.item_base = 0; td.lens_acc_off = -1; td.margin = margin; td.split = td.run = 1;
   td.flush_src = kFlushSrc;
   LensDesc ld{};
   ld.rec = lrec; ld.z = zs; ld.group_start = gstart; ld.group_box = gbox; ld.n_valid = nl_valid;

@@ -464,16 +464,21 @@ __global__ void __launch_bounds__(BT, kPairWarps * 32 / BT) k_pairs(const PairPa
 #endif
   for (int e = 0; e < nb * QA; ++e) hcol[e * BT] = 0.f;
 
+  int item = 0, run_i = 0, run_n = 0;
   while (!aborted) {
-    int item = 0;
-    if (lane == 0) item = atomicAdd(P.queue_head, 1);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= P.n_items) break;
+    if (run_i == run_n) {  // this item's parts are done: the next item
+      if (lane == 0) item = atomicAdd(P.queue_head, 1);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (item >= P.n_items) break;
+      run_i = 0;
+    }
     const int2 it = P.items[item];
     const TaskDesc T = P.tasks[it.x];
+    run_n = T.run;
     const LensDesc LD = P.lenses[T.lens_cat];
     const GridDesc G = P.grids[T.src_cat];
-    const int g = it.y / T.split, part = it.y - g * T.split;
+    const int per = T.split / T.run, g = it.y / per;
+    const int part = (it.y - g * per) * T.run + run_i++;
     const int gs = LD.group_start[g];
     const int nl = LD.group_start[g + 1] - gs;
     const bool act = lane < nl;
@@ -486,7 +491,8 @@ __global__ void __launch_bounds__(BT, kPairWarps * 32 / BT) k_pairs(const PairPa
       vw = (double)r.z * (double)r.w;
       w = (double)r.w;
       if (HAS_Z) lz = LD.z[gs + lane];
-      if (P.lens_acc && T.lens_acc_off >= 0) lens_col = P.lens_acc + T.lens_acc_off + (size_t)part * kQ * nb * LD.n_valid + gs + lane;
+      if (P.lens_acc && T.lens_acc_off >= 0)
+        lens_col = P.lens_acc + T.lens_acc_off + (size_t)(T.run > 1 ? 0 : part) * kQ * nb * LD.n_valid + gs + lane;
     }
     LensP LP;
     LP.nlx = dup2(-lx);
@@ -610,7 +616,7 @@ __global__ void __launch_bounds__(BT, kPairWarps * 32 / BT) k_pairs(const PairPa
     }
     if (aborted) break;
     warp_fold<QA, BT>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, warp, lane);
-    double* out = P.item_sums + (size_t)(T.item_base + it.y) * kQ * nb;
+    double* out = P.item_sums + (size_t)(T.item_base + g * T.split + part) * kQ * nb;
     for (int e = lane; e < kQ * nb; e += 32) {
       const int src = (e / nb == QK && QA == 5) ? e - (QK - QW) * nb : e;
       out[e] = wsum[src];
@@ -934,12 +940,12 @@ __global__ void k_item_cost(const int2* __restrict__ ranges, int n_ranges, int n
   const TaskDesc T = tasks[it.x];
   const LensDesc L = lenses[T.lens_cat];
   const GridDesc G = grids[T.src_cat];
-  const int g = it.y / T.split, part = it.y - g * T.split;
+  const int per = T.split / T.run, g = it.y / per, part = it.y - g * per;
   const float4 box = L.group_box[g];
   int cy0, cy1;
   row_range(G, box, R, T.margin, cy0, cy1);
   unsigned long long s = 0;
-  for (int cy = cy0 + part + v * T.split; cy <= cy1; cy += 8 * T.split) {
+  for (int cy = cy0 + part + v * per; cy <= cy1; cy += 8 * per) {
     const int2 sp = row_span(G, box, R, T.margin, cy);
     if (sp.y > sp.x) s += (unsigned long long)(sp.y - sp.x);
   }

@@ -562,17 +562,22 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
   int issued_end = 0;    // ring index one past the last sub-chunk this warp issued
   bool aborted = false;  // a bounded wait ran out: consume and issue nothing more
 
+  int item = 0, run_i = 0, run_n = 0;
   while (!aborted) {
-    int item = 0;
-    if (lane == 0) item = atomicAdd(P.queue_head, 1);
-    item = __shfl_sync(0xffffffffu, item, 0);
-    if (item >= P.n_items) break;
+    if (run_i == run_n) {  // this item's parts are done: the next item
+      if (lane == 0) item = atomicAdd(P.queue_head, 1);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (item >= P.n_items) break;
+      run_i = 0;
+    }
     const int2 it = P.items[item];
     const TaskDesc T = P.tasks[it.x];
+    run_n = T.run;
     const LensDesc LD = P.lenses[T.lens_cat];
     const GridDesc G = P.grids[T.src_cat];
     const ChunkS* __restrict__ src = reinterpret_cast<const ChunkS*>(G.sph);
-    const int g = it.y / T.split, part = it.y - g * T.split;  // this item's rows: every T.split-th
+    const int per = T.split / T.run, g = it.y / per;
+    const int part = (it.y - g * per) * T.run + run_i++;  // its rows: every T.split-th
     const int gs = LD.group_start[g];
     const bool act = lane < LD.group_start[g + 1] - gs;
     LensS Lf;
@@ -586,7 +591,7 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
       w = (double)r.w;
       if (HAS_Z) lz = LD.z[gs + lane];
       if (P.lens_acc && T.lens_acc_off >= 0)
-        lens_col = P.lens_acc + T.lens_acc_off + (size_t)part * kQ * nb * LD.n_valid + gs + lane;
+        lens_col = P.lens_acc + T.lens_acc_off + (size_t)(T.run > 1 ? 0 : part) * kQ * nb * LD.n_valid + gs + lane;
     } else {
       Lf = lens_frame(make_float4(1.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f));
     }
@@ -688,7 +693,7 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
     }
     if (aborted) break;
     warp_fold<QA, 32>(hist, hcol, wsum, fvw, fw, nb, lens_col, lens_stride, 0, lane);
-    double* out = P.item_sums + (size_t)(T.item_base + it.y) * kQ * nb;
+    double* out = P.item_sums + (size_t)(T.item_base + g * T.split + part) * kQ * nb;
     for (int e = lane; e < kQ * nb; e += 32) {
       const int from = (e / nb == QK && QA == 5) ? e - (QK - QW) * nb : e;
       out[e] = wsum[from];
@@ -818,7 +823,7 @@ __global__ void k_item_cost_sph(const int2* __restrict__ ranges, int n_ranges, i
   const TaskDesc T = tasks[it.x];
   const LensDesc L = lenses[T.lens_cat];
   const GridDesc G = grids[T.src_cat];
-  const int g = it.y / T.split, part = it.y - g * T.split;
+  const int per = T.split / T.run, g = it.y / per, part = it.y - g * per;
   const float4 box = L.group_box[g];
   int cy0, cy1;
   row_range(G, box, R, T.margin, cy0, cy1);
@@ -826,7 +831,7 @@ __global__ void k_item_cost_sph(const int2* __restrict__ ranges, int n_ranges, i
   bool full;
   sph_reach(G, box, R, T.margin, dl, full);
   unsigned long long s = 0;
-  for (int cy = cy0 + part; cy <= cy1; cy += T.split) {
+  for (int cy = cy0 + part; cy <= cy1; cy += per) {
     int2 sp[3];
     const int k = sph_row_spans(G, box, R, T.margin, cy, dl, full, sp);
     for (int j = 0; j < k; ++j)

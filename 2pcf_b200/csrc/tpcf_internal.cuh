@@ -94,7 +94,7 @@ struct LensDesc {
   const float4* pos;        // sphere: {hi.xyz, 0}, {lo.xyz, 0} per sorted lens, else nullptr
 };
 
-// Items that a lens group of a task is cut into at most.
+// Parts that a lens group of a task is cut into at most.
 constexpr int kMaxSplit = 8;
 
 // FP32 histogram folded into FP64 every 4096 sources (each histogram cell then
@@ -111,7 +111,8 @@ struct TaskDesc {
   int src_cat;
   int item_base;            // row of (task, group 0) in item_sums
   float margin;             // FP32 guard on the reach of this task's rows and cells
-  int split;                // work items per lens group, each with every split-th cell row (1 for most)
+  int split;                // parts of a lens group, each with every split-th cell row and sums of its own (1 for most)
+  int run;                  // parts of a work item: 1, or split where their per-lens sums would take too much memory
   int flush_src;            // FP32 sums -> FP64 after this many sources (k_pairs, k_pairs_sph)
   long long lens_acc_off;   // element offset of this task's per-lens sums, -1 = none
 };
@@ -120,7 +121,7 @@ struct PairParams {
   const TaskDesc* tasks;
   const LensDesc* lenses;
   const GridDesc* grids;
-  const int2* items;        // (task, group * split + part) in processing order
+  const int2* items;        // (task, group * (split / run) + part) in processing order
   int n_items;
   int nb;
   int* queue_head;

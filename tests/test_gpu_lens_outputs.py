@@ -47,23 +47,31 @@ def test_large_host_outputs(tpcf, ctx):
         np.testing.assert_array_equal(res.lens_sums[i, 5], np.histogram(d2, bins.bin_edges_sq)[0])
 
 
-def test_workspace_of_a_batch_of_many_tasks(tpcf):
+@pytest.mark.parametrize("sky", [False, True])
+def test_workspace_of_a_batch_of_many_tasks(tpcf, sky):
     """60 tasks with per-lens sums: the split groups' extra columns are bounded for the
-    call, not only per task (1.7 GB of sums in all, 8 times that with 8 parts each);
-    counts as when launched alone, sums to the FP32 partials' order."""
+    call, not only per task (1.7 GB of sums in all, 8 times that with 8 sets each);
+    sums per bin as when launched alone, bit for bit, per lens to FP64 rounding."""
     ctx = tpcf.Context(0)
     L, S = uniform_shear(30_000, 2000, 400.0, 350, w="uniform")
+    unit = np.pi / 180 / 60 if sky else 1.0
+    for c in (L, S):
+        c["x"], c["y"] = (c["x"] * unit).astype(np.float32), ((c["y"] - 200.0) * unit).astype(np.float32)
     lens = tpcf.LensCatalog(L["x"], L["y"], L["val"], L["w"], L["z"])
     src = tpcf.ShapeCatalog(*(S[k] for k in ("x", "y", "e1", "e2", "w", "z", "m")))
-    bins = tpcf.create_bins(1.0, 20.0, 20)
+    bins = tpcf.create_bins(1.0 * unit, 20.0 * unit, 20)
     unsplit = 8 * 6 * 20 * 30_000
-    res = tpcf.batch_shear_2pcf([lens], [src], [(0, 0)] * 60, bins, lens_sums="device", ctx=ctx)
+    res = tpcf.batch_shear_2pcf([lens], [src], [(0, 0)] * 60, bins, lens_sums="device", spherical_coords=sky, ctx=ctx)
     held = ctx.stats()["workspace_bytes"]
-    alone = tpcf.batch_shear_2pcf([lens], [src], [(0, 0)], bins, lens_sums="device", ctx=ctx)[0]
+    alone = tpcf.batch_shear_2pcf([lens], [src], [(0, 0)], bins, lens_sums="device", spherical_coords=sky, ctx=ctx)[0]
     ctx.close()
     assert held <= 1.25 * (60 * unsplit + (1 << 30))   # a slot is a quarter larger than asked for
+    ref = alone.lens_sums.cpu().numpy()
     for r in res:
-        np.testing.assert_array_equal(r.n_pairs, alone.n_pairs)
-        np.testing.assert_allclose(r.sum_w, alone.sum_w, rtol=1e-6)
-        np.testing.assert_array_equal(r.lens_sums[:, 5].cpu().numpy(), alone.lens_sums[:, 5].cpu().numpy())
+        for k in ("n_pairs", "sum_gt", "sum_gx", "sum_w", "sum_dw", "sum_K"):
+            np.testing.assert_array_equal(getattr(r, k), getattr(alone, k))
+        got = r.lens_sums.cpu().numpy()
+        np.testing.assert_array_equal(got[:, 5], ref[:, 5])
+        np.testing.assert_allclose(got[:, 3], ref[:, 3], rtol=1e-12)
+        np.testing.assert_allclose(got[:, 1], ref[:, 1], rtol=1e-12, atol=1e-12)
     assert abs(alone.lens_sums[:, 3].sum().item() - alone.sum_w.sum()) <= 1e-9 * alone.sum_w.sum()
