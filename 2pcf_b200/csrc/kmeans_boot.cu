@@ -662,6 +662,7 @@ tpcf_status tpcf_kmeans(tpcf_ctx* c, const float* x, const float* y, const float
                                                     reassign_tol, max_iter, state);
         counted(c, cudaGetLastError(), "k-means pass");
       }
+      if (batch == 8) expect_outputs(c, {{labels_out, sizeof(int) * (size_t)n}});  // while the first passes run
       check(cudaMemcpyAsync(&hstate, state, sizeof(hstate), cudaMemcpyDeviceToHost, st), "D2H k-means state");
       check(cudaStreamSynchronize(st), "sync k-means");
     }

@@ -48,8 +48,10 @@ struct tpcf_ctx {
   std::string err;
   std::vector<tpcf::Slot> slots;
   size_t next_slot = 0;
-  void* pinned = nullptr;  // staging of large outputs to pageable host memory (copy_out_large), at most kPinnedMax
-  size_t pinned_bytes = 0;
+  void* stage = nullptr;  // kStageBytes of staging for large outputs (copy_out_large), until the context goes
+  void* stage_map = nullptr;
+  size_t stage_map_bytes = 0;
+  bool stage_failed = false;
   int64_t launches = 0;
   int64_t h2d_bytes = 0;
   // statistics of the last call
@@ -77,17 +79,26 @@ const T* stage(tpcf_ctx* c, const T* p, int64_t n);
 // for the caller once the stream is).
 void put_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes);
 void copy_out(tpcf_ctx* c, void* dst, const void* src, size_t bytes);
-// Several outputs at once; complete when it returns for host destinations.
-// Large ones to pageable host memory go through pinned pieces that host threads
-// copy on while the next pieces arrive: a plain copy is one driver thread that
-// also takes the page faults of fresh memory (33.6 MB of marks: 7.4 ms).
+// Large outputs to pageable host memory.  A plain copy is one driver thread that also
+// takes the page faults of fresh memory one by one: 32 MB 16.3 ms, against 1.6 ms into
+// pages that are there.  expect_outputs(), called while the GPU still works on them,
+// has their pages made (contents stay as they are), or from kStagedBytes on the
+// context's staging memory, through which copy_out_large() brings them in pieces that
+// host threads copy on, faults included, while the next pieces land.
+struct HostOut {
+  const void* dst;
+  size_t bytes;
+};
 struct HostCopy {
   void* dst;
   const void* src;
   size_t bytes;
 };
-constexpr size_t kPinnedMax = (size_t)64 << 20, kPinnedPiece = (size_t)2 << 20;
+constexpr size_t kStagePiece = (size_t)2 << 20, kStageBytes = (size_t)16 << 20, kStagedBytes = (size_t)12 << 20;
+void expect_outputs(tpcf_ctx* c, const std::vector<HostOut>& outs);
+// Complete when it returns for host destinations.
 void copy_out_large(tpcf_ctx* c, const std::vector<HostCopy>& v);
+void stage_free(tpcf_ctx* c);
 void begin_call(tpcf_ctx* c);
 cudaStream_t aux_stream(tpcf_ctx* c);
 // The bounding boxes, counts and patch ranges of ncat catalogues on the device

@@ -75,3 +75,28 @@ def test_workspace_of_a_batch_of_many_tasks(tpcf, sky):
         np.testing.assert_allclose(got[:, 3], ref[:, 3], rtol=1e-12)
         np.testing.assert_allclose(got[:, 1], ref[:, 1], rtol=1e-12, atol=1e-12)
     assert abs(alone.lens_sums[:, 3].sum().item() - alone.sum_w.sum()) <= 1e-9 * alone.sum_w.sum()
+
+
+@pytest.mark.parametrize("n", [13_000, 13_108, 200_000])
+def test_large_host_outputs_at_odd_addresses(tpcf, ctx, monkeypatch, n):
+    """Marks of around and well above 1 MiB each into host memory that starts and ends
+    inside pages: the values of the device-independent sums, and nothing outside."""
+    L, S = uniform_shear(n, 3000, 600.0, 360, w="uniform")
+    bins = tpcf.create_bins(1.0, 15.0, 20)
+    alloc, held = tpcf._alloc_result, []
+
+    def odd(nb, nA, *a):
+        r, c = alloc(nb, nA, *a)
+        for k in ("xi_E_marks", "xi_B_marks", "K_marks", "w_marks"):
+            buf = np.full(nA * nb + 64, 7.0, np.float32)
+            held.append(buf)
+            r[k] = buf[3:3 + nA * nb].reshape(nA, nb)
+            setattr(c, k, r[k].ctypes.data)
+        return r, c
+    monkeypatch.setattr(tpcf, "_alloc_result", odd)
+    res = tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"], S["e1"],
+                                     S["e2"], S["w"], S["m"], bins, calculate_marks=True, lens_sums=True, ctx=ctx)
+    for buf in held:
+        assert np.all(buf[:3] == 7.0) and np.all(buf[3 + n * 20:] == 7.0)
+    for k, q in (("xi_E_marks", 1), ("xi_B_marks", 2), ("K_marks", 4), ("w_marks", 3)):
+        np.testing.assert_array_equal(getattr(res, k), res.lens_sums[:, q].astype(np.float32))
