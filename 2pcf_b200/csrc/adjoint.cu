@@ -757,7 +757,8 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     const int li = t.lens, si = nL + t.src;
     if (hc[li] > 0 && hc[si] > 0 && hb[8 * li + 5] > hb[8 * si + 4]) has_z = true;
   }
-  const bool logb = bins->spacing == TPCF_LOG && e2[0] >= kMinLogD2;
+  const BinRule rule = bin_rule(bins, e.data(), e2.data(), false);
+  const bool logb = rule.on;
   const double Rd = bins->x_max;
   const float R = (float)(Rd * (1.0 + 1e-6));
 
@@ -902,15 +903,7 @@ tpcf_status run_adjoint_batch(tpcf_ctx* c, std::vector<AdjLensIn> lens, std::vec
     AdjParams P{};
     P.tasks = d_at; P.items = d_items; P.n_items = n_items; P.nb = nb; P.queue_head = head;
     P.err = (unsigned*)(head + 1); P.e2 = de2; P.e2f = de2f; P.coef = dcoef; P.R = R; P.margin = margin;
-    if (logb) {
-      const double l0 = std::log2(e2[0]), l1 = std::log2(e2[nb]);
-      const double A = nb / (l1 - l0);
-      P.binA = (float)A;
-      P.binB = (float)(-l0 * A);
-      P.eps = 1.0f / 32768.0f;
-    } else {
-      P.eps = 4e-6f;
-    }
+    P.binA = rule.A; P.binB = rule.B; P.eps = rule.eps;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (c->time_pairs) {
       check(cudaEventCreate(&ev0), "event");

@@ -352,6 +352,24 @@ tpcf_status canonical_edges(const tpcf_bins* b, double* e, double* e2) {
   return TPCF_OK;
 }
 
+// The error of t: lg2 is within 2^-22 of its value L (2^-22 at least), theta^2 within
+// 1e-6 of its own (that is 1.5e-6 in L), and the two roundings of L A + B.  Ordinary
+// binnings (20 bins, 1' to 300': 9e-6) stay far below 2^-15; 128 bins from 10' to 11'
+// need 2e-3.  Bins so narrow that the guard would take a good part of them are
+// searched, as are squared distances below kMinLogD2 and, on the sphere, chords beyond
+// the series for theta^2 (0.25).
+BinRule bin_rule(const tpcf_bins* b, const double* e, const double* e2, bool sph) {
+  BinRule r{false, 0.f, 0.f, 4e-6f};
+  const int n = b->n_bin;
+  if (b->spacing != TPCF_LOG || e2[0] < kMinLogD2 || (sph && e2[n] > 0.0625)) return r;
+  const double l0 = std::log2(e[0] * e[0]), l1 = std::log2(e[n] * e[n]);
+  const double A = n / (l1 - l0), L = std::max({1.0, std::fabs(l0), std::fabs(l1)});
+  const double err = A * (std::ldexp(L, -22) + 1.5e-6) + std::ldexp(A * L + std::fabs(l0 * A) + n, -24);
+  const double eps = std::max(std::ldexp(1.0, -15), 1.25 * err);
+  if (eps > 1.0 / 64) return r;
+  return {true, (float)A, (float)(-l0 * A), (float)eps};
+}
+
 // Bin centres in FP32 as create_bins computes them (src/utils.f90:202-229).
 void bin_centers_f32(const tpcf_bins* b, float* centers) {
   const int n = b->n_bin;
@@ -561,8 +579,8 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
       if (lz_max > sz_min) has_z = true;
     }
   }
-  // On the sphere log binning maps theta^2 by a series valid for chords <= 0.25.
-  const bool logb = bins->spacing == TPCF_LOG && e2[0] >= kMinLogD2 && (!sph || e2[nb] <= 0.0625);
+  const BinRule rule = bin_rule(bins, e.data(), e2.data(), sph);
+  const bool logb = rule.on;
   const int qa = has_m ? 6 : 5;
   int bt = 128;
   while (bt > 32 && (size_t)nb * qa * bt * 4 > 100 * 1024) bt /= 2;
@@ -827,16 +845,7 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   P.tasks = d_tasks; P.lenses = d_lens; P.grids = d_grids;
   P.nb = nb; P.item_sums = item_sums; P.lens_acc = lens_acc; P.err = err;
   P.e2 = d_e2; P.e2f = d_e2f; P.R = R;
-  if (logb) {  // t = log2(theta^2) A + B (planar: theta^2 = d2)
-    const double l0 = std::log2(e[0] * e[0]), l1 = std::log2(e[nb] * e[nb]);
-    const double A = nb / (l1 - l0);
-    P.binA = (float)A;
-    P.binB = (float)(-l0 * A);
-    P.eps = 1.0f / 32768.0f;
-  } else {
-    P.binA = P.binB = 0.f;
-    P.eps = 4e-6f;
-  }
+  P.binA = rule.A; P.binB = rule.B; P.eps = rule.eps;
   P.far_bin = series_far_bin(e2.data(), nb);
   int bt_pairs = bt;  // of k_pairs
   if (!sph && B.variant == 0 && c->opts.group_size == 0 && c->opts.tile_chunks == 0) pair_tile_shape(nb, qa, &bt_pairs, &tch);

@@ -143,7 +143,8 @@ tpcf_status run_noalloc(tpcf_ctx* c, const float* xA, const float* yA, const flo
 
   const bool has_m = mB != nullptr && hcnt[1] > 0 && hbox[8 + 6] != 0.f;
   const bool has_z = hcnt[0] > 0 && hcnt[1] > 0 && hbox[5] > hbox[8 + 4];
-  const bool logb = bins->spacing == TPCF_LOG && e2[0] >= kMinLogD2;
+  const BinRule rule = bin_rule(bins, e, e2, false);
+  const bool logb = rule.on;
   const int qa = has_m ? 6 : 5;
   int bt = 128;
   while (bt > 32 && (size_t)nb * qa * bt * 4 > 100 * 1024) bt /= 2;
@@ -260,16 +261,7 @@ tpcf_status run_noalloc(tpcf_ctx* c, const float* xA, const float* yA, const flo
     P.tasks = d_task; P.lenses = d_lens; P.grids = d_grid; P.items = items; P.n_items = n_groups;
     P.nb = nb; P.queue_head = head; P.item_sums = item_sums; P.lens_acc = nullptr; P.err = err;
     P.e2 = d_e2; P.e2f = d_e2f; P.R = R;
-    if (logb) {
-      const double l0 = std::log2(e2[0]), l1 = std::log2(e2[nb]);
-      const double A = nb / (l1 - l0);
-      P.binA = (float)A;
-      P.binB = (float)(-l0 * A);
-      P.eps = 1.0f / 32768.0f;
-    } else {
-      P.binA = P.binB = 0.f;
-      P.eps = 4e-6f;
-    }
+    P.binA = rule.A; P.binB = rule.B; P.eps = rule.eps;
     int grid = 0;
     counted(c, launch_pairs(P, 0, has_m, has_z, logb, bt, 2, 0, c->num_sms, st, &grid), "pair kernel");
     counted(c, launch_patch_reduce(item_sums, 0, 1, pgroups, 1, nb, psum, st), "patch reduce");

@@ -142,4 +142,12 @@ struct Event {
   Event& operator=(const Event&) = delete;
 };
 tpcf_status canonical_edges(const tpcf_bins* b, double* e, double* e2);
+// How the kernels find a bin: for log spacing t = lg2(theta^2) A + B in FP32, with a
+// guard band eps around whole numbers that covers its error; on = false: a search of
+// the squared edges with a relative guard eps.  sph: angle edges e, squared chords e2.
+struct BinRule {
+  bool on;
+  float A, B, eps;
+};
+BinRule bin_rule(const tpcf_bins* b, const double* e, const double* e2, bool sph);
 }  // namespace tpcf

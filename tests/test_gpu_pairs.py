@@ -291,3 +291,15 @@ def test_scalar_auto_correlation_per_lens(tpcf, oracle, ctx):
     can = canon(oracle, oracle.KAPPA, dict(x=x, y=y, val=k, w=w), dict(x=x, y=y, kappa_E=k, kappa_B=k, w=w), bins)
     check_sums("auto-correlation with marks", res, can)
     assert all(np.isfinite(getattr(res, q)).all() for q in ("xi_E_marks", "xi_B_marks", "K_marks", "w_marks"))
+
+
+@pytest.mark.parametrize("lo,hi,nb", [(10.0, 11.0, 128), (50.0, 60.0, 100), (1000.0, 1003.0, 128), (10.0, 20.0, 128)])
+@pytest.mark.parametrize("marks", [False, True])
+def test_narrow_log_bins(tpcf, oracle, ctx, lo, hi, nb, marks):
+    """Log bins so narrow that the FP32 error of lg2(d^2) is a part of them: counts stay
+    those of the FP64 rule."""
+    L, S = uniform_shear(300, 60_000, 6.0 * hi, 34, w="uniform")
+    bins = tpcf.create_bins(lo, hi, nb)
+    res = tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"], S["e1"],
+                                     S["e2"], S["w"], S["m"], bins, calculate_marks=marks, ctx=ctx)
+    check_sums(f"narrow log bins {lo} {hi}", res, canon(oracle, oracle.SHEAR, L, S, bins))
