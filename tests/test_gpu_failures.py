@@ -72,6 +72,30 @@ def test_bounded_wait_runs_out_then_recovery(tpcf, oracle):
     ctx.close()
 
 
+@pytest.mark.parametrize("kind", ["series", "sphere"])
+def test_bounded_wait_of_the_series_and_spherical_kernels(tpcf, oracle, kind):
+    """The same for the kernel of dense source catalogues and the one on the sky."""
+    ctx = tpcf.Context(0)
+    L, S = uniform_shear(400, 60_000, 60.0, 91)
+    unit = np.pi / 180 / 60 if kind == "sphere" else 1.0
+    for c in (L, S):
+        c["x"], c["y"] = (c["x"] * unit).astype(np.float32), (c["y"] * unit).astype(np.float32)
+    bins = tpcf.create_bins(0.5 * unit, 20.0 * unit, 8)
+    kw = dict(calculate_marks=False, spherical_coords=kind == "sphere", ctx=ctx)
+    call = lambda: tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"],  # noqa: E731
+                                              S["e1"], S["e2"], S["w"], S["m"], bins, **kw)
+    for tile, polls in ((0, 1 << 12), (4, 1 << 14)):
+        inject(tpcf, ctx, skip_tile=tile, wait_polls=polls)
+        with pytest.raises(tpcf.TPCFError) as e:
+            call()
+        assert e.value.status == tpcf._lib.TPCF_ERR_TIMEOUT, str(e.value)
+    inject(tpcf, ctx)
+    can = (oracle.canon_sphere(oracle.SHEAR, L, S, bins.chord_edges_sq) if kind == "sphere" else
+           oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
+    check_sums(f"{kind} call after a bounded wait ran out", call(), can)
+    ctx.close()
+
+
 def test_marks_bounded_wait_runs_out_then_recovery(tpcf, oracle):
     ctx = tpcf.Context(0)
     rng = np.random.default_rng(92)

@@ -216,3 +216,49 @@ def test_tasks_of_a_mixed_batch(tpcf, ctx, monkeypatch):
         np.testing.assert_allclose(together[t].sum_K, alone.sum_K, rtol=1e-14)
         if tasks[t][2]:
             np.testing.assert_array_equal(together[t].xi_E_marks, alone.xi_E_marks)
+
+
+@pytest.mark.parametrize("cut,calibration", [(True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("spacing,lo", [("log", 0.3), ("lin", 0.0), ("sqrt", 0.5)])
+def test_cut_and_calibration_apart(tpcf, oracle, ctx, spacing, lo, cut, calibration):
+    L, S = catalogues(82, 97, z=True)
+    if not cut:
+        L["z"][:] = 0.0
+    if not calibration:
+        S["m"][:] = 0.0
+    bins = tpcf.create_bins(lo, 20.0, 9, spacing=spacing, p=0.5)
+    res = shear(tpcf, ctx, L, S, bins)
+    check_sums(f"series {spacing} cut={cut} m={calibration}", res,
+               oracle.canon_pairs(oracle.SHEAR, L, S, bins.bin_edges_sq))
+
+
+@pytest.mark.parametrize("spacing,lo", [("lin", 0.0), ("sqrt", 0.5)])
+def test_kappa_other_spacings(tpcf, oracle, ctx, spacing, lo):
+    """Scalar-scalar, lenses drawn from the sources: d = 0 counts in bin 0 from x_min = 0
+    and leaves the sums finite (they hold no angle)."""
+    L, S = catalogues(83, 70)
+    L["x"][:30], L["y"][:30] = S["x"][:30], S["y"][:30]
+    bins = tpcf.create_bins(lo, 20.0, 9, spacing=spacing)
+    res = tpcf.scalar_kappa_tpcf(L["x"], L["y"], L["val"], L["w"], S["x"], S["y"], S["e1"], S["e2"], S["w"], bins,
+                                 calculate_marks=False, ctx=ctx)
+    K = dict(x=S["x"], y=S["y"], kappa_E=S["e1"], kappa_B=S["e2"], w=S["w"])
+    check_sums(f"series kappa {spacing}", res, oracle.canon_pairs(oracle.KAPPA, L, K, bins.bin_edges_sq))
+
+
+def test_values_that_are_not_finite(tpcf, ctx):
+    """A NaN ellipticity and an infinite weight reach the bins of their own pairs and no
+    others: far away from every lens, none."""
+    L, S = catalogues(84, 40)
+    L["x"], L["y"] = f32(L["x"] * 0.3), f32(L["y"] * 0.3)
+    bins = tpcf.create_bins(0.5, 12.0, 6)
+    clean = shear(tpcf, ctx, L, S, bins)
+    gone = np.flatnonzero((S["x"] > 45) & (S["y"] > 45))
+    S["e1"][gone[0]], S["w"][gone[1]] = np.nan, np.inf
+    res = shear(tpcf, ctx, L, S, bins)
+    for k in ("n_pairs", "sum_gt", "sum_gx", "sum_w", "sum_dw"):
+        np.testing.assert_array_equal(getattr(res, k), getattr(clean, k))
+    one = np.argmin(np.hypot(S["x"] - L["x"][0], S["y"] - L["y"][0]))
+    S["e1"][one] = np.nan
+    res = shear(tpcf, ctx, L, S, bins)
+    np.testing.assert_array_equal(res.n_pairs, clean.n_pairs)
+    assert np.isnan(res.sum_gt).any() and np.all(np.isfinite(res.sum_w)) and np.all(np.isfinite(res.sum_dw))
