@@ -333,6 +333,15 @@ __device__ __forceinline__ void add_bin(const float (&v)[6], int bin, int nb, do
 
 }  // namespace
 
+#ifdef TPCF_MODE_STATS
+// Diagnostic build only: (lens, sub-chunk) combinations [out of range, far, direct with
+// 0, 1, 2, more edges], lists, lenses listed.
+__device__ unsigned long long g_series_stats[8];
+extern "C" int tpcf_debug_series_stats(unsigned long long* out) {
+  return (int)cudaMemcpyFromSymbol(out, g_series_stats, sizeof(g_series_stats));
+}
+#endif
+
 // Far sums of the warp's 32 columns into its FP64 sums; the columns are cleared.
 template <int QA>
 __device__ __forceinline__ void fold_far(float* hist, double* wsum, int nb, int tb, int lane) {
@@ -378,6 +387,10 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
     e2s[i] = P.e2[i];
     e2f[i] = P.e2f[i];
   }
+#ifdef TPCF_MODE_STATS
+  __shared__ unsigned long long sh_stats[8];
+  if (tid < 8) sh_stats[tid] = 0ull;
+#endif
   for (int e = 0; e < (nb - tb) * QA; ++e) hist[e * 32 + lane] = 0.f;
   __syncthreads();
   BinCtx C;
@@ -534,6 +547,16 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
             any_far = any_far || far[l];
             any_dir = any_dir || (in[l] && !far[l]);
           }
+#ifdef TPCF_MODE_STATS
+#pragma unroll
+          for (int l = 0; l < kLpl; ++l) {
+            const int cls = !act[l] ? -1 : !in[l] ? 0 : far[l] ? 1 : 2 + min(b1[l] - b0[l], 3);
+            for (int q = 0; q < 6; ++q) {
+              const unsigned n = __popc(__ballot_sync(0xffffffffu, cls == q));
+              if (lane == 0 && n) atomicAdd(&sh_stats[q], (unsigned long long)n);
+            }
+          }
+#endif
           if (!__any_sync(0xffffffffu, any_in)) continue;
           if (__any_sync(0xffffffffu, any_far)) {
             const float4 sums = ld4(rec + 8);
@@ -646,6 +669,12 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
               cnt += __popc(mem[l]);
             }
             const int kb = (kkey >> 3) - 1, kt = kkey & 7;
+#ifdef TPCF_MODE_STATS
+            if (lane == 0) {
+              atomicAdd(&sh_stats[6], 1ull);
+              atomicAdd(&sh_stats[7], (unsigned long long)cnt);
+            }
+#endif
             __syncwarp();
             int base = 0;
 #pragma unroll
@@ -736,6 +765,10 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
       if (t + 1 != P.debug_skip_tile) mbar_wait_bounded(&full[t % kNbuf], (uint32_t)(t / kNbuf) & 1u, wait_limit);
     if (lane == 0) atomicOr(P.err, kErrTimeout);
   }
+#ifdef TPCF_MODE_STATS
+  __syncthreads();
+  if (tid < 8) atomicAdd(&g_series_stats[tid], sh_stats[tid]);
+#endif
 }
 
 // Sub-chunk records of the cell-sorted sources: one warp per 32-source
@@ -857,6 +890,11 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
 }
 
 // --------------------------------------------------------- host launchers --
+#ifdef TPCF_MODE_STATS
+constexpr int kMaxDynamic = 226 * 1024;  // beside the counters
+#else
+constexpr int kMaxDynamic = 227 * 1024;
+#endif
 template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB>
 static cudaError_t prepare_t(const PairParams& P, int bt, int num_sms, PairLaunch* L) {
   constexpr int QA = (MODE == 0 && HAS_M) ? 6 : 5;
@@ -865,7 +903,7 @@ static cudaError_t prepare_t(const PairParams& P, int bt, int num_sms, PairLaunc
   while (bt > 32 && edge_smem(P.nb) + per * (bt / 32) > 110 * 1024) bt /= 2;
   const size_t smem = edge_smem(P.nb) + per * (bt / 32);
   auto kern = k_pairs_series<MODE, HAS_M, HAS_Z, LOGB>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamic);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, smem);

@@ -619,7 +619,8 @@ O_SHEAR, O_KAPPA = 0, 1   # oracle modes (oracle.SHEAR, oracle.KAPPA)
 
 def path_stats(tpcf, args):
     """One batched call on the diagnostic build; prints the share of warp
-    sub-chunks and lane-pairs per path of k_pairs."""
+    sub-chunks and lane-pairs per path of k_pairs, and of (lens, sub-chunk)
+    combinations per path of k_pairs_series."""
     import ctypes as C
     import torch
     tpcf._lib.LIB_PATH = os.path.join(ROOT, "2pcf_b200", "libtpcf_b200_stats.so")
@@ -634,20 +635,29 @@ def path_stats(tpcf, args):
     ctx = tpcf.Context(0)
     ctx.set_cell_size(bins.x_max / (args.cell_divisor or 64))
     lib = tpcf._lib.lib()
-    st = (C.c_ulonglong * 15)()
-    lib.tpcf_debug_mode_stats(st)
-    base = np.array(st[:])
-    outs = tpcf.batch_shear_2pcf(L, S, w["tasks"], bins, ctx=ctx)
-    lib.tpcf_debug_mode_stats(st)
-    v = np.array(st[:]) - base
+
+    def counters():
+        p, q = (C.c_ulonglong * 15)(), (C.c_ulonglong * 8)()
+        lib.tpcf_debug_mode_stats(p)
+        lib.tpcf_debug_series_stats(q)
+        return np.array(p[:]), np.array(q[:])
+    base = counters()
+    outs = tpcf.batch_shear_2pcf(L, S, w["tasks"], bins, lens_sums="device" if args.per_lens else False, ctx=ctx)
+    v, u = (a - b for a, b in zip(counters(), base))
     binned = sum(int(o.n_pairs.sum()) for o in outs)
     res = {"binned_pairs": binned}
     names = ("skip", "single_bin", "one_edge", "two_edges", "per_pair")
-    for i, name in enumerate(names):
-        res[name] = {"warp_chunks": float(v[i] / v[:5].sum()), "lane_pairs": float(v[5 + i] / v[5:10].sum())}
-    res["computed_lane_pairs_per_binned_pair"] = float(v[6:10].sum() / binned)
-    res["lane_class_of_active_lane_pairs"] = {("out_of_range" if i == 0 else name): float(v[10 + i] / v[10:15].sum())
-                                              for i, name in enumerate(names)}
+    if v[:5].sum():
+        res["k_pairs"] = {name: {"warp_chunks": float(v[i] / v[:5].sum()), "lane_pairs": float(v[5 + i] / v[5:10].sum())}
+                          for i, name in enumerate(names)}
+        res["k_pairs"]["computed_lane_pairs_per_binned_pair"] = float(v[6:10].sum() / binned)
+        res["k_pairs"]["lane_class_of_active_lane_pairs"] = {
+            ("out_of_range" if i == 0 else name): float(v[10 + i] / v[10:15].sum()) for i, name in enumerate(names)}
+    if u[:6].sum():
+        kinds = ("out_of_range", "far", "direct_one_bin", "direct_one_edge", "direct_two_edges", "direct_more_edges")
+        res["k_pairs_series"] = {"lens_sub_chunks": int(u[:6].sum()),
+                                 **{k: float(u[i] / u[:6].sum()) for i, k in enumerate(kinds)},
+                                 "lists": int(u[6]), "lenses_per_list": float(u[7] / max(u[6], 1))}
     print(json.dumps(res), flush=True)
 
 
@@ -710,6 +720,7 @@ def main():
     ap.add_argument("--path-stats", action="store_true",
                     help="diagnostic: load the counting build (make -C 2pcf_b200/csrc stats) and print the "
                          "pair kernel's path mix for one batched call instead of benchmarking")
+    ap.add_argument("--per-lens", action="store_true", help="with --path-stats: per-lens sums (k_pairs for every task)")
     ap.add_argument("--region", type=float, default=0.0,
                     help="profiling: keep only objects with x, y < REGION arcmin (density unchanged)")
     ap.add_argument("--task", type=int, default=-1, help="profiling: run only this task of the 25")
