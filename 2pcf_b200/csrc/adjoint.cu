@@ -593,7 +593,7 @@ template <bool HAS_Z, bool LOGB, bool WX>
 cudaError_t launch_adj_t(const AdjParams& P, int num_sms, cudaStream_t st) {
   const size_t smem = adj_smem(P.nb).total;
   auto kern = k_adj<HAS_Z, LOGB, WX>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dynamic_smem(kern);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BT, smem);

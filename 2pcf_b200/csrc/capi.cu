@@ -71,7 +71,9 @@ bool is_device_ptr(const void* p) {
 }
 
 void check(cudaError_t e, const char* what) {
-  if (e != cudaSuccess) throw Failure(TPCF_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  if (e == cudaSuccess) return;
+  cudaGetLastError();  // the next call's first launch must not find it
+  throw Failure(TPCF_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 void counted(tpcf_ctx* c, cudaError_t e, const char* what) {

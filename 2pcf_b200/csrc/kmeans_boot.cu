@@ -650,7 +650,7 @@ tpcf_status tpcf_kmeans(tpcf_ctx* c, const float* x, const float* y, const float
     k_km_init_labels<<<std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(lab, n, k);
     counted(c, cudaGetLastError(), "init labels");
     const size_t smem = (sizeof(float2) + sizeof(unsigned long long) * 3 + sizeof(float)) * k;
-    check(cudaFuncSetAttribute(k_km_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+    check(allow_dynamic_smem(k_km_pass), "smem attr");
     const int blocks = (int)std::max<long long>(1, std::min<long long>((n + kKmTile - 1) / kKmTile, c->num_sms * 4));
     // Lloyd passes in batches (8, 16, then 32) with the stopping rule evaluated
     // on the device: one host synchronisation per batch; passes after
@@ -829,8 +829,8 @@ tpcf_status tpcf_kmeans_equal(tpcf_ctx* c, const float* x, const float* y, const
     // sweep chunk: at most 1/2048 of the points, 32..1024
     const int chunk = (int)std::max<long long>(32, std::min<long long>(1024, n / 2048));
     const size_t smem = sizeof(float2) * k + sizeof(long long) * k + sizeof(float) * k;
-    check(cudaFuncSetAttribute(k_km_sweep_eq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
-    check(cudaFuncSetAttribute(k_km_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm), "smem attr");
+    check(allow_dynamic_smem(k_km_sweep_eq), "smem attr");
+    check(allow_dynamic_smem(k_km_sums), "smem attr");
     int it = 0;
     unsigned long long hre = 0;
     while (it <= max_iter) {

@@ -657,14 +657,14 @@ cudaError_t launch_marks_partials(const MarksField* fields, int n_field, int nbl
   if (nb <= kDmmaMaxBins) {
     const MarksDmma<Fac> k = marks_dmma_kernel<Fac>(nb);
     const size_t msm = marks_dmma_smem(nb);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess) return e;
     k<<<grid, 32 * kDmmaWarps, msm, st>>>(fields, n_field, fac, n_maps, nb, chunk, part, err, skip_tile, wait_limit);
     return cudaGetLastError();
   }
   const size_t msm = marks_smem(nb);
   const int bt = marks_block_threads(nb), tg = marks_group_threads(nb);
-  cudaError_t e = cudaFuncSetAttribute(k_marks_partials<Fac>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
+  cudaError_t e = allow_dynamic_smem(k_marks_partials<Fac>);
   if (e != cudaSuccess) return e;
   k_marks_partials<Fac><<<grid, bt, msm, st>>>(fields, n_field, fac, n_maps, nb, tg, chunk, part);
   return cudaGetLastError();

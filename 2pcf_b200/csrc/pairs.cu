@@ -1146,7 +1146,7 @@ static cudaError_t prepare_pairs_t(const PairParams& P, int num_sms, PairLaunch*
   constexpr int QA = (MODE == 0 && HAS_M) ? 6 : 5;
   const size_t smem = pair_smem_layout(P.nb, QA, BT, TCH).total;
   auto kern = k_pairs<MODE, HAS_M, HAS_Z, LOGB, BT, TCH, PATH>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_dynamic_smem(kern);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BT, smem);

@@ -890,11 +890,6 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
 }
 
 // --------------------------------------------------------- host launchers --
-#ifdef TPCF_MODE_STATS
-constexpr int kMaxDynamic = 226 * 1024;  // beside the counters
-#else
-constexpr int kMaxDynamic = 227 * 1024;
-#endif
 template <int MODE, bool HAS_M, bool HAS_Z, bool LOGB>
 static cudaError_t prepare_t(const PairParams& P, int bt, int num_sms, PairLaunch* L) {
   constexpr int QA = (MODE == 0 && HAS_M) ? 6 : 5;
@@ -903,7 +898,7 @@ static cudaError_t prepare_t(const PairParams& P, int bt, int num_sms, PairLaunc
   while (bt > 32 && edge_smem(P.nb) + per * (bt / 32) > 110 * 1024) bt /= 2;
   const size_t smem = edge_smem(P.nb) + per * (bt / 32);
   auto kern = k_pairs_series<MODE, HAS_M, HAS_Z, LOGB>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamic);
+  cudaError_t e = allow_dynamic_smem(kern);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, smem);

@@ -850,7 +850,7 @@ static cudaError_t launch_sph_t(const PairParams& P, int num_sms, cudaStream_t s
   const int bt = sph_edge_smem(P.nb) + 2 * per <= 113 * 1024 ? 64 : 32;  // two blocks per SM at least
   const size_t smem = sph_edge_smem(P.nb) + per * (bt / 32);
   auto kern = k_pairs_sph<MODE, HAS_M, HAS_Z, LOGB>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  cudaError_t e = allow_dynamic_smem(kern);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, smem);

@@ -8,6 +8,17 @@
 
 namespace tpcf {
 
+// Lets a kernel be launched with up to 227 KB of shared memory.  The limit belongs to
+// the kernel, not to a launch: set to one launch's size, it would refuse a launch that
+// a plan, another context or another thread has prepared with more.
+template <class Kernel>
+cudaError_t allow_dynamic_smem(Kernel kern) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
+}
+
 size_t pair_smem_bytes(int nb, int qa, int bt, int tch);
 void pair_tile_shape(int nb, int qa, int* bt, int* tch);
 // bt = lenses per group (threads per block), tch = 32-source sub-chunks per

@@ -79,3 +79,25 @@ def test_plan_per_lens_rows_and_misuse(tpcf):
     with pytest.raises(tpcf.TPCFError):
         tpcf.BatchPlan([L0], [S0], [(0, 0)], bins, ctx=ctx)
     ctx.close()
+
+
+@pytest.mark.parametrize("per_lens", [False, True])
+def test_plan_after_calls_with_other_bins(tpcf, ctx, per_lens):
+    """Calls with fewer bins run the same kernels with less shared memory; a plan made
+    before them still launches with its own."""
+    rng = np.random.default_rng(41)
+    f = lambda a: np.ascontiguousarray(a, np.float32)  # noqa: E731
+    n = 3000
+    L = tpcf.LensCatalog(f(rng.uniform(0, 200, n)), f(rng.uniform(0, 200, n)), f(rng.normal(0, .02, n)),
+                         f(rng.uniform(.5, 1.5, n)), f(np.zeros(n)))
+    S = tpcf.ShapeCatalog(f(rng.uniform(0, 200, n)), f(rng.uniform(0, 200, n)), f(rng.normal(0, .3, n)),
+                          f(rng.normal(0, .3, n)), f(np.ones(n)), f(np.ones(n)), f(np.zeros(n)))
+    bins, few = tpcf.create_bins(1.0, 60.0, 20), tpcf.create_bins(1.0, 60.0, 8)
+    ref = tpcf.batch_shear_2pcf([L], [S], [(0, 0)], bins, lens_sums=per_lens, ctx=ctx)[0]
+    plan = tpcf.BatchPlan([L], [S], [(0, 0)], bins, lens_sums=per_lens, ctx=ctx)
+    tpcf.batch_shear_2pcf([L], [S], [(0, 0)], few, lens_sums=per_lens, ctx=ctx)
+    plan.launch()
+    got = plan.results()[0]
+    plan.close()
+    np.testing.assert_array_equal(got.sum_gt, ref.sum_gt)
+    np.testing.assert_array_equal(got.n_pairs, ref.n_pairs)
