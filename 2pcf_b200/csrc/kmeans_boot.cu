@@ -73,7 +73,10 @@ __global__ void k_km_init_labels(int* labels, long long n, int k) {
 // 1 M points, 100 centroids: 21.5 ms for the call when every pass formed every
 // distance and re-summed every point, 8.6 ms with far alone, 6.6 ms with both and
 // one wave of blocks (32 registers; 222 passes of 10 to 30 us: the latency of
-// the chain label -> centroid -> search -> last block, not its traffic).
+// the chain label -> centroid -> search -> last block, not its traffic).  A block
+// takes `tile` points at a time: fewer than kKmTile where that would leave SMs without
+// points (two blocks per SM: 3000 points, 400 centroids 0.99 -> 0.46 ms; 30 k and 20
+// 0.80 -> 0.62; every distance in every pass: 0.53 and 0.73).
 struct KmState {
   int done, passes;
   float drift;
@@ -86,7 +89,7 @@ __global__ void __launch_bounds__(kKmThreads, 4) k_km_pass(const float* __restri
                                                         const float* __restrict__ w, long long n, float2* cen, int k,
                                                         float min_init, int sp, int sw, int* labels, float* far,
                                                         float* half, unsigned long long* acc, float tol, int max_iter,
-                                                        KmState* state) {
+                                                        int tile, KmState* state) {
   if (state->done) return;  // converged in an earlier pass of this batch
   extern __shared__ unsigned char sm[];
   float2* c = reinterpret_cast<float2*>(sm);
@@ -107,13 +110,14 @@ __global__ void __launch_bounds__(kKmThreads, 4) k_km_pass(const float* __restri
   for (int j = threadIdx.x; j < 3 * k; j += blockDim.x) a[j] = 0ull;
   unsigned re = 0;
   if (threadIdx.x == 0) n_changed = 0;
-  for (long long t0 = (long long)blockIdx.x * kKmTile; t0 < n; t0 += (long long)gridDim.x * kKmTile) {
+  for (long long t0 = (long long)blockIdx.x * tile; t0 < n; t0 += (long long)gridDim.x * tile) {
     if (threadIdx.x == 0) n_list = 0;
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < kKmTile / kKmThreads; ++u) {
-      const long long i = t0 + u * kKmThreads + threadIdx.x;
-      bool open = i < n;
+      const int q = u * kKmThreads + threadIdx.x;
+      const long long i = t0 + q;
+      bool open = q < tile && i < n;
       if (open && !first) {
         const int l = labels[i];
         if (l >= 0) {
@@ -122,7 +126,7 @@ __global__ void __launch_bounds__(kKmThreads, 4) k_km_pass(const float* __restri
           open = !((d < h[l] || d < far[i] - D) && d < 0.999f * min_init);
         }
       }
-      if (open) list[atomicAdd(&n_list, 1)] = (int)(i - t0);
+      if (open) list[atomicAdd(&n_list, 1)] = q;
     }
     __syncthreads();
     const int nl = n_list;
@@ -651,18 +655,19 @@ tpcf_status tpcf_kmeans(tpcf_ctx* c, const float* x, const float* y, const float
     counted(c, cudaGetLastError(), "init labels");
     const size_t smem = (sizeof(float2) + sizeof(unsigned long long) * 3 + sizeof(float)) * k;
     check(allow_dynamic_smem(k_km_pass), "smem attr");
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((n + kKmTile - 1) / kKmTile, c->num_sms * 4));
-    // Lloyd passes in batches (8, 16, then 32) with the stopping rule evaluated
+    const int tile = (int)std::clamp<long long>((n + 2 * c->num_sms - 1) / (2 * c->num_sms) + 63, 64, kKmTile) / 64 * 64;
+    const int blocks = (int)std::max<long long>(1, std::min<long long>((n + tile - 1) / tile, c->num_sms * 4));
+    // Lloyd passes in batches (8, later 16 and 32) with the stopping rule evaluated
     // on the device: one host synchronisation per batch; passes after
     // convergence return at once.
     KmState hstate{};
-    for (int batch = 8; !hstate.done; batch = std::min(32, batch * 2)) {
+    for (int batch = 8; !hstate.done; batch = hstate.passes < 16 ? 8 : hstate.passes < 48 ? 16 : 32) {
       for (int b = 0; b < batch; ++b) {
         k_km_pass<<<blocks, kKmThreads, smem, st>>>(x, y, w, n, dcen, k, diam * 10.0f, sp, sw, lab, far, half, acc,
-                                                    reassign_tol, max_iter, state);
+                                                    reassign_tol, max_iter, tile, state);
         counted(c, cudaGetLastError(), "k-means pass");
       }
-      if (batch == 8) expect_outputs(c, {{labels_out, sizeof(int) * (size_t)n}});  // while the first passes run
+      if (hstate.passes == 0) expect_outputs(c, {{labels_out, sizeof(int) * (size_t)n}});  // while the first passes run
       check(cudaMemcpyAsync(&hstate, state, sizeof(hstate), cudaMemcpyDeviceToHost, st), "D2H k-means state");
       check(cudaStreamSynchronize(st), "sync k-means");
     }

@@ -54,3 +54,17 @@ def test_stopping_rules(tpcf, oracle, ctx, max_iter, tol):
     assert it == it_o
     np.testing.assert_array_equal(lab, lab_o)
     np.testing.assert_array_equal(cen, cen_o)
+
+
+@pytest.mark.parametrize("n", [3, 63, 64, 65, 18_943, 18_944, 18_945, 606_207, 606_209])
+def test_points_of_a_block(tpcf, oracle, ctx, n):
+    """Around the steps of the number of points that a block takes at a time."""
+    rng = np.random.default_rng(n)
+    x, y = points("uniform", n, rng)
+    w = f32(rng.uniform(0.2, 1.5, n))
+    k = 2 if n < 63 else 11
+    lab, cen, it = tpcf.partition_data(x, y, w, k, iterations=12, ctx=ctx)
+    lab_o, cen_o, it_o = oracle.kmeans_det(x, y, w, k, 12, 0.0)
+    assert it == it_o
+    np.testing.assert_array_equal(lab, lab_o)
+    np.testing.assert_array_equal(cen, cen_o)
