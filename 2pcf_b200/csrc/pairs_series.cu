@@ -71,7 +71,7 @@ constexpr float kEdgeBand = 1.0e-6f;
 // to its FP64 sums (FP32 sums of at most 8 x 32 pairs per lane).
 constexpr int kKeep = 8;
 
-// One sub-chunk record: {box}{cx cy s (s / kFarRatio)^2}{P Q W K sums}{zmin zmax 0 0},
+// One sub-chunk record: {cx cy s (s / kFarRatio)^2}{P Q W K sums}{zmin zmax 0 0},
 // shear: kOrder + 1 times {M_re N_re M_im N_im}, then the distance series
 // {W00 W11/4 W22/64 0}{W10, -W21/8}{-W20/4, W31/16}{W30/8, -5/128 W41}
 // {-5/64 W40, 7/128 W50}{-W32/64, 0}, then the fields of the 32 sources, each [32]:
@@ -81,7 +81,7 @@ struct RecShape {
 };
 __host__ __device__ constexpr RecShape rec_shape(int mode, bool has_m, bool has_z) {
   RecShape r{};
-  r.g = 16;
+  r.g = 12;
   r.d = r.g + (mode == 0 ? 4 * (kOrder + 1) : 0);
   r.src = r.d + 24;
   r.fields = 5 + (has_m ? 1 : 0) + (has_z ? 1 : 0);
@@ -523,12 +523,12 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
           const int hi = j == tg.n - 1 ? tg.hiL : kChunk;
           const bool whole = lo == 0 && hi == kChunk;
           const float* __restrict__ rec = ring + (size_t)(b * kTch + j) * R.floats;
-          const float4 cen = ld4(rec + 4);
+          const float4 cen = ld4(rec);
           float Zx[kLpl], Zy[kLpl], Z2[kLpl], rs[kLpl], dc[kLpl];
           int b0[kLpl], b1[kLpl];
           bool in[kLpl], far[kLpl], any_in = false, any_far = false, any_dir = false;
           float2 zr = make_float2(0.f, 0.f);
-          if (HAS_Z) zr = *reinterpret_cast<const float2*>(rec + 12);
+          if (HAS_Z) zr = *reinterpret_cast<const float2*>(rec + 8);
 #pragma unroll
           for (int l = 0; l < kLpl; ++l) {
             Zx[l] = cen.x - lx[l];
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kSeriesThreads, kSeriesBlocks) k_pairs_series(
 #endif
           if (!__any_sync(0xffffffffu, any_in)) continue;
           if (__any_sync(0xffffffffu, any_far)) {
-            const float4 sums = ld4(rec + 8);
+            const float4 sums = ld4(rec + 4);
             float r[kLpl], tx[kLpl], ty[kLpl], gt[kLpl], gx[kLpl], dw[kLpl];
 #pragma unroll
             for (int l = 0; l < kLpl; ++l) {
@@ -839,12 +839,11 @@ __global__ void k_src_series(const int* __restrict__ idx, int n_valid, int n_chu
   const double sp = red(dp), sq = red(dq), sw = red(dw), sk = red((double)K);
   if (lane == 0) {
     float4* o4 = reinterpret_cast<float4*>(out);
-    o4[0] = make_float4(mnx, mny, mxx, mxy);
     // never 0: a lens on the centre of a sub-chunk without extent has no series
     const float far2 = (float)((double)rad * rad / ((double)kFarRatio * kFarRatio));
-    o4[1] = make_float4(cx, cy, rad, fmaxf(far2, kMinNormal));
-    o4[2] = make_float4((float)sp, (float)sq, (float)sw, (float)sk);
-    o4[3] = make_float4(mnz, mxz, 0.f, 0.f);
+    o4[0] = make_float4(cx, cy, rad, fmaxf(far2, kMinNormal));
+    o4[1] = make_float4((float)sp, (float)sq, (float)sw, (float)sk);
+    o4[2] = make_float4(mnz, mxz, 0.f, 0.f);
   }
   const double uu = ux * ux + uy * uy;
   double re = 1.0, im = 0.0;  // (delta / s)^k

@@ -163,7 +163,7 @@ __device__ __forceinline__ int pair_bin_s(float d2, const LensS& L, const float4
 // Conservative bin class of a 3-D box (min mn, max mx of the chunk's hi parts,
 // already widened by the hi/lo split error) for one lens; classes as in the
 // planar kernel.
-template <bool LOGB, bool HAS_Z>
+template <bool LOGB>
 __device__ __forceinline__ int classify_s(const LensS& L, const float4 mn, const float4 mx, const BinCtx& C,
                                           int& blo) {
   const float dxl = fmaxf(fmaxf(mn.x - L.h.x, L.h.x - mx.x), 0.f);
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(64, 6) k_pairs_sph(const PairParams P) {
         const int lo = tg.lo0, hi = tg.hiL;
         const bool partial = lo > 0 || hi < kChunk;
         int blo = 0;
-        const int cls = act ? classify_s<LOGB, HAS_Z>(Lf, ch->mn, ch->mx, C, blo) : 0;
+        const int cls = act ? classify_s<LOGB>(Lf, ch->mn, ch->mx, C, blo) : 0;
         const int m = (int)__reduce_max_sync(0xffffffffu, (unsigned)cls);
         const float4 ss = ch->sum;
         if (m == 1) {
