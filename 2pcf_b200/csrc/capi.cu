@@ -467,13 +467,29 @@ bool wants_lens(const tpcf_result& o) {
 // ratio 0.08: 3.3 / 5.0, 0.12: 2.08 / 2.22, 0.17: 1.60 / 1.38 and 6.7 / 6.0,
 // 0.26: 4.5 / 2.6 -- wider sub-chunks straddle several edges and few
 // combinations are far.  In the other spacings k_pairs searches the bin of
-// every pair: 0.34: 7.3 / 12.9, 0.77: 3.2 / 4.7, 1.1: 3.0 / 3.4, 1.7: 2.9 / 1.6.
+// every pair, and the mean over the pairs of the bins that a sub-chunk spans
+// decides (each bin's share of the pairs over its width).  Times of the call before
+// there was a series kernel / now, 100 k lenses, by that span (sources 10 k to 400 k):
+//   linear              1.3: 1.8, 1.8: 1.29, 2.0: 1.37 (k_pairs from 2.2 on: 1.14 to 1.26)
+//   square root         1.5: 1.47, 1.8: 1.41, 2.2: 0.98 (k_pairs: 1.25 to 1.3)
+//   inverse hyperbolic  0.8: 1.4, 1.0: 1.5, 1.15: 0.84, 1.6: 0.88 (k_pairs: 1.1 to 1.3);
+//     sine              its narrow bins at small separations make short lists
 bool series_pays(int n_valid, double ex, double ey, const tpcf_bins* bins, const double* edges) {
   if (n_valid < kChunk) return false;
   const double half = std::sqrt(0.5 * kChunk * ex * ey / n_valid);
-  const double width = edges[bins->n_bin] - edges[bins->n_bin - 1];
-  return half <= (bins->spacing == TPCF_LOG ? 0.14 : 1.1) * width;
+  const int nb = bins->n_bin;
+  if (bins->spacing == TPCF_LOG) return half <= 0.14 * (edges[nb] - edges[nb - 1]);
+  double span = 0.0;  // sum of (e1^2 - e0^2) / (e1 - e0)
+  for (int i = 0; i < nb; ++i) span += edges[i] + edges[i + 1];
+  const double most = bins->spacing == TPCF_LIN ? 2.2 : bins->spacing == TPCF_SQRT ? 1.8 : 1.0;
+  return 2.0 * half * span <= most * (edges[nb] * edges[nb] - edges[0] * edges[0]);
 }
+
+// Lenses from which k_pairs_series takes a source grid of one row: its groups are not
+// cut into parts there, and they are half as many as those of k_pairs.  (No grid,
+// 100 k sources; k_pairs / series: 20 k lenses, 15 log bins to 500' 5.4 / 7.5 ms, 60 k
+// 8.0 / 8.1.)
+constexpr unsigned long long kOneRowLenses = 75000;
 
 // A task with fewer lens groups than kSplitItems / 2 is cut into several items
 // per group (at most kMaxSplit).
@@ -613,21 +629,21 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
     }
     double cell = c->opts.cell_size > 0 ? c->opts.cell_size : Rd / 16.0;
     const double span = std::max((double)ex, (double)ey);
-    // the pair kernel of each of its tasks, by the task and this catalogue alone;
-    // records for each kernel that reads it
-    const bool dense = !sph && B.variant == 0 && series_pays(n_valid, ex, ey, bins, e.data());
-    bool series = false, other = false;
-    for (int t = 0; t < nT; ++t)
-      if (ts[t] == i) {
-        B.kind[t] = dense && !wants_lens(outs[t]);
-        (B.kind[t] ? series : other) = true;
-      }
     if (!c->opts.use_grid) cell = span * 2.0 + 1.0;
     // keep the grid below 2^24 cells
     while ((span / cell + 2.0) * (span / cell + 2.0) > (double)(1 << 24)) cell *= 1.5;
     if (!(cell > 0)) cell = 1.0;
     int ncx = (int)std::floor(ex / cell) + 1, ncy = (int)std::floor(ey / cell) + 1;
     ncx = std::max(1, ncx); ncy = std::max(1, ncy);
+    // the pair kernel of each of its tasks, by its two catalogues and outputs alone;
+    // records for each kernel that reads it
+    const bool dense = !sph && B.variant == 0 && series_pays(n_valid, ex, ey, bins, e.data());
+    bool series = false, other = false;
+    for (int t = 0; t < nT; ++t)
+      if (ts[t] == i) {
+        B.kind[t] = dense && !wants_lens(outs[t]) && (ncy > 1 || hcnt[tl[t]] >= kOneRowLenses);
+        (B.kind[t] ? series : other) = true;
+      }
     const unsigned ncells = (unsigned)ncx * (unsigned)ncy;
     g.x0 = x0; g.y0 = y0; g.cell = (float)cell; g.inv_cell = (float)(1.0 / cell);
     g.ncx = ncx; g.ncy = ncy; g.n_valid = n_valid;
