@@ -804,7 +804,9 @@ void batch_setup(tpcf_ctx* c, int mode, std::vector<LensIn> lens, std::vector<Sr
   for (int t = 0; t < nT; ++t) {
     TaskDesc& d = tdesc[t];
     const int ng = lb[tl[t]].by[(int)B.kind[t]].n_groups;
-    d.split = ng > 0 ? std::max(1, std::min(kMaxSplit, kSplitItems / ng)) : 1;
+    // (parts take cell rows: no more of them than rows, or they hold nothing and crowd
+    // the rest; no grid, 20 k x 100 k: 5.4 -> 6.2 ms)
+    d.split = ng > 0 ? std::max(1, std::min({kMaxSplit, kSplitItems / ng, grids[ts[t]].ncy})) : 1;
     const size_t lens_bytes = sizeof(double) * kQ * nb * (size_t)std::max(lb[tl[t]].n_valid, 1);
     if (!wants_lens(outs[t])) continue;
     while (d.split > 1 && lens_bytes * d.split > kSplitLensBytes) --d.split;
