@@ -1072,7 +1072,9 @@ __global__ void __launch_bounds__(32 * kReduceWarps) k_patch_reduce(const double
 // shared memory and both sides are runs of 160 to 256 bytes; with one thread per
 // lens every store of a warp touched 32 sectors: 60 k lenses in 4 parts, 15 bins,
 // raw FP64 sums: 195 us, against 50 now (32 at 6650 GB/s; 71 with the parts loaded
-// one after the other).
+// one after the other).  20 bins a chunk keep seven blocks on an SM: 100 k
+// lenses in 2 parts, 20 / 24 / 31 / 32 bins 96 / 127 / 152 / 147 us, against 121 / 131 /
+// 160 / 196 with chunks of 31.
 constexpr int kOutBins = 20;
 __global__ void __launch_bounds__(128) k_lens_outputs(const double* __restrict__ acc, int split,
                                                       const float4* __restrict__ rec, const int* __restrict__ perm,

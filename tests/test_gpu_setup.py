@@ -50,3 +50,43 @@ def test_item_counts(tpcf, ctx, n_lens):
     ctx.set_shard(0, 0)
     np.testing.assert_array_equal(sum(p.n_pairs for p in parts), n)
     np.testing.assert_allclose(sum(p.sum_gt for p in parts), res.sum_gt, rtol=0, atol=1e-12 * np.abs(res.sum_w).max())
+
+
+def test_contexts_on_several_threads(tpcf):
+    """One context per host thread, each with its own bins, clusters and marks (other
+    amounts of shared memory for the same kernels): the results of a thread alone."""
+    import threading
+    rng = np.random.default_rng(91)
+    f = lambda a: np.ascontiguousarray(a, np.float32)  # noqa: E731
+    L, S = uniform_shear(3000, 20_000, 100.0, 92, w="uniform")
+    work = [(8, False, 5), (20, True, 90), (31, True, 400), (60, True, 20)]
+    marks = [[tpcf.MarksField(x=f(rng.normal(size=4000)), y=f(rng.normal(size=4000)), w=f(rng.uniform(.5, 1, 4000)),
+                              xi_E=f(rng.normal(size=(4000, nb))), xi_B=f(rng.normal(size=(4000, nb))),
+                              K=f(rng.uniform(.5, 1, (4000, nb))))] for nb, _, _ in work]
+
+    def calls(ctx, i):
+        nb, per_lens, k = work[i]
+        r = tpcf.tangential_shear_tpcf(L["x"], L["y"], L["z"], L["val"], L["w"], S["x"], S["y"], S["z"], S["e1"],
+                                       S["e2"], S["w"], S["m"], tpcf.create_bins(1.0, 30.0, nb),
+                                       calculate_marks=per_lens, ctx=ctx)
+        b = tpcf.marks_bootstrap(marks[i], 20, seed=2, covariance=False, ctx=ctx)
+        q = tpcf.partition_data(S["x"], S["y"], S["w"], k, iterations=15, ctx=ctx)
+        return [r.n_pairs, r.sum_gt, b["g_t"], q[0], q[1]] + ([r.xi_E_marks] if per_lens else [])
+    ctx = tpcf.Context(0)
+    alone = [calls(ctx, i) for i in range(len(work))]
+    ctx.close()
+    wrong = []
+
+    def thread(i):
+        try:
+            c = tpcf.Context(0)
+            for _ in range(15):
+                for a, b in zip(calls(c, i), alone[i]):
+                    np.testing.assert_array_equal(a, b)
+            c.close()
+        except BaseException as e:  # noqa: BLE001
+            wrong.append((i, repr(e)[:300]))
+    threads = [threading.Thread(target=thread, args=(i,)) for i in range(len(work))]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not wrong, wrong
