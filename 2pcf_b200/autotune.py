@@ -11,7 +11,9 @@ in flight in each warp's ring).  ``autotune`` times the pair kernel
 field that keeps the object density: first every cell side theta_max/d with
 the default shape, then every shape with the best cell side, and sets the
 fastest on the context.  Results do not depend on either choice (every pair
-is binned by the same rule); only speed does.
+is binned by the same rule); only speed does.  Calls without per-lens outputs over
+dense sources run a kernel with one shape: the shapes then time alike and the pick
+serves the context's other calls.
 """
 from __future__ import annotations
 

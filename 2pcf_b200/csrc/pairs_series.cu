@@ -48,9 +48,9 @@ namespace tpcf {
 namespace {
 
 // At least 14 warps per SM, at most 144 registers: the tomography call (25 tasks,
-// 1.24e12 pairs) takes 869 ms against 952 ms with 12 warps at 168 registers; where
-// the compiler needs 128 or less, as without z cut and calibration, 16 warps fit
-// and gain nothing more.
+// 1.24e12 pairs) took 869 ms against 952 ms with 12 warps at 168 registers (874 now,
+// with one more order in both series); where the compiler needs 128 or less, as without
+// z cut and calibration, 16 warps fit and gain nothing more.
 constexpr int kSeriesThreads = 64, kSeriesBlocks = 7;
 constexpr float kFarRatio = 0.08f;
 constexpr float kNullPos = 1.0e18f;  // coordinate of a source that takes no part: every term stays finite
@@ -67,8 +67,9 @@ constexpr int kOrder = 6;            // M_0 .. M_6, N_0 .. N_5
 // Guard band around a squared edge, relative: FP32 d2 is within 3e-7 of its
 // exact value and the FP32 edge within 6e-8.
 constexpr float kEdgeBand = 1.0e-6f;
-// Sub-chunks whose one-edge sums a warp keeps in registers before it adds them
-// to its FP64 sums (FP32 sums of at most 8 x 32 pairs per lane).
+// Lists whose one-edge sums a warp keeps in registers before it adds them to its FP64
+// sums: FP32 sums of at most 8 x 64 pairs per lane (a list holds up to 64 lenses), in
+// runs of 32 and 8, then a tree over the 32 lanes.
 constexpr int kKeep = 8;
 
 // One sub-chunk record: {cx cy s (s / kFarRatio)^2}{P Q W K sums}{zmin zmax 0 0},

@@ -111,9 +111,10 @@ __device__ __forceinline__ int2 row_span(const GridDesc& G, float4 box, float R,
 }
 
 // Cost band of a work item: log2 of its cost in steps of 2^(1/8) (about 9%),
-// below kCostBands.  The costliest bands start first (load balance); inside
-// one band the items run in task and space order, so that the warps resident
-// at one time read the same rows of one source grid and those stay in L2.
+// below kCostBands.  The costliest bands start first (load balance).  Where
+// a radix sort orders the items (more than k_item_order takes, or shards), those of one
+// band keep their task and space order, so that the warps resident at one time read
+// the same rows of one source grid and those stay in L2.
 constexpr int kCostBands = 512;
 __device__ __forceinline__ unsigned cost_band(unsigned long long cost) {
   return min((unsigned)(__log2f((float)cost) * 8.f), (unsigned)kCostBands - 1u);

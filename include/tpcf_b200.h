@@ -77,12 +77,14 @@ typedef struct tpcf_opts {
                             must be summed over shards (one all-reduce);
                             normalised outputs are not written            */
   int32_t shard_count;   /* 0 or 1: no sharding                              */
-  int32_t group_size;    /* planar pair kernel tile shape: threads per block
-                            (32, 64 or 128; 0 = 128, halved while the
-                            per-lens histogram would exceed 100 KB); each
-                            warp takes 32-lens work items of its own         */
+  int32_t group_size;    /* tile shape of the planar pair kernel for per-lens
+                            outputs and sparse sources: threads per block
+                            (32, 64 or 128; 0 = the shape that keeps most
+                            warps on an SM for the binning); each warp takes
+                            32-lens work items of its own.  The kernel for
+                            dense sources has one shape                      */
   int32_t tile_chunks;   /* 32-source sub-chunks per source tile (1 or 2;
-                            0 = 2), in a 4 KB ring per warp                 */
+                            0 = as above), in two buffers per warp          */
   int32_t reserved[3];
 } tpcf_opts;
 
