@@ -1379,7 +1379,9 @@ tpcf_status tpcf_plan_shear_scalar(tpcf_ctx* c, int32_t n_lens_cat, const tpcf_l
   tpcf_ctx* pc = nullptr;
   tpcf_status st = tpcf_create(&pc, c->device, &c->opts);
   if (st != TPCF_OK) return st;
-  pc->stream = c->stream;
+  // the stream a caller has set on the context; its own one goes with the context, which
+  // the plan may outlive
+  if (c->stream != c->own_stream) pc->stream = c->stream;
   tpcf_plan* pl = new tpcf_plan();
   pl->ctx = pc;
   pl->bins = *bins;

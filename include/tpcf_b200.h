@@ -416,14 +416,14 @@ tpcf_status tpcf_batch_scalar_scalar(tpcf_ctx* ctx,
  * has (non-null fields; the pointers are not kept).
  *
  * tpcf_plan_launch enqueues the persistent pair kernel and the per-patch
- * reductions on the plan's stream (the context's stream when the plan was
- * made, or tpcf_plan_set_stream): no host synchronisation, no allocation and
+ * reductions on the plan's stream (the one set on the context when the plan was
+ * made, else one of its own; or tpcf_plan_set_stream): no host synchronisation, no allocation and
  * no other API call, so the sequence may be recorded into a CUDA graph
  * (stream capture) and replayed.  tpcf_plan_results waits for the last launch
  * and writes the outputs of every task, as tpcf_batch_shear_scalar would
  * (same sums bit for bit); its outs must have the per-lens outputs the plan
  * was made with.  The plan keeps its own device workspace; the context it was
- * made from stays free for other calls.  Spherical contexts return
+ * made from stays free for other calls and may be destroyed before it.  Spherical contexts return
  * TPCF_ERR_NOT_SUPPORTED. */
 typedef struct tpcf_plan tpcf_plan;
 tpcf_status tpcf_plan_shear_scalar(tpcf_ctx* ctx,

@@ -101,3 +101,17 @@ def test_plan_after_calls_with_other_bins(tpcf, ctx, per_lens):
     plan.close()
     np.testing.assert_array_equal(got.sum_gt, ref.sum_gt)
     np.testing.assert_array_equal(got.n_pairs, ref.n_pairs)
+
+
+def test_plan_outlives_its_context(tpcf, ctx):
+    rng = np.random.default_rng(42)
+    L, S = catalogues(tpcf, rng, 2000, 4000, 100.0, False)
+    bins = tpcf.create_bins(1.0, 40.0, 10)
+    direct = tpcf.batch_shear_2pcf([L], [S], [(0, 0)], bins, ctx=ctx)
+    own = tpcf.Context(0)
+    plan = tpcf.BatchPlan([L], [S], [(0, 0)], bins, ctx=own)
+    own.close()
+    for _ in range(2):
+        plan.launch()
+        same(plan.results(), direct)
+    plan.close()
