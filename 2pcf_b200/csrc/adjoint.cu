@@ -963,7 +963,8 @@ extern "C" tpcf_status tpcf_shear_scalar_adjoint(
     std::vector<AdjSrcIn> S{{nB, xB, yB, zB, e1B, e2B, wB, mB, grad_e1B, grad_e2B, grad_wB, grad_mB}};
     std::vector<AdjTaskIn> T{{0, 0, sum_gt, sum_gx, sum_K, lens_raw, dL_dgt, dL_dgx}};
     return run_adjoint_batch(c, L, S, T, bins);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     c->err = f.msg;
     return f.status;
   }
@@ -996,7 +997,8 @@ extern "C" tpcf_status tpcf_batch_shear_scalar_adjoint(
       T.push_back({task_lens[t], task_src[t], a.sum_gt, a.sum_gx, a.sum_K, a.lens_raw, a.dL_dgt, a.dL_dgx});
     }
     return run_adjoint_batch(c, L, S, T, bins);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     c->err = f.msg;
     return f.status;
   }

@@ -18,6 +18,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <stdexcept>
 #include <string>
 #include <thread>
 #include <utility>
@@ -33,6 +34,18 @@ using namespace tpcf;
 
 // ------------------------------------------------------------- ctx helpers --
 namespace tpcf {
+
+Failure caught() {
+  try {
+    throw;
+  } catch (const Failure& f) {
+    return f;
+  } catch (const std::length_error& e) {
+    return Failure(TPCF_ERR_OVERFLOW, std::string("size out of range: ") + e.what());
+  } catch (const std::exception& e) {  // std::bad_alloc
+    return Failure(TPCF_ERR_OOM, std::string("host memory: ") + e.what());
+  }
+}
 
 void* ws_alloc(tpcf_ctx* c, size_t bytes) {
   if (bytes == 0) bytes = 16;
@@ -1206,7 +1219,8 @@ tpcf_status tpcf_unit_vectors(tpcf_ctx* c, const float* lam, const float* phi, i
     if (dlo != lo) copy_out(c, lo, dlo, sizeof(float) * 3 * (size_t)n);
     check(cudaStreamSynchronize(c->stream), "sync unit vectors");
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -1238,7 +1252,8 @@ tpcf_status tpcf_measure_fp32_peak(tpcf_ctx* c, double* tflops) {
     cudaEventDestroy(e1);
     *tflops = 2.0 * 8.0 * (double)iters * threads * blocks / (ms * 1e-3) / 1e12;
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -1263,7 +1278,8 @@ tpcf_status tpcf_measure_fp64_peak(tpcf_ctx* c, double* tflops) {
     cudaEventDestroy(e1);
     *tflops = 2.0 * 8.0 * (double)iters * threads * blocks / (ms * 1e-3) / 1e12;
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -1303,7 +1319,8 @@ tpcf_status tpcf_shear_scalar(tpcf_ctx* c, const float* xA, const float* yA, con
     std::vector<LensIn> L{{nA, xA, yA, zA, valA, wA, patchA}};
     std::vector<SrcIn> S{{nB, xB, yB, zB, e1B, e2B, wB, mB}};
     return run_batch(c, 0, L, S, {0}, {0}, bins, n_patch, out);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -1317,7 +1334,8 @@ tpcf_status tpcf_scalar_scalar(tpcf_ctx* c, const float* xA, const float* yA, co
     std::vector<LensIn> L{{nA, xA, yA, nullptr, valA, wA, patchA}};
     std::vector<SrcIn> S{{nB, xB, yB, nullptr, kE, kB, wB, nullptr}};
     return run_batch(c, 1, L, S, {0}, {0}, bins, n_patch, out);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -1342,7 +1360,8 @@ tpcf_status tpcf_batch_shear_scalar(tpcf_ctx* c, int32_t n_lens_cat, const tpcf_
     }
     std::vector<int> tl(task_lens, task_lens + n_task), ts(task_src, task_src + n_task);
     return run_batch(c, 0, L, S, tl, ts, bins, n_patch, outs);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -1401,7 +1420,8 @@ tpcf_status tpcf_plan_shear_scalar(tpcf_ctx* c, int32_t n_lens_cat, const tpcf_l
     batch_setup(pc, 0, L, S, tl, ts, bins, n_patch, outs, pl->B);
     check(cudaStreamSynchronize(pc->stream), "sync plan");
     pl->slot_mark = pc->next_slot;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     c->err = f.msg;
     tpcf_destroy(pc);
     delete pl;
@@ -1415,7 +1435,8 @@ tpcf_status tpcf_plan_launch(tpcf_plan* pl) {
   if (!pl) return TPCF_ERR_INVALID_ARG;
   try {
     batch_launch(pl->ctx, pl->B, false);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(pl->ctx, f);
   }
   return TPCF_OK;
@@ -1436,7 +1457,8 @@ tpcf_status tpcf_plan_results(tpcf_plan* pl, tpcf_result* outs) {
   try {
     pl->ctx->next_slot = pl->slot_mark;  // the outputs' staging reuses the same slots every time
     batch_finish(pl->ctx, pl->B, &pl->bins, outs);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(pl->ctx, f);
   }
   return TPCF_OK;
@@ -1477,7 +1499,8 @@ tpcf_status tpcf_batch_scalar_scalar(tpcf_ctx* c, int32_t n_lens_cat, const tpcf
     }
     std::vector<int> tl(task_lens, task_lens + n_task), ts(task_kappa, task_kappa + n_task);
     return run_batch(c, 1, L, S, tl, ts, bins, n_patch, outs);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }

@@ -169,7 +169,8 @@ extern "C" tpcf_status tpcf_rotate_from_poles(tpcf_ctx* c, float* xA, float* yA,
     *rotated = rot ? 1 : 0;
     if (center) { center[0] = cx; center[1] = cy; }
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     c->err = f.msg;
     return f.status;
   }

@@ -677,7 +677,8 @@ tpcf_status tpcf_kmeans(tpcf_ctx* c, const float* x, const float* y, const float
     check(cudaStreamSynchronize(st), "sync outputs");
     if (n_iter_out) *n_iter_out = it;
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -727,7 +728,8 @@ tpcf_status tpcf_bootstrap(tpcf_ctx* c, const double* patch_sums, int32_t n_task
     }
     check(cudaStreamSynchronize(st), "sync bootstrap");
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }
@@ -909,7 +911,8 @@ tpcf_status tpcf_kmeans_equal(tpcf_ctx* c, const float* x, const float* y, const
     if (n_iter_out) *n_iter_out = it;
     if (max_dev_out) *max_dev_out = dev;
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     return fail(c, f);
   }
 }

@@ -977,7 +977,8 @@ extern "C" tpcf_status tpcf_xi_from_marks(tpcf_ctx* c, int32_t n_field, const tp
       if (weights_stacked) weights_stacked[m] = sw;
     }
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     c->err = f.msg;
     return f.status;
   }
@@ -1143,7 +1144,8 @@ extern "C" tpcf_status tpcf_marks_bootstrap(tpcf_ctx* c, int32_t n_field, const 
       }
     }
     return TPCF_OK;
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     c->err = f.msg;
     return f.status;
   }

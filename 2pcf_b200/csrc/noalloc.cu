@@ -314,7 +314,8 @@ extern "C" tpcf_status tpcf_shear_scalar_noalloc(tpcf_ctx* c, const float* xA, c
   if (!c || !bins || !out) return TPCF_ERR_INVALID_ARG;
   try {
     return run_noalloc(c, xA, yA, zA, valA, wA, nA, xB, yB, zB, e1B, e2B, wB, mB, nB, bins, out);
-  } catch (const Failure& f) {
+  } catch (...) {
+    const Failure f = caught();
     c->err = f.msg;
     return f.status;
   }

@@ -18,6 +18,9 @@ struct Failure {
   std::string msg;
   Failure(tpcf_status s, std::string m) : status(s), msg(std::move(m)) {}
 };
+// The exception being handled, as a Failure (for the handlers of the C entry points,
+// which let none through).
+Failure caught();
 
 // NVTX range over one phase of a call (grid build, pair kernel, reduction,
 // k-means, resampling), visible in Nsight timelines; free when no tool is

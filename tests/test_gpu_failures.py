@@ -120,3 +120,38 @@ def test_marks_bounded_wait_runs_out_then_recovery(tpcf, oracle):
         np.testing.assert_allclose(out["g_t"][m, 0], per[0]["g_t"], rtol=1e-9)
         np.testing.assert_allclose(out["weights"][m, 0], per[0]["weights"], rtol=1e-12)
     ctx.close()
+
+
+HOST_MEMORY = """
+import importlib, resource, sys
+import numpy as np
+sys.path.insert(0, {root!r})
+tpcf = importlib.import_module("2pcf_b200")
+from importlib import import_module
+rng = np.random.default_rng(1)
+f = lambda *s: rng.uniform(0.5, 1.0, s).astype(np.float32)
+marks = [tpcf.MarksField(x=f(64), y=f(64), w=f(64), xi_E=f(64, 20), xi_B=f(64, 20), K=f(64, 20))]
+ctx = tpcf.Context(0)
+ref = tpcf.marks_bootstrap(marks, 8, seed=1, covariance=False, ctx=ctx)["g_t"]
+held = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (held + (4 << 30), resource.RLIM_INFINITY))
+files = import_module("2pcf_b200.files")
+arr, keep = files._cfields(marks)
+st = tpcf._lib.lib().tpcf_marks_bootstrap(ctx.handle, 1, arr, None, 0, None, 1, 50_000_000, 1.0, 1, None, None, None,
+                                          None, None)
+assert st == tpcf._lib.TPCF_ERR_OOM, st
+again = tpcf.marks_bootstrap(marks, 8, seed=1, covariance=False, ctx=ctx)["g_t"]
+assert np.array_equal(ref, again)
+print("returned")
+"""
+
+
+def test_host_allocation_failure_is_a_status():
+    """Sums that do not fit the process's address space (a limit set for it): the entry
+    point returns TPCF_ERR_OOM, and the context stays usable."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", HOST_MEMORY.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "returned" in r.stdout, (r.returncode, r.stderr[-800:])
