@@ -201,9 +201,10 @@ __device__ __forceinline__ void adj_terms2(float2 nsx, float2 nsy, float sz, con
 }
 
 // Sub-chunk sums of a source whose pairs cross up to NE bin edges (class cls = 1 +
-// its edges, lowest bin blo; a side outside [0, nb) contributes nothing): per edge
-// the sums over the pairs at or above it, by selects on the sign of d2 - E.  False
-// when a pair lies within the guard band of an edge (A is then not complete).
+// its edges, lowest bin blo; a side outside [0, nb) contributes nothing), by selects
+// on the sign of d2 - E: one edge, all pairs and those at or above it; two edges, each
+// side on its own (a difference of sums would carry the rounding of the pairs beyond a
+// bin with few).  False when a pair lies within the guard band of an edge (A is then not complete).
 template <bool HAS_Z, bool LOGB, bool WX, int NE>
 __device__ __forceinline__ bool adj_edges(const LensPair* __restrict__ Sc, int np, float2 nsx, float2 nsy, float sz,
                                           int cls, int blo, const float4* coef, const BinCtx& C, float sum_w,
@@ -222,6 +223,29 @@ __device__ __forceinline__ bool adj_edges(const LensPair* __restrict__ Sc, int n
     float2 d2, F, Pq, Q, w;
     bool z0, z1;
     adj_terms2<HAS_Z, LOGB>(nsx, nsy, sz, Sc[q], d2, F, Pq, Q, w, z0, z1);
+    if (NE == 2) {
+      bool u[2][2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float2 dE = add2(d2, dup2(-E[e < NE ? e : 0]));
+        close[e < NE ? e : 0] = fminf(close[e < NE ? e : 0], fminf(fabsf(dE.x), fabsf(dE.y)));
+        u[e][0] = dE.x >= 0.f;
+        u[e][1] = dE.y >= 0.f;
+      }
+      const float2 F0 = make_float2(u[0][0] ? 0.f : F.x, u[0][1] ? 0.f : F.y);
+      const float2 F2 = make_float2(u[1][0] ? F.x : 0.f, u[1][1] ? F.y : 0.f);
+      const float2 F1 = make_float2(u[0][0] && !u[1][0] ? F.x : 0.f, u[0][1] && !u[1][1] ? F.y : 0.f);
+      T1 = fma2(F0, Pq, T1);
+      T2 = fma2(F0, Q, T2);
+      TN = add2(TN, make_float2(u[0][0] ? 0.f : w.x, u[0][1] ? 0.f : w.y));
+      H1[0] = fma2(F1, Pq, H1[0]);
+      H2[0] = fma2(F1, Q, H2[0]);
+      HN[0] = add2(HN[0], make_float2(u[0][0] && !u[1][0] ? w.x : 0.f, u[0][1] && !u[1][1] ? w.y : 0.f));
+      H1[NE - 1] = fma2(F2, Pq, H1[NE - 1]);
+      H2[NE - 1] = fma2(F2, Q, H2[NE - 1]);
+      HN[NE - 1] = add2(HN[NE - 1], make_float2(u[1][0] ? w.x : 0.f, u[1][1] ? w.y : 0.f));
+      continue;
+    }
     T1 = fma2(F, Pq, T1);
     T2 = fma2(F, Q, T2);
     if (!LI) TN = add2(TN, w);
@@ -236,14 +260,17 @@ __device__ __forceinline__ bool adj_edges(const LensPair* __restrict__ Sc, int n
       HN[e] = add2(HN[e], make_float2(u0 ? w.x : 0.f, u1 ? w.y : 0.f));
     }
   }
-  float p1 = sum2(T1), p2 = sum2(T2), pn = LI ? sum_w : sum2(TN);
+  float p1 = sum2(T1), p2 = sum2(T2), pn = LI && NE == 1 ? sum_w : sum2(TN);
   bool band = false;
 #pragma unroll
   for (int j = 0; j <= NE; ++j) {
     const float h1 = j < NE ? sum2(H1[j < NE ? j : 0]) : 0.f, h2 = j < NE ? sum2(H2[j < NE ? j : 0]) : 0.f,
                 hn = j < NE ? sum2(HN[j < NE ? j : 0]) : 0.f;
     const int bin = blo + j;
-    if (j <= cls - 1 && bin >= 0 && bin < C.nb) adj_apply<WX>(coef[bin], p1 - h1, p2 - h2, pn - hn, A);
+    if (j <= cls - 1 && bin >= 0 && bin < C.nb) {
+      if (NE == 2) adj_apply<WX>(coef[bin], p1, p2, pn, A);
+      else adj_apply<WX>(coef[bin], p1 - h1, p2 - h2, pn - hn, A);
+    }
     p1 = h1;
     p2 = h2;
     pn = hn;

@@ -290,8 +290,10 @@ __device__ __forceinline__ void sph_terms2(const LensS2& L, const SrcPairS& s, f
   }
 }
 
-// Register sums of one lens over a sub-chunk: all pairs (s*) and, per edge,
-// the upper side (h*).
+// Register sums of one lens over a sub-chunk.  One edge: all pairs (s*) and the
+// upper side (h*).  Two edges: each side on its own (s*, h*[0], h*[1]), since a bin
+// between two edges may hold one pair of a sub-chunk whose others are far beyond: a
+// difference of sums would carry their rounding (1.8e-5 of a bin's d w).  Counts are at or above each edge.
 template <int NE>
 struct SphAcc {
   float2 sgt, sgx, sw, sdw, sk, sn;
@@ -334,6 +336,40 @@ __device__ __forceinline__ void sph_step(const LensS2& L, float lz, const SrcPai
     w = mul2(w, vm);
     if (MODE == 0 && HAS_M) K = mul2(K, vm);
     A.sn = add2(A.sn, vm);
+  }
+  if (NE == 2) {
+    const float2 one_neg = dup2(-1.f);
+    float2 m[2], rk[3], wk[3], kk[3];
+    rk[0] = r; wk[0] = w; kk[0] = K;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float2 t = add2(d2, dup2(-E[NE ? e : 0]));
+      A.close[e] = fminf(A.close[e], fminf(fabsf(t.x), fabsf(t.y)));
+      m[e] = make_float2(t.x >= 0.f ? 1.f : 0.f, t.y >= 0.f ? 1.f : 0.f);
+      rk[e + 1] = mul2(r, m[e]);  // r, w, K carry the validity mask already
+      wk[e + 1] = mul2(w, m[e]);
+      rk[e] = fma2(rk[e + 1], one_neg, rk[e]);  // exactly 0 or the value
+      wk[e] = fma2(wk[e + 1], one_neg, wk[e]);
+      if (MODE == 0 && HAS_M) {
+        kk[e + 1] = mul2(K, m[e]);
+        kk[e] = fma2(kk[e + 1], one_neg, kk[e]);
+      }
+      A.hn[e] = add2(A.hn[e], LI ? m[e] : mul2(m[e], vm));
+    }
+    A.sgt = fma2(rk[0], X, A.sgt);
+    A.sgx = fma2(rk[0], Y, A.sgx);
+    A.sw = add2(A.sw, wk[0]);
+    A.sdw = fma2(th, wk[0], A.sdw);
+    if (MODE == 0 && HAS_M) A.sk = add2(A.sk, kk[0]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      A.hgt[e] = fma2(rk[e + 1], X, A.hgt[e]);
+      A.hgx[e] = fma2(rk[e + 1], Y, A.hgx[e]);
+      A.hw[e] = add2(A.hw[e], wk[e + 1]);
+      A.hdw[e] = fma2(th, wk[e + 1], A.hdw[e]);
+      if (MODE == 0 && HAS_M) A.hk[e] = add2(A.hk[e], kk[e + 1]);
+    }
+    return;
   }
   if (!(LI && MODE == 1)) {
     A.sgt = fma2(r, X, A.sgt);
@@ -395,8 +431,8 @@ __device__ __forceinline__ void chunk_single_s(const SrcPairS* __restrict__ S, i
 }
 
 // Classes 2 and 3: pairs in bins blo .. blo + NE across NE = 1 or 2 edges (a bin
-// outside [0, nb) is dropped); edge e is e2f[blo + 1 + e].  Bin blo + j receives
-// h[j-1] - h[j] with h[-1] = all and h[NE] = 0, as in the planar kernel.
+// outside [0, nb) is dropped); edge e is e2f[blo + 1 + e].  One edge: bin blo + j receives
+// h[j-1] - h[j] with h[-1] = all and h[1] = 0, as in the planar kernel; two: its own sums.
 template <int MODE, bool HAS_M, bool HAS_Z, bool SMALL, bool PART, int NC, int QA, int NE>
 __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, int lo, int hi, const LensS& Lf,
                                               const LensS2& L, float lz, int cls, int blo, float* __restrict__ hcol,
@@ -419,7 +455,8 @@ __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, in
     return;
   }
   float prev[QA];
-  sph_totals<MODE, HAS_M, !(HAS_Z || PART), QA>(A, ss, prev);
+  sph_totals<MODE, HAS_M, NE == 1 && !(HAS_Z || PART), QA>(A, ss, prev);
+  if (NE == 2 && !(HAS_Z || PART)) prev[QN] = (float)kChunk;
 #pragma unroll
   for (int j = 0; j <= NE; ++j) {
     float up[QA];
@@ -437,7 +474,7 @@ __device__ __forceinline__ void chunk_edges_s(const SrcPairS* __restrict__ S, in
     if (j <= cls - 1 && bin >= 0 && bin < C.nb) {
       float v[QA];
 #pragma unroll
-      for (int q = 0; q < QA; ++q) v[q] = prev[q] - up[q];
+      for (int q = 0; q < QA; ++q) v[q] = NE == 2 && q != QN ? prev[q] : prev[q] - up[q];
       hist_add<QA, NC>(hcol, bin, v);
     }
 #pragma unroll

@@ -193,3 +193,22 @@ def test_lenses_on_sources(tpcf, oracle, sctx, spacing):
     bins = tpcf.create_bins(0.7 * ARCMIN, 20 * ARCMIN, 5, spacing=spacing)
     res = run_shear(tpcf, sctx, L, S, bins, calculate_marks=False)
     assert_parity(res, oracle.canon_sphere(oracle.SHEAR, L, S, bins.chord_edges_sq))
+
+
+@pytest.mark.parametrize("spacing", ["log", "lin"])
+@pytest.mark.parametrize("z", [False, True])
+def test_bins_smaller_than_a_sub_chunk(tpcf, oracle, sctx, spacing, z):
+    """A few pairs in one small bin, from sub-chunks whose other sources lie far beyond
+    both of its edges: each bin's sums are its own pairs', to 1e-6 of them."""
+    rng = np.random.default_rng(23)
+    L, S = shear_cats(rng, 40, 320, (30, 31, -1, 0), w="uniform")
+    a, d = rng.uniform(0, 2 * np.pi, 40), rng.uniform(0.28, 0.47, 40) * ARCMIN
+    S["x"][:40], S["y"][:40] = f32(L["x"] + d * np.cos(a)), f32(L["y"] + d * np.sin(a))
+    S["m"][:] = f32(rng.normal(0, .05, 320))
+    if z:
+        L["z"], S["z"] = f32(rng.uniform(0, 0.5, 40)), f32(rng.uniform(0.3, 1.0, 320))
+    bins = tpcf.create_bins(0.25 * ARCMIN, 0.5 * ARCMIN, 1, spacing=spacing)
+    res = run_shear(tpcf, sctx, L, S, bins, calculate_marks=False)
+    can = oracle.canon_sphere(oracle.SHEAR, L, S, bins.chord_edges_sq)
+    assert 10 <= can["n_pairs"][0] <= 60
+    assert_parity(res, can)
